@@ -18,6 +18,7 @@
 // scalars on the device and the loop in a CUDA graph WHILE node.  Step 2 is
 // one element pass over the evaluation API's tiles.
 #include "kernels.h"
+#include "pdl.cuh"
 #include "solver.h"
 #include "tile.cuh"
 
@@ -29,9 +30,6 @@ constexpr int kCgThreads = 128;
 constexpr int kCgWarps = kCgThreads / 32;
 constexpr int kCgVerts = kTileVerts / kCgThreads;
 constexpr int kVThreadsCg = 256;
-
-__device__ __forceinline__ void pdl_wait_cg() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_trigger_cg() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 template <class R>
 __device__ __forceinline__ V4<R>* cg_p_prev(const CgArgs& c, int pb) {
@@ -142,8 +140,8 @@ __global__ void __launch_bounds__(kCgThreads) cg_prod_kernel(CgArgs c) {
     if (lane < n) load_elem_m<R, MAT>(a.fv, e0 + lane, geo, ids);
   }
   const int vs = a.fv.tile_vstart[tile], nv = a.fv.tile_vstart[tile + 1] - vs;
-  pdl_trigger_cg();
-  pdl_wait_cg();
+  pdl_trigger();
+  pdl_wait();
   CgState* cs = c.cs;
   if (c.cond && blockIdx.x == 0 && threadIdx.x == 0)
     cudaGraphSetConditional((cudaGraphConditionalHandle)c.cond, 0u);  // the second vertex pass re-arms
@@ -269,8 +267,8 @@ template <class R>
 __global__ void __launch_bounds__(kVThreadsCg) cg_vertex1_kernel(CgArgs c) {
   __shared__ Acc<R> red[(kVThreadsCg / 32) * 1];
   const SolveArgs& a = c.a;
-  pdl_trigger_cg();
-  pdl_wait_cg();
+  pdl_trigger();
+  pdl_wait();
   CgState* cs = c.cs;
   if (cs->done) return;
   const V4<R>* XA = (const V4<R>*)a.xa;
@@ -313,8 +311,8 @@ template <class R>
 __global__ void __launch_bounds__(kVThreadsCg) cg_vertex2_kernel(CgArgs c) {
   __shared__ Acc<R> red[(kVThreadsCg / 32) * 2];
   const SolveArgs& a = c.a;
-  pdl_trigger_cg();
-  pdl_wait_cg();
+  pdl_trigger();
+  pdl_wait();
   CgState* cs = c.cs;
   if (cs->done) return;
   const R alpha = (R)cs->alpha;
@@ -374,28 +372,13 @@ __global__ void __launch_bounds__(256) cg_unpack_kernel(int n, const V4<R>* __re
 
 __global__ void cg_set_limit_kernel(CgState* cs, int n) { cs->iter_limit = cs->iter + n; }
 
-template <class... P, class... A>
-cudaError_t launch_pdl_cg(void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = grid;
-  cfg.blockDim = block;
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, k, args...);
-}
-
 template <class R, int MAT>
 cudaError_t cg_iteration_t(const CgArgs& c, cudaStream_t s) {
   // the element pass opens the loop body: a plain launch
   cg_prod_kernel<R, MAT><<<c.a.fv.n_tiles, kCgThreads, cg_smem_bytes<R>(), s>>>(c);
   cudaError_t e = cudaGetLastError();
-  if (e == cudaSuccess) e = launch_pdl_cg(cg_vertex1_kernel<R>, dim3(c.vblocks), dim3(kVThreadsCg), 0, s, c);
-  if (e == cudaSuccess) e = launch_pdl_cg(cg_vertex2_kernel<R>, dim3(c.vblocks), dim3(kVThreadsCg), 0, s, c);
+  if (e == cudaSuccess) e = launch_pdl(cg_vertex1_kernel<R>, dim3(c.vblocks), dim3(kVThreadsCg), 0, s, c);
+  if (e == cudaSuccess) e = launch_pdl(cg_vertex2_kernel<R>, dim3(c.vblocks), dim3(kVThreadsCg), 0, s, c);
   return e;
 }
 
@@ -413,8 +396,8 @@ cudaError_t cg_prepare_t() {
 // material VJP: out_mu[c] += d(w . g)/d mu_c, out_lambda[c] += d(w . g)/d lambda_c
 // ---------------------------------------------------------------------------
 template <class R, int MAT>
-__global__ void __launch_bounds__(kElemThreads) param_vjp_kernel(FemView fv, const V4<R>* __restrict__ u,
-                                                                 const V4<R>* __restrict__ w,
+__global__ void __launch_bounds__(kElemThreads) param_vjp_kernel(FemView fv, const R* __restrict__ u,
+                                                                 const R* __restrict__ w,
                                                                  const R* __restrict__ vol,
                                                                  const int32_t* __restrict__ elem_user,
                                                                  R* __restrict__ out_mu, R* __restrict__ out_lam) {
@@ -423,9 +406,9 @@ __global__ void __launch_bounds__(kElemThreads) param_vjp_kernel(FemView fv, con
   const int tile = blockIdx.x;
   const int vs = fv.tile_vstart[tile], nv = fv.tile_vstart[tile + 1] - vs;
   for (int i = threadIdx.x; i < nv; i += blockDim.x) {
-    const int v = fv.tv_vid[vs + i];
-    su[i] = ldg4(u + v);
-    sw[i] = ldg4(w + v);
+    const size_t k = 3 * (size_t)fv.tv_user[vs + i];
+    su[i] = V4<R>{u[k], u[k + 1], u[k + 2], R(0)};
+    sw[i] = V4<R>{w[k], w[k + 1], w[k + 2], R(0)};
   }
   __syncthreads();
   for (int e = fv.tile_estart[tile] + threadIdx.x; e < fv.tile_estart[tile + 1]; e += blockDim.x) {
@@ -478,8 +461,8 @@ __global__ void __launch_bounds__(kElemThreads) param_vjp_kernel(FemView fv, con
 // and d/da = (Z00, Z11, Z22, Z01 + Z10, Z02 + Z20, Z12 + Z21)
 // (warp/fem/_stable_neo_hookean_muscle.py:18-46, func/_misc.py:48-53).
 template <class R>
-__global__ void __launch_bounds__(kElemThreads) activation_vjp_kernel(FemView fv, const V4<R>* __restrict__ u,
-                                                                      const V4<R>* __restrict__ w,
+__global__ void __launch_bounds__(kElemThreads) activation_vjp_kernel(FemView fv, const R* __restrict__ u,
+                                                                      const R* __restrict__ w,
                                                                       const int32_t* __restrict__ elem_user,
                                                                       R* __restrict__ out_act) {
   __shared__ V4<R> su[kTileVerts];
@@ -487,9 +470,9 @@ __global__ void __launch_bounds__(kElemThreads) activation_vjp_kernel(FemView fv
   const int tile = blockIdx.x;
   const int vs = fv.tile_vstart[tile], nv = fv.tile_vstart[tile + 1] - vs;
   for (int i = threadIdx.x; i < nv; i += blockDim.x) {
-    const int v = fv.tv_vid[vs + i];
-    su[i] = ldg4(u + v);
-    sw[i] = ldg4(w + v);
+    const size_t k = 3 * (size_t)fv.tv_user[vs + i];
+    su[i] = V4<R>{u[k], u[k + 1], u[k + 2], R(0)};
+    sw[i] = V4<R>{w[k], w[k + 1], w[k + 2], R(0)};
   }
   __syncthreads();
   for (int e = fv.tile_estart[tile] + threadIdx.x; e < fv.tile_estart[tile + 1]; e += blockDim.x) {
@@ -606,28 +589,28 @@ cudaError_t launch_param_vjp(const FemView& fv, int precision, const void* u, co
   if (precision == AGB_F64) {
     if (muscle)
       param_vjp_kernel<double, AGB_STABLE_NEO_HOOKEAN_MUSCLE><<<g, b, 0, s>>>(
-          fv, (const V4<double>*)u, (const V4<double>*)w, (const double*)vol, elem_user, (double*)out_mu,
+          fv, (const double*)u, (const double*)w, (const double*)vol, elem_user, (double*)out_mu,
           (double*)out_lam);
     else if (fv.material == AGB_ARAP)
-      param_vjp_kernel<double, AGB_ARAP><<<g, b, 0, s>>>(fv, (const V4<double>*)u, (const V4<double>*)w,
+      param_vjp_kernel<double, AGB_ARAP><<<g, b, 0, s>>>(fv, (const double*)u, (const double*)w,
                                                           (const double*)vol, elem_user, (double*)out_mu,
                                                           (double*)out_lam);
     else
       param_vjp_kernel<double, AGB_STABLE_NEO_HOOKEAN><<<g, b, 0, s>>>(
-          fv, (const V4<double>*)u, (const V4<double>*)w, (const double*)vol, elem_user, (double*)out_mu,
+          fv, (const double*)u, (const double*)w, (const double*)vol, elem_user, (double*)out_mu,
           (double*)out_lam);
   } else {
     if (muscle)
       param_vjp_kernel<float, AGB_STABLE_NEO_HOOKEAN_MUSCLE><<<g, b, 0, s>>>(
-          fv, (const V4<float>*)u, (const V4<float>*)w, (const float*)vol, elem_user, (float*)out_mu,
+          fv, (const float*)u, (const float*)w, (const float*)vol, elem_user, (float*)out_mu,
           (float*)out_lam);
     else if (fv.material == AGB_ARAP)
-      param_vjp_kernel<float, AGB_ARAP><<<g, b, 0, s>>>(fv, (const V4<float>*)u, (const V4<float>*)w,
+      param_vjp_kernel<float, AGB_ARAP><<<g, b, 0, s>>>(fv, (const float*)u, (const float*)w,
                                                          (const float*)vol, elem_user, (float*)out_mu,
                                                          (float*)out_lam);
     else
       param_vjp_kernel<float, AGB_STABLE_NEO_HOOKEAN><<<g, b, 0, s>>>(
-          fv, (const V4<float>*)u, (const V4<float>*)w, (const float*)vol, elem_user, (float*)out_mu,
+          fv, (const float*)u, (const float*)w, (const float*)vol, elem_user, (float*)out_mu,
           (float*)out_lam);
   }
   return cudaGetLastError();
@@ -639,10 +622,10 @@ cudaError_t launch_activation_vjp(const FemView& fv, int precision, const void* 
   if (fv.material != AGB_STABLE_NEO_HOOKEAN_MUSCLE || !fv.act) return cudaErrorInvalidValue;
   const dim3 g(fv.n_tiles), b(kElemThreads);
   if (precision == AGB_F64)
-    activation_vjp_kernel<double><<<g, b, 0, s>>>(fv, (const V4<double>*)u, (const V4<double>*)w, elem_user,
+    activation_vjp_kernel<double><<<g, b, 0, s>>>(fv, (const double*)u, (const double*)w, elem_user,
                                                   (double*)out_act);
   else
-    activation_vjp_kernel<float><<<g, b, 0, s>>>(fv, (const V4<float>*)u, (const V4<float>*)w, elem_user,
+    activation_vjp_kernel<float><<<g, b, 0, s>>>(fv, (const float*)u, (const float*)w, elem_user,
                                                  (float*)out_act);
   return cudaGetLastError();
 }

@@ -108,6 +108,7 @@ struct FemView {
   const int32_t* tile_gstart;
   const int32_t* group_estart;
   const int32_t* tv_vid;
+  const int32_t* tv_user;  // the caller's point id of each tile vertex (evaluation API)
   // FP32: rec = float4[3][n_cells]; FP64: rec = double[11][n_cells] + ids
   const void* rec;
   const uint32_t* ids;
@@ -132,6 +133,7 @@ struct agb_fem {
   int32_t* d_tile_gstart = nullptr;
   int32_t* d_group_estart = nullptr;
   int32_t* d_tv_vid = nullptr;
+  int32_t* d_tv_user = nullptr;   // tile-vertex -> caller's point id
   int32_t* d_own_slot = nullptr;  // tile-vertex -> slot (standalone)
   int32_t* d_own_off = nullptr;   // n_points + 1
   void* d_rec = nullptr;
@@ -143,9 +145,7 @@ struct agb_fem {
   int32_t* d_elem_user = nullptr;    // internal -> caller's cell index (on first use)
   void* d_vol = nullptr;             // R per internal element (on first use)
   // scratch for the standalone evaluation API
-  void* d_u = nullptr;      // V4<R> n_points
-  void* d_p = nullptr;      // V4<R> n_points
-  void* d_slots = nullptr;  // V4<R> [3][n_tv]
+  void* d_slots = nullptr;  // up to 9 R per tile vertex
   double* d_partials = nullptr;
   unsigned* d_counter = nullptr;
   agb::FemView view() const;
@@ -167,9 +167,7 @@ struct agb_model {
   std::vector<int32_t*> d_slot_of_tv;  // per potential
   void* d_fixed = nullptr;             // V4<R> n_points: fixed values, w = mask bits
   void* d_force = nullptr;             // V4<R> n_points or null
-  void* d_u = nullptr;
-  void* d_p = nullptr;
-  void* d_slots = nullptr;             // V4<R> [3][n_slots]
+  void* d_slots = nullptr;             // up to 9 R per slot
   double* d_partials = nullptr;
   unsigned* d_counter = nullptr;
 };

@@ -351,41 +351,26 @@ __global__ void batch_init_state_kernel(BatchArgs b, SolverState proto) {
 
 __global__ void batch_set_limit_kernel(BatchState* bs, int n) { bs->iter_limit = bs->iter + n; }
 
-template <class... P, class... A>
-cudaError_t launch_pdl_b(void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = grid;
-  cfg.blockDim = block;
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, k, args...);
-}
-
 cudaError_t batch_refresh(const BatchArgs& b, cudaStream_t s) {
   cudaError_t e = b.a.fv.material == AGB_STABLE_NEO_HOOKEAN_MUSCLE
-                      ? launch_pdl_b(batch_ref_elem_kernel<AGB_STABLE_NEO_HOOKEAN_MUSCLE>,
+                      ? launch_pdl(batch_ref_elem_kernel<AGB_STABLE_NEO_HOOKEAN_MUSCLE>,
                                      dim3(ref_blocks(b.a.fv.n_tiles)), dim3(kGradThreads), ref_smem_bytes(), s, b)
-                      : launch_pdl_b(batch_ref_elem_kernel<AGB_STABLE_NEO_HOOKEAN>, dim3(ref_blocks(b.a.fv.n_tiles)),
+                      : launch_pdl(batch_ref_elem_kernel<AGB_STABLE_NEO_HOOKEAN>, dim3(ref_blocks(b.a.fv.n_tiles)),
                                      dim3(kGradThreads), ref_smem_bytes(), s, b);
   const int vb = b.n_chunks < kSMs * 8 ? b.n_chunks : kSMs * 8;
-  if (e == cudaSuccess) e = launch_pdl_b(batch_ref_vertex_kernel, dim3(vb > 0 ? vb : 1), dim3(kVThreads), 0, s, b);
+  if (e == cudaSuccess) e = launch_pdl(batch_ref_vertex_kernel, dim3(vb > 0 ? vb : 1), dim3(kVThreads), 0, s, b);
   return e;
 }
 
 template <class R, int MAT, bool DELTA>
 cudaError_t batch_grad_and_vertex_d(const BatchArgs& b, cudaStream_t s, int fallback = 0) {
   const int phase = fallback ? 2 : 0;
-  cudaError_t e = launch_pdl_b(batch_grad_kernel<R, MAT, DELTA>, dim3(b.a.fv.n_tiles), dim3(kGradThreads),
+  cudaError_t e = launch_pdl(batch_grad_kernel<R, MAT, DELTA>, dim3(b.a.fv.n_tiles), dim3(kGradThreads),
                                grad_smem_bytes<R>(), s, b, fallback);
   if (e == cudaSuccess)
-    e = launch_pdl_b(batch_vertex_kernel<R, DELTA>, dim3(b.n_chunks), dim3(kVThreads), 0, s, b, phase);
+    e = launch_pdl(batch_vertex_kernel<R, DELTA>, dim3(b.n_chunks), dim3(kVThreads), 0, s, b, phase);
   if (e == cudaSuccess)
-    e = launch_pdl_b(batch_vertex_tail_kernel<R>, dim3(b.n_meshes), dim3(kTailThreads), 0, s, b, phase);
+    e = launch_pdl(batch_vertex_tail_kernel<R>, dim3(b.n_meshes), dim3(kTailThreads), 0, s, b, phase);
   if (e == cudaSuccess && DELTA) e = batch_refresh(b, s);
   return e;
 }
@@ -412,7 +397,7 @@ cudaError_t batch_iteration_m(const BatchArgs& b, cudaStream_t s) {
   batch_dir_kernel<R, MAT><<<b.a.fv.n_tiles, kElemThreads, 0, s>>>(b);
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess)
-    e = launch_pdl_b(batch_dir_tail_kernel<R, MAT>, dim3(b.n_meshes), dim3(kTailThreads), 0, s, b);
+    e = launch_pdl(batch_dir_tail_kernel<R, MAT>, dim3(b.n_meshes), dim3(kTailThreads), 0, s, b);
   if (e == cudaSuccess) e = batch_grad_and_vertex_m<R, MAT>(b, s);
   return e;
 }
@@ -427,14 +412,14 @@ cudaError_t batch_iteration_arap(const BatchArgs& b, cudaStream_t s) {
   const int nt = b.a.fv.n_tiles, max_bt = b.a.max_bt;
   batch_dir_kernel<R, A><<<nt, kElemThreads, 0, s>>>(b);
   cudaError_t e = cudaGetLastError();
-  if (e == cudaSuccess) e = launch_pdl_b(batch_dir_tail_kernel<R, A>, dim3(b.n_meshes), dim3(kTailThreads), 0, s, b);
+  if (e == cudaSuccess) e = launch_pdl(batch_dir_tail_kernel<R, A>, dim3(b.n_meshes), dim3(kTailThreads), 0, s, b);
   if (e == cudaSuccess)
-    e = launch_pdl_b(batch_grad_spec_kernel<R>, dim3(nt), dim3(kGradThreads), grad_spec_smem_bytes<R>(), s, b);
-  if (e == cudaSuccess) e = launch_pdl_b(batch_spec_tail_kernel<R>, dim3(b.n_meshes), dim3(kTailThreads), 0, s, b);
+    e = launch_pdl(batch_grad_spec_kernel<R>, dim3(nt), dim3(kGradThreads), grad_spec_smem_bytes<R>(), s, b);
+  if (e == cudaSuccess) e = launch_pdl(batch_spec_tail_kernel<R>, dim3(b.n_meshes), dim3(kTailThreads), 0, s, b);
   if (e == cudaSuccess)
-    e = launch_pdl_b(batch_vertex_kernel<R, false>, dim3(b.n_chunks), dim3(kVThreads), 0, s, b, 1);
+    e = launch_pdl(batch_vertex_kernel<R, false>, dim3(b.n_chunks), dim3(kVThreads), 0, s, b, 1);
   if (e == cudaSuccess)
-    e = launch_pdl_b(batch_vertex_tail_kernel<R>, dim3(b.n_meshes), dim3(kTailThreads), 0, s, b, 1);
+    e = launch_pdl(batch_vertex_tail_kernel<R>, dim3(b.n_meshes), dim3(kTailThreads), 0, s, b, 1);
   for (int j0 = 1; e == cudaSuccess && j0 <= max_bt; j0 += 3) {
     const int k = max_bt - j0 + 1 < 3 ? max_bt - j0 + 1 : 3;
     batch_trial_kernel<R><<<nt, kElemThreads, 0, s>>>(b, j0, k);

@@ -245,6 +245,7 @@ FemView agb_fem::view() const {
   v.tile_gstart = d_tile_gstart;
   v.group_estart = d_group_estart;
   v.tv_vid = d_tv_vid;
+  v.tv_user = d_tv_user;
   v.rec = d_rec;
   v.ids = d_ids;
   v.act = d_act;
@@ -327,9 +328,8 @@ int agb_region_compute(int32_t n_cells, const int32_t* cells, int32_t n_points,
 int agb_fem_destroy(agb_fem* f) {
   if (!f) return AGB_OK;
   for (void* p : {(void*)f->d_tile_estart, (void*)f->d_tile_vstart, (void*)f->d_tile_gstart,
-                  (void*)f->d_group_estart, (void*)f->d_tv_vid,
-                  (void*)f->d_own_slot, (void*)f->d_own_off, f->d_rec, (void*)f->d_ids, f->d_u,
-                  f->d_p, f->d_slots, (void*)f->d_partials, (void*)f->d_counter,
+                  (void*)f->d_group_estart, (void*)f->d_tv_vid, (void*)f->d_tv_user,
+                  (void*)f->d_own_slot, (void*)f->d_own_off, f->d_rec, (void*)f->d_ids, f->d_slots, (void*)f->d_partials, (void*)f->d_counter,
                   (void*)f->d_elem_user, f->d_vol, f->d_act, (void*)f->d_D, (void*)f->d_act_user})
     dfree(p);
   delete f;
@@ -416,21 +416,23 @@ int agb_fem_create(agb_space* space, int material, int precision, int32_t n_cell
     for (int e = 0; e < n_cells; ++e) f->vol_internal[e] = vol[f->plan.elem_user[e]];
   }
   const TilePlan& P = f->plan;
-  const size_t v4 = v4_bytes(precision);
   const size_t n_part = (size_t)std::max(P.n_tiles, unpack_blocks(np)) * 2;
   if (!rc) rc = dupload(&f->d_tile_estart, P.tile_estart);
   if (!rc) rc = dupload(&f->d_tile_vstart, P.tile_vstart);
   if (!rc) rc = dupload(&f->d_tile_gstart, P.tile_gstart);
   if (!rc) rc = dupload(&f->d_group_estart, P.group_estart);
   if (!rc) rc = dupload(&f->d_tv_vid, P.tv_vid);
+  if (!rc) {
+    std::vector<int32_t> tv_user(P.tv_vid.size());
+    for (size_t i = 0; i < tv_user.size(); ++i) tv_user[i] = space->user_of_internal[P.tv_vid[i]];
+    rc = dupload(&f->d_tv_user, tv_user);
+  }
   if (!rc) rc = dupload(&f->d_own_slot, f->own_slots.slot_of_tv);
   if (!rc) rc = dupload(&f->d_own_off, f->own_off);
   if (!rc) rc = upload_records(P, precision, &f->d_rec, &f->d_ids);
   if (!rc && material == AGB_STABLE_NEO_HOOKEAN_MUSCLE)
     rc = upload_act(std::vector<double>(6 * (size_t)n_cells, 0.0), (size_t)n_cells, precision, &f->d_act);
-  if (!rc) rc = dalloc_bytes(&f->d_u, v4 * np);
-  if (!rc) rc = dalloc_bytes(&f->d_p, v4 * np);
-  if (!rc) rc = dalloc_bytes(&f->d_slots, v4 * 3 * (size_t)P.n_tv);
+  if (!rc) rc = dalloc_bytes(&f->d_slots, 9 * real_bytes(precision) * (size_t)P.n_tv);
   if (!rc) rc = dalloc(&f->d_partials, n_part);
   if (!rc) rc = dalloc(&f->d_counter, 1);
   if (!rc && cudaMemset(f->d_counter, 0, sizeof(unsigned)) != cudaSuccess) rc = AGB_E_CUDA;
@@ -537,18 +539,14 @@ int agb_fem_eval(agb_fem* f, unsigned flags, const void* u, const void* p, doubl
   if (!flags) return AGB_OK;
   cudaStream_t s = as_stream(stream);
   const int np = f->space->n_points;
-  RC(check_launch(launch_pack(f->precision, np, f->space->d_user_of_internal, u, f->d_u,
-                              need_p ? p : nullptr, f->d_p, s),
-                  "pack"));
-  RC(check_launch(launch_fem_eval(f->precision, f->view(), flags, f->d_u, f->d_p, f->d_own_slot,
-                                  f->d_slots, f->plan.n_tv, f->d_partials, f->d_counter, energy,
-                                  quad, s),
+  RC(check_launch(launch_fem_eval(f->precision, f->view(), flags, u, p, f->d_own_slot, f->d_slots, f->plan.n_tv,
+                                  f->d_partials, f->d_counter, energy, quad, 0, s),
                   "fem_eval"));
   const unsigned vec = flags & (AGB_GRAD | AGB_HESS_DIAG | AGB_HESS_PROD);
   if (vec)
-    RC(check_launch(launch_unpack(f->precision, np, f->space->d_user_of_internal, f->d_own_off,
-                                  f->d_slots, f->plan.n_tv, vec, grad, diag, prod, nullptr,
-                                  f->d_u, f->d_partials, f->d_counter, nullptr, s),
+    RC(check_launch(launch_unpack(f->precision, np, f->space->d_user_of_internal, f->d_own_off, f->d_slots,
+                                  f->plan.n_tv, vec, grad, diag, prod, 0, nullptr, u, f->d_partials, f->d_counter,
+                                  nullptr, s),
                     "unpack"));
   return AGB_OK;
 }
@@ -575,7 +573,7 @@ int agb_fem_hess_quad(agb_fem* f, const void* u, const void* p, double* out, voi
 int agb_model_destroy(agb_model* m) {
   if (!m) return AGB_OK;
   for (int32_t* p : m->d_slot_of_tv) dfree(p);
-  for (void* p : {(void*)m->d_off, m->d_fixed, m->d_force, m->d_u, m->d_p, m->d_slots,
+  for (void* p : {(void*)m->d_off, m->d_fixed, m->d_force, m->d_slots,
                   (void*)m->d_partials, (void*)m->d_counter})
     dfree(p);
   delete m;
@@ -662,9 +660,7 @@ int agb_model_create(agb_space* space, int precision, int32_t n_pot, agb_fem* co
   int max_tiles = 0;
   for (agb_fem* f : m->fems) max_tiles = std::max(max_tiles, f->plan.n_tiles);
   const size_t n_part = (size_t)std::max(max_tiles, unpack_blocks(np)) * 2;
-  if (!rc) rc = dalloc_bytes(&m->d_u, v4 * np);
-  if (!rc) rc = dalloc_bytes(&m->d_p, v4 * np);
-  if (!rc) rc = dalloc_bytes(&m->d_slots, v4 * 3 * (size_t)m->n_slots);
+  if (!rc) rc = dalloc_bytes(&m->d_slots, 9 * real_bytes(prec) * (size_t)m->n_slots);
   if (!rc) rc = dalloc(&m->d_partials, n_part);
   if (!rc) rc = dalloc(&m->d_counter, 1);
   if (!rc && cudaMemset(m->d_counter, 0, sizeof(unsigned)) != cudaSuccess) rc = AGB_E_CUDA;
@@ -710,28 +706,27 @@ int agb_model_eval(agb_model* m, unsigned flags, const void* u, const void* p, d
   AGB_REQUIRE(!(flags & AGB_HESS_QUAD) || quad, AGB_E_INVALID, "agb_model_eval: hess_quad is null");
   cudaStream_t s = as_stream(stream);
   const int np = m->space->n_points;
-  const size_t vec_bytes = 3 * (size_t)np * real_bytes(m->precision);
-  // WarpModel: zero, then every potential accumulates (warp/model/_model.py:13-36)
-  if (flags & AGB_FUN) AGB_CHECK_CUDA(cudaMemsetAsync(energy, 0, sizeof(double), s));
-  if (flags & AGB_HESS_QUAD) AGB_CHECK_CUDA(cudaMemsetAsync(quad, 0, sizeof(double), s));
-  if (flags & AGB_GRAD) AGB_CHECK_CUDA(cudaMemsetAsync(grad, 0, vec_bytes, s));
-  if (flags & AGB_HESS_DIAG) AGB_CHECK_CUDA(cudaMemsetAsync(diag, 0, vec_bytes, s));
-  if (flags & AGB_HESS_PROD) AGB_CHECK_CUDA(cudaMemsetAsync(prod, 0, vec_bytes, s));
+  // WarpModel: zero, then every potential accumulates (warp/model/_model.py:13-36).
+  // The vertex pass covers every point and stores the vectors, and the first
+  // element pass stores the scalars; only scalars no element pass writes are
+  // zeroed here.
+  const bool any_tiles =
+      std::any_of(m->fems.begin(), m->fems.end(), [](const agb_fem* f) { return f->plan.n_tiles > 0; });
+  if ((flags & AGB_FUN) && !any_tiles) AGB_CHECK_CUDA(cudaMemsetAsync(energy, 0, sizeof(double), s));
+  if ((flags & AGB_HESS_QUAD) && !any_tiles) AGB_CHECK_CUDA(cudaMemsetAsync(quad, 0, sizeof(double), s));
   if (!flags) return AGB_OK;
-  RC(check_launch(launch_pack(m->precision, np, m->space->d_user_of_internal, u, m->d_u,
-                              need_p ? p : nullptr, m->d_p, s),
-                  "pack"));
-  for (size_t k = 0; k < m->fems.size(); ++k)
-    RC(check_launch(launch_fem_eval(m->precision, m->fems[k]->view(), flags, m->d_u, m->d_p,
-                                    m->d_slot_of_tv[k], m->d_slots, m->n_slots, m->d_partials,
-                                    m->d_counter, energy, quad, s),
+  int assign = 1;
+  for (size_t k = 0; k < m->fems.size(); ++k) {
+    RC(check_launch(launch_fem_eval(m->precision, m->fems[k]->view(), flags, u, p, m->d_slot_of_tv[k], m->d_slots,
+                                    m->n_slots, m->d_partials, m->d_counter, energy, quad, assign, s),
                     "fem_eval"));
+    if (m->fems[k]->plan.n_tiles > 0) assign = 0;
+  }
   const unsigned vec = flags & (AGB_GRAD | AGB_HESS_DIAG | AGB_HESS_PROD | AGB_FUN);
   const bool ext = m->d_force != nullptr;
   if ((vec & ~AGB_FUN) || (ext && (flags & AGB_FUN)))
-    RC(check_launch(launch_unpack(m->precision, np, m->space->d_user_of_internal, m->d_off,
-                                  m->d_slots, m->n_slots, vec, grad, diag, prod, m->d_force,
-                                  m->d_u, m->d_partials, m->d_counter, energy, s),
+    RC(check_launch(launch_unpack(m->precision, np, m->space->d_user_of_internal, m->d_off, m->d_slots, m->n_slots,
+                                  vec, grad, diag, prod, 1, m->d_force, u, m->d_partials, m->d_counter, energy, s),
                     "unpack"));
   return AGB_OK;
 }
@@ -1449,10 +1444,7 @@ int agb_fem_grad_param_vjp(agb_fem* f, const void* u, const void* w, void* out_m
   AGB_REQUIRE(f && u && w && out_mu, AGB_E_INVALID, "agb_fem_grad_param_vjp: null argument");
   cudaStream_t s = as_stream(stream);
   RC(ensure_vjp_tables(f));
-  const int np = f->space->n_points;
-  RC(check_launch(launch_pack(f->precision, np, f->space->d_user_of_internal, u, f->d_u, w, f->d_p, s),
-                  "pack"));
-  RC(check_launch(launch_param_vjp(f->view(), f->precision, f->d_u, f->d_p, f->d_vol, f->d_elem_user,
+  RC(check_launch(launch_param_vjp(f->view(), f->precision, u, w, f->d_vol, f->d_elem_user,
                                    out_mu, f->material != AGB_ARAP ? out_lambda : nullptr, s),
                   "param_vjp"));
   return AGB_OK;
@@ -1837,9 +1829,7 @@ int agb_fem_grad_activation_vjp(agb_fem* f, const void* u, const void* w, void* 
               "agb_fem_grad_activation_vjp: not a muscle potential");
   cudaStream_t s = as_stream(stream);
   RC(ensure_vjp_tables(f));
-  const int np = f->space->n_points;
-  RC(check_launch(launch_pack(f->precision, np, f->space->d_user_of_internal, u, f->d_u, w, f->d_p, s), "pack"));
-  RC(check_launch(launch_activation_vjp(f->view(), f->precision, f->d_u, f->d_p, f->d_elem_user, out_activation, s),
+  RC(check_launch(launch_activation_vjp(f->view(), f->precision, u, w, f->d_elem_user, out_activation, s),
                   "activation_vjp"));
   return AGB_OK;
 }

@@ -2,289 +2,469 @@
 // tiled pass over the mesh (warp/fem/_base.py:243-383).
 //
 // One CTA per tile: the tile's vertices (<= kTileVerts) are staged in
-// shared memory, each thread evaluates elements of the tile, the
-// element-to-vertex scatter (the reference's 4 x vec3 global atomics per tet,
-// _base.py:288-289, 321-322, 348-349) becomes shared-memory accumulation,
-// and each tile writes one slot per vertex that a vertex pass sums in a
-// fixed order.  Scalar outputs (energy, p^T H p) are reduced in float-float
-// and finished by the last block, replacing the single-address scalar
-// atomics of _base.py:261, 381.
+// shared memory straight from the caller's arrays, and each warp evaluates
+// conflict-free groups of the tile's elements.  The element-to-vertex scatter
+// (the reference's 4 x vec3 global atomics per tet, _base.py:288-289,
+// 321-322, 348-349) becomes plain read-modify-writes of the warp's private
+// shared-memory accumulator; each tile writes one slot per vertex that a
+// vertex pass sums in a fixed order.  Scalar outputs (energy, p^T H p) are
+// reduced in float-float and finished by the last block, replacing the
+// single-address scalar atomics of _base.py:261, 381.  Every output is
+// bitwise reproducible.
 #include <algorithm>
 
 #include "kernels.h"
+#include "pdl.cuh"
 #include "tile.cuh"
 
 namespace agb {
 
-template <class R>
-__global__ void __launch_bounds__(256) pack_kernel(int n, const int32_t* __restrict__ uoi,
-                                                   const R* __restrict__ u, V4<R>* __restrict__ ui,
-                                                   const R* __restrict__ p, V4<R>* __restrict__ pi) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const size_t k = 3 * (size_t)uoi[i];
-    ui[i] = V4<R>{u[k], u[k + 1], u[k + 2], R(0)};
-    if (p) pi[i] = V4<R>{p[k], p[k + 1], p[k + 2], R(0)};
+namespace {
+
+// The NVEC vectors requested (of gradient, diagonal, product, in that order)
+// as 3 NVEC reals per vertex: NVEC 1: one V4 (last lane unused); 2: V4 + V2;
+// 3: two V4 and one real.  The accumulators and the slots share this layout.
+template <int NVEC>
+struct VecLayout {
+  static constexpr int n4 = NVEC == 3 ? 2 : (NVEC ? 1 : 0);
+  static constexpr int n2 = NVEC == 2 ? 1 : 0;
+  static constexpr int n1 = NVEC == 3 ? 1 : 0;
+  static constexpr int reals = 4 * n4 + 2 * n2 + n1;
+};
+
+// arrays of `n` entries each: n4 of V4, then n2 of V2, then n1 of R
+template <class R, int NVEC>
+struct VecArrays {
+  using L = VecLayout<NVEC>;
+  unsigned char* base;
+  size_t n;
+  __device__ __forceinline__ V4<R>* v4(int j) const { return reinterpret_cast<V4<R>*>(base) + j * n; }
+  __device__ __forceinline__ V2<R>* v2() const { return reinterpret_cast<V2<R>*>(base + n * L::n4 * sizeof(V4<R>)); }
+  __device__ __forceinline__ R* v1() const {
+    return reinterpret_cast<R*>(base + n * (L::n4 * sizeof(V4<R>) + L::n2 * sizeof(V2<R>)));
   }
+  __device__ __forceinline__ void load(size_t i, R (&x)[9]) const {
+    if constexpr (NVEC >= 1) {
+      const V4<R> a = v4(0)[i];
+      x[0] = a.x;
+      x[1] = a.y;
+      x[2] = a.z;
+      if constexpr (NVEC >= 2) x[3] = a.w;
+    }
+    if constexpr (NVEC == 2) {
+      const V2<R> b = v2()[i];
+      x[4] = b.x;
+      x[5] = b.y;
+    }
+    if constexpr (NVEC == 3) {
+      const V4<R> b = v4(1)[i];
+      x[4] = b.x;
+      x[5] = b.y;
+      x[6] = b.z;
+      x[7] = b.w;
+      x[8] = v1()[i];
+    }
+  }
+  __device__ __forceinline__ void store(size_t i, const R (&x)[9]) const {
+    if constexpr (NVEC >= 1) v4(0)[i] = V4<R>{x[0], x[1], x[2], NVEC >= 2 ? x[3] : R(0)};
+    if constexpr (NVEC == 2) v2()[i] = V2<R>{x[4], x[5]};
+    if constexpr (NVEC == 3) {
+      v4(1)[i] = V4<R>{x[4], x[5], x[6], x[7]};
+      v1()[i] = x[8];
+    }
+  }
+};
+
+// staging: (x y z p.x) and, with p, (p.y p.z) per vertex
+template <class R>
+constexpr size_t eval_stage_bytes() {
+  return (size_t)kTileVerts * (sizeof(V4<R>) + sizeof(V2<R>));
+}
+template <class R, int NVEC>
+constexpr size_t eval_smem_bytes(int warps) {
+  return eval_stage_bytes<R>() + (size_t)warps * kTileVerts * VecLayout<NVEC>::reals * sizeof(R);
 }
 
-template <class R, int MAT>
-__global__ void __launch_bounds__(kElemThreads) fem_eval_kernel(
-    FemView fv, unsigned flags, const V4<R>* __restrict__ u, const V4<R>* __restrict__ p,
-    const int32_t* __restrict__ slot_of_tv, V4<R>* __restrict__ slots, int n_slots,
-    AccStore<R>* __restrict__ partials, unsigned* counter, double* energy, double* quad) {
-  __shared__ R sx[3][kTileVerts];
-  __shared__ R sp[3][kTileVerts];
-  __shared__ R acc[9][kTileVerts];
-  __shared__ Acc<R> red[(kElemThreads / 32) * 2];
+// Bound: the shared-memory pipe and latency in FP32 (staging, gathers and
+// read-modify-writes of 3 NVEC reals per corner), the FP64 pipe in FP64.  The
+// records of a warp's next group are loaded while the current one computes.
+// MAXT 128: four warps per tile and five CTAs per SM in FP32, for meshes with
+// enough tiles to fill the SMs; MAXT 512 (FP64: 256): 8 or 16 warps per tile (blockDim),
+// for meshes with fewer tiles than SMs, where one tile's serial chain of
+// groups is the whole pass (eval_warps below).
+// A call for scalars alone runs the NVEC 1 kernel without its accumulators:
+// with the vector branches compiled in, the invariants are formed the same
+// way, and the energy and p^T H p have the same element values whatever else
+// is asked for.
+// Measured, all five quantities on the 1.5M-tet grid in FP32: element pass 81 us
+// (119 us with shared-memory float atomics on one accumulator), the call
+// 130 us (170 us with that, a packing pass and separate zeroing).
+template <class R, int MAT, int NVEC, int MAXT>
+__global__ void __launch_bounds__(MAXT, MAXT == 128 ? (sizeof(R) == 4 ? 5 : 2) : 1) fem_eval_kernel(
+    FemView fv, unsigned flags, const R* __restrict__ u, const R* __restrict__ p,
+    const int32_t* __restrict__ slot_of_tv, void* __restrict__ slots, int n_slots, AccStore<R>* __restrict__ partials,
+    unsigned* counter, double* energy, double* quad, int assign) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  V4<R>* sx = reinterpret_cast<V4<R>*>(smem_raw);
+  V2<R>* sq = reinterpret_cast<V2<R>*>(sx + kTileVerts);
+  unsigned char* acc = smem_raw + eval_stage_bytes<R>();
+  constexpr size_t kAccBytes = (size_t)kTileVerts * VecLayout<NVEC>::reals * sizeof(R);
+  __shared__ Acc<R> red[(MAXT / 32) * 2];
 
   const bool do_fun = flags & AGB_FUN, do_grad = flags & AGB_GRAD, do_diag = flags & AGB_HESS_DIAG;
   const bool do_prod = flags & AGB_HESS_PROD, do_quad = flags & AGB_HESS_QUAD;
-  const bool need_p = do_prod || do_quad;
+  const bool need_p = do_prod || do_quad, vectors = do_grad || do_diag || do_prod;
 
   const int tile = blockIdx.x;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+  const int ge = fv.tile_gstart[tile + 1];
+  int g = fv.tile_gstart[tile] + warp, n = 0;
+  ElemGeo<R> geo;
+  uint32_t ids = 0;
+  if (g < ge) {
+    const int e0 = fv.group_estart[g];
+    n = fv.group_estart[g + 1] - e0;
+    if (lane < n) load_elem_m<R, MAT>(fv, e0 + lane, geo, ids);
+  }
   const int vs = fv.tile_vstart[tile], nv = fv.tile_vstart[tile + 1] - vs;
-  const int es = fv.tile_estart[tile], ee = fv.tile_estart[tile + 1];
-
+  pdl_trigger();
   for (int i = threadIdx.x; i < nv; i += blockDim.x) {
-    const int v = fv.tv_vid[vs + i];
-    const V4<R> a = ldg4(u + v);
-    sx[0][i] = a.x;
-    sx[1][i] = a.y;
-    sx[2][i] = a.z;
+    const size_t k = 3 * (size_t)fv.tv_user[vs + i];
+    V4<R> a{u[k], u[k + 1], u[k + 2], R(0)};
     if (need_p) {
-      const V4<R> b = ldg4(p + v);
-      sp[0][i] = b.x;
-      sp[1][i] = b.y;
-      sp[2][i] = b.z;
+      a.w = p[k];
+      sq[i] = V2<R>{p[k + 1], p[k + 2]};
     }
-#pragma unroll
-    for (int q = 0; q < 9; ++q) acc[q][i] = R(0);
+    sx[i] = a;
+  }
+  if (vectors) {
+    V4<R>* z = reinterpret_cast<V4<R>*>(acc);
+    const int nz = (int)(warps * kAccBytes / sizeof(V4<R>));
+    for (int i = threadIdx.x; i < nz; i += blockDim.x) z[i] = V4<R>{R(0), R(0), R(0), R(0)};
   }
   __syncthreads();
 
+  const VecArrays<R, NVEC> my{acc + warp * kAccBytes, (size_t)kTileVerts};
   Acc<R> sums[2] = {};
-  for (int e = es + threadIdx.x; e < ee; e += blockDim.x) {
-    ElemGeo<R> geo;
-    uint32_t ids;
-    load_elem_m<R, MAT>(fv, e, geo, ids);
-    int l[4];
-    R uc[4][3];
-#pragma unroll
-    for (int a = 0; a < 4; ++a) {
-      l[a] = corner(ids, a);
-#pragma unroll
-      for (int c = 0; c < 3; ++c) uc[a][c] = sx[c][l[a]];
+  while (g < ge) {
+    const int gn = g + warps;
+    int nn = 0;
+    ElemGeo<R> geon;
+    uint32_t idsn = 0;
+    if (gn < ge) {
+      const int e0n = fv.group_estart[gn];
+      nn = fv.group_estart[gn + 1] - e0n;
+      if (lane < nn) load_elem_m<R, MAT>(fv, e0n + lane, geon, idsn);
     }
-    R G[3][3];
-    corner_gradient(uc, geo.D, G);
-    add_act<MAT>(geo, G);
-    R dF[3][3];
-    if (need_p) {
-      R pc[4][3];
-#pragma unroll
-      for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int c = 0; c < 3; ++c) pc[a][c] = sp[c][l[a]];
-      corner_gradient(pc, geo.D, dF);
-    }
-    R f[4][3];
-    if constexpr (snh_family(MAT)) {
-      SnhPoint<R> s;
-      snh_prepare(G, s);
-      if (do_fun) sums[0].add(snh_energy(s, geo.mu, geo.lam));
-      if (do_grad) {
-        R P[3][3];
-        snh_pk1(s, geo.mu, geo.lam, P);
-        corner_vjp(P, geo.D, f);
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-          for (int c = 0; c < 3; ++c) atomicAdd(&acc[c][l[a]], f[a][c]);
-      }
-      if (do_diag) {
-        snh_hess_diag(s, geo.D, geo.mu, geo.lam, f);
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-          for (int c = 0; c < 3; ++c) atomicAdd(&acc[3 + c][l[a]], fmax(f[a][c], R(0)));
-      }
+    const int l[4] = {corner(ids, 0), corner(ids, 1), corner(ids, 2), corner(ids, 3)};
+    // f[q]: corner values of the q-th requested vector
+    R f[NVEC][4][3];
+    if (lane < n) {
+      R G[3][3], dF[3][3];
       if (need_p) {
+        dir_gradients(sx, sq, l, geo.D, G, dF);
+      } else {
+        vec_gradient(sx, l, geo.D, G);
+      }
+      add_act<MAT>(geo, G);
+      // which vector each f[q] holds: with one or two requested the choice is
+      // uniform over the launch
+      auto fill = [&](auto grad, auto diag, auto prod) {
+        if constexpr (NVEC == 1) {
+          if (do_grad)
+            grad(f[0]);
+          else if (do_diag)
+            diag(f[0]);
+          else if (do_prod)
+            prod(f[0]);
+        } else if constexpr (NVEC == 2) {
+          if (do_grad)
+            grad(f[0]);
+          else
+            diag(f[0]);
+          if (do_prod)
+            prod(f[1]);
+          else
+            diag(f[1]);
+        } else {
+          grad(f[0]);
+          diag(f[1]);
+          prod(f[2]);
+        }
+      };
+      auto clamp = [](R(&h)[4][3]) {
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+#pragma unroll
+          for (int c = 0; c < 3; ++c) h[a][c] = fmax(h[a][c], R(0));
+      };
+      if constexpr (snh_family(MAT)) {
+        SnhPoint<R> s;
+        snh_prepare(G, s);
         SnhDir<R> d;
-        snh_dir(s, dF, d);
+        if (need_p) snh_dir(s, dF, d);
+        if (do_fun) sums[0].add(snh_energy(s, geo.mu, geo.lam));
         if (do_quad) sums[1].add(fmax(snh_hess_quad(s, d, geo.mu, geo.lam), R(0)));
-        if (do_prod) {
-          R M[3][3];
-          snh_hess_prod(s, d, dF, geo.mu, geo.lam, M);
-          corner_vjp(M, geo.D, f);
+        fill(
+            [&](R(&h)[4][3]) {
+              R P[3][3];
+              snh_pk1(s, geo.mu, geo.lam, P);
+              corner_vjp(P, geo.D, h);
+            },
+            [&](R(&h)[4][3]) {
+              snh_hess_diag(s, geo.D, geo.mu, geo.lam, h);
+              clamp(h);
+            },
+            [&](R(&h)[4][3]) {
+              R M[3][3];
+              snh_hess_prod(s, d, dF, geo.mu, geo.lam, M);
+              corner_vjp(M, geo.D, h);
+            });
+      } else {
+        const R jm1 = (G[0][0] + G[1][1] + G[2][2]) + inv2(G) + det3(G);
+        Svd<R> sv;
+        svd_rv(G, jm1, sv);
+        R lk[3];
+        arap_lambdas(sv, lk);
+        if (do_fun) sums[0].add(arap_energy(sv, geo.mu));
+        if (do_quad) sums[1].add(fmax(arap_hess_quad(sv, lk, dF, geo.mu), R(0)));
+        fill(
+            [&](R(&h)[4][3]) {
+              R P[3][3];
+              arap_pk1(sv, geo.mu, P);
+              corner_vjp(P, geo.D, h);
+            },
+            [&](R(&h)[4][3]) {
+              arap_hess_diag(sv, lk, geo.D, geo.mu, h);
+              clamp(h);
+            },
+            [&](R(&h)[4][3]) {
+              R M[3][3];
+              arap_hess_prod(sv, lk, dF, geo.mu, M);
+              corner_vjp(M, geo.D, h);
+            });
+      }
+    }
+    if (vectors) {
+      // corner k of the group's lanes is a distinct vertex for every lane
 #pragma unroll
-          for (int a = 0; a < 4; ++a)
+      for (int k = 0; k < 4; ++k) {
+        __syncwarp();
+        if (lane < n) {
+          R x[9];
+          my.load(l[k], x);
 #pragma unroll
-            for (int c = 0; c < 3; ++c) atomicAdd(&acc[6 + c][l[a]], f[a][c]);
+          for (int q = 0; q < NVEC; ++q)
+#pragma unroll
+            for (int c = 0; c < 3; ++c) x[3 * q + c] += f[q][k][c];
+          my.store(l[k], x);
         }
       }
-    } else {
-      const R jm1 = (G[0][0] + G[1][1] + G[2][2]) + inv2(G) + det3(G);
-      Svd<R> sv;
-      svd_rv(G, jm1, sv);
-      if (do_fun) sums[0].add(arap_energy(sv, geo.mu));
-      if (do_grad) {
-        R P[3][3];
-        arap_pk1(sv, geo.mu, P);
-        corner_vjp(P, geo.D, f);
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-          for (int c = 0; c < 3; ++c) atomicAdd(&acc[c][l[a]], f[a][c]);
-      }
-      R lk[3];
-      arap_lambdas(sv, lk);
-      if (do_diag) {
-        arap_hess_diag(sv, lk, geo.D, geo.mu, f);
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-          for (int c = 0; c < 3; ++c) atomicAdd(&acc[3 + c][l[a]], fmax(f[a][c], R(0)));
-      }
-      if (do_quad) sums[1].add(fmax(arap_hess_quad(sv, lk, dF, geo.mu), R(0)));
-      if (do_prod) {
-        R M[3][3];
-        arap_hess_prod(sv, lk, dF, geo.mu, M);
-        corner_vjp(M, geo.D, f);
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-          for (int c = 0; c < 3; ++c) atomicAdd(&acc[6 + c][l[a]], f[a][c]);
-      }
+      __syncwarp();
     }
+    g = gn;
+    n = nn;
+    geo = geon;
+    ids = idsn;
   }
-  __syncthreads();
-
-  for (int i = threadIdx.x; i < nv; i += blockDim.x) {
-    const int s = slot_of_tv[vs + i];
-    if (do_grad) slots[s] = V4<R>{acc[0][i], acc[1][i], acc[2][i], R(0)};
-    if (do_diag) slots[(size_t)n_slots + s] = V4<R>{acc[3][i], acc[4][i], acc[5][i], R(0)};
-    if (do_prod) slots[2 * (size_t)n_slots + s] = V4<R>{acc[6][i], acc[7][i], acc[8][i], R(0)};
+  if (vectors) {
+    __syncthreads();
+    const VecArrays<R, NVEC> out{(unsigned char*)slots, (size_t)n_slots};
+    for (int i = threadIdx.x; i < nv; i += blockDim.x) {
+      R x[9];
+      VecArrays<R, NVEC>{acc, (size_t)kTileVerts}.load(i, x);
+      for (int w = 1; w < warps; ++w) {
+        R y[9];
+        VecArrays<R, NVEC>{acc + w * kAccBytes, (size_t)kTileVerts}.load(i, y);
+#pragma unroll
+        for (int c = 0; c < 3 * NVEC; ++c) x[c] += y[c];
+      }
+      out.store(slot_of_tv[vs + i], x);
+    }
   }
 
   if (do_fun || do_quad) {
     double tot[2];
     if (grid_reduce<2, R>(sums, partials, counter, gridDim.x, red, tot) && threadIdx.x == 0) {
-      if (do_fun) *energy += tot[0];
-      if (do_quad) *quad += tot[1];
+      if (do_fun) *energy = assign ? tot[0] : *energy + tot[0];
+      if (do_quad) *quad = assign ? tot[1] : *quad + tot[1];
     }
   }
 }
 
 constexpr int kUnpackThreads = 256;
 
+// The vertex pass: a vertex's slots (contiguous, fixed order), the external
+// force, and one write per requested vector in the caller's order.  Bound by
+// the latency of offsets -> slots -> output, so a dependent launch reads the
+// offsets before the element pass ends.
+template <class R, int NVEC>
+__global__ void __launch_bounds__(kUnpackThreads) unpack_kernel(
+    int n, const int32_t* __restrict__ uoi, const int32_t* __restrict__ off, const void* __restrict__ slots,
+    int n_slots, R* o0, R* o1, R* o2, int assign, int force_grad, int force_fun, const V4<R>* __restrict__ force,
+    const R* __restrict__ u, AccStore<R>* partials, unsigned* counter, double* energy) {
+  __shared__ Acc<R> red[kUnpackThreads / 32];
+  const VecArrays<R, NVEC> in{(unsigned char*)slots, (size_t)n_slots};
+  Acc<R> ext[1] = {};
+  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  int s0 = 0, s1 = 0, user = 0;
+  if (i < n) {
+    user = uoi[i];
+    s0 = off[i];
+    s1 = off[i + 1];
+  }
+  pdl_wait();
+  while (i < n) {
+    const size_t k = 3 * (size_t)user;
+    V4<R> f{R(0), R(0), R(0), R(0)};
+    if (force_grad || force_fun) f = ldg4(force + i);
+    if constexpr (NVEC > 0) {
+      R x[9];
+#pragma unroll
+      for (int c = 0; c < 3 * NVEC; ++c) x[c] = R(0);
+      for (int s = s0; s < s1; ++s) {
+        R y[9];
+        in.load(s, y);
+#pragma unroll
+        for (int c = 0; c < 3 * NVEC; ++c) x[c] += y[c];
+      }
+      if (force_grad) {  // the gradient, when requested, is the first vector
+        x[0] -= f.x;
+        x[1] -= f.y;
+        x[2] -= f.z;
+      }
+      R* const outs[3] = {o0, o1, o2};
+#pragma unroll
+      for (int q = 0; q < NVEC; ++q)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) outs[q][k + c] = assign ? x[3 * q + c] : outs[q][k + c] + x[3 * q + c];
+    }
+    if (force_fun) ext[0].add(-(f.x * u[k] + f.y * u[k + 1] + f.z * u[k + 2]));
+    i += gridDim.x * blockDim.x;
+    if (i < n) {
+      user = uoi[i];
+      s0 = off[i];
+      s1 = off[i + 1];
+    }
+  }
+  if (force_fun) {
+    double tot[1];
+    if (grid_reduce<1, R>(ext, partials, counter, gridDim.x, red, tot) && threadIdx.x == 0) *energy += tot[0];
+  }
+}
+
+int popcount3(unsigned vec) { return (int)((vec & 1u) + ((vec >> 1) & 1u) + ((vec >> 2) & 1u)); }
+
+// the vectors among the flags, as a 3-bit mask (gradient, diagonal, product)
+unsigned vec_mask(unsigned flags) {
+  return (flags & AGB_GRAD ? 1u : 0u) | (flags & AGB_HESS_DIAG ? 2u : 0u) | (flags & AGB_HESS_PROD ? 4u : 0u);
+}
+
+// Warps per tile.  With at least two tiles per SM, four (five CTAs per SM
+// keep the SM busy, and fewer accumulator copies are summed); below that the
+// SMs have room, and more warps shorten each tile's chain of groups: 8 up to
+// two tiles per SM, 16 (FP32; 8 in FP64, by shared memory) up to one.
+int eval_warps(int precision, int n_tiles) {
+  if (n_tiles > 2 * kSMs) return 4;
+  return n_tiles > kSMs || precision == AGB_F64 ? 8 : 16;
+}
+
+template <class R, int MAT, int NVEC, int MAXT>
+cudaError_t eval_launch(const FemView& fv, int warps, unsigned flags, const void* u, const void* p,
+                        const int32_t* slot_of_tv, void* slots, int32_t n_slots, void* partials, unsigned* counter,
+                        double* energy, double* quad, int assign, cudaStream_t s) {
+  const bool vectors = flags & (AGB_GRAD | AGB_HESS_DIAG | AGB_HESS_PROD);
+  const size_t smem = vectors ? eval_smem_bytes<R, NVEC>(warps) : eval_stage_bytes<R>();
+  if (smem > 48 * 1024) {  // above the default limit the kernel has to opt in
+    const cudaError_t e = cudaFuncSetAttribute(fem_eval_kernel<R, MAT, NVEC, MAXT>,
+                                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+  }
+  fem_eval_kernel<R, MAT, NVEC, MAXT><<<fv.n_tiles, 32 * warps, smem, s>>>(
+      fv, flags, (const R*)u, (const R*)p, slot_of_tv, slots, n_slots, (AccStore<R>*)partials, counter, energy, quad,
+      assign);
+  return cudaGetLastError();
+}
+
+template <class R, int MAT, int NVEC, class... A>
+cudaError_t eval_warps_of(const FemView& fv, int warps, A... args) {
+  return warps == 4 ? eval_launch<R, MAT, NVEC, 128>(fv, warps, args...)
+                    : eval_launch<R, MAT, NVEC, sizeof(R) == 4 ? 512 : 256>(fv, warps, args...);
+}
+
+template <class R, int MAT, class... A>
+cudaError_t eval_vectors(int nvec, const FemView& fv, A... args) {
+  switch (nvec) {
+    case 0:
+    case 1: return eval_warps_of<R, MAT, 1>(fv, args...);
+    case 2: return eval_warps_of<R, MAT, 2>(fv, args...);
+    default: return eval_warps_of<R, MAT, 3>(fv, args...);
+  }
+}
+
+template <class R, class... A>
+cudaError_t eval_material(int nvec, const FemView& fv, A... args) {
+  if (fv.material == AGB_ARAP) return eval_vectors<R, AGB_ARAP>(nvec, fv, args...);
+  if (fv.material == AGB_STABLE_NEO_HOOKEAN_MUSCLE)
+    return eval_vectors<R, AGB_STABLE_NEO_HOOKEAN_MUSCLE>(nvec, fv, args...);
+  return eval_vectors<R, AGB_STABLE_NEO_HOOKEAN>(nvec, fv, args...);
+}
+
+template <class R, int NVEC>
+cudaError_t unpack_launch(int n, const int32_t* uoi, const int32_t* off, const void* slots, int32_t n_slots,
+                          unsigned flags, void* grad, void* diag, void* prod, int assign, const void* force,
+                          const void* u, void* partials, unsigned* counter, double* energy, cudaStream_t s) {
+  R* outs[3] = {nullptr, nullptr, nullptr};
+  int k = 0;
+  if (flags & AGB_GRAD) outs[k++] = (R*)grad;
+  if (flags & AGB_HESS_DIAG) outs[k++] = (R*)diag;
+  if (flags & AGB_HESS_PROD) outs[k++] = (R*)prod;
+  const int force_grad = force && (flags & AGB_GRAD) ? 1 : 0, force_fun = force && (flags & AGB_FUN) ? 1 : 0;
+  return launch_pdl(unpack_kernel<R, NVEC>, dim3(unpack_blocks(n)), dim3(kUnpackThreads), 0, s, n, uoi, off, slots,
+                    n_slots, outs[0], outs[1], outs[2], assign, force_grad, force_fun, (const V4<R>*)force,
+                    (const R*)u, (AccStore<R>*)partials, counter, energy);
+}
+
+template <class R, class... A>
+cudaError_t unpack_vectors(int nvec, A... args) {
+  switch (nvec) {
+    case 0: return unpack_launch<R, 0>(args...);
+    case 1: return unpack_launch<R, 1>(args...);
+    case 2: return unpack_launch<R, 2>(args...);
+    default: return unpack_launch<R, 3>(args...);
+  }
+}
+
+}  // namespace
+
 int unpack_blocks(int n_points) {
   int b = (n_points + kUnpackThreads - 1) / kUnpackThreads;
   return b < 1 ? 1 : (b > 1216 ? 1216 : b);
 }
 
-template <class R>
-__global__ void __launch_bounds__(kUnpackThreads) unpack_kernel(
-    int n, const int32_t* __restrict__ uoi, const int32_t* __restrict__ off,
-    const V4<R>* __restrict__ slots, int n_slots, unsigned flags, R* grad, R* diag, R* prod,
-    const V4<R>* __restrict__ force, const V4<R>* __restrict__ u, AccStore<R>* partials,
-    unsigned* counter, double* energy) {
-  __shared__ Acc<R> red[kUnpackThreads / 32];
-  Acc<R> ext[1] = {};
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const size_t k = 3 * (size_t)uoi[i];
-    const int s0 = off[i], s1 = off[i + 1];
-    R* outs[3] = {grad, diag, prod};
-    const unsigned fl[3] = {AGB_GRAD, AGB_HESS_DIAG, AGB_HESS_PROD};
-#pragma unroll
-    for (int q = 0; q < 3; ++q) {
-      if (!(flags & fl[q])) continue;
-      R sx = R(0), sy = R(0), sz = R(0);
-      for (int s = s0; s < s1; ++s) {
-        const V4<R> v = slots[(size_t)q * n_slots + s];
-        sx += v.x;
-        sy += v.y;
-        sz += v.z;
-      }
-      if (q == 0 && force) {
-        const V4<R> f = ldg4(force + i);
-        sx -= f.x;
-        sy -= f.y;
-        sz -= f.z;
-      }
-      outs[q][k] += sx;
-      outs[q][k + 1] += sy;
-      outs[q][k + 2] += sz;
-    }
-    if ((flags & AGB_FUN) && force) {
-      const V4<R> f = ldg4(force + i);
-      const V4<R> x = ldg4(u + i);
-      ext[0].add(-(f.x * x.x + f.y * x.y + f.z * x.z));
-    }
-  }
-  if ((flags & AGB_FUN) && force) {
-    double tot[1];
-    if (grid_reduce<1, R>(ext, partials, counter, gridDim.x, red, tot) && threadIdx.x == 0)
-      *energy += tot[0];
-  }
-}
-
-cudaError_t launch_pack(int precision, int n, const int32_t* uoi, const void* u, void* ui,
-                        const void* p, void* pi, cudaStream_t stream) {
-  const int blocks = unpack_blocks(n);
-  if (precision == AGB_F64)
-    pack_kernel<double><<<blocks, 256, 0, stream>>>(n, uoi, (const double*)u, (V4<double>*)ui,
-                                                    (const double*)p, (V4<double>*)pi);
-  else
-    pack_kernel<float><<<blocks, 256, 0, stream>>>(n, uoi, (const float*)u, (V4<float>*)ui,
-                                                   (const float*)p, (V4<float>*)pi);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_fem_eval(int precision, const FemView& fv, unsigned flags, const void* u,
-                            const void* p, const int32_t* slot_of_tv, void* slots, int32_t n_slots,
-                            void* partials, unsigned* counter, double* energy, double* quad,
-                            cudaStream_t stream) {
+cudaError_t launch_fem_eval(int precision, const FemView& fv, unsigned flags, const void* u, const void* p,
+                            const int32_t* slot_of_tv, void* slots, int32_t n_slots, void* partials,
+                            unsigned* counter, double* energy, double* quad, int assign, cudaStream_t stream) {
   if (fv.n_tiles == 0) return cudaSuccess;
-  const dim3 grid(fv.n_tiles), block(kElemThreads);
-#define AGB_EVAL_LAUNCH(R, MAT)                                                                \
-  fem_eval_kernel<R, MAT><<<grid, block, 0, stream>>>(                                        \
-      fv, flags, (const V4<R>*)u, (const V4<R>*)p, slot_of_tv, (V4<R>*)slots, n_slots,          \
-      (AccStore<R>*)partials, counter, energy, quad)
-  if (precision == AGB_F64) {
-    if (fv.material == AGB_ARAP)
-      AGB_EVAL_LAUNCH(double, AGB_ARAP);
-    else if (fv.material == AGB_STABLE_NEO_HOOKEAN_MUSCLE)
-      AGB_EVAL_LAUNCH(double, AGB_STABLE_NEO_HOOKEAN_MUSCLE);
-    else
-      AGB_EVAL_LAUNCH(double, AGB_STABLE_NEO_HOOKEAN);
-  } else {
-    if (fv.material == AGB_ARAP)
-      AGB_EVAL_LAUNCH(float, AGB_ARAP);
-    else if (fv.material == AGB_STABLE_NEO_HOOKEAN_MUSCLE)
-      AGB_EVAL_LAUNCH(float, AGB_STABLE_NEO_HOOKEAN_MUSCLE);
-    else
-      AGB_EVAL_LAUNCH(float, AGB_STABLE_NEO_HOOKEAN);
-  }
-#undef AGB_EVAL_LAUNCH
-  return cudaGetLastError();
+  const int nvec = popcount3(vec_mask(flags)), warps = eval_warps(precision, fv.n_tiles);
+  if (precision == AGB_F64)
+    return eval_material<double>(nvec, fv, warps, flags, u, p, slot_of_tv, slots, n_slots, partials, counter, energy,
+                                 quad, assign, stream);
+  return eval_material<float>(nvec, fv, warps, flags, u, p, slot_of_tv, slots, n_slots, partials, counter, energy,
+                              quad, assign, stream);
 }
 
-cudaError_t launch_unpack(int precision, int n, const int32_t* uoi, const int32_t* off,
-                          const void* slots, int32_t n_slots, unsigned flags, void* grad,
-                          void* diag, void* prod, const void* force, const void* u, void* partials,
-                          unsigned* counter, double* energy, cudaStream_t stream) {
-  const int blocks = unpack_blocks(n);
+cudaError_t launch_unpack(int precision, int n, const int32_t* uoi, const int32_t* off, const void* slots,
+                          int32_t n_slots, unsigned flags, void* grad, void* diag, void* prod, int assign,
+                          const void* force, const void* u, void* partials, unsigned* counter, double* energy,
+                          cudaStream_t stream) {
+  if (n <= 0) return cudaSuccess;
+  const int nvec = popcount3(vec_mask(flags));
   if (precision == AGB_F64)
-    unpack_kernel<double><<<blocks, kUnpackThreads, 0, stream>>>(
-        n, uoi, off, (const V4<double>*)slots, n_slots, flags, (double*)grad, (double*)diag,
-        (double*)prod, (const V4<double>*)force, (const V4<double>*)u,
-        (AccStore<double>*)partials, counter, energy);
-  else
-    unpack_kernel<float><<<blocks, kUnpackThreads, 0, stream>>>(
-        n, uoi, off, (const V4<float>*)slots, n_slots, flags, (float*)grad, (float*)diag,
-        (float*)prod, (const V4<float>*)force, (const V4<float>*)u, (AccStore<float>*)partials,
-        counter, energy);
-  return cudaGetLastError();
+    return unpack_vectors<double>(nvec, n, uoi, off, slots, n_slots, flags, grad, diag, prod, assign, force, u,
+                                  partials, counter, energy, stream);
+  return unpack_vectors<float>(nvec, n, uoi, off, slots, n_slots, flags, grad, diag, prod, assign, force, u, partials,
+                               counter, energy, stream);
 }
 
 // ---------------------------------------------------------------------------

@@ -31,15 +31,14 @@ static __device__ __align__(256) unsigned char g_fun_noalloc_scratch[kNoAllocPar
 
 template <class R, int MAT>
 __global__ void __launch_bounds__(kElemThreads)
-    fem_fun_noalloc_kernel(FemView fv, const int32_t* __restrict__ user_of_internal,
-                           const R* __restrict__ u, unsigned char* scratch, double* out) {
+    fem_fun_noalloc_kernel(FemView fv, const R* __restrict__ u, unsigned char* scratch, double* out) {
   __shared__ R sx[3][kTileVerts];
   __shared__ Acc<R> red[kElemThreads / 32];
   const int tile = blockIdx.x;
   const int vs = fv.tile_vstart[tile], nv = fv.tile_vstart[tile + 1] - vs;
   const int es = fv.tile_estart[tile], ee = fv.tile_estart[tile + 1];
   for (int i = threadIdx.x; i < nv; i += blockDim.x) {
-    const size_t k = 3 * (size_t)user_of_internal[fv.tv_vid[vs + i]];
+    const size_t k = 3 * (size_t)fv.tv_user[vs + i];
     sx[0][i] = u[k];
     sx[1][i] = u[k + 1];
     sx[2][i] = u[k + 2];
@@ -106,20 +105,19 @@ extern "C" int agb_fem_fun_noalloc(agb_fem* fem, const void* u, double* output, 
   if (rc) return rc;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   AGB_CHECK_CUDA(cudaMemsetAsync(scratch + kNoAllocPartialBytes, 0, sizeof(unsigned), s));
-  const int32_t* uoi = fem->space->d_user_of_internal;
   const dim3 grid(fv.n_tiles), block(kElemThreads);
   if (fem->precision == AGB_F64) {
     if (fv.material == AGB_ARAP)
-      fem_fun_noalloc_kernel<double, AGB_ARAP><<<grid, block, 0, s>>>(fv, uoi, (const double*)u, scratch, output);
+      fem_fun_noalloc_kernel<double, AGB_ARAP><<<grid, block, 0, s>>>(fv, (const double*)u, scratch, output);
     else
       fem_fun_noalloc_kernel<double, AGB_STABLE_NEO_HOOKEAN>
-          <<<grid, block, 0, s>>>(fv, uoi, (const double*)u, scratch, output);
+          <<<grid, block, 0, s>>>(fv, (const double*)u, scratch, output);
   } else {
     if (fv.material == AGB_ARAP)
-      fem_fun_noalloc_kernel<float, AGB_ARAP><<<grid, block, 0, s>>>(fv, uoi, (const float*)u, scratch, output);
+      fem_fun_noalloc_kernel<float, AGB_ARAP><<<grid, block, 0, s>>>(fv, (const float*)u, scratch, output);
     else
       fem_fun_noalloc_kernel<float, AGB_STABLE_NEO_HOOKEAN>
-          <<<grid, block, 0, s>>>(fv, uoi, (const float*)u, scratch, output);
+          <<<grid, block, 0, s>>>(fv, (const float*)u, scratch, output);
   }
   AGB_CHECK_CUDA(cudaGetLastError());
   return AGB_OK;

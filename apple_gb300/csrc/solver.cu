@@ -652,24 +652,6 @@ cudaError_t launch_solver_energy(const SolveArgs& a, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-// launch with programmatic stream serialisation: the kernel may start while
-// the previous kernel in the stream finishes and waits in griddepcontrol.wait
-template <class... P, class... A>
-static cudaError_t launch_pdl(void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
-                              A... args) {
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = grid;
-  cfg.blockDim = block;
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, k, args...);
-}
-
 // the direction pass (pdl: as a programmatic dependent)
 template <class R, int MAT>
 static cudaError_t launch_dir(const SolveArgs& a, int use_cond, bool pdl, cudaStream_t s) {

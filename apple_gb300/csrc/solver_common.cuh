@@ -6,20 +6,17 @@
 
 #include <math.h>
 
+#include "pdl.cuh"
 #include "solver.h"
 #include "tile.cuh"
 
 namespace agb {
 
-constexpr int kSMs = 152;
 constexpr int kVThreads = 256;
 constexpr int kWarps = kElemThreads / 32;
 // gradient pass: 4 warps per tile, one private accumulator copy per warp
 constexpr int kGradThreads = 128;
 constexpr int kGradWarps = kGradThreads / 32;
-
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // the passes of a guarded iteration (SolveArgs::guard) skip it when the one
 // before it ended the solve's run: limit reached or refresh due
@@ -177,47 +174,11 @@ __device__ __forceinline__ void stage_dir_packed(const SolveArgs& a, int v, R be
   sq[threadIdx.x] = V2<R>{p[1], p[2]};
 }
 
-// G = sum_a (x_a - x_0) D_a^T and dF = sum_a (p_a - p_0) D_a^T from the
-// packed staging (the same arithmetic as vec_gradient on each field)
-template <class R>
-__device__ __forceinline__ void dir_gradients(const V4<R>* sxp, const V2<R>* sq, const int (&l)[4],
-                                              const R (&D)[3][3], R (&G)[3][3], R (&dF)[3][3]) {
-  const V4<R> w0 = sxp[l[0]], w1 = sxp[l[1]], w2 = sxp[l[2]], w3 = sxp[l[3]];
-  const V2<R> q0 = sq[l[0]], q1 = sq[l[1]], q2 = sq[l[2]], q3 = sq[l[3]];
-  const R e[3][3] = {{w1.x - w0.x, w2.x - w0.x, w3.x - w0.x},
-                     {w1.y - w0.y, w2.y - w0.y, w3.y - w0.y},
-                     {w1.z - w0.z, w2.z - w0.z, w3.z - w0.z}};
-  const R f[3][3] = {{w1.w - w0.w, w2.w - w0.w, w3.w - w0.w},
-                     {q1.x - q0.x, q2.x - q0.x, q3.x - q0.x},
-                     {q1.y - q0.y, q2.y - q0.y, q3.y - q0.y}};
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-#pragma unroll
-    for (int j = 0; j < 3; ++j) {
-      G[i][j] = e[i][0] * D[0][j] + e[i][1] * D[1][j] + e[i][2] * D[2][j];
-      dF[i][j] = f[i][0] * D[0][j] + f[i][1] * D[1][j] + f[i][2] * D[2][j];
-    }
-}
-
 // the thread's vertex of a tile, or -1
 __device__ __forceinline__ int tile_vertex(const FemView& fv, int tile, int i) {
   if (tile >= fv.n_tiles) return -1;
   const int vs = fv.tile_vstart[tile];
   return i < fv.tile_vstart[tile + 1] - vs ? fv.tv_vid[vs + i] : -1;
-}
-
-// W = sum_a (w_a - w_0) D_a^T from 16-byte staged corners
-template <class R>
-__device__ __forceinline__ void vec_gradient(const V4<R>* s, const int (&l)[4], const R (&D)[3][3],
-                                             R (&W)[3][3]) {
-  const V4<R> w0 = s[l[0]], w1 = s[l[1]], w2 = s[l[2]], w3 = s[l[3]];
-  const R e[3][3] = {{w1.x - w0.x, w2.x - w0.x, w3.x - w0.x},
-                     {w1.y - w0.y, w2.y - w0.y, w3.y - w0.y},
-                     {w1.z - w0.z, w2.z - w0.z, w3.z - w0.z}};
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-#pragma unroll
-    for (int j = 0; j < 3; ++j) W[i][j] = e[i][0] * D[0][j] + e[i][1] * D[1][j] + e[i][2] * D[2][j];
 }
 
 template <class R>

@@ -179,4 +179,40 @@ __device__ __forceinline__ void pdir(const V4<R>& g, const V4<R>& d, const V4<R>
 
 __device__ __forceinline__ int corner(uint32_t ids, int a) { return (int)((ids >> (8 * a)) & 0xffu); }
 
+// G = sum_a (x_a - x_0) D_a^T and dF = sum_a (p_a - p_0) D_a^T from the
+// packed staging (the same arithmetic as vec_gradient on each field)
+template <class R>
+__device__ __forceinline__ void dir_gradients(const V4<R>* sxp, const V2<R>* sq, const int (&l)[4],
+                                              const R (&D)[3][3], R (&G)[3][3], R (&dF)[3][3]) {
+  const V4<R> w0 = sxp[l[0]], w1 = sxp[l[1]], w2 = sxp[l[2]], w3 = sxp[l[3]];
+  const V2<R> q0 = sq[l[0]], q1 = sq[l[1]], q2 = sq[l[2]], q3 = sq[l[3]];
+  const R e[3][3] = {{w1.x - w0.x, w2.x - w0.x, w3.x - w0.x},
+                     {w1.y - w0.y, w2.y - w0.y, w3.y - w0.y},
+                     {w1.z - w0.z, w2.z - w0.z, w3.z - w0.z}};
+  const R f[3][3] = {{w1.w - w0.w, w2.w - w0.w, w3.w - w0.w},
+                     {q1.x - q0.x, q2.x - q0.x, q3.x - q0.x},
+                     {q1.y - q0.y, q2.y - q0.y, q3.y - q0.y}};
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      G[i][j] = e[i][0] * D[0][j] + e[i][1] * D[1][j] + e[i][2] * D[2][j];
+      dF[i][j] = f[i][0] * D[0][j] + f[i][1] * D[1][j] + f[i][2] * D[2][j];
+    }
+}
+
+// W = sum_a (w_a - w_0) D_a^T from 16-byte staged corners
+template <class R>
+__device__ __forceinline__ void vec_gradient(const V4<R>* s, const int (&l)[4], const R (&D)[3][3],
+                                             R (&W)[3][3]) {
+  const V4<R> w0 = s[l[0]], w1 = s[l[1]], w2 = s[l[2]], w3 = s[l[3]];
+  const R e[3][3] = {{w1.x - w0.x, w2.x - w0.x, w3.x - w0.x},
+                     {w1.y - w0.y, w2.y - w0.y, w3.y - w0.y},
+                     {w1.z - w0.z, w2.z - w0.z, w3.z - w0.z}};
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int j = 0; j < 3; ++j) W[i][j] = e[i][0] * D[0][j] + e[i][1] * D[1][j] + e[i][2] * D[2][j];
+}
+
 }  // namespace agb
