@@ -758,7 +758,7 @@ int agb_solver_destroy(agb_solver* sv) {
                   (void*)sv->d_group_estart, (void*)sv->d_tv_vid,
                   (void*)sv->d_slot_of_tv, sv->d_rec, (void*)sv->d_ids, sv->d_xa, sv->d_gd, sv->d_p0,
                   sv->d_p1, sv->d_xref, sv->d_gref, sv->d_svd, sv->d_slots, sv->d_part, (void*)sv->d_cnt,
-                  (void*)sv->d_state, sv->d_u_tmp, sv->d_act})
+                  (void*)sv->d_state, sv->d_u_tmp, sv->d_act, sv->d_res_part, (void*)sv->d_res_counters})
     dfree(p);
   if (sv->h_state) cudaFreeHost(sv->h_state);
   delete sv;
@@ -954,8 +954,29 @@ int agb_solver_create(agb_model* m, const agb_pncg_params* params, agb_solver** 
   a.cond_outer = 0;
   a.refresh_exits = 0;
   a.guard = 0;
+  // resident iterations when every tile's CTA fits the device at once; a
+  // point that no cell uses has no tile to own it there
+  bool covered = true;
+  for (int v = 0; v < np && covered; ++v) covered = m->off[v + 1] > m->off[v];
+  if (covered) {
+    rc = check_launch(resident_prepare(a, &sv->resident), "resident_prepare");
+    if (!rc && sv->resident) rc = dalloc_bytes(&sv->d_res_part, 8 * 18 * nt);
+    if (!rc && sv->resident) rc = dalloc(&sv->d_res_counters, 2);
+    if (!rc && sv->resident && cudaMemset(sv->d_res_counters, 0, 2 * sizeof(unsigned)) != cudaSuccess) rc = AGB_E_CUDA;
+    if (rc) {
+      if (rc == AGB_E_CUDA && agb::last_error()[0] == 0) set_error("agb_solver_create: CUDA allocation failed");
+      agb_solver_destroy(sv);
+      return rc;
+    }
+  }
   *out = sv;
   return AGB_OK;
+}
+
+// the solver's iterations up to its limit, or a due refresh, in one launch
+static cudaError_t run_resident(agb_solver* sv, const SolveArgs& a, cudaStream_t s) {
+  return launch_resident(a, sv->d_res_part, (char*)sv->d_res_part + 8 * 6 * (size_t)a.fv.n_tiles, sv->d_res_counters,
+                         s);
 }
 
 int agb_solver_reset(agb_solver* sv, const void* u, void* stream) {
@@ -975,7 +996,8 @@ int agb_solver_reset(agb_solver* sv, const void* u, void* stream) {
 
 // Capture into `graph` after `deps` (which may be empty): the three passes
 // of one iteration (refresh = false) or the two refresh passes as plain
-// launches (refresh = true).
+// launches (refresh = true); for resident iterations their launch and the
+// refresh passes.
 // Iterations per body of agb_solver_iterate's WHILE loop: the second of two
 // is guarded (its passes return at once when the first ended the run), its
 // direction pass a programmatic dependent of the first's vertex pass, and
@@ -989,6 +1011,13 @@ static cudaError_t capture_into(agb_solver* sv, cudaGraph_t graph, const cudaGra
   cudaStream_t cs = sv->capture_stream;
   cudaError_t e = cudaStreamBeginCaptureToGraph(cs, graph, deps, nullptr, n_deps, cudaStreamCaptureModeThreadLocal);
   if (e != cudaSuccess) return e;
+  if (sv->resident) {
+    cudaError_t le = run_resident(sv, a, cs);
+    if (le == cudaSuccess) le = launch_solver_refresh(a, cs, false);
+    cudaGraph_t captured = nullptr;
+    e = cudaStreamEndCapture(cs, &captured);
+    return e == cudaSuccess ? le : e;
+  }
   cudaError_t le = refresh ? launch_solver_refresh(a, cs, false) : launch_solver_iteration(a, a.cond != 0, cs);
   for (int k = 1; !refresh && le == cudaSuccess && k < AGB_LOOP_UNROLL; ++k) {
     SolveArgs ag = a;
@@ -1021,6 +1050,7 @@ static cudaError_t add_conditional(cudaGraph_t g, const cudaGraphNode_t* deps, s
 // iteration limit or asks for a refresh; the refresh vertex pass (which does
 // the refresh only if it was asked for) continues the outer loop and re-arms
 // the inner one unless the solve ended or reached the limit.
+// Resident iterations: WHILE(outer) { resident run; refresh passes }.
 static int build_loop_graph(agb_solver* sv) {
   cudaGraph_t g = nullptr;
   AGB_CHECK_CUDA(cudaGraphCreate(&g, 0));
@@ -1029,7 +1059,13 @@ static int build_loop_graph(agb_solver* sv) {
   cudaGraphNode_t w_out = nullptr, w_in = nullptr;
   cudaGraph_t body_out = nullptr, body_in = nullptr;
   cudaError_t e = cudaSuccess;
-  if (a.delta) {
+  if (sv->resident) {
+    e = cudaGraphConditionalHandleCreate(&h_out, g, 1u, cudaGraphCondAssignDefault);
+    if (e == cudaSuccess) e = add_conditional(g, nullptr, 0, h_out, cudaGraphCondTypeWhile, &w_out, &body_out);
+    SolveArgs ar = a;
+    ar.cond_outer = (unsigned long long)h_out;
+    if (e == cudaSuccess) e = capture_into(sv, body_out, nullptr, 0, ar, true);
+  } else if (a.delta) {
     e = cudaGraphConditionalHandleCreate(&h_out, g, 1u, cudaGraphCondAssignDefault);
     if (e == cudaSuccess) e = add_conditional(g, nullptr, 0, h_out, cudaGraphCondTypeWhile, &w_out, &body_out);
     if (e == cudaSuccess) e = cudaGraphConditionalHandleCreate(&h_in, body_out, 1u, cudaGraphCondAssignDefault);
@@ -1073,8 +1109,15 @@ static int build_step_graph(agb_solver* sv) {
   cudaError_t e = cudaStreamBeginCaptureToGraph(cs, g, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
   size_t n_nodes = 0;
   if (e == cudaSuccess) {
-    cudaError_t le = launch_solver_iteration(a, false, cs);
-    if (le == cudaSuccess && a.delta) le = launch_solver_refresh(a, cs, true);
+    cudaError_t le;
+    if (sv->resident) {
+      le = launch_solver_set_limit(a, 1, cs);
+      if (le == cudaSuccess) le = run_resident(sv, a, cs);
+      if (le == cudaSuccess && a.delta) le = launch_solver_refresh(a, cs, false);
+    } else {
+      le = launch_solver_iteration(a, false, cs);
+      if (le == cudaSuccess && a.delta) le = launch_solver_refresh(a, cs, true);
+    }
     cudaGraph_t captured = nullptr;
     e = cudaStreamEndCapture(cs, &captured);
     if (e == cudaSuccess) e = le;
@@ -1096,8 +1139,12 @@ int agb_solver_step_kernels(agb_solver* sv, int32_t* n_kernels) {
 int agb_solver_iterate(agb_solver* sv, int32_t n_steps, void* stream) {
   AGB_REQUIRE(sv && n_steps >= 0, AGB_E_INVALID, "agb_solver_iterate: bad argument");
   if (n_steps == 0) return AGB_OK;
-  if (!sv->loop_exec) RC(build_loop_graph(sv));
   cudaStream_t s = as_stream(stream);
+  if (sv->resident && !sv->args.delta) {  // no refresh ends the run: no loop around it
+    RC(check_launch(launch_solver_set_limit(sv->args, n_steps, s), "set_limit"));
+    return check_launch(run_resident(sv, sv->args, s), "resident iterations");
+  }
+  if (!sv->loop_exec) RC(build_loop_graph(sv));
   RC(check_launch(launch_solver_set_limit(sv->args, n_steps, s), "set_limit"));
   AGB_CHECK_CUDA(cudaGraphLaunch(sv->loop_exec, s));
   return AGB_OK;

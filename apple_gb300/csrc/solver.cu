@@ -507,7 +507,7 @@ __global__ void __launch_bounds__(kVThreads) solver_ref_vertex_kernel(SolveArgs 
     const SolverState* st = a.st;
     const bool go = !st->done && st->iter < st->iter_limit;
     cudaGraphSetConditional((cudaGraphConditionalHandle)a.cond_outer, go ? 1u : 0u);
-    cudaGraphSetConditional((cudaGraphConditionalHandle)a.cond, go ? 1u : 0u);
+    if (a.cond) cudaGraphSetConditional((cudaGraphConditionalHandle)a.cond, go ? 1u : 0u);
   }
   if (!a.st->refresh) return;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.n_points; i += gridDim.x * blockDim.x) ref_vertex(a, i);

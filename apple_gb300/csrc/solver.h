@@ -135,6 +135,13 @@ cudaError_t launch_solver_refresh(const SolveArgs& a, cudaStream_t s, bool pdl =
 // set st->refresh (the next refresh passes run unconditionally)
 cudaError_t launch_solver_force_refresh(const SolveArgs& a, cudaStream_t s);
 
+// Resident iterations (solver_resident.cu): one cooperative launch runs until
+// the iteration limit, termination or a due refresh.  resident_prepare tells
+// whether every tile's CTA fits the device at once; part_d and part_v hold 6
+// and 12 partials per tile, counters two zeroed words.
+cudaError_t resident_prepare(const SolveArgs& a, bool* fits);
+cudaError_t launch_resident(const SolveArgs& a, void* part_d, void* part_v, unsigned* counters, cudaStream_t s);
+
 // Adjoint CG (adjoint.cu): scalars of H lam = rhs on the free DOFs at the
 // solver's current x, kept on the device like SolverState.
 struct CgState {
@@ -266,6 +273,10 @@ struct agb_solver {
   cudaGraphExec_t step_exec = nullptr;
   int step_kernels = 0;  // kernel nodes of one iteration
   cudaStream_t capture_stream = nullptr;
+  // resident iterations, when the mesh fits (solver_resident.cu)
+  bool resident = false;
+  void* d_res_part = nullptr;         // 18 partials per tile
+  unsigned* d_res_counters = nullptr;
   bool has_state = false;  // vertex state written (reset or checkpoint load)
   uint64_t fingerprint = 0;  // of the model and parameters, checked by agb_solver_load
 };

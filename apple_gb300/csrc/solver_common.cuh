@@ -469,33 +469,26 @@ __device__ __forceinline__ void vertex_load(const SolveArgs& a, int i, int s0, i
   in.s1 = s1;
 }
 
-// the rest of a vertex once its slots are summed (gs, ds in slot order)
+// g and d of a vertex from its slot sums (gs, ds in slot order; r the reference
+// gradient, f the external force, xn the new position), masked, and its terms
+// of vertex_decide's sums
 template <class R, bool DELTA>
-__device__ __forceinline__ void vertex_apply(const SolveArgs& a, int i, const VertexIn<R>& in, R t,
-                                             R (&gs)[3], const R (&ds)[3], R (&s)[12]) {
-  V4<R>* XA = (V4<R>*)a.xa;
-  V4<R>* GD = (V4<R>*)a.gd;
-  const bool ext = a.force != nullptr;
-  const int mask = (int)in.x.w;
-  const R p[3] = {in.p.x, in.p.y, in.p.z};
-  R xh[3] = {in.x.x, in.x.y, in.x.z}, xlo[3] = {in.xl.x, in.xl.y, in.xl.z};
-#pragma unroll
-  for (int c = 0; c < 3; ++c) pair_add(xh[c], xlo[c], mul_rn(t, p[c]));
-  const R xn[3] = {xh[0] + xlo[0], xh[1] + xlo[1], xh[2] + xlo[2]};
+__device__ __forceinline__ void vertex_terms(bool ext, int mask, const R (&xn)[3], const R (&p)[3],
+                                             const V4<R>& go4, const V4<R>& r, const V4<R>& f, R (&gs)[3],
+                                             const R (&ds)[3], R (&gn)[3], R (&dn)[3], R (&s)[12]) {
   if constexpr (DELTA) {
     // g = g(x_ref) + sum_e (f_e(x) - f_e(x_ref)); the force is folded into g(x_ref)
-    gs[0] += in.r.x;
-    gs[1] += in.r.y;
-    gs[2] += in.r.z;
-    if (ext) s[11] += -(in.f.x * xn[0] + in.f.y * xn[1] + in.f.z * xn[2]);
+    gs[0] += r.x;
+    gs[1] += r.y;
+    gs[2] += r.z;
+    if (ext) s[11] += -(f.x * xn[0] + f.y * xn[1] + f.z * xn[2]);
   } else if (ext) {
-    gs[0] -= in.f.x;
-    gs[1] -= in.f.y;
-    gs[2] -= in.f.z;
-    s[11] += -(in.f.x * xn[0] + in.f.y * xn[1] + in.f.z * xn[2]);
+    gs[0] -= f.x;
+    gs[1] -= f.y;
+    gs[2] -= f.z;
+    s[11] += -(f.x * xn[0] + f.y * xn[1] + f.z * xn[2]);
   }
-  const R go[3] = {in.g.x, in.g.y, in.g.z};
-  R gn[3], dn[3];
+  const R go[3] = {go4.x, go4.y, go4.z};
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
     const bool fixed = (mask >> c) & 1;
@@ -520,6 +513,22 @@ __device__ __forceinline__ void vertex_apply(const SolveArgs& a, int i, const Ve
     s[9] += p[c] * gn[c];
     s[10] += gn[c] * gn[c];
   }
+}
+
+// the rest of a vertex once its slots are summed (gs, ds in slot order)
+template <class R, bool DELTA>
+__device__ __forceinline__ void vertex_apply(const SolveArgs& a, int i, const VertexIn<R>& in, R t,
+                                             R (&gs)[3], const R (&ds)[3], R (&s)[12]) {
+  V4<R>* XA = (V4<R>*)a.xa;
+  V4<R>* GD = (V4<R>*)a.gd;
+  const int mask = (int)in.x.w;
+  const R p[3] = {in.p.x, in.p.y, in.p.z};
+  R xh[3] = {in.x.x, in.x.y, in.x.z}, xlo[3] = {in.xl.x, in.xl.y, in.xl.z};
+#pragma unroll
+  for (int c = 0; c < 3; ++c) pair_add(xh[c], xlo[c], mul_rn(t, p[c]));
+  const R xn[3] = {xh[0] + xlo[0], xh[1] + xlo[1], xh[2] + xlo[2]};
+  R gn[3], dn[3];
+  vertex_terms<R, DELTA>(a.force != nullptr, mask, xn, p, in.g, in.r, in.f, gs, ds, gn, dn, s);
   XA[2 * i] = V4<R>{xh[0], xh[1], xh[2], in.x.w};
   XA[2 * i + 1] = V4<R>{xlo[0], xlo[1], xlo[2], R(0)};
   GD[2 * i] = V4<R>{gn[0], gn[1], gn[2], R(0)};

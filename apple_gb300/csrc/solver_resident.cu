@@ -1,0 +1,468 @@
+// PNCG iterations of a small or medium mesh in one cooperative launch.
+//
+// A mesh of a few hundred tiles has too little work per pass to cover the
+// fixed costs of the three-kernel iteration (solver.cu): a launch, a drain, a
+// completion counter and a one-thread scalar tail per pass.  Here every tile
+// stays on one resident CTA for the whole run, three grid barriers separate
+// the passes, and all CTAs sum the partials and take the scalar decisions
+// themselves (the same numbers in the same order, so they agree bit for bit):
+//
+//   direction   the CTA's tile vertices read (g, d), form p = -P g + beta
+//               p_prev; per element p^T H_e p and the line-search polynomial
+//   -- barrier: sums, alpha_0, Armijo step t --
+//   gradient    x <- x + t p; forces and clamped diagonal -> slots
+//   -- barrier --
+//   vertex      the first tile that holds a vertex sums its slots, writes
+//               (g, d) and adds the 12 dot products
+//   -- barrier: sums, beta, preconditioner mean, termination --
+//
+// Every tile keeps x (hi + lo), p, x_ref and the previous g of its vertices in
+// shared memory between iterations and updates x and p itself (each tile that
+// holds a vertex computes the same values); only (g, d), the slots and the
+// partials pass through L2.  The run ends at the iteration limit, at
+// termination or when a reference-state refresh is due; the vertex state and
+// SolverState are then written back, so a run cut into pieces continues bit
+// for bit.
+//
+// Measured (40 iterations with the reset and the refreshes): 5,000-tet cube in
+// FP32 1,108 us against 1,377 with the three-kernel loop, 138,240 tets 1,467
+// against 1,976; 20 iterations of 138,240 tets in FP64 5,507 against 7,307.
+#include <math.h>
+
+#include "gridsync.cuh"
+#include "kernels.h"
+#include "solver.h"
+#include "solver_common.cuh"
+
+namespace agb {
+
+namespace {
+
+constexpr int kStateWords = (int)(sizeof(SolverState) / 4);
+
+// Warps per tile: in FP32 16 while every tile has an SM to itself, 8 up to two
+// tiles per SM (128 registers each way); FP64 is bound by its arithmetic pipe,
+// which 8 warps per SM fill: 4 per tile.  Above two tiles per SM the
+// three-kernel iteration is the faster one: with four 4-warp CTAs per SM this
+// kernel took 2.46 against 2.23 ms on 245,760 tets (376 tiles) and 2.88
+// against 2.55 ms on 400,000 (592 tiles), for 40 iterations and the reset.
+template <class R>
+constexpr int ctas_per_sm(int nw) {
+  return nw == 16 ? 1 : 2;
+}
+
+// per-vertex words kept between iterations: x hi, x lo, p, previous g, mask,
+// and with the reference-state correction x_ref
+template <bool DELTA>
+constexpr int kVertexWords = DELTA ? 16 : 13;
+
+template <class R, bool DELTA>
+constexpr size_t resident_smem(int nw) {
+  return (size_t)kTileVerts *
+         ((size_t)(nw + 1) * (sizeof(V4<R>) + sizeof(V2<R>)) + kVertexWords<DELTA> * sizeof(R) + 4 * sizeof(int));
+}
+
+template <class R>
+__device__ __forceinline__ V4<R> ldcg4(const V4<R>* p);
+template <>
+__device__ __forceinline__ V4<float> ldcg4<float>(const V4<float>* p) {
+  const float4 v = __ldcg(reinterpret_cast<const float4*>(p));
+  return V4<float>{v.x, v.y, v.z, v.w};
+}
+template <>
+__device__ __forceinline__ V4<double> ldcg4<double>(const V4<double>* p) {
+  const double2 a = __ldcg(reinterpret_cast<const double2*>(p));
+  const double2 b = __ldcg(reinterpret_cast<const double2*>(p) + 1);
+  return V4<double>{a.x, a.y, b.x, b.y};
+}
+
+template <class R, int MAT, bool DELTA, int NW>
+__global__ void __launch_bounds__(32 * NW, ctas_per_sm<R>(NW)) solver_resident_kernel(SolveArgs a, void* part_d,
+                                                                                     void* part_v, unsigned* counters) {
+  constexpr int T = 32 * NW, ND = 6, NVT = 12;
+  constexpr unsigned FFD = 0x2u, FFV = (1u << 1) | (1u << 6) | (1u << 8) | (1u << 9);
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  V4<R>* s4 = reinterpret_cast<V4<R>*>(smem_raw);           // staging
+  V4<R>* acc4 = s4 + kTileVerts;                            // [warp][vertex]: gx gy gz dx
+  V2<R>* s2 = reinterpret_cast<V2<R>*>(acc4 + NW * kTileVerts);
+  V2<R>* acc2 = s2 + kTileVerts;                            // [warp][vertex]: dy dz
+  R* vw = reinterpret_cast<R*>(acc2 + NW * kTileVerts);     // kept vertex words, [word][vertex]
+  int* vi = reinterpret_cast<int*>(vw + kVertexWords<DELTA> * kTileVerts);  // vertex, slot, first and end slot
+  __shared__ Acc<R> red[NW * NVT];
+  __shared__ double tot[NVT];
+  __shared__ SolverState sst;
+  R* const xh = vw;
+  R* const xl = vw + 3 * kTileVerts;
+  R* const vp = vw + 6 * kTileVerts;
+  R* const vg = vw + 9 * kTileVerts;
+  R* const vmask = vw + 12 * kTileVerts;
+  R* const xr = vw + 13 * kTileVerts;  // DELTA only
+
+  if (a.st->done) return;
+  const int tile = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int gs = a.fv.tile_gstart[tile], ge = a.fv.tile_gstart[tile + 1];
+  const int vs = a.fv.tile_vstart[tile], nv = a.fv.tile_vstart[tile + 1] - vs;
+  GridBar bar{counters, gridDim.x, 0};
+  if (tid < kStateWords) ((uint32_t*)&sst)[tid] = ((const uint32_t*)a.st)[tid];
+  __syncthreads();
+  const V4<R>* XA = (const V4<R>*)a.xa;
+  V4<R>* GD = (V4<R>*)a.gd;
+  V4<R>* slots = (V4<R>*)a.slots;
+  {
+    const V4<R>* P = p_prev<R>(a, sst.pbuf);
+    for (int i = tid; i < nv; i += T) {
+      const int v = a.fv.tv_vid[vs + i], sl = a.slot_of_tv[vs + i];
+      const int s0 = a.off[v], s1 = a.off[v + 1];
+      vi[i] = v;
+      vi[kTileVerts + i] = sl;
+      // the tile with a vertex's first slot owns it
+      vi[2 * kTileVerts + i] = s0;
+      vi[3 * kTileVerts + i] = sl == s0 ? s1 : s0;
+      const V4<R> x = XA[2 * v], l = XA[2 * v + 1], p = P[v];
+      xh[i] = x.x;
+      xh[kTileVerts + i] = x.y;
+      xh[2 * kTileVerts + i] = x.z;
+      vmask[i] = x.w;
+      xl[i] = l.x;
+      xl[kTileVerts + i] = l.y;
+      xl[2 * kTileVerts + i] = l.z;
+      vp[i] = p.x;
+      vp[kTileVerts + i] = p.y;
+      vp[2 * kTileVerts + i] = p.z;
+      if constexpr (DELTA) {
+        const V4<R> r = ((const V4<R>*)a.xref)[v];
+        xr[i] = r.x;
+        xr[kTileVerts + i] = r.y;
+        xr[2 * kTileVerts + i] = r.z;
+      }
+    }
+  }
+  __syncthreads();  // every thread has read sst.pbuf
+  if (tid == 0) sst.refresh = 0;  // the refresh passes, if any, ran after the last vertex pass
+
+  bool ok = true;
+  for (;;) {
+    // ---- direction ----
+    __syncthreads();
+    {
+      const R beta = (R)sst.beta, inv_mean = (R)sst.inv_mean;
+      for (int i = tid; i < nv; i += T) {
+        const int v = vi[i];
+        const V4<R> g = ldcg4(GD + 2 * v), d = ldcg4(GD + 2 * v + 1);
+        const V4<R> po{vp[i], vp[kTileVerts + i], vp[2 * kTileVerts + i], R(0)};
+        R p[3];
+        pdir(g, d, po, beta, inv_mean, p);
+        vg[i] = g.x;
+        vg[kTileVerts + i] = g.y;
+        vg[2 * kTileVerts + i] = g.z;
+        vp[i] = p[0];
+        vp[kTileVerts + i] = p[1];
+        vp[2 * kTileVerts + i] = p[2];
+        s4[i] = V4<R>{xh[i], xh[kTileVerts + i], xh[2 * kTileVerts + i], p[0]};
+        s2[i] = V2<R>{p[1], p[2]};
+      }
+    }
+    int g = gs + warp, n = 0;
+    ElemGeo<R> geo;
+    uint32_t ids = 0;
+    if (g < ge) {
+      const int e0 = a.fv.group_estart[g];
+      n = a.fv.group_estart[g + 1] - e0;
+      if (lane < n) load_elem_m<R, MAT>(a.fv, e0 + lane, geo, ids);
+    }
+    for (int w = 0; w < NW; ++w)
+      for (int i = tid; i < nv; i += T) {
+        acc4[w * kTileVerts + i] = V4<R>{R(0), R(0), R(0), R(0)};
+        acc2[w * kTileVerts + i] = V2<R>{R(0), R(0)};
+      }
+    __syncthreads();
+    {
+      R plain[ND] = {};
+      Acc<R> c2acc = {};
+      while (g < ge) {
+        const int gn = g + NW;
+        int nn = 0;
+        ElemGeo<R> geon;
+        uint32_t idsn = 0;
+        if (gn < ge) {
+          const int e0n = a.fv.group_estart[gn];
+          nn = a.fv.group_estart[gn + 1] - e0n;
+          if (lane < nn) load_elem_m<R, MAT>(a.fv, e0n + lane, geon, idsn);
+        }
+        if (lane < n) {
+          const int l[4] = {corner(ids, 0), corner(ids, 1), corner(ids, 2), corner(ids, 3)};
+          R G[3][3], dF[3][3];
+          dir_gradients(s4, s2, l, geo.D, G, dF);
+          add_act<MAT>(geo, G);
+          SnhPoint<R> s;
+          snh_prepare(G, s);
+          SnhDir<R> d;
+          snh_dir(s, dF, d);
+          plain[0] += fmax(snh_hess_quad(s, d, geo.mu, geo.lam), R(0));
+          R c[5];
+          snh_poly(s, d, geo.mu, geo.lam, c);
+          c2acc.add(c[0]);
+#pragma unroll
+          for (int m = 1; m < 5; ++m) plain[1 + m] += c[m];
+        }
+        g = gn;
+        n = nn;
+        geo = geon;
+        ids = idsn;
+      }
+      Acc<R> sums[ND];
+#pragma unroll
+      for (int k = 0; k < ND; ++k) {
+        sums[k] = Acc<R>{};
+        sums[k].add(plain[k]);
+      }
+      sums[1] = c2acc;
+      cta_partials<ND, FFD, R>(sums, red, (AccStore<R>*)part_d, gridDim.x);
+    }
+    if (!(ok = bar.sync())) break;
+    grid_totals<ND, R>((const AccStore<R>*)part_d, gridDim.x, tot);
+    if (tid == 0) dir_decide<MAT>(&sst, tot);
+    // the gradient pass's first record, in flight during the decision
+    g = gs + warp;
+    n = 0;
+    if (g < ge) {
+      const int e0 = a.fv.group_estart[g];
+      n = a.fv.group_estart[g + 1] - e0;
+      if (lane < n) load_elem_m<R, MAT>(a.fv, e0 + lane, geo, ids);
+    }
+    __syncthreads();
+
+    // ---- gradient at x + t p ----
+    {
+      const R t = (R)sst.t;
+      for (int i = tid; i < nv; i += T) {
+        R h[3], l[3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          h[c] = xh[c * kTileVerts + i];
+          l[c] = xl[c * kTileVerts + i];
+          pair_add(h[c], l[c], mul_rn(t, vp[c * kTileVerts + i]));
+          xh[c * kTileVerts + i] = h[c];
+          xl[c * kTileVerts + i] = l[c];
+        }
+        if constexpr (DELTA) {
+          const R r[3] = {xr[i], xr[kTileVerts + i], xr[2 * kTileVerts + i]};
+          s4[i] = V4<R>{r[0], r[1], r[2], add_rn(sub_rn(h[0], r[0]), l[0])};
+          s2[i] = V2<R>{add_rn(sub_rn(h[1], r[1]), l[1]), add_rn(sub_rn(h[2], r[2]), l[2])};
+        } else {
+          s4[i] = V4<R>{h[0], h[1], h[2], l[0]};
+          s2[i] = V2<R>{l[1], l[2]};
+        }
+      }
+    }
+    __syncthreads();
+    {
+      V4<R>* my4 = acc4 + warp * kTileVerts;
+      V2<R>* my2 = acc2 + warp * kTileVerts;
+      while (g < ge) {
+        const int gn = g + NW;
+        int nn = 0;
+        ElemGeo<R> geon;
+        uint32_t idsn = 0;
+        if (gn < ge) {
+          const int e0n = a.fv.group_estart[gn];
+          nn = a.fv.group_estart[gn + 1] - e0n;
+          if (lane < nn) load_elem_m<R, MAT>(a.fv, e0n + lane, geon, idsn);
+        }
+        const int l[4] = {corner(ids, 0), corner(ids, 1), corner(ids, 2), corner(ids, 3)};
+        R f[4][3], hd[4][3];
+        if (lane < n) {
+          R G[3][3], P[3][3];
+          if constexpr (DELTA) {
+            R dG[3][3];
+            delta_gradient(s4, s2, l, geo.D, G, dG);
+            add_act<MAT>(geo, G);
+            SnhPoint<R> s, sn;
+            snh_prepare(G, s);
+            snh_pk1_delta(s, dG, geo.mu, geo.lam, P, sn);
+            corner_vjp(P, geo.D, f);
+            snh_hess_diag(sn, geo.D, geo.mu, geo.lam, hd);
+          } else {
+            pair_gradient(s4, s2, l, geo.D, G);
+            add_act<MAT>(geo, G);
+            SnhPoint<R> s;
+            snh_prepare(G, s);
+            snh_pk1(s, geo.mu, geo.lam, P);
+            corner_vjp(P, geo.D, f);
+            snh_hess_diag(s, geo.D, geo.mu, geo.lam, hd);
+          }
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          __syncwarp();
+          if (lane < n) {
+            const int v = l[k];
+            V4<R> q4 = my4[v];
+            V2<R> q2 = my2[v];
+            q4.x += f[k][0];
+            q4.y += f[k][1];
+            q4.z += f[k][2];
+            q4.w += fmax(hd[k][0], R(0));
+            q2.x += fmax(hd[k][1], R(0));
+            q2.y += fmax(hd[k][2], R(0));
+            my4[v] = q4;
+            my2[v] = q2;
+          }
+        }
+        __syncwarp();
+        g = gn;
+        n = nn;
+        geo = geon;
+        ids = idsn;
+      }
+    }
+    __syncthreads();
+    for (int i = tid; i < nv; i += T) {
+      V4<R> q4 = acc4[i];
+      V2<R> q2 = acc2[i];
+#pragma unroll
+      for (int w = 1; w < NW; ++w) {
+        const V4<R> r4 = acc4[w * kTileVerts + i];
+        const V2<R> r2 = acc2[w * kTileVerts + i];
+        q4.x += r4.x;
+        q4.y += r4.y;
+        q4.z += r4.z;
+        q4.w += r4.w;
+        q2.x += r2.x;
+        q2.y += r2.y;
+      }
+      const size_t sl = 2 * (size_t)vi[kTileVerts + i];
+      slots[sl] = V4<R>{q4.x, q4.y, q4.z, R(0)};
+      slots[sl + 1] = V4<R>{q4.w, q2.x, q2.y, R(0)};
+    }
+    if (!(ok = bar.sync())) break;
+
+    // ---- vertex ----
+    {
+      R s[NVT] = {};
+      for (int i = tid; i < nv; i += T) {
+        const int s0 = vi[2 * kTileVerts + i], s1 = vi[3 * kTileVerts + i];
+        if (s0 == s1) continue;  // another tile's vertex
+        const int v = vi[i];
+        V4<R> r{}, f{};
+        if constexpr (DELTA) r = ldg4((const V4<R>*)a.gref + v);
+        if (a.force) f = ldg4((const V4<R>*)a.force + v);
+        R ss[3] = {R(0), R(0), R(0)}, ds[3] = {R(0), R(0), R(0)};
+        for (int k = s0; k < s1; ++k) {
+          const V4<R> sg = ldcg4(slots + 2 * (size_t)k), sd = ldcg4(slots + 2 * (size_t)k + 1);
+          ss[0] += sg.x;
+          ss[1] += sg.y;
+          ss[2] += sg.z;
+          ds[0] += sd.x;
+          ds[1] += sd.y;
+          ds[2] += sd.z;
+        }
+        R xn[3], p[3], gn[3], dn[3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          xn[c] = xh[c * kTileVerts + i] + xl[c * kTileVerts + i];
+          p[c] = vp[c * kTileVerts + i];
+        }
+        const V4<R> go{vg[i], vg[kTileVerts + i], vg[2 * kTileVerts + i], R(0)};
+        vertex_terms<R, DELTA>(a.force != nullptr, (int)vmask[i], xn, p, go, r, f, ss, ds, gn, dn, s);
+        GD[2 * v] = V4<R>{gn[0], gn[1], gn[2], R(0)};
+        GD[2 * v + 1] = V4<R>{dn[0], dn[1], dn[2], R(0)};
+      }
+      Acc<R> acc[NVT];
+#pragma unroll
+      for (int k = 0; k < NVT; ++k) {
+        acc[k] = Acc<R>{};
+        acc[k].add(s[k]);
+      }
+      cta_partials<NVT, FFV, R>(acc, red, (AccStore<R>*)part_v, gridDim.x);
+    }
+    if (!(ok = bar.sync())) break;
+    grid_totals<NVT, R>((const AccStore<R>*)part_v, gridDim.x, tot);
+    if (tid == 0) vertex_decide(&sst, tot);
+    __syncthreads();
+    if (sst.done || sst.iter >= sst.iter_limit || sst.refresh) break;
+  }
+
+  if (ok) {
+    V4<R>* X = (V4<R>*)a.xa;
+    V4<R>* P = p_prev<R>(a, sst.pbuf);  // the last direction, flipped to p_prev by the decision
+    for (int i = tid; i < nv; i += T) {
+      if (vi[2 * kTileVerts + i] == vi[3 * kTileVerts + i]) continue;
+      const int v = vi[i];
+      X[2 * v] = V4<R>{xh[i], xh[kTileVerts + i], xh[2 * kTileVerts + i], vmask[i]};
+      X[2 * v + 1] = V4<R>{xl[i], xl[kTileVerts + i], xl[2 * kTileVerts + i], R(0)};
+      P[v] = V4<R>{vp[i], vp[kTileVerts + i], vp[2 * kTileVerts + i], R(0)};
+    }
+    if (tile == 0 && tid < kStateWords) ((uint32_t*)a.st)[tid] = ((const uint32_t*)&sst)[tid];
+  } else if (tid == 0) {  // a barrier gave up: the solve stops with a device error
+    atomicMax(&a.st->error, 3);
+    a.st->done = 1;
+  }
+  bar.leave();
+}
+
+using ResidentKernel = void (*)(SolveArgs, void*, void*, unsigned*);
+
+struct ResidentShape {
+  ResidentKernel kernel = nullptr;
+  int threads = 0;
+  size_t smem = 0;
+};
+
+template <class R, int MAT, bool DELTA, int NW>
+ResidentShape shape_nw() {
+  return ResidentShape{solver_resident_kernel<R, MAT, DELTA, NW>, 32 * NW, resident_smem<R, DELTA>(NW)};
+}
+
+template <int MAT, bool DELTA>
+ResidentShape shape_f32(int n_tiles) {
+  return n_tiles <= kSMs ? shape_nw<float, MAT, DELTA, 16>() : shape_nw<float, MAT, DELTA, 8>();
+}
+
+ResidentShape resident_shape(const SolveArgs& a) {
+  const int nt = a.fv.n_tiles;
+  if (nt > 2 * kSMs) return ResidentShape{};
+  constexpr int SNH = AGB_STABLE_NEO_HOOKEAN, MU = AGB_STABLE_NEO_HOOKEAN_MUSCLE;
+  if (!snh_family(a.fv.material)) return ResidentShape{};
+  const bool mu = a.fv.material == MU;
+  if (a.precision == AGB_F64) return mu ? shape_nw<double, MU, false, 4>() : shape_nw<double, SNH, false, 4>();
+  if (a.delta) return mu ? shape_f32<MU, true>(nt) : shape_f32<SNH, true>(nt);
+  return mu ? shape_f32<MU, false>(nt) : shape_f32<SNH, false>(nt);
+}
+
+}  // namespace
+
+// Whether the solver's iterations can run resident: every tile's CTA fits the
+// device at once (the kernel prepared on the way).
+cudaError_t resident_prepare(const SolveArgs& a, bool* fits) {
+  *fits = false;
+  const ResidentShape sh = resident_shape(a);
+  if (!sh.kernel || a.fv.n_tiles == 0) return cudaSuccess;
+  int dev = 0, sms = 0, coop = 0, occ = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(sh.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh.smem);
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, sh.kernel, sh.threads, sh.smem);
+  if (e == cudaSuccess) *fits = coop && (int64_t)a.fv.n_tiles <= (int64_t)occ * sms;
+  return e;
+}
+
+cudaError_t launch_resident(const SolveArgs& a, void* part_d, void* part_v, unsigned* counters, cudaStream_t s) {
+  const ResidentShape sh = resident_shape(a);
+  if (!sh.kernel) return cudaErrorInvalidValue;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(a.fv.n_tiles);
+  cfg.blockDim = dim3(sh.threads);
+  cfg.dynamicSmemBytes = sh.smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, sh.kernel, a, part_d, part_v, counters);
+}
+
+}  // namespace agb
