@@ -63,7 +63,7 @@ __global__ void __launch_bounds__(kVThreadsCg) cg_init_kernel(CgArgs c, const R*
   const SolveArgs& a = c.a;
   const V4<R>* XA = (const V4<R>*)a.xa;
   const V4<R>* GD = (const V4<R>*)a.gd;
-  const R inv_mean = (R)a.st->inv_mean;
+  const R inv_mean = to_real<R>(a.st->inv_mean);
   Acc<R> s[2] = {};
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.n_points; i += gridDim.x * blockDim.x) {
     const int mask = (int)XA[2 * i].w;
@@ -146,7 +146,7 @@ __global__ void __launch_bounds__(kCgThreads) cg_prod_kernel(CgArgs c) {
   if (c.cond && blockIdx.x == 0 && threadIdx.x == 0)
     cudaGraphSetConditional((cudaGraphConditionalHandle)c.cond, 0u);  // the second vertex pass re-arms
   if (cs->done) return;
-  const R beta = (R)cs->beta;
+  const R beta = to_real<R>(cs->beta);
   const int pb = cs->pbuf;
   const V4<R>* po = cg_p_prev<R>(c, pb);
   V4<R>* pc = cg_p_cur<R>(c, pb);
@@ -315,7 +315,7 @@ __global__ void __launch_bounds__(kVThreadsCg) cg_vertex2_kernel(CgArgs c) {
   pdl_wait();
   CgState* cs = c.cs;
   if (cs->done) return;
-  const R alpha = (R)cs->alpha;
+  const R alpha = to_real<R>(cs->alpha);
   const V4<R>* pc = cg_p_cur<R>(c, cs->pbuf);
   V4<R>* L = (V4<R>*)c.lam;
   V4<R>* Rs = (V4<R>*)c.res;

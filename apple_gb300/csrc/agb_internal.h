@@ -79,6 +79,14 @@ int build_tiles(int n_cells, const int32_t* cells_int, const double* centroid_xy
                 const double* D9, const double* mudv, const double* lamdv, int tile_elems,
                 TilePlan* plan);
 
+// Cut the tiles of a plan with at most sms * per_sm of them into as many
+// pieces (of at least 8 warp groups, each with its tile's vertex list), for
+// kernels that hold one piece per CTA: with more tiles than SMs, the first
+// `sms` stay whole -- one per SM -- and the others are cut to fill the second
+// CTAs evenly.  Fills the tile arrays and tv_vid of `out`; groups, elements
+// and corner ids are the plan's.
+void split_tiles(const TilePlan& plan, int sms, int per_sm, TilePlan* out);
+
 // One slot map over several plans (a model); plans[k]->n_tv entries each.
 void build_slots(int n_points, const std::vector<const TilePlan*>& plans,
                  std::vector<SlotMap>* per_plan, std::vector<int32_t>* off);

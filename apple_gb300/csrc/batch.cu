@@ -41,7 +41,7 @@ __global__ void __launch_bounds__(kElemThreads) batch_dir_kernel(BatchArgs b) {
   pdl_trigger();
   SolverState* st = b.st + b.tile_mesh[tile];
   if (st->done) return;
-  const R beta = (R)st->beta, inv_mean = (R)st->inv_mean;
+  const R beta = to_real<R>(st->beta), inv_mean = to_real<R>(st->inv_mean);
   const int pb = st->pbuf;
   stage_dir<R>(a, tile_vertex(a.fv, tile, threadIdx.x), beta, inv_mean, p_prev<R>(a, pb), p_cur<R>(a, pb), sx,
                sp);
@@ -101,12 +101,7 @@ __global__ void __launch_bounds__(kTailThreads) batch_dir_tail_kernel(BatchArgs 
     for (int k = 0; k < N; ++k) s[k].add(acc_load<R>((const AccStore<R>*)b.part_dir + (size_t)t * N + k));
   }
   block_reduce<N, 0xffffffffu, R>(s, red);
-  if (threadIdx.x == 0) {
-    double tot[N];
-#pragma unroll
-    for (int k = 0; k < N; ++k) tot[k] = s[k].value();
-    dir_decide<MAT>(st, tot);
-  }
+  if (threadIdx.x < 32) dir_decide<MAT, R>(st, red);  // the sums are in red[0 .. N-1]
 }
 
 // ARAP: the gradient pass at the first trial step x + alpha_0 p of each
@@ -194,7 +189,7 @@ __global__ void __launch_bounds__(kVThreads) batch_vertex_kernel(BatchArgs b, in
   pdl_wait();
   if (st->done) return;
   if ((phase == 1 && !st->spec_ok) || (phase == 2 && st->spec_ok)) return;
-  const R t = (R)st->t;
+  const R t = to_real<R>(st->t);
   const V4<R>* P = p_cur<R>(a, st->pbuf);
   R s[N] = {};
   for (int i = v0 + threadIdx.x; i < v1; i += blockDim.x) vertex_update<R, DELTA>(a, i, a.off[i], a.off[i + 1], t, P, s);
@@ -233,13 +228,9 @@ __global__ void __launch_bounds__(kTailThreads) batch_vertex_tail_kernel(BatchAr
       for (int k = 0; k < N; ++k) s[k].add(acc_load<R>((const AccStore<R>*)b.part_vert + (size_t)c * N + k));
     }
     block_reduce<N, 0xffffffffu, R>(s, red);
-    if (threadIdx.x == 0) {
-      double tot[N];
-#pragma unroll
-      for (int k = 0; k < N; ++k) tot[k] = s[k].value();
-      vertex_decide(st, tot);
-      if (b.a.svd) st->sbuf ^= 1;  // the gradient pass's SVDs are those at the new x
-    }
+    vertex_decide<R>(st, red);  // the sums are in red[0 .. N-1]
+    // the gradient pass's SVDs are those at the new x
+    if (threadIdx.x == 0 && b.a.svd) st->sbuf ^= 1;
   }
   if (phase == 1) return;
   if (threadIdx.x == 0) {

@@ -758,7 +758,8 @@ int agb_solver_destroy(agb_solver* sv) {
                   (void*)sv->d_group_estart, (void*)sv->d_tv_vid,
                   (void*)sv->d_slot_of_tv, sv->d_rec, (void*)sv->d_ids, sv->d_xa, sv->d_gd, sv->d_p0,
                   sv->d_p1, sv->d_xref, sv->d_gref, sv->d_svd, sv->d_slots, sv->d_part, (void*)sv->d_cnt,
-                  (void*)sv->d_state, sv->d_u_tmp, sv->d_act, sv->d_res_part, (void*)sv->d_res_counters})
+                  (void*)sv->d_state, sv->d_u_tmp, sv->d_act, sv->d_res_part, (void*)sv->d_res_counters,
+                  (void*)sv->d_off})
     dfree(p);
   if (sv->h_state) cudaFreeHost(sv->h_state);
   delete sv;
@@ -872,6 +873,36 @@ int agb_solver_create(agb_model* m, const agb_pncg_params* params, agb_solver** 
     sv->fv.ids = sv->d_ids;
     sv->fv.act = sv->d_act;
   }
+  // meshes small enough for resident iterations: tiles cut to fill the device,
+  // with slots of their own (a point that no cell uses has no tile to own it
+  // there, so such a mesh keeps the three-kernel iteration)
+  bool covered = true;
+  for (int v = 0; v < np && covered; ++v) covered = m->off[v + 1] > m->off[v];
+  const bool small = covered && mat != AGB_ARAP && sv->fv.n_tiles > 0 && sv->fv.n_tiles <= kResidentMaxTiles;
+  TilePlan pieces;
+  std::vector<int32_t> off;
+  int32_t n_slots = m->n_slots;
+  if (!rc && small) {
+    split_tiles(m->fems.size() == 1 ? m->fems[0]->plan : sv->plan, kResidentMaxTiles / 2, 2, &pieces);
+    std::vector<SlotMap> sm;
+    build_slots(np, {&pieces}, &sm, &off);
+    slot_of_tv = sm[0].slot_of_tv;
+    n_slots = off[np];
+    for (int32_t** d : {&sv->d_tile_estart, &sv->d_tile_vstart, &sv->d_tile_gstart, &sv->d_tv_vid}) {
+      dfree(*d);
+      *d = nullptr;
+    }
+    rc = dupload(&sv->d_tile_estart, pieces.tile_estart);
+    if (!rc) rc = dupload(&sv->d_tile_vstart, pieces.tile_vstart);
+    if (!rc) rc = dupload(&sv->d_tile_gstart, pieces.tile_gstart);
+    if (!rc) rc = dupload(&sv->d_tv_vid, pieces.tv_vid);
+    if (!rc) rc = dupload(&sv->d_off, off);
+    sv->fv.n_tiles = pieces.n_tiles;
+    sv->fv.tile_estart = sv->d_tile_estart;
+    sv->fv.tile_vstart = sv->d_tile_vstart;
+    sv->fv.tile_gstart = sv->d_tile_gstart;
+    sv->fv.tv_vid = sv->d_tv_vid;
+  }
   if (!rc) rc = dupload(&sv->d_slot_of_tv, slot_of_tv);
   const size_t v4 = v4_bytes(sv->precision);
   const int vblocks = solver_vertex_blocks(np);
@@ -889,7 +920,7 @@ int agb_solver_create(agb_model* m, const agb_pncg_params* params, agb_solver** 
   if (!rc && delta) rc = dalloc_bytes(&sv->d_xref, v4 * np);
   if (!rc && delta) rc = dalloc_bytes(&sv->d_gref, v4 * np);
   if (!rc && mat == AGB_ARAP) rc = dalloc_bytes(&sv->d_svd, svd_cache_bytes(sv));
-  if (!rc) rc = dalloc_bytes(&sv->d_slots, v4 * 2 * (size_t)m->n_slots);
+  if (!rc) rc = dalloc_bytes(&sv->d_slots, v4 * 2 * (size_t)n_slots);
   if (!rc) rc = dalloc_bytes(&sv->d_part, 8 * n_part);
   if (!rc) rc = dalloc(&sv->d_cnt, n_cnt);
   if (!rc && cudaMemset(sv->d_cnt, 0, n_cnt * sizeof(unsigned)) != cudaSuccess) rc = AGB_E_CUDA;
@@ -933,9 +964,9 @@ int agb_solver_create(agb_model* m, const agb_pncg_params* params, agb_solver** 
   a.delta = delta ? 1 : 0;
   a.force = m->d_force;
   a.slot_of_tv = sv->d_slot_of_tv;
-  a.off = m->d_off;
+  a.off = small ? sv->d_off : m->d_off;
   a.slots = sv->d_slots;
-  a.n_slots = m->n_slots;
+  a.n_slots = n_slots;
   a.st = sv->d_state;
   char* part = (char*)sv->d_part;
   a.part_a = part;
@@ -954,15 +985,19 @@ int agb_solver_create(agb_model* m, const agb_pncg_params* params, agb_solver** 
   a.cond_outer = 0;
   a.refresh_exits = 0;
   a.guard = 0;
-  // resident iterations when every tile's CTA fits the device at once; a
-  // point that no cell uses has no tile to own it there
-  bool covered = true;
-  for (int v = 0; v < np && covered; ++v) covered = m->off[v + 1] > m->off[v];
-  if (covered) {
+  // resident iterations when every tile's CTA fits the device at once
+  if (small) {
+    for (int t = 0; t < pieces.n_tiles; ++t) {
+      sv->resident.max_elems = std::max(sv->resident.max_elems, pieces.tile_estart[t + 1] - pieces.tile_estart[t]);
+      sv->resident.max_groups = std::max(sv->resident.max_groups, pieces.tile_gstart[t + 1] - pieces.tile_gstart[t]);
+    }
+    const int n_whole = m->fems.size() == 1 ? m->fems[0]->plan.n_tiles : sv->plan.n_tiles;
+    sv->resident.whole = n_whole > kResidentMaxTiles / 2 ? kResidentMaxTiles / 2 : 0;
     rc = check_launch(resident_prepare(a, &sv->resident), "resident_prepare");
-    if (!rc && sv->resident) rc = dalloc_bytes(&sv->d_res_part, 8 * 18 * nt);
-    if (!rc && sv->resident) rc = dalloc(&sv->d_res_counters, 2);
-    if (!rc && sv->resident && cudaMemset(sv->d_res_counters, 0, 2 * sizeof(unsigned)) != cudaSuccess) rc = AGB_E_CUDA;
+    const bool fits = sv->resident.shape != 0;
+    if (!rc && fits) rc = dalloc_bytes(&sv->d_res_part, 8 * 18 * nt);
+    if (!rc && fits) rc = dalloc(&sv->d_res_counters, kResidentCounters);
+    if (!rc && fits && cudaMemset(sv->d_res_counters, 0, kResidentCounters * sizeof(unsigned)) != cudaSuccess) rc = AGB_E_CUDA;
     if (rc) {
       if (rc == AGB_E_CUDA && agb::last_error()[0] == 0) set_error("agb_solver_create: CUDA allocation failed");
       agb_solver_destroy(sv);
@@ -975,8 +1010,8 @@ int agb_solver_create(agb_model* m, const agb_pncg_params* params, agb_solver** 
 
 // the solver's iterations up to its limit, or a due refresh, in one launch
 static cudaError_t run_resident(agb_solver* sv, const SolveArgs& a, cudaStream_t s) {
-  return launch_resident(a, sv->d_res_part, (char*)sv->d_res_part + 8 * 6 * (size_t)a.fv.n_tiles, sv->d_res_counters,
-                         s);
+  return launch_resident(a, sv->resident, sv->d_res_part, (char*)sv->d_res_part + 8 * 6 * (size_t)a.fv.n_tiles,
+                         sv->d_res_counters, s);
 }
 
 int agb_solver_reset(agb_solver* sv, const void* u, void* stream) {
@@ -1011,7 +1046,7 @@ static cudaError_t capture_into(agb_solver* sv, cudaGraph_t graph, const cudaGra
   cudaStream_t cs = sv->capture_stream;
   cudaError_t e = cudaStreamBeginCaptureToGraph(cs, graph, deps, nullptr, n_deps, cudaStreamCaptureModeThreadLocal);
   if (e != cudaSuccess) return e;
-  if (sv->resident) {
+  if (sv->resident.shape) {
     cudaError_t le = run_resident(sv, a, cs);
     if (le == cudaSuccess) le = launch_solver_refresh(a, cs, false);
     cudaGraph_t captured = nullptr;
@@ -1059,7 +1094,7 @@ static int build_loop_graph(agb_solver* sv) {
   cudaGraphNode_t w_out = nullptr, w_in = nullptr;
   cudaGraph_t body_out = nullptr, body_in = nullptr;
   cudaError_t e = cudaSuccess;
-  if (sv->resident) {
+  if (sv->resident.shape) {
     e = cudaGraphConditionalHandleCreate(&h_out, g, 1u, cudaGraphCondAssignDefault);
     if (e == cudaSuccess) e = add_conditional(g, nullptr, 0, h_out, cudaGraphCondTypeWhile, &w_out, &body_out);
     SolveArgs ar = a;
@@ -1110,7 +1145,7 @@ static int build_step_graph(agb_solver* sv) {
   size_t n_nodes = 0;
   if (e == cudaSuccess) {
     cudaError_t le;
-    if (sv->resident) {
+    if (sv->resident.shape) {
       le = launch_solver_set_limit(a, 1, cs);
       if (le == cudaSuccess) le = run_resident(sv, a, cs);
       if (le == cudaSuccess && a.delta) le = launch_solver_refresh(a, cs, false);
@@ -1140,7 +1175,7 @@ int agb_solver_iterate(agb_solver* sv, int32_t n_steps, void* stream) {
   AGB_REQUIRE(sv && n_steps >= 0, AGB_E_INVALID, "agb_solver_iterate: bad argument");
   if (n_steps == 0) return AGB_OK;
   cudaStream_t s = as_stream(stream);
-  if (sv->resident && !sv->args.delta) {  // no refresh ends the run: no loop around it
+  if (sv->resident.shape && !sv->args.delta) {  // no refresh ends the run: no loop around it
     RC(check_launch(launch_solver_set_limit(sv->args, n_steps, s), "set_limit"));
     return check_launch(run_resident(sv, sv->args, s), "resident iterations");
   }

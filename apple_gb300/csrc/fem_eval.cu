@@ -376,8 +376,7 @@ cudaError_t eval_launch(const FemView& fv, int warps, unsigned flags, const void
   const bool vectors = flags & (AGB_GRAD | AGB_HESS_DIAG | AGB_HESS_PROD);
   const size_t smem = vectors ? eval_smem_bytes<R, NVEC>(warps) : eval_stage_bytes<R>();
   if (smem > 48 * 1024) {  // above the default limit the kernel has to opt in
-    const cudaError_t e = cudaFuncSetAttribute(fem_eval_kernel<R, MAT, NVEC, MAXT>,
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = allow_max_smem(fem_eval_kernel<R, MAT, NVEC, MAXT>);
     if (e != cudaSuccess) return e;
   }
   fem_eval_kernel<R, MAT, NVEC, MAXT><<<fv.n_tiles, 32 * warps, smem, s>>>(

@@ -15,26 +15,36 @@
 namespace agb {
 
 struct GridBar {
-  unsigned* counters;  // [0] arrivals, [1] exits; zero before the first launch
+  static constexpr uint64_t kLimit = 2000000000ull;  // ns
+  unsigned* counters;  // [0] arrivals, [1] exits; `words` of them, zero before the first launch
+  int words;           // reset by the last CTA to leave
   unsigned n;          // CTAs
   unsigned round;      // barriers passed
 
-  // every thread of the CTA calls it; false when the wait gave up
-  __device__ __forceinline__ bool sync() {
-    __shared__ int s_ok;
+  // every thread of the CTA calls it; what the CTA wrote before is visible to
+  // the others after their wait().  Work that needs nothing from them can go
+  // between arrive() and wait().
+  __device__ __forceinline__ void arrive() {
     ++round;
     __syncthreads();
     if (threadIdx.x == 0) {
       __threadfence();
       atomicAdd(&counters[0], 1u);
+    }
+  }
+
+  // wait until every CTA has arrived; false when the wait gave up
+  __device__ __forceinline__ bool wait() {
+    __shared__ int s_ok;
+    if (threadIdx.x == 0) {
       const unsigned want = round * n;
       const uint64_t t0 = global_ns();
       bool ok = true;
       for (;;) {
         unsigned v;
         asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(counters) : "memory");
-        if (v >= want) break;
-        if (global_ns() - t0 > 2000000000ull) {
+        if ((int)(v - want) >= 0) break;  // the counter may wrap
+        if (global_ns() - t0 > kLimit) {
           ok = false;
           break;
         }
@@ -50,54 +60,103 @@ struct GridBar {
     __syncthreads();
     if (threadIdx.x != 0) return;
     __threadfence();
-    if (atomicAdd(&counters[1], 1u) == n - 1u) {
-      counters[0] = 0u;
-      counters[1] = 0u;
-    }
+    if (atomicAdd(&counters[1], 1u) == n - 1u)
+      for (int k = 0; k < words; ++k) counters[k] = 0u;
   }
 };
 
-// The CTA's sums of N quantities into part[k * n + block]: float-float warp
-// trees for the quantities in FF, plain ones for the others, then the warps
-// in order (as block_reduce).
-template <int N, unsigned FF, class R>
-__device__ __forceinline__ void cta_partials(Acc<R> (&a)[N], Acc<R>* scratch, AccStore<R>* part, int n) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+// The CTA's sum of each of N quantities into part[k * n + block].  x: the
+// thread's terms; lo: the low word of quantity LO (float-float), or unused
+// with LO < 0.  The terms go through shared memory (`rows`: N + 1 rows of
+// THREADS reals) so that one warp adds one quantity, instead of every warp
+// reducing all N by shuffles: quantities in FF in float-float, the others
+// (sums of same-sign terms) in R.
+template <int N, unsigned FF, int LO, int THREADS, class R>
+__device__ __forceinline__ void cta_partials(const R (&x)[N], R lo, R* rows, AccStore<R>* part, int n, int block) {
+  constexpr int NW = THREADS / 32;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-  for (int k = 0; k < N; ++k) {
-    if ((FF >> k) & 1u) {
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1) a[k].add(a[k].shfl_down(off));
-    } else {
-      a[k].warp_plain_sum();
-    }
-  }
-  if (lane == 0) {
-#pragma unroll
-    for (int k = 0; k < N; ++k) scratch[warp * N + k] = a[k];
-  }
+  for (int k = 0; k < N; ++k) rows[k * THREADS + threadIdx.x] = x[k];
+  if constexpr (LO >= 0) rows[N * THREADS + threadIdx.x] = lo;
   __syncthreads();
-  if (threadIdx.x < N) {
-    Acc<R> s = scratch[threadIdx.x];
-    for (int w = 1; w < nw; ++w) s.add(scratch[w * N + threadIdx.x]);
-    part[(size_t)threadIdx.x * n + blockIdx.x] = acc_store(s);
+  for (int k = warp; k < N; k += NW) {
+    const R* row = rows + k * THREADS;
+    Acc<R> s{};
+    if ((FF >> k) & 1u) {
+#pragma unroll 4
+      for (int j = 0; j < NW; ++j) s.add(row[lane + 32 * j]);
+      if (k == LO) {
+        R l = R(0);
+#pragma unroll 4
+        for (int j = 0; j < NW; ++j) l += rows[N * THREADS + lane + 32 * j];
+        s.add(l);
+      }
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) s.add(s.shfl_down(off));
+    } else {
+      R p = R(0);
+#pragma unroll 4
+      for (int j = 0; j < NW; ++j) p += row[lane + 32 * j];
+      s.add(p);
+      s.warp_plain_sum();
+    }
+    if (lane == 0) part[(size_t)k * n + block] = acc_store(s);
   }
 }
 
-// After a barrier: the sums over all CTAs, in every CTA.  Warp w adds
-// quantities w, w + nw, ...; tot is complete after the closing __syncthreads.
-template <int N, class R>
-__device__ __forceinline__ void grid_totals(const AccStore<R>* part, int n, double* tot) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int k = warp; k < N; k += nw) {
-    Acc<R> s{};
-#pragma unroll 4
-    for (int b = lane; b < n; b += 32) s.add(acc_load<R>(part + (size_t)k * n + b));
+// After a barrier: the sums over all CTAs in every CTA, into shared tot: a
+// warp per quantity (its KPW quantities interleaved, so that their loads are
+// in flight together); complete after the closing __syncthreads.
+template <int N, int THREADS, class R>
+__device__ __forceinline__ void grid_totals(const AccStore<R>* part, int n, Acc<R>* tot) {
+  constexpr int NW = THREADS / 32, KPW = (N + NW - 1) / NW, U = 4;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  Acc<R> s[KPW] = {};
+  for (int b0 = lane; b0 < n; b0 += 32 * U) {
+    Acc<R> v[KPW][U] = {};
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) s.add(s.shfl_down(off));
-    if (lane == 0) tot[k] = s.value();
+    for (int j = 0; j < KPW; ++j)
+#pragma unroll
+      for (int q = 0; q < U; ++q)
+        if (warp + j * NW < N && b0 + 32 * q < n)
+          v[j][q] = acc_load<R>(part + (size_t)(warp + j * NW) * n + b0 + 32 * q);
+#pragma unroll
+    for (int j = 0; j < KPW; ++j)
+#pragma unroll
+      for (int q = 0; q < U; ++q) s[j].add(v[j][q]);
   }
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) {
+#pragma unroll
+    for (int j = 0; j < KPW; ++j) s[j].add(s[j].shfl_down(off));
+  }
+#pragma unroll
+  for (int j = 0; j < KPW; ++j)
+    if (lane == 0 && warp + j * NW < N) tot[warp + j * NW] = s[j];
   __syncthreads();
+}
+
+// The work item of this CTA when the first `whole` of n items are large: the
+// first CTA to arrive on an SM takes the next large one, a second CTA there
+// the next of the others, so that no SM holds two large items while another
+// holds none.  counters[2], [3]: items taken; counters[4 + k]: CTAs on SM k
+// (kPlaceWords words after the barrier's two, zero before the launch).
+// Called by one thread.
+constexpr int kPlaceSms = 256;
+constexpr int kPlaceWords = 2 + kPlaceSms;
+
+__device__ __forceinline__ int place_cta(unsigned* counters, int whole, int n) {
+  unsigned sm;
+  asm volatile("mov.u32 %0, %%smid;" : "=r"(sm));
+  const bool first = atomicAdd(&counters[4 + (sm & (kPlaceSms - 1))], 1u) == 0u;
+  if (first) {
+    const int k = (int)atomicAdd(&counters[2], 1u);
+    if (k < whole) return k;
+    return min(whole + (int)atomicAdd(&counters[3], 1u), n - 1);
+  }
+  const int k = (int)atomicAdd(&counters[3], 1u);
+  if (whole + k < n) return whole + k;
+  return min((int)atomicAdd(&counters[2], 1u), n - 1);
 }
 
 }  // namespace agb

@@ -1,4 +1,5 @@
-// Programmatic dependent launch, and the SM count the launch rules use.
+// Launch helpers: programmatic dependent launch, the shared-memory opt-in and
+// the SM count the launch rules use.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -25,6 +26,22 @@ inline cudaError_t launch_pdl(void (*k)(P...), dim3 grid, dim3 block, size_t sme
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, k, args...);
+}
+
+// Opt a kernel in to as much dynamic shared memory as the device grants
+// beside the kernel's static use.  The same value on every call: launches of
+// one kernel with different sizes from several threads do not disturb each
+// other.
+template <class... P>
+inline cudaError_t allow_max_smem(void (*k)(P...)) {
+  int dev = 0, limit = 0;
+  cudaFuncAttributes at{};
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&at, k);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, limit - (int)at.sharedSizeBytes);
+  return e;
 }
 
 }  // namespace agb

@@ -297,6 +297,37 @@ int build_tiles(int n_cells, const int32_t* cells, const double* centroid, const
   return AGB_OK;
 }
 
+void split_tiles(const TilePlan& plan, int sms, int per_sm, TilePlan* out) {
+  const int T = plan.n_tiles, most = sms * per_sm;
+  out->n_cells = plan.n_cells;
+  out->n_tiles = 0;
+  out->tile_estart.assign(1, 0);
+  out->tile_vstart.assign(1, 0);
+  out->tile_gstart.assign(1, 0);
+  out->tv_vid.clear();
+  int left = most;  // pieces still to be given
+  for (int t = 0; t < T; ++t) {
+    const int g0 = plan.tile_gstart[t], g1 = plan.tile_gstart[t + 1], ng = g1 - g0;
+    int k;
+    if (T > sms)  // one whole tile per SM first, the rest shared out over the other CTAs
+      k = t < sms ? 1 : left / (T - t);
+    else
+      k = left / (T - t);
+    k = std::max(1, std::min(k, ng / 8));
+    for (int j = 0; j < k; ++j) {
+      const int b = g0 + (int)((int64_t)ng * (j + 1) / k);
+      out->tile_gstart.push_back(b);
+      out->tile_estart.push_back(b < (int)plan.group_estart.size() ? plan.group_estart[b] : plan.n_cells);
+      out->tv_vid.insert(out->tv_vid.end(), plan.tv_vid.begin() + plan.tile_vstart[t],
+                         plan.tv_vid.begin() + plan.tile_vstart[t + 1]);
+      out->tile_vstart.push_back((int32_t)out->tv_vid.size());
+    }
+    left -= k;
+    out->n_tiles += k;
+  }
+  out->n_tv = (int)out->tv_vid.size();
+}
+
 void build_slots(int n_points, const std::vector<const TilePlan*>& plans,
                  std::vector<SlotMap>* per_plan, std::vector<int32_t>* off) {
   std::vector<int32_t> count(n_points + 1, 0);

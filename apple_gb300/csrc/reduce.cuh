@@ -12,8 +12,40 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include <stdint.h>
 
 namespace agb {
+
+// float <-> double in the integer pipe: GB300's conversion instructions take
+// about 270 cycles each.  Exact, and rounded to nearest even, like them; the
+// values they leave to the instruction are zero-exponent and non-finite ones
+// (and, narrowing, results near the limits of float).
+__device__ __forceinline__ double widen(float x) {
+  const uint32_t b = __float_as_uint(x), m = b & 0x7fffffffu;
+  if (m - 0x00800000u < 0x7f000000u)  // normal
+    return __hiloint2double((int)((b & 0x80000000u) | ((m >> 3) + 0x38000000u)), (int)(b << 29));
+  return m == 0u ? __hiloint2double((int)b, 0) : (double)x;
+}
+__device__ __forceinline__ float narrow(double x) {
+  const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
+  const uint32_t e = (hi >> 20) & 0x7ffu;
+  if (e - 900u < 240u) {  // float exponent 4 .. 243: no overflow from rounding up
+    const uint32_t m = ((hi & 0x7fffffffu) - 0x38000000u) << 3 | lo >> 29, rest = lo & 0x1fffffffu;
+    return __uint_as_float((hi & 0x80000000u) | (m + (rest > 0x10000000u || (rest == 0x10000000u && (m & 1u)))));
+  }
+  return (hi & 0x7fffffffu) == 0u && lo == 0u ? __uint_as_float(hi) : (float)x;
+}
+// a scalar of the solver's state in the kernels' real type
+template <class R>
+__device__ __forceinline__ R to_real(double x);
+template <>
+__device__ __forceinline__ float to_real<float>(double x) {
+  return narrow(x);
+}
+template <>
+__device__ __forceinline__ double to_real<double>(double x) {
+  return x;
+}
 
 template <class R>
 struct Acc;
@@ -41,7 +73,7 @@ struct Acc<float> {
     r.lo = __shfl_down_sync(0xffffffffu, lo, off);
     return r;
   }
-  __device__ __forceinline__ double value() const { return (double)hi + (double)lo; }
+  __device__ __forceinline__ double value() const { return widen(hi) + widen(lo); }
   // lane 0 gets the float sum of hi + lo over the warp
   __device__ __forceinline__ void warp_plain_sum() {
     float v = hi + lo;
@@ -236,16 +268,15 @@ __device__ __forceinline__ bool grid_reduce_masked(Acc<R> (&a)[N], AccStore<R>* 
   return true;
 }
 
-// grid_reduce_masked, and the last block also copies `words` 32-bit words of
-// `src` (the solver's scalar state) into shared `dst` in the same round trip
-// as the partials, so that its scalar logic reads shared memory instead of
-// making one dependent global load per field.  `dst` is complete in every
-// thread of the last block on return.
+// grid_reduce_masked, but the sums stay in scratch[0 .. N-1] (every thread of
+// the last block may read them on return), and the last block also copies
+// `words` 32-bit words of `src` (the solver's scalar state) into shared `dst`
+// in the same round trip as the partials, so that its scalar logic reads
+// shared memory instead of making one dependent global load per field.
 template <int N, unsigned FF, class R>
 __device__ __forceinline__ bool grid_reduce_masked_state(Acc<R> (&a)[N], AccStore<R>* partials,
                                                          unsigned* counter, int nblocks, Acc<R>* scratch,
-                                                         double (&total)[N], const uint32_t* src,
-                                                         uint32_t* dst, int words) {
+                                                         const uint32_t* src, uint32_t* dst, int words) {
   __shared__ bool s_last;
   block_reduce<N, FF, R>(a, scratch);
   if (threadIdx.x == 0) {
@@ -270,12 +301,8 @@ __device__ __forceinline__ bool grid_reduce_masked_state(Acc<R> (&a)[N], AccStor
     for (int k = 0; k < N; ++k) b[k].add(v[k]);
   }
   if ((int)threadIdx.x < words) dst[threadIdx.x] = w;
-  block_reduce<N, 0xffffffffu, R>(b, scratch);  // ends with a barrier: dst is complete
-  if (threadIdx.x == 0) {
-#pragma unroll
-    for (int k = 0; k < N; ++k) total[k] = b[k].value();
-    *counter = 0u;
-  }
+  block_reduce<N, 0xffffffffu, R>(b, scratch);  // ends with a barrier: scratch and dst are complete
+  if (threadIdx.x == 0) *counter = 0u;
   return true;
 }
 

@@ -91,7 +91,7 @@ __global__ void __launch_bounds__(kElemThreads, kDirCtasPerSM) solver_dir_kernel
     if (!a.guard) st->refresh = 0;
   }
   if (st->done || guard_skip(a, st)) return;
-  const R beta = (R)st->beta, inv_mean = (R)st->inv_mean;
+  const R beta = to_real<R>(st->beta), inv_mean = to_real<R>(st->inv_mean);
   const int pb = st->pbuf;
   const V4<R>* pprev = p_prev<R>(a, pb);
   V4<R>* pcur = p_cur<R>(a, pb);
@@ -156,7 +156,6 @@ __global__ void __launch_bounds__(kElemThreads, kDirCtasPerSM) solver_dir_kernel
     ee = een;
     __syncthreads();
   }
-  double tot[N];
   Acc<R> sums[N];
 #pragma unroll
   for (int k = 0; k < N; ++k) {
@@ -165,10 +164,10 @@ __global__ void __launch_bounds__(kElemThreads, kDirCtasPerSM) solver_dir_kernel
   }
   if constexpr (N > 1) sums[1] = c2acc;
   // the last block decides on a shared copy of the state (see the vertex pass)
-  if (!grid_reduce_masked_state<N, FF, R>(sums, (AccStore<R>*)a.part_a, a.cnt_a, gridDim.x, red, tot,
+  if (!grid_reduce_masked_state<N, FF, R>(sums, (AccStore<R>*)a.part_a, a.cnt_a, gridDim.x, red,
                                           (const uint32_t*)st, (uint32_t*)&sst, kStateWords))
     return;
-  if (threadIdx.x == 0) dir_decide<MAT>(&sst, tot);
+  if (threadIdx.x < 32) dir_decide<MAT, R>(&sst, red);
   __syncthreads();
   if ((int)threadIdx.x < kStateWords) ((uint32_t*)st)[threadIdx.x] = ((const uint32_t*)&sst)[threadIdx.x];
 }
@@ -261,7 +260,7 @@ __global__ void __launch_bounds__(kVThreads, kVertexCtasPerSM) solver_vertex_ker
   // ARAP: the pass after the speculative gradient pass, or the one after the
   // fallback passes, whichever applies (the other leaves the condition alone)
   if ((phase == 1 && !st->spec_ok) || (phase == 2 && st->spec_ok)) return;
-  const R t = (R)st->t;
+  const R t = to_real<R>(st->t);
   const V4<R>* P = p_cur<R>(a, st->pbuf);
   // 0 gPg 1 gPy 2 yPy 3 sum|d| 4 count 5 zgg 6 zgy 7 zyy 8 y.p 9 p.g 10 g.g 11 ext energy
   // a thread sums its few vertices in R; float-float starts at the warp trees
@@ -273,23 +272,28 @@ __global__ void __launch_bounds__(kVThreads, kVertexCtasPerSM) solver_vertex_ker
     }
     vertex_update<R, DELTA>(a, i, s0, s1, t, P, s);
   }
-  double tot[N];
   // float-float block sums for the quantities whose terms change sign
   constexpr unsigned FF = (1u << 1) | (1u << 6) | (1u << 8) | (1u << 9);
+  __shared__ SolverState sst;
   Acc<R> acc[N];
 #pragma unroll
   for (int k = 0; k < N; ++k) {
     acc[k] = Acc<R>{};
     acc[k].add(s[k]);
   }
-  if (!grid_reduce_masked<N, FF, R>(acc, (AccStore<R>*)a.part_v, a.cnt_v, gridDim.x, red, tot)) return;
-  if (threadIdx.x != 0) return;
-  vertex_decide(st, tot);
-  if (a.svd) st->sbuf ^= 1;  // the gradient pass's SVDs are those at the new x
-  const bool go = !st->done && st->iter < st->iter_limit;
-  if (use_cond)
-    cudaGraphSetConditional((cudaGraphConditionalHandle)a.cond,
-                            (go && !(a.refresh_exits && st->refresh)) ? 1u : 0u);
+  if (!grid_reduce_masked_state<N, FF, R>(acc, (AccStore<R>*)a.part_v, a.cnt_v, gridDim.x, red, (const uint32_t*)st,
+                                          (uint32_t*)&sst, kStateWords))
+    return;
+  vertex_decide<R>(&sst, red);
+  if (threadIdx.x == 0) {
+    if (a.svd) sst.sbuf ^= 1;  // the gradient pass's SVDs are those at the new x
+    const bool go = !sst.done && sst.iter < sst.iter_limit;
+    if (use_cond)
+      cudaGraphSetConditional((cudaGraphConditionalHandle)a.cond,
+                              (go && !(a.refresh_exits && sst.refresh)) ? 1u : 0u);
+  }
+  __syncthreads();
+  if ((int)threadIdx.x < kStateWords) ((uint32_t*)st)[threadIdx.x] = ((const uint32_t*)&sst)[threadIdx.x];
 }
 
 // The FP32 vertex pass with its inputs streamed by bulk copies.  Each CTA
@@ -355,7 +359,7 @@ __global__ void __launch_bounds__(kVThreads, kVertexCtasPerSM) solver_vertex_bul
   }
   if (guard_skip(a, st)) return;
   if ((phase == 1 && !st->spec_ok) || (phase == 2 && st->spec_ok)) return;
-  const R t = (R)st->t;
+  const R t = to_real<R>(st->t);
   const V4<R>* P = p_cur<R>(a, st->pbuf);
   const V4<R>* XA = (const V4<R>*)a.xa;
   const V4<R>* GD = (const V4<R>*)a.gd;
@@ -439,7 +443,6 @@ __global__ void __launch_bounds__(kVThreads, kVertexCtasPerSM) solver_vertex_bul
     __syncthreads();  // this stage is read before it is refilled
   }
   if (bad) atomicMax(&st->error, 2);  // a copy never completed: the solve stops with a device error
-  double tot[N];
   constexpr unsigned FF = (1u << 1) | (1u << 6) | (1u << 8) | (1u << 9);
   Acc<R> acc[N];
 #pragma unroll
@@ -449,16 +452,15 @@ __global__ void __launch_bounds__(kVThreads, kVertexCtasPerSM) solver_vertex_bul
   }
   // the last block decides on a shared copy of the state, loaded with the
   // block partials, and writes it back in one coalesced store
-  if (!grid_reduce_masked_state<N, FF, R>(acc, (AccStore<R>*)a.part_v, a.cnt_v, gridDim.x, red, tot,
+  if (!grid_reduce_masked_state<N, FF, R>(acc, (AccStore<R>*)a.part_v, a.cnt_v, gridDim.x, red,
                                           (const uint32_t*)st, (uint32_t*)&sst, kStateWords))
     return;
+  if (!sst.error) vertex_decide<R>(&sst, red);
   if (tid == 0) {
-    if (sst.error) {
+    if (sst.error)
       sst.done = 1;
-    } else {
-      vertex_decide(&sst, tot);
-      if (a.svd) sst.sbuf ^= 1;
-    }
+    else if (a.svd)
+      sst.sbuf ^= 1;
     const bool go = !sst.done && sst.iter < sst.iter_limit;
     if (use_cond)
       cudaGraphSetConditional((cudaGraphConditionalHandle)a.cond,

@@ -136,11 +136,22 @@ cudaError_t launch_solver_refresh(const SolveArgs& a, cudaStream_t s, bool pdl =
 cudaError_t launch_solver_force_refresh(const SolveArgs& a, cudaStream_t s);
 
 // Resident iterations (solver_resident.cu): one cooperative launch runs until
-// the iteration limit, termination or a due refresh.  resident_prepare tells
-// whether every tile's CTA fits the device at once; part_d and part_v hold 6
-// and 12 partials per tile, counters two zeroed words.
-cudaError_t resident_prepare(const SolveArgs& a, bool* fits);
-cudaError_t launch_resident(const SolveArgs& a, void* part_d, void* part_v, unsigned* counters, cudaStream_t s);
+// the iteration limit, termination or a due refresh.  resident_prepare fills
+// `shape` when every tile's CTA fits the device at once (0: it does not) from
+// the largest tile's elements and warp groups; part_d and part_v hold 6 and
+// 12 partials per tile, counters kResidentCounters zeroed words.
+constexpr int kResidentMaxTiles = 2 * 152;  // two CTAs on each of the 152 SMs
+struct ResidentPlan {
+  int shape = 0;
+  int max_elems = 0;
+  int max_groups = 0;
+  int whole = 0;  // the first tiles are this many whole ones, the others cut (0: all alike)
+};
+// words of `counters` below
+constexpr int kResidentCounters = 4 + 256;
+cudaError_t resident_prepare(const SolveArgs& a, ResidentPlan* p);
+cudaError_t launch_resident(const SolveArgs& a, const ResidentPlan& p, void* part_d, void* part_v, unsigned* counters,
+                            cudaStream_t s);
 
 // Adjoint CG (adjoint.cu): scalars of H lam = rhs on the free DOFs at the
 // solver's current x, kept on the device like SolverState.
@@ -274,9 +285,10 @@ struct agb_solver {
   int step_kernels = 0;  // kernel nodes of one iteration
   cudaStream_t capture_stream = nullptr;
   // resident iterations, when the mesh fits (solver_resident.cu)
-  bool resident = false;
+  agb::ResidentPlan resident;
   void* d_res_part = nullptr;         // 18 partials per tile
   unsigned* d_res_counters = nullptr;
+  int32_t* d_off = nullptr;           // slot offsets of the split tiles
   bool has_state = false;  // vertex state written (reset or checkpoint load)
   uint64_t fingerprint = 0;  // of the model and parameters, checked by agb_solver_load
 };

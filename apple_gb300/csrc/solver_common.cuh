@@ -24,12 +24,29 @@ __device__ __forceinline__ bool guard_skip(const SolveArgs& a, const SolverState
   return a.guard && (st->iter >= st->iter_limit || st->refresh);
 }
 
+// Scalar decisions.  A GB300 warp issues one FP64 instruction per 65 cycles,
+// whatever its lanes and its parallelism (measured: 65.4 cycles per DFMA in
+// one chain or in four; a division 690, a square root 706), and its four
+// schedulers work independently.  The decisions therefore convert all sums in
+// one instruction (a sum per lane), test signs, finiteness and magnitudes in
+// the integer pipe, and give independent quotients and roots to different
+// warps.
+__device__ __forceinline__ bool finite_bits(double x) {
+  return (__double2hiint(x) & 0x7ff00000) != 0x7ff00000;
+}
+__device__ __forceinline__ bool positive_finite(double x) {  // 0 < x < inf
+  const long long b = __double_as_longlong(x);
+  return b > 0 && b < 0x7ff0000000000000ll;
+}
+__device__ __forceinline__ bool negative_finite(double x) {
+  return positive_finite(__longlong_as_double(__double_as_longlong(x) ^ (long long)0x8000000000000000ull));
+}
+
+// the reference's first trial step: overstep * (-gd / hq), 1 in place of a
+// quotient that is not positive and finite
 __device__ __forceinline__ double initial_alpha(double gd, double hq, double overstep) {
-  double a = -gd / hq;
-  if (isnan(a)) a = 0.0;
-  if (isinf(a)) a = a > 0 ? 1.0 : 0.0;
-  if (!(a > 0.0 && isfinite(a))) a = 1.0;
-  return a * overstep;
+  const double a = -gd / hq;
+  return positive_finite(a) ? a * overstep : overstep;
 }
 
 // A rejected line search restarts with steepest descent; along steepest
@@ -253,27 +270,36 @@ __device__ __forceinline__ void pair_gradient(const V4<R>* sh, const V2<R>* sl, 
 }
 
 
-// Last block of the direction pass (thread 0): alpha_0 from p^T H p and, for
+// After the direction pass, by one whole warp: alpha_0 from p^T H p and, for
 // stable Neo-Hookean, the reference's Armijo backtracking on the closed-form
 // energy change dE(t) = t g.p + sum_m C_m t^m; tot = {p^T H p, C_2..C_6}.
-template <int MAT>
-__device__ __forceinline__ void dir_decide(SolverState* st, const double* tot) {
-  const double hq = tot[0];
-  st->hq = hq;
-  const double gd = st->gd;
+template <int MAT, class R>
+__device__ __forceinline__ void dir_decide(SolverState* st, const Acc<R>* tot) {
+  constexpr unsigned ALL = 0xffffffffu;
+  constexpr int N = snh_family(MAT) ? 6 : 1;
+  const int lane = threadIdx.x & 31;
+  const double v = tot[lane < N ? lane : 0].value();
+  const double hq = __shfl_sync(ALL, v, 0), gd = st->gd;
   const double a0 = initial_alpha(gd, hq, st->overstep);
-  st->alpha0 = a0;
   if constexpr (snh_family(MAT)) {
+    const double c1 = __shfl_sync(ALL, v, 1), c2 = __shfl_sync(ALL, v, 2), c3 = __shfl_sync(ALL, v, 3),
+                 c4 = __shfl_sync(ALL, v, 4), c5 = __shfl_sync(ALL, v, 5);
+    const int max_bt = st->max_bt;
+    const double armijo = st->armijo_c;
     double t = a0, de = 0.0;
     int ls = 0;
     bool ok = false;
     for (;;) {
-      de = t * (gd + t * (tot[1] + t * (tot[2] + t * (tot[3] + t * (tot[4] + t * tot[5])))));
-      ok = isfinite(de) && de <= st->armijo_c * t * gd;
-      if (ok || ls >= st->max_bt || !(t > 0.0)) break;
+      de = t * (gd + t * (c1 + t * (c2 + t * (c3 + t * (c4 + t * c5)))));
+      ok = finite_bits(de) && de <= armijo * t * gd;
+      if (ok || ls >= max_bt || !(t > 0.0)) break;
       t *= 0.5;
       ++ls;
     }
+    __syncwarp();
+    if (lane != 0) return;
+    st->hq = hq;
+    st->alpha0 = a0;
     if (ok) {
       st->t = t;
       st->delta_e = de;
@@ -284,7 +310,10 @@ __device__ __forceinline__ void dir_decide(SolverState* st, const double* tot) {
     }
     st->decided = 1;
   } else {
+    if (lane != 0) return;
     // ARAP: the speculative gradient pass evaluates alpha_0
+    st->hq = hq;
+    st->alpha0 = a0;
     st->t = 0.0;
     st->decided = 0;
     st->spec_ok = 0;
@@ -325,7 +354,7 @@ __device__ __forceinline__ void trial_tile(const SolveArgs& a, int tile, const S
   const double a0 = st->alpha0;
   R tj[3];
 #pragma unroll
-  for (int j = 0; j < 3; ++j) tj[j] = (R)ldexp(a0, -(j0 + j));
+  for (int j = 0; j < 3; ++j) tj[j] = to_real<R>(ldexp(a0, -(j0 + j)));
   const int vs = a.fv.tile_vstart[tile], nv = a.fv.tile_vstart[tile + 1] - vs;
   const int es = a.fv.tile_estart[tile], ee = a.fv.tile_estart[tile + 1];
   stage_direction<R>(a, vs, nv, p_cur<R>(a, st->pbuf), sh, sl, sp);
@@ -384,25 +413,66 @@ __device__ __forceinline__ void trial_decide(SolverState* st, double a0, int j0,
   }
 }
 
-// Last block of the vertex pass (thread 0): Dai-Kou beta, preconditioner
-// mean, descent check and termination from the 12 sums
+// After the vertex pass, by every thread of the CTA (at least 96): Dai-Kou
+// beta, preconditioner mean, descent check and termination from the 12 sums
 // 0 gPg 1 gPy 2 yPy 3 sum|d| 4 count 5 zgg 6 zgy 7 zyy 8 y.p 9 p.g 10 g.g 11 ext energy
-__device__ __forceinline__ void vertex_decide(SolverState* st, const double* tot) {
-  const double cnt = tot[4], sad = tot[3];
-  const double inv_m = (cnt > 0.0 && sad > 0.0) ? cnt / sad : 1.0;
-  const double gPg = tot[0] + inv_m * tot[5];
-  const double gPy = tot[1] + inv_m * tot[6];
-  const double yPy = tot[2] + inv_m * tot[7];
-  const double yp = tot[8], pg = tot[9], gg = tot[10];
-  const double gnorm = sqrt(gg);
+// Of three warps from `w0` on, the first forms the mean fill and its three
+// products, the second 1 / y.p, the third the gradient norm and its tests; the
+// first finishes.
+template <class R>
+__device__ __forceinline__ void vertex_decide(SolverState* st, const Acc<R>* tot, int w0 = 0) {
+  constexpr unsigned ALL = 0xffffffffu;
+  __shared__ double s_d[3];
+  __shared__ int s_flags;
+  const int lane = threadIdx.x & 31, warp = (int)(threadIdx.x >> 5) - w0;
+  double v = 0.0, inv_m = 1.0, filled = 0.0;
+  if (warp >= 0 && warp < 3) v = tot[lane < 12 ? lane : 0].value();
+  if (warp == 0) {
+    const double sad = __shfl_sync(ALL, v, 3), cnt = __shfl_sync(ALL, v, 4);
+    const double mean = cnt / sad;
+    if (positive_finite(cnt) && sad > 0.0) inv_m = mean;
+    const double z = __shfl_sync(ALL, v, (lane + 5) & 31);
+    filled = v + inv_m * z;  // lanes 0..2: gPg, gPy, yPy
+  } else if (warp == 1) {
+    const double yp = __shfl_sync(ALL, v, 8), pg = __shfl_sync(ALL, v, 9);
+    const double r = 1.0 / yp;
+    const double q = pg * r;
+    if (lane == 0) {
+      s_d[0] = fabs(yp) > 1.0e-12 ? r : INFINITY;
+      s_d[1] = q;
+    }
+  } else if (warp == 2) {
+    const double gnorm = sqrt(__shfl_sync(ALL, v, 10));
+    const bool first = st->init != 0;
+    const double g0 = first ? gnorm : st->gnorm0;
+    const bool converged = gnorm <= fmax(st->atol, st->rtol * g0);
+    const double ref = st->ref_ratio;
+    const bool due = !first && ref > 0.0 && gnorm <= ref * st->gnorm_ref;
+    if (lane == 0) {
+      s_d[2] = gnorm;
+      s_flags = (converged ? 1 : 0) | (due ? 2 : 0);
+    }
+  }
+  __syncthreads();
+  if (warp != 0) return;
+  const double r = s_d[0], pg_yp = s_d[1], gnorm = s_d[2];
+  const int flags = s_flags;
+  const double pg = __shfl_sync(ALL, v, 9), ext = __shfl_sync(ALL, v, 11);
+  const double q = filled * r;  // lanes 1, 2: gPy / yp, yPy / yp
+  const double gPy_yp = __shfl_sync(ALL, q, 1), yPy_yp = __shfl_sync(ALL, q, 2);
+  const double gPg = __shfl_sync(ALL, filled, 0);
+  if (lane != 0) return;
   const bool first = st->init != 0;
   double b = 0.0;
-  if (!first) {
-    b = fabs(yp) > 1.0e-12 ? gPy / yp - (yPy / yp) * (pg / yp) : INFINITY;
-    if (st->reset_beta || !isfinite(b) || fabs(b) > st->beta_max) b = 0.0;
+  if (!first && !st->reset_beta && finite_bits(r)) {
+    b = gPy_yp - yPy_yp * pg_yp;
+    // |b| > beta_max on the bits: both orders agree for non-negative doubles
+    if (!finite_bits(b) ||
+        (__double_as_longlong(b) & 0x7fffffffffffffffll) > __double_as_longlong(st->beta_max))
+      b = 0.0;
   }
   double gd = -gPg + b * pg;
-  if (!(isfinite(gd) && gd < 0.0)) {
+  if (!negative_finite(gd)) {
     b = 0.0;
     gd = -gPg;
   }
@@ -411,7 +481,7 @@ __device__ __forceinline__ void vertex_decide(SolverState* st, const double* tot
   st->pbuf ^= 1;  // this iteration's p becomes p_prev
   st->gd = gd;
   st->gnorm = gnorm;
-  st->ext_energy = tot[11];
+  st->ext_energy = ext;
   st->reset_beta = 0;
   if (first) {
     st->gnorm0 = gnorm;
@@ -420,24 +490,22 @@ __device__ __forceinline__ void vertex_decide(SolverState* st, const double* tot
     st->iter += 1;
   }
   int result = AGB_RUNNING;
-  if (!isfinite(gnorm) || !isfinite(gPg) || !isfinite(tot[11]))
+  if (!finite_bits(gnorm) || !finite_bits(gPg) || !finite_bits(ext))
     result = AGB_NAN_ENCOUNTERED;
   else if (!first && st->ls_fail)
     result = AGB_LINE_SEARCH_FAILED;
-  else if (gnorm <= fmax(st->atol, st->rtol * st->gnorm0))
+  else if (flags & 1)
     result = AGB_PRIMARY_SUCCESS;
   else if (st->iter >= st->max_steps)
     result = AGB_MAX_STEPS_REACHED;
   if (result != AGB_RUNNING) {
     st->done = 1;
     st->result = result;
-  } else if (st->ref_ratio > 0.0) {
-    if (first)
-      st->gnorm_ref = gnorm;
-    else if (gnorm <= st->ref_ratio * st->gnorm_ref) {
-      st->refresh = 1;
-      st->gnorm_ref = gnorm;
-    }
+  } else if (first) {
+    st->gnorm_ref = gnorm;  // read only with ref_ratio > 0
+  } else if (flags & 2) {
+    st->refresh = 1;
+    st->gnorm_ref = gnorm;
   }
 }
 
@@ -680,10 +748,10 @@ __device__ __forceinline__ bool grad_tile(const SolveArgs& a, int tile, const So
   }
   R t;
   if constexpr (SPEC) {
-    t = (R)st->alpha0;
+    t = to_real<R>(st->alpha0);
     stage_point_dir<R>(a, vid, p_cur<R>(a, st->pbuf), sh, sl, sp);
   } else {
-    t = (R)st->t;
+    t = to_real<R>(st->t);
     if constexpr (DELTA)
       stage_point_delta<R>(a, vid, p_cur<R>(a, st->pbuf), t, sh, sl);
     else
@@ -846,7 +914,7 @@ __device__ __forceinline__ void ref_tile(const SolveArgs& a, int tile) {
     const int v = a.fv.tv_vid[vs + i];
     const V4<float> x = XA[2 * v];
     XR[v] = V4<float>{x.x, x.y, x.z, 0.f};  // tiles sharing v store equal values
-    sx[i] = V4<double>{(double)x.x, (double)x.y, (double)x.z, 0.0};
+    sx[i] = V4<double>{widen(x.x), widen(x.y), widen(x.z), 0.0};
   }
   for (int i = threadIdx.x; i < kGradWarps * kTileVerts; i += blockDim.x) acc[i] = V4<double>{0.0, 0.0, 0.0, 0.0};
   __syncthreads();
@@ -863,11 +931,11 @@ __device__ __forceinline__ void ref_tile(const SolveArgs& a, int tile) {
 #pragma unroll
       for (int i = 0; i < 3; ++i)
 #pragma unroll
-        for (int j = 0; j < 3; ++j) geo.D[i][j] = (double)gf.D[i][j];
-      geo.mu = (double)gf.mu;
-      geo.lam = (double)gf.lam;
+        for (int j = 0; j < 3; ++j) geo.D[i][j] = widen(gf.D[i][j]);
+      geo.mu = widen(gf.mu);
+      geo.lam = widen(gf.lam);
 #pragma unroll
-      for (int k = 0; k < 6; ++k) geo.S[k] = (double)gf.S[k];
+      for (int k = 0; k < 6; ++k) geo.S[k] = widen(gf.S[k]);
 #pragma unroll
       for (int k = 0; k < 4; ++k) l[k] = corner(ids, k);
       double G[3][3], P[3][3];
@@ -919,13 +987,13 @@ __device__ __forceinline__ void ref_vertex(const SolveArgs& a, int i) {
   }
   if (a.force) {
     const V4<float> f = ((const V4<float>*)a.force)[i];
-    g[0] -= (double)f.x;
-    g[1] -= (double)f.y;
-    g[2] -= (double)f.z;
+    g[0] -= widen(f.x);
+    g[1] -= widen(f.y);
+    g[2] -= widen(f.z);
   }
   // one float suffices: g(x_ref) is itself a residual (at most 1/ref_ratio
   // times the current one), so its rounding is far below the current ||g||
-  const V4<float> gr{(float)g[0], (float)g[1], (float)g[2], 0.f};
+  const V4<float> gr{narrow(g[0]), narrow(g[1]), narrow(g[2]), 0.f};
   ((V4<float>*)a.gref)[i] = gr;
   // the stored g of this iterate becomes the new reference's value too
   // (x_ref = x_hi differs from x by x_lo only), so the next y = g - g_prev

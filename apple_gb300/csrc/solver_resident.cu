@@ -5,7 +5,8 @@
 // completion counter and a one-thread scalar tail per pass.  Here every tile
 // stays on one resident CTA for the whole run, three grid barriers separate
 // the passes, and all CTAs sum the partials and take the scalar decisions
-// themselves (the same numbers in the same order, so they agree bit for bit):
+// themselves (the same numbers in the same order, so they agree bit for bit;
+// one CTA deciding and publishing took 2 us more per decision):
 //
 //   direction   the CTA's tile vertices read (g, d), form p = -P g + beta
 //               p_prev; per element p^T H_e p and the line-search polynomial
@@ -25,8 +26,10 @@
 // for bit.
 //
 // Measured (40 iterations with the reset and the refreshes): 5,000-tet cube in
-// FP32 1,108 us against 1,377 with the three-kernel loop, 138,240 tets 1,467
-// against 1,976; 20 iterations of 138,240 tets in FP64 5,507 against 7,307.
+// FP32 833 us against 1,369 with the three-kernel loop, 138,240 tets 1,176
+// against 1,976; 20 iterations of 138,240 tets in FP64 4,458 against 7,306.
+// An iteration of the cube takes 15.7 us, of which the three barriers are 4,
+// the element groups 3, the sums 1.3 and the two decisions 2.5.
 #include <math.h>
 
 #include "gridsync.cuh"
@@ -40,22 +43,26 @@ namespace {
 
 constexpr int kStateWords = (int)(sizeof(SolverState) / 4);
 
-// Warps per tile: in FP32 16 while every tile has an SM to itself, 8 up to two
-// tiles per SM (128 registers each way); FP64 is bound by its arithmetic pipe,
-// which 8 warps per SM fill: 4 per tile.  Above two tiles per SM the
-// three-kernel iteration is the faster one: with four 4-warp CTAs per SM this
-// kernel took 2.46 against 2.23 ms on 245,760 tets (376 tiles) and 2.88
-// against 2.55 ms on 400,000 (592 tiles), for 40 iterations and the reset.
+// Warps per tile (two CTAs per SM): 8 in FP32; FP64 is bound by its
+// arithmetic pipe, which 8 warps per SM fill: 4.  Meshes with fewer tiles
+// than CTAs are cut finer first (split_tiles in prep.cpp): a whole tile's
+// groups are issue-bound on one SM while others idle.  Above two tiles
+// per SM the three-kernel iteration is the faster one: with four 4-warp CTAs
+// per SM this kernel took 2.46 against 2.23 ms on 245,760 tets (376 tiles) and
+// 2.88 against 2.55 ms on 400,000 (592 tiles), for 40 iterations and the reset.
 template <class R>
-constexpr int ctas_per_sm(int nw) {
-  return nw == 16 ? 1 : 2;
-}
+constexpr int kResidentWarps = sizeof(R) == 4 ? 8 : 4;
 
 // per-vertex words kept between iterations: x hi, x lo, p, previous g, mask,
 // and with the reference-state correction x_ref
 template <bool DELTA>
 constexpr int kVertexWords = DELTA ? 16 : 13;
 
+// records kept in shared memory (FP32): their float4 streams
+template <int MAT>
+constexpr int kRecStreams = MAT == AGB_STABLE_NEO_HOOKEAN_MUSCLE ? 5 : 3;
+
+// the accumulators' space also takes the block sums' rows (13 per thread)
 template <class R, bool DELTA>
 constexpr size_t resident_smem(int nw) {
   return (size_t)kTileVerts *
@@ -76,10 +83,14 @@ __device__ __forceinline__ V4<double> ldcg4<double>(const V4<double>* p) {
   return V4<double>{a.x, a.y, b.x, b.y};
 }
 
-template <class R, int MAT, bool DELTA, int NW>
-__global__ void __launch_bounds__(32 * NW, ctas_per_sm<R>(NW)) solver_resident_kernel(SolveArgs a, void* part_d,
-                                                                                     void* part_v, unsigned* counters) {
-  constexpr int T = 32 * NW, ND = 6, NVT = 12;
+// REC: the tile's element records stay in shared memory after the first read
+// (a barrier's acquire leaves nothing in L1, so every pass would fetch them
+// from L2); otherwise each group's records are loaded one group ahead.
+template <class R, int MAT, bool DELTA, int NW, bool REC>
+__global__ void __launch_bounds__(32 * NW, 2) solver_resident_kernel(SolveArgs a, int max_elems, int whole,
+                                                                                     void* part_d, void* part_v,
+                                                                                     unsigned* counters) {
+  constexpr int T = 32 * NW, ND = 6, NVT = 12, kSlotBatch = 4;
   constexpr unsigned FFD = 0x2u, FFV = (1u << 1) | (1u << 6) | (1u << 8) | (1u << 9);
   extern __shared__ __align__(16) unsigned char smem_raw[];
   V4<R>* s4 = reinterpret_cast<V4<R>*>(smem_raw);           // staging
@@ -88,8 +99,12 @@ __global__ void __launch_bounds__(32 * NW, ctas_per_sm<R>(NW)) solver_resident_k
   V2<R>* acc2 = s2 + kTileVerts;                            // [warp][vertex]: dy dz
   R* vw = reinterpret_cast<R*>(acc2 + NW * kTileVerts);     // kept vertex words, [word][vertex]
   int* vi = reinterpret_cast<int*>(vw + kVertexWords<DELTA> * kTileVerts);  // vertex, slot, first and end slot
-  __shared__ Acc<R> red[NW * NVT];
-  __shared__ double tot[NVT];
+  float4* srec = reinterpret_cast<float4*>(vi + 4 * kTileVerts);  // REC: [stream][element]
+  int* sgrp = reinterpret_cast<int*>(srec + (size_t)kRecStreams<MAT> * max_elems);  // REC: group starts
+  R* const rows = reinterpret_cast<R*>(acc4);  // the block sums' terms, while no accumulation runs
+  static_assert(NW * kTileVerts * sizeof(V4<R>) >= (NVT + 1) * T * sizeof(R), "rows fit the accumulators");
+  static_assert(kResidentCounters == 2 + kPlaceWords, "barrier and placement");
+  __shared__ Acc<R> tot[NVT];
   __shared__ SolverState sst;
   R* const xh = vw;
   R* const xl = vw + 3 * kTileVerts;
@@ -99,10 +114,14 @@ __global__ void __launch_bounds__(32 * NW, ctas_per_sm<R>(NW)) solver_resident_k
   R* const xr = vw + 13 * kTileVerts;  // DELTA only
 
   if (a.st->done) return;
-  const int tile = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  __shared__ int s_tile;
+  if (tid == 0) s_tile = whole > 0 ? place_cta(counters, whole, gridDim.x) : (int)blockIdx.x;
+  __syncthreads();
+  const int tile = s_tile;
   const int gs = a.fv.tile_gstart[tile], ge = a.fv.tile_gstart[tile + 1];
   const int vs = a.fv.tile_vstart[tile], nv = a.fv.tile_vstart[tile + 1] - vs;
-  GridBar bar{counters, gridDim.x, 0};
+  GridBar bar{counters, kResidentCounters, gridDim.x, 0};
   if (tid < kStateWords) ((uint32_t*)&sst)[tid] = ((const uint32_t*)a.st)[tid];
   __syncthreads();
   const V4<R>* XA = (const V4<R>*)a.xa;
@@ -115,9 +134,9 @@ __global__ void __launch_bounds__(32 * NW, ctas_per_sm<R>(NW)) solver_resident_k
       const int s0 = a.off[v], s1 = a.off[v + 1];
       vi[i] = v;
       vi[kTileVerts + i] = sl;
-      // the tile with a vertex's first slot owns it
+      // one of the tiles that hold a vertex owns it, spread over its slots
       vi[2 * kTileVerts + i] = s0;
-      vi[3 * kTileVerts + i] = sl == s0 ? s1 : s0;
+      vi[3 * kTileVerts + i] = sl == s0 + v % (s1 - s0) ? s1 : s0;
       const V4<R> x = XA[2 * v], l = XA[2 * v + 1], p = P[v];
       xh[i] = x.x;
       xh[kTileVerts + i] = x.y;
@@ -137,15 +156,78 @@ __global__ void __launch_bounds__(32 * NW, ctas_per_sm<R>(NW)) solver_resident_k
       }
     }
   }
-  __syncthreads();  // every thread has read sst.pbuf
+  const int e_first = a.fv.tile_estart[tile];
+  if constexpr (REC) {
+    const int ne = a.fv.tile_estart[tile + 1] - e_first;
+    const float4* rec = static_cast<const float4*>(a.fv.rec);
+    const float4* act = static_cast<const float4*>(a.fv.act);
+    const size_t nc = (size_t)a.fv.n_cells;
+    for (int i = tid; i < ne; i += T) {
+#pragma unroll
+      for (int k = 0; k < 3; ++k) srec[(size_t)k * max_elems + i] = __ldg(rec + k * nc + e_first + i);
+#pragma unroll
+      for (int k = 3; k < kRecStreams<MAT>; ++k) srec[(size_t)k * max_elems + i] = __ldg(act + (k - 3) * nc + e_first + i);
+    }
+    for (int i = tid; i <= ge - gs; i += T) sgrp[i] = a.fv.group_estart[gs + i] - e_first;
+  }
+  // the record of lane `lane` in group q; its size into n
+  auto load_group = [&](int q, int& n, ElemGeo<R>& geo, uint32_t& ids) {
+    if constexpr (REC) {
+      const int e0 = sgrp[q - gs];
+      n = sgrp[q - gs + 1] - e0;
+      if (lane < n) {
+        const float4* r = srec + e0 + lane;
+        const float4 A = r[0], B = r[max_elems], C = r[2 * max_elems];
+        geo.D[0][0] = A.x; geo.D[0][1] = A.y; geo.D[0][2] = A.z;
+        geo.D[1][0] = A.w; geo.D[1][1] = B.x; geo.D[1][2] = B.y;
+        geo.D[2][0] = B.z; geo.D[2][1] = B.w; geo.D[2][2] = C.x;
+        geo.mu = C.y;
+        geo.lam = C.z;
+        ids = __float_as_uint(C.w);
+        if constexpr (kRecStreams<MAT> == 5) {
+          const float4 s0 = r[3 * max_elems], s1 = r[4 * max_elems];
+          geo.S[0] = s0.x; geo.S[1] = s0.y; geo.S[2] = s0.z;
+          geo.S[3] = s0.w; geo.S[4] = s1.x; geo.S[5] = s1.y;
+        }
+      }
+    } else {
+      const int e0 = a.fv.group_estart[q];
+      n = a.fv.group_estart[q + 1] - e0;
+      if (lane < n) load_elem_m<R, MAT>(a.fv, e0 + lane, geo, ids);
+    }
+  };
+  // The accumulators are cleared while a barrier is waited for: those that
+  // the block sums' rows overlay after the direction pass, the others after
+  // the vertex pass.
+  constexpr int kRowCopies = (int)(((NVT + 1) * T * sizeof(R) + kTileVerts * sizeof(V4<R>) - 1) /
+                                   (kTileVerts * sizeof(V4<R>)));
+  auto zero4 = [&](int w) {
+    for (int i = tid; i < nv; i += T) acc4[w * kTileVerts + i] = V4<R>{R(0), R(0), R(0), R(0)};
+  };
+  auto zero_rest = [&]() {
+    for (int w = kRowCopies; w < NW; ++w) zero4(w);
+    for (int w = 0; w < NW; ++w)
+      for (int i = tid; i < nv; i += T) acc2[w * kTileVerts + i] = V2<R>{R(0), R(0)};
+  };
+  zero_rest();
+  __syncthreads();  // every thread has read sst.pbuf; records and groups are in place
   if (tid == 0) sst.refresh = 0;  // the refresh passes, if any, ran after the last vertex pass
+
+  // the scheduler whose FP64 pipe takes the decisions: the second CTA of an SM
+  // uses another one
+  unsigned warp_slot;
+  asm volatile("mov.u32 %0, %%warpid;" : "=r"(warp_slot));
+  __shared__ int s_w0;
+  if (tid == 0) s_w0 = (warp_slot / NW) & 1u ? 1 : 0;
+  __syncthreads();
+  const int w0 = s_w0;
 
   bool ok = true;
   for (;;) {
     // ---- direction ----
     __syncthreads();
     {
-      const R beta = (R)sst.beta, inv_mean = (R)sst.inv_mean;
+      const R beta = to_real<R>(sst.beta), inv_mean = to_real<R>(sst.inv_mean);
       for (int i = tid; i < nv; i += T) {
         const int v = vi[i];
         const V4<R> g = ldcg4(GD + 2 * v), d = ldcg4(GD + 2 * v + 1);
@@ -165,16 +247,7 @@ __global__ void __launch_bounds__(32 * NW, ctas_per_sm<R>(NW)) solver_resident_k
     int g = gs + warp, n = 0;
     ElemGeo<R> geo;
     uint32_t ids = 0;
-    if (g < ge) {
-      const int e0 = a.fv.group_estart[g];
-      n = a.fv.group_estart[g + 1] - e0;
-      if (lane < n) load_elem_m<R, MAT>(a.fv, e0 + lane, geo, ids);
-    }
-    for (int w = 0; w < NW; ++w)
-      for (int i = tid; i < nv; i += T) {
-        acc4[w * kTileVerts + i] = V4<R>{R(0), R(0), R(0), R(0)};
-        acc2[w * kTileVerts + i] = V2<R>{R(0), R(0)};
-      }
+    if (!REC && g < ge) load_group(g, n, geo, ids);
     __syncthreads();
     {
       R plain[ND] = {};
@@ -184,11 +257,10 @@ __global__ void __launch_bounds__(32 * NW, ctas_per_sm<R>(NW)) solver_resident_k
         int nn = 0;
         ElemGeo<R> geon;
         uint32_t idsn = 0;
-        if (gn < ge) {
-          const int e0n = a.fv.group_estart[gn];
-          nn = a.fv.group_estart[gn + 1] - e0n;
-          if (lane < nn) load_elem_m<R, MAT>(a.fv, e0n + lane, geon, idsn);
-        }
+        if constexpr (REC)
+          load_group(g, n, geo, ids);
+        else if (gn < ge)
+          load_group(gn, nn, geon, idsn);
         if (lane < n) {
           const int l[4] = {corner(ids, 0), corner(ids, 1), corner(ids, 2), corner(ids, 3)};
           R G[3][3], dF[3][3];
@@ -206,35 +278,35 @@ __global__ void __launch_bounds__(32 * NW, ctas_per_sm<R>(NW)) solver_resident_k
           for (int m = 1; m < 5; ++m) plain[1 + m] += c[m];
         }
         g = gn;
-        n = nn;
-        geo = geon;
-        ids = idsn;
+        if constexpr (!REC) {
+          n = nn;
+          geo = geon;
+          ids = idsn;
+        }
       }
-      Acc<R> sums[ND];
-#pragma unroll
-      for (int k = 0; k < ND; ++k) {
-        sums[k] = Acc<R>{};
-        sums[k].add(plain[k]);
+      R lo = R(0);
+      if constexpr (sizeof(R) == 4) {
+        plain[1] = c2acc.hi;
+        lo = c2acc.lo;
+      } else {
+        plain[1] = c2acc.v;
       }
-      sums[1] = c2acc;
-      cta_partials<ND, FFD, R>(sums, red, (AccStore<R>*)part_d, gridDim.x);
+      cta_partials<ND, FFD, sizeof(R) == 4 ? 1 : -1, T, R>(plain, lo, rows, (AccStore<R>*)part_d, gridDim.x, tile);
     }
-    if (!(ok = bar.sync())) break;
-    grid_totals<ND, R>((const AccStore<R>*)part_d, gridDim.x, tot);
-    if (tid == 0) dir_decide<MAT>(&sst, tot);
+    bar.arrive();
+    for (int w = 0; w < kRowCopies; ++w) zero4(w);
+    if (!(ok = bar.wait())) break;
     // the gradient pass's first record, in flight during the decision
     g = gs + warp;
     n = 0;
-    if (g < ge) {
-      const int e0 = a.fv.group_estart[g];
-      n = a.fv.group_estart[g + 1] - e0;
-      if (lane < n) load_elem_m<R, MAT>(a.fv, e0 + lane, geo, ids);
-    }
+    if (!REC && g < ge) load_group(g, n, geo, ids);
+    grid_totals<ND, T, R>((const AccStore<R>*)part_d, gridDim.x, tot);
+    if (warp == w0) dir_decide<MAT, R>(&sst, tot);
     __syncthreads();
+    const R t = to_real<R>(sst.t);
 
     // ---- gradient at x + t p ----
     {
-      const R t = (R)sst.t;
       for (int i = tid; i < nv; i += T) {
         R h[3], l[3];
 #pragma unroll
@@ -264,11 +336,10 @@ __global__ void __launch_bounds__(32 * NW, ctas_per_sm<R>(NW)) solver_resident_k
         int nn = 0;
         ElemGeo<R> geon;
         uint32_t idsn = 0;
-        if (gn < ge) {
-          const int e0n = a.fv.group_estart[gn];
-          nn = a.fv.group_estart[gn + 1] - e0n;
-          if (lane < nn) load_elem_m<R, MAT>(a.fv, e0n + lane, geon, idsn);
-        }
+        if constexpr (REC)
+          load_group(g, n, geo, ids);
+        else if (gn < ge)
+          load_group(gn, nn, geon, idsn);
         const int l[4] = {corner(ids, 0), corner(ids, 1), corner(ids, 2), corner(ids, 3)};
         R f[4][3], hd[4][3];
         if (lane < n) {
@@ -311,9 +382,11 @@ __global__ void __launch_bounds__(32 * NW, ctas_per_sm<R>(NW)) solver_resident_k
         }
         __syncwarp();
         g = gn;
-        n = nn;
-        geo = geon;
-        ids = idsn;
+        if constexpr (!REC) {
+          n = nn;
+          geo = geon;
+          ids = idsn;
+        }
       }
     }
     __syncthreads();
@@ -335,8 +408,8 @@ __global__ void __launch_bounds__(32 * NW, ctas_per_sm<R>(NW)) solver_resident_k
       slots[sl] = V4<R>{q4.x, q4.y, q4.z, R(0)};
       slots[sl + 1] = V4<R>{q4.w, q2.x, q2.y, R(0)};
     }
-    if (!(ok = bar.sync())) break;
-
+    bar.arrive();
+    if (!(ok = bar.wait())) break;
     // ---- vertex ----
     {
       R s[NVT] = {};
@@ -348,14 +421,24 @@ __global__ void __launch_bounds__(32 * NW, ctas_per_sm<R>(NW)) solver_resident_k
         if constexpr (DELTA) r = ldg4((const V4<R>*)a.gref + v);
         if (a.force) f = ldg4((const V4<R>*)a.force + v);
         R ss[3] = {R(0), R(0), R(0)}, ds[3] = {R(0), R(0), R(0)};
-        for (int k = s0; k < s1; ++k) {
-          const V4<R> sg = ldcg4(slots + 2 * (size_t)k), sd = ldcg4(slots + 2 * (size_t)k + 1);
-          ss[0] += sg.x;
-          ss[1] += sg.y;
-          ss[2] += sg.z;
-          ds[0] += sd.x;
-          ds[1] += sd.y;
-          ds[2] += sd.z;
+        for (int k = s0; k < s1; k += kSlotBatch) {  // a batch of slots in flight together
+          V4<R> sg[kSlotBatch], sd[kSlotBatch];
+#pragma unroll
+          for (int q = 0; q < kSlotBatch; ++q)
+            if (k + q < s1) {
+              sg[q] = ldcg4(slots + 2 * (size_t)(k + q));
+              sd[q] = ldcg4(slots + 2 * (size_t)(k + q) + 1);
+            }
+#pragma unroll
+          for (int q = 0; q < kSlotBatch; ++q)
+            if (k + q < s1) {
+              ss[0] += sg[q].x;
+              ss[1] += sg[q].y;
+              ss[2] += sg[q].z;
+              ds[0] += sd[q].x;
+              ds[1] += sd[q].y;
+              ds[2] += sd[q].z;
+            }
         }
         R xn[3], p[3], gn[3], dn[3];
 #pragma unroll
@@ -368,17 +451,13 @@ __global__ void __launch_bounds__(32 * NW, ctas_per_sm<R>(NW)) solver_resident_k
         GD[2 * v] = V4<R>{gn[0], gn[1], gn[2], R(0)};
         GD[2 * v + 1] = V4<R>{dn[0], dn[1], dn[2], R(0)};
       }
-      Acc<R> acc[NVT];
-#pragma unroll
-      for (int k = 0; k < NVT; ++k) {
-        acc[k] = Acc<R>{};
-        acc[k].add(s[k]);
-      }
-      cta_partials<NVT, FFV, R>(acc, red, (AccStore<R>*)part_v, gridDim.x);
+      cta_partials<NVT, FFV, -1, T, R>(s, R(0), rows, (AccStore<R>*)part_v, gridDim.x, tile);
     }
-    if (!(ok = bar.sync())) break;
-    grid_totals<NVT, R>((const AccStore<R>*)part_v, gridDim.x, tot);
-    if (tid == 0) vertex_decide(&sst, tot);
+    bar.arrive();
+    zero_rest();
+    if (!(ok = bar.wait())) break;
+    grid_totals<NVT, T, R>((const AccStore<R>*)part_v, gridDim.x, tot);
+    vertex_decide<R>(&sst, tot, w0);
     __syncthreads();
     if (sst.done || sst.iter >= sst.iter_limit || sst.refresh) break;
   }
@@ -386,6 +465,7 @@ __global__ void __launch_bounds__(32 * NW, ctas_per_sm<R>(NW)) solver_resident_k
   if (ok) {
     V4<R>* X = (V4<R>*)a.xa;
     V4<R>* P = p_prev<R>(a, sst.pbuf);  // the last direction, flipped to p_prev by the decision
+    if (tile == 0 && tid < kStateWords) ((uint32_t*)a.st)[tid] = ((const uint32_t*)&sst)[tid];
     for (int i = tid; i < nv; i += T) {
       if (vi[2 * kTileVerts + i] == vi[3 * kTileVerts + i]) continue;
       const int v = vi[i];
@@ -393,7 +473,6 @@ __global__ void __launch_bounds__(32 * NW, ctas_per_sm<R>(NW)) solver_resident_k
       X[2 * v + 1] = V4<R>{xl[i], xl[kTileVerts + i], xl[2 * kTileVerts + i], R(0)};
       P[v] = V4<R>{vp[i], vp[kTileVerts + i], vp[2 * kTileVerts + i], R(0)};
     }
-    if (tile == 0 && tid < kStateWords) ((uint32_t*)a.st)[tid] = ((const uint32_t*)&sst)[tid];
   } else if (tid == 0) {  // a barrier gave up: the solve stops with a device error
     atomicMax(&a.st->error, 3);
     a.st->done = 1;
@@ -401,57 +480,73 @@ __global__ void __launch_bounds__(32 * NW, ctas_per_sm<R>(NW)) solver_resident_k
   bar.leave();
 }
 
-using ResidentKernel = void (*)(SolveArgs, void*, void*, unsigned*);
+using ResidentKernel = void (*)(SolveArgs, int, int, void*, void*, unsigned*);
 
-struct ResidentShape {
-  ResidentKernel kernel = nullptr;
-  int threads = 0;
-  size_t smem = 0;
+struct Shape {
+  ResidentKernel kernel;
+  int threads;
+  size_t smem;
 };
 
-template <class R, int MAT, bool DELTA, int NW>
-ResidentShape shape_nw() {
-  return ResidentShape{solver_resident_kernel<R, MAT, DELTA, NW>, 32 * NW, resident_smem<R, DELTA>(NW)};
+template <class R, int MAT, bool DELTA, int NW, bool REC>
+Shape shape(const ResidentPlan& p) {
+  size_t smem = resident_smem<R, DELTA>(NW);
+  if (REC) smem += (size_t)p.max_elems * kRecStreams<MAT> * sizeof(float4) + ((size_t)p.max_groups + 1) * sizeof(int);
+  return Shape{solver_resident_kernel<R, MAT, DELTA, NW, REC>, 32 * NW, smem};
 }
 
 template <int MAT, bool DELTA>
-ResidentShape shape_f32(int n_tiles) {
-  return n_tiles <= kSMs ? shape_nw<float, MAT, DELTA, 16>() : shape_nw<float, MAT, DELTA, 8>();
+Shape shape_f32(const ResidentPlan& p) {
+  constexpr int W = kResidentWarps<float>;
+  return p.shape == 1 ? shape<float, MAT, DELTA, W, true>(p) : shape<float, MAT, DELTA, W, false>(p);
 }
 
-ResidentShape resident_shape(const SolveArgs& a) {
-  const int nt = a.fv.n_tiles;
-  if (nt > 2 * kSMs) return ResidentShape{};
+Shape shape_of(const SolveArgs& a, const ResidentPlan& p) {
   constexpr int SNH = AGB_STABLE_NEO_HOOKEAN, MU = AGB_STABLE_NEO_HOOKEAN_MUSCLE;
-  if (!snh_family(a.fv.material)) return ResidentShape{};
   const bool mu = a.fv.material == MU;
-  if (a.precision == AGB_F64) return mu ? shape_nw<double, MU, false, 4>() : shape_nw<double, SNH, false, 4>();
-  if (a.delta) return mu ? shape_f32<MU, true>(nt) : shape_f32<SNH, true>(nt);
-  return mu ? shape_f32<MU, false>(nt) : shape_f32<SNH, false>(nt);
+  if (a.precision == AGB_F64)
+    return mu ? shape<double, MU, false, kResidentWarps<double>, false>(p)
+              : shape<double, SNH, false, kResidentWarps<double>, false>(p);
+  if (a.delta) return mu ? shape_f32<MU, true>(p) : shape_f32<SNH, true>(p);
+  return mu ? shape_f32<MU, false>(p) : shape_f32<SNH, false>(p);
 }
 
 }  // namespace
 
-// Whether the solver's iterations can run resident: every tile's CTA fits the
-// device at once (the kernel prepared on the way).
-cudaError_t resident_prepare(const SolveArgs& a, bool* fits) {
-  *fits = false;
-  const ResidentShape sh = resident_shape(a);
-  if (!sh.kernel || a.fv.n_tiles == 0) return cudaSuccess;
-  int dev = 0, sms = 0, coop = 0, occ = 0;
+// The first shape whose CTAs, one per tile, fit the device at once: in FP32
+// with the records in shared memory, or without (tiles with too many
+// elements for two CTAs per SM).
+cudaError_t resident_prepare(const SolveArgs& a, ResidentPlan* p) {
+  p->shape = 0;
+  if (!snh_family(a.fv.material) || a.fv.n_tiles == 0 || a.fv.n_tiles > kResidentMaxTiles) return cudaSuccess;
+  int dev = 0, sms = 0, coop = 0, limit = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(sh.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh.smem);
-  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, sh.kernel, sh.threads, sh.smem);
-  if (e == cudaSuccess) *fits = coop && (int64_t)a.fv.n_tiles <= (int64_t)occ * sms;
-  return e;
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  if (e != cudaSuccess || !coop) return e;
+  const int shapes = a.precision == AGB_F64 ? 1 : 2;
+  for (int k = 1; k <= shapes; ++k) {
+    ResidentPlan q = *p;
+    q.shape = k;
+    const Shape sh = shape_of(a, q);
+    if (sh.smem + 8 * 1024 > (size_t)limit) continue;  // beside the kernel's static arrays
+    int occ = 0;
+    e = allow_max_smem(sh.kernel);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, sh.kernel, sh.threads, sh.smem);
+    if (e != cudaSuccess) return e;
+    if ((int64_t)a.fv.n_tiles <= (int64_t)occ * sms) {
+      p->shape = k;
+      return cudaSuccess;
+    }
+  }
+  return cudaSuccess;
 }
 
-cudaError_t launch_resident(const SolveArgs& a, void* part_d, void* part_v, unsigned* counters, cudaStream_t s) {
-  const ResidentShape sh = resident_shape(a);
-  if (!sh.kernel) return cudaErrorInvalidValue;
+cudaError_t launch_resident(const SolveArgs& a, const ResidentPlan& p, void* part_d, void* part_v, unsigned* counters,
+                            cudaStream_t s) {
+  if (!p.shape) return cudaErrorInvalidValue;
+  const Shape sh = shape_of(a, p);
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(a.fv.n_tiles);
   cfg.blockDim = dim3(sh.threads);
@@ -462,7 +557,7 @@ cudaError_t launch_resident(const SolveArgs& a, void* part_d, void* part_v, unsi
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, sh.kernel, a, part_d, part_v, counters);
+  return cudaLaunchKernelEx(&cfg, sh.kernel, a, p.max_elems, p.whole, part_d, part_v, counters);
 }
 
 }  // namespace agb
