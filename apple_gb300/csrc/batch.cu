@@ -64,7 +64,7 @@ __global__ void __launch_bounds__(kElemThreads) batch_dir_kernel(BatchArgs b) {
       snh_prepare(G, s);
       SnhDir<R> d;
       snh_dir(s, dF, d);
-      sums[0].add(fmax(snh_hess_quad(s, d, geo.mu, geo.lam), R(0)));
+      sums[0].add(clamp0(snh_hess_quad(s, d, geo.mu, geo.lam)));
       R c[5];
       snh_poly(s, d, geo.mu, geo.lam, c);
 #pragma unroll
@@ -75,7 +75,7 @@ __global__ void __launch_bounds__(kElemThreads) batch_dir_kernel(BatchArgs b) {
       svd_get(csvd, (size_t)a.fv.n_cells, e, sv);
       R lk[3];
       arap_lambdas(sv, lk);
-      sums[0].add(fmax(arap_hess_quad(sv, lk, dF, geo.mu), R(0)));
+      sums[0].add(clamp0(arap_hess_quad(sv, lk, dF, geo.mu)));
     }
   }
   block_reduce<N, FF, R>(sums, red);

@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(kElemThreads, kDirCtasPerSM) solver_dir_kernel
         snh_prepare(G, s);
         SnhDir<R> d;
         snh_dir(s, dF, d);
-        plain[0] += fmax(snh_hess_quad(s, d, geo.mu, geo.lam), R(0));
+        plain[0] += clamp0(snh_hess_quad(s, d, geo.mu, geo.lam));
         R c[5];
         snh_poly(s, d, geo.mu, geo.lam, c);
         c2acc.add(c[0]);
@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(kElemThreads, kDirCtasPerSM) solver_dir_kernel
         svd_get(csvd, (size_t)a.fv.n_cells, e, sv);
         R lk[3];
         arap_lambdas(sv, lk);
-        plain[0] += fmax(arap_hess_quad(sv, lk, dF, geo.mu), R(0));
+        plain[0] += clamp0(arap_hess_quad(sv, lk, dF, geo.mu));
       }
       geo = geon;
       ids = idsn;

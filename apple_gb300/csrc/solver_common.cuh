@@ -847,9 +847,9 @@ __device__ __forceinline__ bool grad_tile(const SolveArgs& a, int tile, const So
         q4.x += f[k][0];
         q4.y += f[k][1];
         q4.z += f[k][2];
-        q4.w += fmax(hd[k][0], R(0));
-        q2.x += fmax(hd[k][1], R(0));
-        q2.y += fmax(hd[k][2], R(0));
+        q4.w += clamp0(hd[k][0]);
+        q2.x += clamp0(hd[k][1]);
+        q2.y += clamp0(hd[k][2]);
         my4[v] = q4;
         my2[v] = q2;
       }
