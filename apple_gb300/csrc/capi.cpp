@@ -759,7 +759,8 @@ int agb_solver_destroy(agb_solver* sv) {
                   (void*)sv->d_slot_of_tv, sv->d_rec, (void*)sv->d_ids, sv->d_xa, sv->d_gd, sv->d_p0,
                   sv->d_p1, sv->d_xref, sv->d_gref, sv->d_svd, sv->d_slots, sv->d_part, (void*)sv->d_cnt,
                   (void*)sv->d_state, sv->d_u_tmp, sv->d_act, sv->d_res_part, (void*)sv->d_res_counters,
-                  (void*)sv->d_off})
+                  (void*)sv->d_piece_estart, (void*)sv->d_piece_vstart, (void*)sv->d_piece_gstart,
+                  (void*)sv->d_piece_vid, (void*)sv->d_piece_slot, (void*)sv->d_piece_off})
     dfree(p);
   if (sv->h_state) cudaFreeHost(sv->h_state);
   delete sv;
@@ -880,33 +881,30 @@ int agb_solver_create(agb_model* m, const agb_pncg_params* params, agb_solver** 
   for (int v = 0; v < np && covered; ++v) covered = m->off[v + 1] > m->off[v];
   const bool small = covered && mat != AGB_ARAP && sv->fv.n_tiles > 0 && sv->fv.n_tiles <= kResidentMaxTiles;
   TilePlan pieces;
-  std::vector<int32_t> off;
+  FemView fv = sv->fv;
   int32_t n_slots = m->n_slots;
   if (!rc && small) {
     split_tiles(m->fems.size() == 1 ? m->fems[0]->plan : sv->plan, kResidentMaxTiles / 2, 2, &pieces);
     std::vector<SlotMap> sm;
+    std::vector<int32_t> off;
     build_slots(np, {&pieces}, &sm, &off);
-    slot_of_tv = sm[0].slot_of_tv;
     n_slots = off[np];
-    for (int32_t** d : {&sv->d_tile_estart, &sv->d_tile_vstart, &sv->d_tile_gstart, &sv->d_tv_vid}) {
-      dfree(*d);
-      *d = nullptr;
-    }
-    rc = dupload(&sv->d_tile_estart, pieces.tile_estart);
-    if (!rc) rc = dupload(&sv->d_tile_vstart, pieces.tile_vstart);
-    if (!rc) rc = dupload(&sv->d_tile_gstart, pieces.tile_gstart);
-    if (!rc) rc = dupload(&sv->d_tv_vid, pieces.tv_vid);
-    if (!rc) rc = dupload(&sv->d_off, off);
-    sv->fv.n_tiles = pieces.n_tiles;
-    sv->fv.tile_estart = sv->d_tile_estart;
-    sv->fv.tile_vstart = sv->d_tile_vstart;
-    sv->fv.tile_gstart = sv->d_tile_gstart;
-    sv->fv.tv_vid = sv->d_tv_vid;
+    rc = dupload(&sv->d_piece_estart, pieces.tile_estart);
+    if (!rc) rc = dupload(&sv->d_piece_vstart, pieces.tile_vstart);
+    if (!rc) rc = dupload(&sv->d_piece_gstart, pieces.tile_gstart);
+    if (!rc) rc = dupload(&sv->d_piece_vid, pieces.tv_vid);
+    if (!rc) rc = dupload(&sv->d_piece_slot, sm[0].slot_of_tv);
+    if (!rc) rc = dupload(&sv->d_piece_off, off);
+    fv.n_tiles = pieces.n_tiles;
+    fv.tile_estart = sv->d_piece_estart;
+    fv.tile_vstart = sv->d_piece_vstart;
+    fv.tile_gstart = sv->d_piece_gstart;
+    fv.tv_vid = sv->d_piece_vid;
   }
   if (!rc) rc = dupload(&sv->d_slot_of_tv, slot_of_tv);
   const size_t v4 = v4_bytes(sv->precision);
   const int vblocks = solver_vertex_blocks(np);
-  const size_t nt = (size_t)sv->fv.n_tiles;
+  const size_t nt = (size_t)fv.n_tiles;
   const size_t gt = (nt + 31) / 32, gv = ((size_t)vblocks + 31) / 32;
   // partials: direction (nt x 6 + gt x 6), gradient (nt), vertex (vb x 12 + gv x 12), trial (nt x 3 + gt x 3)
   const size_t off_ga = nt * 6, off_b = off_ga + gt * 6, off_v = off_b + nt, off_gv = off_v + (size_t)vblocks * 12,
@@ -951,7 +949,7 @@ int agb_solver_create(agb_model* m, const agb_pncg_params* params, agb_solver** 
     return rc;
   }
   SolveArgs& a = sv->args;
-  a.fv = sv->fv;
+  a.fv = fv;
   a.n_points = np;
   a.precision = sv->precision;
   a.xa = sv->d_xa;
@@ -963,8 +961,8 @@ int agb_solver_create(agb_model* m, const agb_pncg_params* params, agb_solver** 
   a.svd = sv->d_svd;
   a.delta = delta ? 1 : 0;
   a.force = m->d_force;
-  a.slot_of_tv = sv->d_slot_of_tv;
-  a.off = small ? sv->d_off : m->d_off;
+  a.slot_of_tv = small ? sv->d_piece_slot : sv->d_slot_of_tv;
+  a.off = small ? sv->d_piece_off : m->d_off;
   a.slots = sv->d_slots;
   a.n_slots = n_slots;
   a.st = sv->d_state;
@@ -985,6 +983,12 @@ int agb_solver_create(agb_model* m, const agb_pncg_params* params, agb_solver** 
   a.cond_outer = 0;
   a.refresh_exits = 0;
   a.guard = 0;
+  // sums over whole tiles do not depend on how the iterations run
+  sv->whole = a;
+  sv->whole.fv = sv->fv;
+  sv->whole.slot_of_tv = sv->d_slot_of_tv;
+  sv->whole.off = m->d_off;
+  sv->whole.n_slots = m->n_slots;
   // resident iterations when every tile's CTA fits the device at once
   if (small) {
     for (int t = 0; t < pieces.n_tiles; ++t) {
@@ -1017,14 +1021,14 @@ static cudaError_t run_resident(agb_solver* sv, const SolveArgs& a, cudaStream_t
 int agb_solver_reset(agb_solver* sv, const void* u, void* stream) {
   AGB_REQUIRE(sv && u, AGB_E_INVALID, "agb_solver_reset: null argument");
   cudaStream_t s = as_stream(stream);
-  RC(check_launch(launch_solver_init(sv->args, u, sv->model->d_fixed,
+  RC(check_launch(launch_solver_init(sv->whole, u, sv->model->d_fixed,
                                      sv->model->space->d_user_of_internal, s),
                   "solver_init"));
-  if (sv->args.delta) {  // x_ref = x_0 and g(x_0) in FP64 before the first gradient pass
-    RC(check_launch(launch_solver_force_refresh(sv->args, s), "solver_refresh"));
-    RC(check_launch(launch_solver_refresh(sv->args, s), "solver_refresh"));
+  if (sv->whole.delta) {  // x_ref = x_0 and g(x_0) in FP64 before the first gradient pass
+    RC(check_launch(launch_solver_force_refresh(sv->whole, s), "solver_refresh"));
+    RC(check_launch(launch_solver_refresh(sv->whole, s), "solver_refresh"));
   }
-  RC(check_launch(launch_solver_first(sv->args, s), "solver_first"));
+  RC(check_launch(launch_solver_first(sv->whole, s), "solver_first"));
   sv->has_state = true;
   return AGB_OK;
 }
@@ -1202,7 +1206,7 @@ int agb_solver_read(agb_solver* sv, void* u_out, agb_pncg_stats* stats, void* st
     RC(check_launch(launch_solver_unpack_x(sv->args, nullptr, sv->model->space->d_user_of_internal,
                                            u_out, s),
                     "unpack_x"));
-  RC(check_launch(launch_solver_energy(sv->args, s), "solver_energy"));
+  RC(check_launch(launch_solver_energy(sv->whole, s), "solver_energy"));
   AGB_CHECK_CUDA(cudaMemcpyAsync(sv->h_state, sv->d_state, sizeof(SolverState),
                                  cudaMemcpyDeviceToHost, s));
   AGB_CHECK_CUDA(cudaStreamSynchronize(s));
@@ -1373,7 +1377,7 @@ int agb_solver_time_passes(agb_solver* sv, int32_t reps, void* flush, size_t flu
     for (int r = 0; r < reps && !rc; ++r) {
       if (flush && flush_bytes && cudaMemsetAsync(flush, r & 0xff, flush_bytes, s) != cudaSuccess) rc = AGB_E_CUDA;
       if (!rc && cudaEventRecord(e0, s) != cudaSuccess) rc = AGB_E_CUDA;
-      if (!rc) rc = check_launch(launch_solver_pass(sv->args, which, s), "time_passes");
+      if (!rc) rc = check_launch(launch_solver_pass(sv->whole, which, s), "time_passes");
       if (!rc && cudaEventRecord(e1, s) != cudaSuccess) rc = AGB_E_CUDA;
       float t = 0.0f;
       if (!rc && (cudaEventSynchronize(e1) != cudaSuccess || cudaEventElapsedTime(&t, e0, e1) != cudaSuccess))
@@ -1431,7 +1435,7 @@ static int cg_setup(agb_solver* sv) {
     return rc;
   }
   CgArgs& c = sv->cg;
-  c.a = sv->args;
+  c.a = sv->whole;
   char* base = (char*)sv->d_cg;
   const size_t vb = v4 * (size_t)np;
   c.lam = base;

@@ -270,7 +270,8 @@ struct agb_solver {
   agb::SolverState* h_state = nullptr;  // pinned
   void* d_act = nullptr;                // several potentials: concatenated activation stream (muscle)
   void* d_u_tmp = nullptr;              // caller-order staging for host I/O
-  agb::SolveArgs args{};
+  agb::SolveArgs args{};   // the iterations' tiles (split ones for resident iterations)
+  agb::SolveArgs whole{};  // the whole tiles: reset, energy, adjoint CG
   // adjoint CG (allocated on first use)
   void* d_cg = nullptr;            // lam, res, q, minv, p0, p1: 6 x V4<R> x n_points
   void* d_cg_part = nullptr;
@@ -288,7 +289,13 @@ struct agb_solver {
   agb::ResidentPlan resident;
   void* d_res_part = nullptr;         // 18 partials per tile
   unsigned* d_res_counters = nullptr;
-  int32_t* d_off = nullptr;           // slot offsets of the split tiles
+  // the split tiles of resident iterations
+  int32_t* d_piece_estart = nullptr;
+  int32_t* d_piece_vstart = nullptr;
+  int32_t* d_piece_gstart = nullptr;
+  int32_t* d_piece_vid = nullptr;
+  int32_t* d_piece_slot = nullptr;
+  int32_t* d_piece_off = nullptr;
   bool has_state = false;  // vertex state written (reset or checkpoint load)
   uint64_t fingerprint = 0;  // of the model and parameters, checked by agb_solver_load
 };

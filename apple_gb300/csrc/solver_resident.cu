@@ -33,7 +33,7 @@
 #include <math.h>
 
 #include "gridsync.cuh"
-#include "kernels.h"
+#include "resident.cuh"
 #include "solver.h"
 #include "solver_common.cuh"
 
@@ -43,24 +43,10 @@ namespace {
 
 constexpr int kStateWords = (int)(sizeof(SolverState) / 4);
 
-// Warps per tile (two CTAs per SM): 8 in FP32; FP64 is bound by its
-// arithmetic pipe, which 8 warps per SM fill: 4.  Meshes with fewer tiles
-// than CTAs are cut finer first (split_tiles in prep.cpp): a whole tile's
-// groups are issue-bound on one SM while others idle.  Above two tiles
-// per SM the three-kernel iteration is the faster one: with four 4-warp CTAs
-// per SM this kernel took 2.46 against 2.23 ms on 245,760 tets (376 tiles) and
-// 2.88 against 2.55 ms on 400,000 (592 tiles), for 40 iterations and the reset.
-template <class R>
-constexpr int kResidentWarps = sizeof(R) == 4 ? 8 : 4;
-
 // per-vertex words kept between iterations: x hi, x lo, p, previous g, mask,
 // and with the reference-state correction x_ref
 template <bool DELTA>
 constexpr int kVertexWords = DELTA ? 16 : 13;
-
-// records kept in shared memory (FP32): their float4 streams
-template <int MAT>
-constexpr int kRecStreams = MAT == AGB_STABLE_NEO_HOOKEAN_MUSCLE ? 5 : 3;
 
 // the accumulators' space also takes the block sums' rows (13 per thread)
 template <class R, bool DELTA>
@@ -69,23 +55,8 @@ constexpr size_t resident_smem(int nw) {
          ((size_t)(nw + 1) * (sizeof(V4<R>) + sizeof(V2<R>)) + kVertexWords<DELTA> * sizeof(R) + 4 * sizeof(int));
 }
 
-template <class R>
-__device__ __forceinline__ V4<R> ldcg4(const V4<R>* p);
-template <>
-__device__ __forceinline__ V4<float> ldcg4<float>(const V4<float>* p) {
-  const float4 v = __ldcg(reinterpret_cast<const float4*>(p));
-  return V4<float>{v.x, v.y, v.z, v.w};
-}
-template <>
-__device__ __forceinline__ V4<double> ldcg4<double>(const V4<double>* p) {
-  const double2 a = __ldcg(reinterpret_cast<const double2*>(p));
-  const double2 b = __ldcg(reinterpret_cast<const double2*>(p) + 1);
-  return V4<double>{a.x, a.y, b.x, b.y};
-}
-
-// REC: the tile's element records stay in shared memory after the first read
-// (a barrier's acquire leaves nothing in L1, so every pass would fetch them
-// from L2); otherwise each group's records are loaded one group ahead.
+// REC: the tile's element records stay in shared memory after the first read;
+// otherwise each group's records are loaded one group ahead.
 template <class R, int MAT, bool DELTA, int NW, bool REC>
 __global__ void __launch_bounds__(32 * NW, 2) solver_resident_kernel(SolveArgs a, int max_elems, int whole,
                                                                                      void* part_d, void* part_v,
@@ -103,7 +74,6 @@ __global__ void __launch_bounds__(32 * NW, 2) solver_resident_kernel(SolveArgs a
   int* sgrp = reinterpret_cast<int*>(srec + (size_t)kRecStreams<MAT> * max_elems);  // REC: group starts
   R* const rows = reinterpret_cast<R*>(acc4);  // the block sums' terms, while no accumulation runs
   static_assert(NW * kTileVerts * sizeof(V4<R>) >= (NVT + 1) * T * sizeof(R), "rows fit the accumulators");
-  static_assert(kResidentCounters == 2 + kPlaceWords, "barrier and placement");
   __shared__ Acc<R> tot[NVT];
   __shared__ SolverState sst;
   R* const xh = vw;
@@ -156,46 +126,8 @@ __global__ void __launch_bounds__(32 * NW, 2) solver_resident_kernel(SolveArgs a
       }
     }
   }
-  const int e_first = a.fv.tile_estart[tile];
-  if constexpr (REC) {
-    const int ne = a.fv.tile_estart[tile + 1] - e_first;
-    const float4* rec = static_cast<const float4*>(a.fv.rec);
-    const float4* act = static_cast<const float4*>(a.fv.act);
-    const size_t nc = (size_t)a.fv.n_cells;
-    for (int i = tid; i < ne; i += T) {
-#pragma unroll
-      for (int k = 0; k < 3; ++k) srec[(size_t)k * max_elems + i] = __ldg(rec + k * nc + e_first + i);
-#pragma unroll
-      for (int k = 3; k < kRecStreams<MAT>; ++k) srec[(size_t)k * max_elems + i] = __ldg(act + (k - 3) * nc + e_first + i);
-    }
-    for (int i = tid; i <= ge - gs; i += T) sgrp[i] = a.fv.group_estart[gs + i] - e_first;
-  }
-  // the record of lane `lane` in group q; its size into n
-  auto load_group = [&](int q, int& n, ElemGeo<R>& geo, uint32_t& ids) {
-    if constexpr (REC) {
-      const int e0 = sgrp[q - gs];
-      n = sgrp[q - gs + 1] - e0;
-      if (lane < n) {
-        const float4* r = srec + e0 + lane;
-        const float4 A = r[0], B = r[max_elems], C = r[2 * max_elems];
-        geo.D[0][0] = A.x; geo.D[0][1] = A.y; geo.D[0][2] = A.z;
-        geo.D[1][0] = A.w; geo.D[1][1] = B.x; geo.D[1][2] = B.y;
-        geo.D[2][0] = B.z; geo.D[2][1] = B.w; geo.D[2][2] = C.x;
-        geo.mu = C.y;
-        geo.lam = C.z;
-        ids = __float_as_uint(C.w);
-        if constexpr (kRecStreams<MAT> == 5) {
-          const float4 s0 = r[3 * max_elems], s1 = r[4 * max_elems];
-          geo.S[0] = s0.x; geo.S[1] = s0.y; geo.S[2] = s0.z;
-          geo.S[3] = s0.w; geo.S[4] = s1.x; geo.S[5] = s1.y;
-        }
-      }
-    } else {
-      const int e0 = a.fv.group_estart[q];
-      n = a.fv.group_estart[q + 1] - e0;
-      if (lane < n) load_elem_m<R, MAT>(a.fv, e0 + lane, geo, ids);
-    }
-  };
+  if constexpr (REC) keep_records<MAT>(a.fv, tile, max_elems, srec, sgrp);
+  const GroupLoader<R, MAT, REC> load_group{a.fv, gs, max_elems, srec, sgrp};
   // The accumulators are cleared while a barrier is waited for: those that
   // the block sums' rows overlay after the direction pass, the others after
   // the vertex pass.
@@ -213,14 +145,7 @@ __global__ void __launch_bounds__(32 * NW, 2) solver_resident_kernel(SolveArgs a
   __syncthreads();  // every thread has read sst.pbuf; records and groups are in place
   if (tid == 0) sst.refresh = 0;  // the refresh passes, if any, ran after the last vertex pass
 
-  // the scheduler whose FP64 pipe takes the decisions: the second CTA of an SM
-  // uses another one
-  unsigned warp_slot;
-  asm volatile("mov.u32 %0, %%warpid;" : "=r"(warp_slot));
-  __shared__ int s_w0;
-  if (tid == 0) s_w0 = (warp_slot / NW) & 1u ? 1 : 0;
-  __syncthreads();
-  const int w0 = s_w0;
+  const int w0 = decision_warp<NW>();
 
   bool ok = true;
   for (;;) {
@@ -270,7 +195,7 @@ __global__ void __launch_bounds__(32 * NW, 2) solver_resident_kernel(SolveArgs a
           snh_prepare(G, s);
           SnhDir<R> d;
           snh_dir(s, dF, d);
-          plain[0] += fmax(snh_hess_quad(s, d, geo.mu, geo.lam), R(0));
+          plain[0] += clamp0(snh_hess_quad(s, d, geo.mu, geo.lam));
           R c[5];
           snh_poly(s, d, geo.mu, geo.lam, c);
           c2acc.add(c[0]);
@@ -373,9 +298,9 @@ __global__ void __launch_bounds__(32 * NW, 2) solver_resident_kernel(SolveArgs a
             q4.x += f[k][0];
             q4.y += f[k][1];
             q4.z += f[k][2];
-            q4.w += fmax(hd[k][0], R(0));
-            q2.x += fmax(hd[k][1], R(0));
-            q2.y += fmax(hd[k][2], R(0));
+            q4.w += clamp0(hd[k][0]);
+            q2.x += clamp0(hd[k][1]);
+            q2.y += clamp0(hd[k][2]);
             my4[v] = q4;
             my2[v] = q2;
           }
@@ -410,6 +335,7 @@ __global__ void __launch_bounds__(32 * NW, 2) solver_resident_kernel(SolveArgs a
     }
     bar.arrive();
     if (!(ok = bar.wait())) break;
+
     // ---- vertex ----
     {
       R s[NVT] = {};
@@ -491,7 +417,7 @@ struct Shape {
 template <class R, int MAT, bool DELTA, int NW, bool REC>
 Shape shape(const ResidentPlan& p) {
   size_t smem = resident_smem<R, DELTA>(NW);
-  if (REC) smem += (size_t)p.max_elems * kRecStreams<MAT> * sizeof(float4) + ((size_t)p.max_groups + 1) * sizeof(int);
+  if (REC) smem += records_bytes<MAT>(p);
   return Shape{solver_resident_kernel<R, MAT, DELTA, NW, REC>, 32 * NW, smem};
 }
 
@@ -513,51 +439,22 @@ Shape shape_of(const SolveArgs& a, const ResidentPlan& p) {
 
 }  // namespace
 
-// The first shape whose CTAs, one per tile, fit the device at once: in FP32
-// with the records in shared memory, or without (tiles with too many
-// elements for two CTAs per SM).
+// Above two tiles per SM the three-kernel iteration is the faster one: with
+// four 4-warp CTAs per SM this kernel took 2.46 against 2.23 ms on 245,760 tets
+// (376 tiles) and 2.88 against 2.55 ms on 400,000 (592 tiles), for 40
+// iterations and the reset.
 cudaError_t resident_prepare(const SolveArgs& a, ResidentPlan* p) {
   p->shape = 0;
-  if (!snh_family(a.fv.material) || a.fv.n_tiles == 0 || a.fv.n_tiles > kResidentMaxTiles) return cudaSuccess;
-  int dev = 0, sms = 0, coop = 0, limit = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
-  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-  if (e != cudaSuccess || !coop) return e;
-  const int shapes = a.precision == AGB_F64 ? 1 : 2;
-  for (int k = 1; k <= shapes; ++k) {
-    ResidentPlan q = *p;
-    q.shape = k;
-    const Shape sh = shape_of(a, q);
-    if (sh.smem + 8 * 1024 > (size_t)limit) continue;  // beside the kernel's static arrays
-    int occ = 0;
-    e = allow_max_smem(sh.kernel);
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, sh.kernel, sh.threads, sh.smem);
-    if (e != cudaSuccess) return e;
-    if ((int64_t)a.fv.n_tiles <= (int64_t)occ * sms) {
-      p->shape = k;
-      return cudaSuccess;
-    }
-  }
-  return cudaSuccess;
+  if (!snh_family(a.fv.material)) return cudaSuccess;
+  return choose_shape(a, p, [&](const ResidentPlan& q) { return shape_of(a, q); });
 }
 
 cudaError_t launch_resident(const SolveArgs& a, const ResidentPlan& p, void* part_d, void* part_v, unsigned* counters,
                             cudaStream_t s) {
   if (!p.shape) return cudaErrorInvalidValue;
   const Shape sh = shape_of(a, p);
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(a.fv.n_tiles);
-  cfg.blockDim = dim3(sh.threads);
-  cfg.dynamicSmemBytes = sh.smem;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeCooperative;
-  attr[0].val.cooperative = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, sh.kernel, a, p.max_elems, p.whole, part_d, part_v, counters);
+  return launch_cooperative(sh.kernel, a.fv.n_tiles, sh.threads, sh.smem, s, a, p.max_elems, p.whole, part_d, part_v,
+                            counters);
 }
 
 }  // namespace agb
