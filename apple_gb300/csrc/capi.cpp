@@ -750,7 +750,9 @@ int agb_solver_destroy(agb_solver* sv) {
   if (!sv) return AGB_OK;
   if (sv->loop_exec) cudaGraphExecDestroy(sv->loop_exec);
   if (sv->cg_exec) cudaGraphExecDestroy(sv->cg_exec);
-  for (void* p : {sv->d_cg, sv->d_cg_part, (void*)sv->d_cg_cnt, (void*)sv->d_cg_state}) dfree(p);
+  for (void* p : {sv->d_cg, sv->d_cg_part, (void*)sv->d_cg_cnt, (void*)sv->d_cg_state, sv->d_cg_res_part,
+                  (void*)sv->d_cg_res_counters})
+    dfree(p);
   if (sv->h_cg_state) cudaFreeHost(sv->h_cg_state);
   if (sv->step_exec) cudaGraphExecDestroy(sv->step_exec);
   if (sv->capture_stream) cudaStreamDestroy(sv->capture_stream);
@@ -770,6 +772,14 @@ int agb_solver_destroy(agb_solver* sv) {
 // ARAP: both per-element SVD caches, 3 V4 per cell each
 static size_t svd_cache_bytes(const agb_solver* sv) {
   return 2 * 3 * v4_bytes(sv->precision) * (size_t)sv->fv.n_cells;
+}
+
+// the most elements and warp groups of one tile
+static void largest_tile(const TilePlan& P, ResidentPlan* p) {
+  for (int t = 0; t < P.n_tiles; ++t) {
+    p->max_elems = std::max(p->max_elems, P.tile_estart[t + 1] - P.tile_estart[t]);
+    p->max_groups = std::max(p->max_groups, P.tile_gstart[t + 1] - P.tile_gstart[t]);
+  }
 }
 
 int agb_solver_create(agb_model* m, const agb_pncg_params* params, agb_solver** out) {
@@ -991,10 +1001,7 @@ int agb_solver_create(agb_model* m, const agb_pncg_params* params, agb_solver** 
   sv->whole.n_slots = m->n_slots;
   // resident iterations when every tile's CTA fits the device at once
   if (small) {
-    for (int t = 0; t < pieces.n_tiles; ++t) {
-      sv->resident.max_elems = std::max(sv->resident.max_elems, pieces.tile_estart[t + 1] - pieces.tile_estart[t]);
-      sv->resident.max_groups = std::max(sv->resident.max_groups, pieces.tile_gstart[t + 1] - pieces.tile_gstart[t]);
-    }
+    largest_tile(pieces, &sv->resident);
     const int n_whole = m->fems.size() == 1 ? m->fems[0]->plan.n_tiles : sv->plan.n_tiles;
     sv->resident.whole = n_whole > kResidentMaxTiles / 2 ? kResidentMaxTiles / 2 : 0;
     rc = check_launch(resident_prepare(a, &sv->resident), "resident_prepare");
@@ -1430,6 +1437,16 @@ static int cg_setup(agb_solver* sv) {
   if (!rc) rc = dalloc(&sv->d_cg_state, 1);
   if (!rc && cudaMallocHost((void**)&sv->h_cg_state, sizeof(CgState)) != cudaSuccess) rc = AGB_E_CUDA;
   if (!rc && cg_prepare_kernels(sv->precision) != cudaSuccess) rc = AGB_E_CUDA;
+  if (!rc) {
+    largest_tile(sv->model->fems.size() == 1 ? sv->model->fems[0]->plan : sv->plan, &sv->cg_resident);
+    rc = check_launch(cg_resident_prepare(sv->whole, &sv->cg_resident), "cg_resident_prepare");
+  }
+  if (!rc && sv->cg_resident.shape) {
+    rc = dalloc_bytes(&sv->d_cg_res_part, 8 * 3 * (size_t)sv->fv.n_tiles);
+    if (!rc) rc = dalloc(&sv->d_cg_res_counters, kResidentCounters);
+    if (!rc && cudaMemset(sv->d_cg_res_counters, 0, kResidentCounters * sizeof(unsigned)) != cudaSuccess)
+      rc = AGB_E_CUDA;
+  }
   if (rc) {
     if (rc == AGB_E_CUDA && agb::last_error()[0] == 0) set_error("agb_solver_adjoint: CUDA allocation failed");
     return rc;
@@ -1497,7 +1514,8 @@ int agb_solver_adjoint(agb_solver* sv, const void* rhs, void* lam, const agb_cg_
   AGB_REQUIRE(prm.max_iter >= 0 && prm.rtol >= 0.0 && prm.atol >= 0.0, AGB_E_INVALID,
               "agb_solver_adjoint: bad parameters");
   RC(cg_setup(sv));
-  if (!sv->cg_exec) RC(build_cg_graph(sv));
+  const bool resident = sv->cg_resident.shape != 0;
+  if (!resident && !sv->cg_exec) RC(build_cg_graph(sv));
   cudaStream_t s = as_stream(stream);
   CgState init{};
   init.rtol = prm.rtol;
@@ -1510,12 +1528,19 @@ int agb_solver_adjoint(agb_solver* sv, const void* rhs, void* lam, const agb_cg_
   RC(check_launch(launch_cg_init(sv->cg, rhs, uoi, s), "cg_init"));
   if (prm.max_iter > 0) {
     RC(check_launch(launch_cg_set_limit(sv->cg, prm.max_iter, s), "cg_set_limit"));
-    AGB_CHECK_CUDA(cudaGraphLaunch(sv->cg_exec, s));
+    if (resident)
+      RC(check_launch(launch_cg_resident(sv->cg, sv->cg_resident, sv->d_cg_res_part,
+                                         (char*)sv->d_cg_res_part + 8 * (size_t)sv->fv.n_tiles, sv->d_cg_res_counters,
+                                         s),
+                      "resident CG"));
+    else
+      AGB_CHECK_CUDA(cudaGraphLaunch(sv->cg_exec, s));
   }
   RC(check_launch(launch_cg_unpack(sv->cg, uoi, lam, s), "cg_unpack"));
   AGB_CHECK_CUDA(cudaMemcpyAsync(sv->h_cg_state, sv->d_cg_state, sizeof(CgState), cudaMemcpyDeviceToHost, s));
   AGB_CHECK_CUDA(cudaStreamSynchronize(s));
   const CgState& cs = *sv->h_cg_state;
+  AGB_REQUIRE(cs.result != AGB_E_DEVICE, AGB_E_DEVICE, "adjoint CG: a grid barrier gave up");
   if (stats) {
     stats->result = cs.done ? cs.result : AGB_MAX_STEPS_REACHED;
     stats->n_iter = cs.iter;
