@@ -87,6 +87,10 @@ _SIGNATURES = {
         c_int,
         [c_void_p, c_uint, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p],
     ),
+    "agb_fem_eval_store": (
+        c_int,
+        [c_void_p, c_uint, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p],
+    ),
     "agb_model_create": (
         c_int,
         [c_void_p, c_int, c_int32, c_void_p, c_void_p, c_void_p, c_int32, c_void_p, c_void_p, POINTER(c_void_p)],
@@ -95,6 +99,10 @@ _SIGNATURES = {
     "agb_model_eval": (
         c_int,
         [c_void_p, c_uint, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p],
+    ),
+    "agb_model_eval_free": (
+        c_int,
+        [c_void_p, c_uint, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p],
     ),
     "agb_dof_to_free": (c_int, [c_int32, ctypes.c_int64, c_void_p, c_void_p, c_void_p, c_void_p]),
     "agb_dof_to_full": (c_int, [c_int32, ctypes.c_int64, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p]),
@@ -161,4 +169,6 @@ def check(rc: int) -> None:
 
 
 def call(name: str, *args) -> None:
-    check(getattr(load(), name)(*args))
+    rc = getattr(_lib if _lib is not None else load(), name)(*args)
+    if rc != OK:
+        check(rc)

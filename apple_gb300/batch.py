@@ -60,7 +60,8 @@ class BatchedForward:
         return npt.value, nc.value
 
     def initial_u(self, device="cuda") -> torch.Tensor:
-        parts = [m.init().u.to(device) for m in self.models]
+        # Model.init() of each: the fixed values, zero elsewhere
+        parts = [m.dof_map._fill_for(m.dtype).reshape(-1, 3).to(device) for m in self.models]
         return torch.cat(parts, 0).contiguous()
 
     def reset(self, u: torch.Tensor | None = None) -> None:

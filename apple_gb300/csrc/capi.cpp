@@ -525,8 +525,8 @@ int agb_fem_cells(const agb_fem* f, int32_t* cells_out, uint32_t* tile_color_has
   return AGB_OK;
 }
 
-int agb_fem_eval(agb_fem* f, unsigned flags, const void* u, const void* p, double* energy,
-                 void* grad, void* diag, void* prod, double* quad, void* stream) {
+static int fem_eval(agb_fem* f, unsigned flags, const void* u, const void* p, double* energy, void* grad, void* diag,
+                    void* prod, double* quad, int assign, void* stream) {
   AGB_REQUIRE(f && u, AGB_E_INVALID, "agb_fem_eval: null handle or u");
   AGB_REQUIRE(!(flags & ~31u), AGB_E_INVALID, "agb_fem_eval: unknown flags %u", flags);
   AGB_REQUIRE(!(flags & AGB_FUN) || energy, AGB_E_INVALID, "agb_fem_eval: energy output is null");
@@ -539,16 +539,30 @@ int agb_fem_eval(agb_fem* f, unsigned flags, const void* u, const void* p, doubl
   if (!flags) return AGB_OK;
   cudaStream_t s = as_stream(stream);
   const int np = f->space->n_points;
-  RC(check_launch(launch_fem_eval(f->precision, f->view(), flags, u, p, f->d_own_slot, f->d_slots, f->plan.n_tv,
-                                  f->d_partials, f->d_counter, energy, quad, 0, s),
+  if (assign && f->plan.n_tiles == 0) {  // no element pass stores the scalars
+    if (flags & AGB_FUN) AGB_CHECK_CUDA(cudaMemsetAsync(energy, 0, sizeof(double), s));
+    if (flags & AGB_HESS_QUAD) AGB_CHECK_CUDA(cudaMemsetAsync(quad, 0, sizeof(double), s));
+  }
+  RC(check_launch(launch_fem_eval(f->precision, f->view(), flags, u, p, nullptr, f->d_own_slot, f->d_slots,
+                                  f->plan.n_tv, f->d_partials, f->d_counter, energy, quad, assign, s),
                   "fem_eval"));
   const unsigned vec = flags & (AGB_GRAD | AGB_HESS_DIAG | AGB_HESS_PROD);
   if (vec)
     RC(check_launch(launch_unpack(f->precision, np, f->space->d_user_of_internal, f->d_own_off, f->d_slots,
-                                  f->plan.n_tv, vec, grad, diag, prod, 0, nullptr, u, f->d_partials, f->d_counter,
+                                  f->plan.n_tv, vec, grad, diag, prod, nullptr, assign, nullptr, u, f->d_partials, f->d_counter,
                                   nullptr, s),
                     "unpack"));
   return AGB_OK;
+}
+
+int agb_fem_eval(agb_fem* f, unsigned flags, const void* u, const void* p, double* energy,
+                 void* grad, void* diag, void* prod, double* quad, void* stream) {
+  return fem_eval(f, flags, u, p, energy, grad, diag, prod, quad, 0, stream);
+}
+
+int agb_fem_eval_store(agb_fem* f, unsigned flags, const void* u, const void* p, double* energy,
+                       void* grad, void* diag, void* prod, double* quad, void* stream) {
+  return fem_eval(f, flags, u, p, energy, grad, diag, prod, quad, 1, stream);
 }
 
 int agb_fem_fun(agb_fem* f, const void* u, double* out, void* s) {
@@ -693,8 +707,8 @@ int agb_dof_to_full(int32_t precision, int64_t n_full, const int32_t* slot, cons
                       "dof_to_full");
 }
 
-int agb_model_eval(agb_model* m, unsigned flags, const void* u, const void* p, double* energy,
-                   void* grad, void* diag, void* prod, double* quad, void* stream) {
+static int model_eval(agb_model* m, unsigned flags, const int32_t* slot, const void* u, const void* p, double* energy,
+                      void* grad, void* diag, void* prod, double* quad, void* stream) {
   AGB_REQUIRE(m && u, AGB_E_INVALID, "agb_model_eval: null handle or u");
   AGB_REQUIRE(!(flags & ~31u), AGB_E_INVALID, "agb_model_eval: unknown flags %u", flags);
   const bool need_p = flags & (AGB_HESS_PROD | AGB_HESS_QUAD);
@@ -717,7 +731,7 @@ int agb_model_eval(agb_model* m, unsigned flags, const void* u, const void* p, d
   if (!flags) return AGB_OK;
   int assign = 1;
   for (size_t k = 0; k < m->fems.size(); ++k) {
-    RC(check_launch(launch_fem_eval(m->precision, m->fems[k]->view(), flags, u, p, m->d_slot_of_tv[k], m->d_slots,
+    RC(check_launch(launch_fem_eval(m->precision, m->fems[k]->view(), flags, u, p, slot, m->d_slot_of_tv[k], m->d_slots,
                                     m->n_slots, m->d_partials, m->d_counter, energy, quad, assign, s),
                     "fem_eval"));
     if (m->fems[k]->plan.n_tiles > 0) assign = 0;
@@ -726,9 +740,20 @@ int agb_model_eval(agb_model* m, unsigned flags, const void* u, const void* p, d
   const bool ext = m->d_force != nullptr;
   if ((vec & ~AGB_FUN) || (ext && (flags & AGB_FUN)))
     RC(check_launch(launch_unpack(m->precision, np, m->space->d_user_of_internal, m->d_off, m->d_slots, m->n_slots,
-                                  vec, grad, diag, prod, 1, m->d_force, u, m->d_partials, m->d_counter, energy, s),
+                                  vec, grad, diag, prod, slot, 1, m->d_force, u, m->d_partials, m->d_counter, energy, s),
                     "unpack"));
   return AGB_OK;
+}
+
+int agb_model_eval(agb_model* m, unsigned flags, const void* u, const void* p, double* energy,
+                   void* grad, void* diag, void* prod, double* quad, void* stream) {
+  return model_eval(m, flags, nullptr, u, p, energy, grad, diag, prod, quad, stream);
+}
+
+int agb_model_eval_free(agb_model* m, unsigned flags, const int32_t* slot, const void* u, const void* p_free,
+                        double* energy, void* grad, void* diag, void* prod, double* quad, void* stream) {
+  AGB_REQUIRE(slot, AGB_E_INVALID, "agb_model_eval_free: slot is null");
+  return model_eval(m, flags, slot, u, p_free, energy, grad, diag, prod, quad, stream);
 }
 
 // ---------------------------------------------------------------------------

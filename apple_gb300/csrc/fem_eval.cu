@@ -102,7 +102,7 @@ constexpr size_t eval_smem_bytes(int warps) {
 template <class R, int MAT, int NVEC, int MAXT>
 __global__ void __launch_bounds__(MAXT, MAXT == 128 ? (sizeof(R) == 4 ? 5 : 2) : 1) fem_eval_kernel(
     FemView fv, unsigned flags, const R* __restrict__ u, const R* __restrict__ p,
-    const int32_t* __restrict__ slot_of_tv, void* __restrict__ slots, int n_slots, AccStore<R>* __restrict__ partials,
+    const int32_t* __restrict__ p_slot, const int32_t* __restrict__ slot_of_tv, void* __restrict__ slots, int n_slots, AccStore<R>* __restrict__ partials,
     unsigned* counter, double* energy, double* quad, int assign) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   V4<R>* sx = reinterpret_cast<V4<R>*>(smem_raw);
@@ -132,8 +132,14 @@ __global__ void __launch_bounds__(MAXT, MAXT == 128 ? (sizeof(R) == 4 ? 5 : 2) :
     const size_t k = 3 * (size_t)fv.tv_user[vs + i];
     V4<R> a{u[k], u[k + 1], u[k + 2], R(0)};
     if (need_p) {
-      a.w = p[k];
-      sq[i] = V2<R>{p[k + 1], p[k + 2]};
+      if (p_slot) {  // p over the free components
+        const int32_t s0 = p_slot[k], s1 = p_slot[k + 1], s2 = p_slot[k + 2];
+        a.w = s0 >= 0 ? p[s0] : R(0);
+        sq[i] = V2<R>{s1 >= 0 ? p[s1] : R(0), s2 >= 0 ? p[s2] : R(0)};
+      } else {
+        a.w = p[k];
+        sq[i] = V2<R>{p[k + 1], p[k + 2]};
+      }
     }
     sx[i] = a;
   }
@@ -301,7 +307,7 @@ constexpr int kUnpackThreads = 256;
 template <class R, int NVEC>
 __global__ void __launch_bounds__(kUnpackThreads) unpack_kernel(
     int n, const int32_t* __restrict__ uoi, const int32_t* __restrict__ off, const void* __restrict__ slots,
-    int n_slots, R* o0, R* o1, R* o2, int assign, int force_grad, int force_fun, const V4<R>* __restrict__ force,
+    int n_slots, R* o0, R* o1, R* o2, const int32_t* __restrict__ out_slot, int assign, int force_grad, int force_fun, const V4<R>* __restrict__ force,
     const R* __restrict__ u, AccStore<R>* partials, unsigned* counter, double* energy) {
   __shared__ Acc<R> red[kUnpackThreads / 32];
   const VecArrays<R, NVEC> in{(unsigned char*)slots, (size_t)n_slots};
@@ -334,10 +340,18 @@ __global__ void __launch_bounds__(kUnpackThreads) unpack_kernel(
         x[2] -= f.z;
       }
       R* const outs[3] = {o0, o1, o2};
+      int64_t at[3] = {(int64_t)k, (int64_t)k + 1, (int64_t)k + 2};
+      if (out_slot) {  // outputs over the free components
 #pragma unroll
-      for (int q = 0; q < NVEC; ++q)
+        for (int c = 0; c < 3; ++c) at[c] = out_slot[k + c];
+      }
 #pragma unroll
-        for (int c = 0; c < 3; ++c) outs[q][k + c] = assign ? x[3 * q + c] : outs[q][k + c] + x[3 * q + c];
+      for (int c = 0; c < 3; ++c) {
+        if (at[c] < 0) continue;
+#pragma unroll
+        for (int q = 0; q < NVEC; ++q)
+          outs[q][at[c]] = assign ? x[3 * q + c] : outs[q][at[c]] + x[3 * q + c];
+      }
     }
     if (force_fun) ext[0].add(-(f.x * u[k] + f.y * u[k + 1] + f.z * u[k + 2]));
     i += gridDim.x * blockDim.x;
@@ -371,7 +385,7 @@ int eval_warps(int precision, int n_tiles) {
 
 template <class R, int MAT, int NVEC, int MAXT>
 cudaError_t eval_launch(const FemView& fv, int warps, unsigned flags, const void* u, const void* p,
-                        const int32_t* slot_of_tv, void* slots, int32_t n_slots, void* partials, unsigned* counter,
+                        const int32_t* p_slot, const int32_t* slot_of_tv, void* slots, int32_t n_slots, void* partials, unsigned* counter,
                         double* energy, double* quad, int assign, cudaStream_t s) {
   const bool vectors = flags & (AGB_GRAD | AGB_HESS_DIAG | AGB_HESS_PROD);
   const size_t smem = vectors ? eval_smem_bytes<R, NVEC>(warps) : eval_stage_bytes<R>();
@@ -380,8 +394,8 @@ cudaError_t eval_launch(const FemView& fv, int warps, unsigned flags, const void
     if (e != cudaSuccess) return e;
   }
   fem_eval_kernel<R, MAT, NVEC, MAXT><<<fv.n_tiles, 32 * warps, smem, s>>>(
-      fv, flags, (const R*)u, (const R*)p, slot_of_tv, slots, n_slots, (AccStore<R>*)partials, counter, energy, quad,
-      assign);
+      fv, flags, (const R*)u, (const R*)p, p_slot, slot_of_tv, slots, n_slots, (AccStore<R>*)partials, counter, energy,
+      quad, assign);
   return cudaGetLastError();
 }
 
@@ -411,8 +425,9 @@ cudaError_t eval_material(int nvec, const FemView& fv, A... args) {
 
 template <class R, int NVEC>
 cudaError_t unpack_launch(int n, const int32_t* uoi, const int32_t* off, const void* slots, int32_t n_slots,
-                          unsigned flags, void* grad, void* diag, void* prod, int assign, const void* force,
-                          const void* u, void* partials, unsigned* counter, double* energy, cudaStream_t s) {
+                          unsigned flags, void* grad, void* diag, void* prod, const int32_t* out_slot, int assign,
+                          const void* force, const void* u, void* partials, unsigned* counter, double* energy,
+                          cudaStream_t s) {
   R* outs[3] = {nullptr, nullptr, nullptr};
   int k = 0;
   if (flags & AGB_GRAD) outs[k++] = (R*)grad;
@@ -420,7 +435,7 @@ cudaError_t unpack_launch(int n, const int32_t* uoi, const int32_t* off, const v
   if (flags & AGB_HESS_PROD) outs[k++] = (R*)prod;
   const int force_grad = force && (flags & AGB_GRAD) ? 1 : 0, force_fun = force && (flags & AGB_FUN) ? 1 : 0;
   return launch_pdl(unpack_kernel<R, NVEC>, dim3(unpack_blocks(n)), dim3(kUnpackThreads), 0, s, n, uoi, off, slots,
-                    n_slots, outs[0], outs[1], outs[2], assign, force_grad, force_fun, (const V4<R>*)force,
+                    n_slots, outs[0], outs[1], outs[2], out_slot, assign, force_grad, force_fun, (const V4<R>*)force,
                     (const R*)u, (AccStore<R>*)partials, counter, energy);
 }
 
@@ -442,27 +457,27 @@ int unpack_blocks(int n_points) {
 }
 
 cudaError_t launch_fem_eval(int precision, const FemView& fv, unsigned flags, const void* u, const void* p,
-                            const int32_t* slot_of_tv, void* slots, int32_t n_slots, void* partials,
+                            const int32_t* p_slot, const int32_t* slot_of_tv, void* slots, int32_t n_slots, void* partials,
                             unsigned* counter, double* energy, double* quad, int assign, cudaStream_t stream) {
   if (fv.n_tiles == 0) return cudaSuccess;
   const int nvec = popcount3(vec_mask(flags)), warps = eval_warps(precision, fv.n_tiles);
   if (precision == AGB_F64)
-    return eval_material<double>(nvec, fv, warps, flags, u, p, slot_of_tv, slots, n_slots, partials, counter, energy,
+    return eval_material<double>(nvec, fv, warps, flags, u, p, p_slot, slot_of_tv, slots, n_slots, partials, counter, energy,
                                  quad, assign, stream);
-  return eval_material<float>(nvec, fv, warps, flags, u, p, slot_of_tv, slots, n_slots, partials, counter, energy,
+  return eval_material<float>(nvec, fv, warps, flags, u, p, p_slot, slot_of_tv, slots, n_slots, partials, counter, energy,
                               quad, assign, stream);
 }
 
 cudaError_t launch_unpack(int precision, int n, const int32_t* uoi, const int32_t* off, const void* slots,
-                          int32_t n_slots, unsigned flags, void* grad, void* diag, void* prod, int assign,
-                          const void* force, const void* u, void* partials, unsigned* counter, double* energy,
+                          int32_t n_slots, unsigned flags, void* grad, void* diag, void* prod,
+                          const int32_t* out_slot, int assign, const void* force, const void* u, void* partials, unsigned* counter, double* energy,
                           cudaStream_t stream) {
   if (n <= 0) return cudaSuccess;
   const int nvec = popcount3(vec_mask(flags));
   if (precision == AGB_F64)
-    return unpack_vectors<double>(nvec, n, uoi, off, slots, n_slots, flags, grad, diag, prod, assign, force, u,
+    return unpack_vectors<double>(nvec, n, uoi, off, slots, n_slots, flags, grad, diag, prod, out_slot, assign, force, u,
                                   partials, counter, energy, stream);
-  return unpack_vectors<float>(nvec, n, uoi, off, slots, n_slots, flags, grad, diag, prod, assign, force, u, partials,
+  return unpack_vectors<float>(nvec, n, uoi, off, slots, n_slots, flags, grad, diag, prod, out_slot, assign, force, u, partials,
                                counter, energy, stream);
 }
 

@@ -39,11 +39,14 @@ def dtype_code(dtype: torch.dtype) -> int:
 
 
 def stream_ptr(device=None) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    # the handle of torch.cuda.current_stream(device) without building the
+    # stream object (2 us a call)
+    index = None if device is None else device.index
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
 
 
-def ptr(t: torch.Tensor | None):
-    return None if t is None else ctypes.c_void_p(t.data_ptr())
+def ptr(t: torch.Tensor | None) -> int | None:
+    return None if t is None else t.data_ptr()
 
 
 def check_vec(t: torch.Tensor, n_points: int, dtype: torch.dtype, name: str) -> torch.Tensor:
@@ -267,8 +270,7 @@ class WarpPotentialFem(WarpPotential):
         check_vec(u, self.n_points, self.dtype, "u")
         w = check_vec(w.to(self.dtype), self.n_points, self.dtype, "w")
         n = self.cells.shape[0]
-        dmu = torch.zeros(n, dtype=self.dtype, device=u.device)
-        dlam = torch.zeros(n, dtype=self.dtype, device=u.device)
+        dmu, dlam = torch.zeros((2, n), dtype=self.dtype, device=u.device)
         _lib.call("agb_fem_grad_param_vjp", self._standalone(), ptr(u), ptr(w), ptr(dmu), ptr(dlam),
                   stream_ptr(u.device))
         out = {"mu": dmu}
@@ -287,8 +289,8 @@ class WarpPotentialFem(WarpPotential):
                 raise ValueError("p is required for hess_prod / hess_quad")
             p = check_vec(p.to(self.dtype), self.n_points, self.dtype, "p")
         out = {}
-        z = lambda: torch.zeros((self.n_points, 3), dtype=self.dtype, device=u.device)  # noqa: E731
-        s = lambda: torch.zeros((1,), dtype=torch.float64, device=u.device)  # noqa: E731
+        z = lambda: torch.empty((self.n_points, 3), dtype=self.dtype, device=u.device)  # noqa: E731
+        s = lambda: torch.empty((1,), dtype=torch.float64, device=u.device)  # noqa: E731
         if fun:
             out["fun"] = s()
         if grad:
@@ -300,7 +302,7 @@ class WarpPotentialFem(WarpPotential):
         if hess_quad:
             out["hess_quad"] = s()
         _lib.call(
-            "agb_fem_eval", self._standalone(), flags, ptr(u), ptr(p), ptr(out.get("fun")), ptr(out.get("grad")),
+            "agb_fem_eval_store", self._standalone(), flags, ptr(u), ptr(p), ptr(out.get("fun")), ptr(out.get("grad")),
             ptr(out.get("hess_diag")), ptr(out.get("hess_prod")), ptr(out.get("hess_quad")), stream_ptr(u.device),
         )
         return out
@@ -326,7 +328,9 @@ def _activation_array(activation, n_cells: int) -> np.ndarray:
     a = np.asarray(activation, np.float64)
     if a.shape == (6,):
         a = np.broadcast_to(a, (n_cells, 6))
-    return np.ascontiguousarray(a.reshape(n_cells, 6)).copy()
+    a = np.ascontiguousarray(a.reshape(n_cells, 6))
+    # a copy of its own; torch copies large arrays on all cores
+    return torch.from_numpy(a).clone().numpy() if a.flags.writeable else a.copy()
 
 
 class StableNeoHookeanMuscle(WarpPotentialFem):

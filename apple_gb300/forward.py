@@ -36,18 +36,33 @@ class ForwardProblem:
     def fun(self, state: ModelState) -> torch.Tensor:
         return self.model.fun(state.u)
 
+    # The free-component forms map inside the evaluation's own passes when the
+    # model and its map are this package's (Model.eval_free), and by separate
+    # gathers otherwise.
     def grad(self, state: ModelState) -> torch.Tensor:
-        return self.model.dof_map.to_free_grad(self.model.grad(state.u))
+        out = _eval_free(self.model, state.u, "grad")
+        return self.model.dof_map.to_free_grad(self.model.grad(state.u)) if out is None else out
 
     def hess_diag(self, state: ModelState) -> torch.Tensor:
-        return self.model.dof_map.to_free_hess_diag(self.model.hess_diag(state.u))
+        out = _eval_free(self.model, state.u, "hess_diag")
+        return self.model.dof_map.to_free_hess_diag(self.model.hess_diag(state.u)) if out is None else out
 
     def hess_prod(self, state: ModelState, p: torch.Tensor) -> torch.Tensor:
+        out = _eval_free(self.model, state.u, "hess_prod", p)
+        if out is not None:
+            return out
         p_full = self.model.dof_map.to_full_grad(p)
         return self.model.dof_map.to_free_grad(self.model.hess_prod(state.u, p_full))
 
     def hess_quad(self, state: ModelState, p: torch.Tensor) -> torch.Tensor:
-        return self.model.hess_quad(state.u, self.model.dof_map.to_full_grad(p))
+        out = _eval_free(self.model, state.u, "hess_quad", p)
+        return self.model.hess_quad(state.u, self.model.dof_map.to_full_grad(p)) if out is None else out
+
+
+def _eval_free(model, u: torch.Tensor, what: str, p: torch.Tensor | None = None):
+    if type(model) is not Model or type(model.dof_map) is not DofMap:
+        return None
+    return model.eval_free(u, what, p)
 
 
 class Forward:

@@ -203,6 +203,9 @@ class WarpModel:
         self._eval(_lib.HESS_QUAD, u, p, quad=output)
 
 
+_FLAGS = {"grad": _lib.GRAD, "hess_diag": _lib.HESS_DIAG, "hess_prod": _lib.HESS_PROD, "hess_quad": _lib.HESS_QUAD}
+
+
 class Model:
     """Pure functions of the full displacement (forward/_model.py:46-74)."""
 
@@ -264,6 +267,27 @@ class Model:
         out = torch.empty((1,), dtype=torch.float64, device=u.device)
         self.warp_model.hess_quad(u, p, out)
         return out[0]
+
+    def eval_free(self, u: torch.Tensor, what: str, p: torch.Tensor | None = None) -> torch.Tensor | None:
+        """``what`` (``grad``, ``hess_diag``, ``hess_prod`` or ``hess_quad``) at
+        the full ``u`` over the free components, ``p`` free too; None where
+        the separate maps have to say what is wrong with the arguments or
+        convert them."""
+        dm, wm = self.dof_map, self.warp_model
+        if not isinstance(u, torch.Tensor) or not u.is_cuda or u.device != dm.slot.device or dm.dim != 3 \
+                or dm.n_points != wm.n_points or dm.n_free == 0:
+            return None
+        if p is not None and not (isinstance(p, torch.Tensor) and p.dtype == wm.dtype and p.device == u.device
+                                  and p.numel() == dm.n_free and p.is_contiguous()):
+            return None
+        check_vec(u, wm.n_points, wm.dtype, "u")
+        quad = what == "hess_quad"
+        out = torch.empty((1,) if quad else (dm.n_free,), dtype=torch.float64 if quad else wm.dtype, device=u.device)
+        o = out.data_ptr()
+        _lib.call("agb_model_eval_free", wm.handle, _FLAGS[what], ptr(dm.slot), ptr(u), ptr(p), None,
+                  o if what == "grad" else None, o if what == "hess_diag" else None,
+                  o if what == "hess_prod" else None, o if quad else None, stream_ptr(u.device))
+        return out[0] if quad else out
 
     def init(self):
         from .forward import ModelState

@@ -166,6 +166,9 @@ int agb_fem_fun_noalloc(agb_fem* fem, const void* u, double* output, void* strea
  * for unset flags.  p is needed for HESS_PROD and HESS_QUAD. */
 int agb_fem_eval(agb_fem* fem, unsigned flags, const void* u, const void* p, double* energy,
                  void* grad, void* hess_diag, void* hess_prod, double* hess_quad, void* stream);
+/* agb_fem_eval, but the outputs are stored instead of accumulated into */
+int agb_fem_eval_store(agb_fem* fem, unsigned flags, const void* u, const void* p, double* energy,
+                       void* grad, void* hess_diag, void* hess_prod, double* hess_quad, void* stream);
 
 /* ---------------------------------------------------------------------------
  * Model = potentials + fixed DOFs + external force over one space
@@ -184,6 +187,13 @@ int agb_model_destroy(agb_model* model);
  * (warp/model/_model.py:13-36, potential/_ext_force.py:17-39). */
 int agb_model_eval(agb_model* model, unsigned flags, const void* u, const void* p, double* energy,
                    void* grad, void* hess_diag, void* hess_prod, double* hess_quad, void* stream);
+/* agb_model_eval over the free components (ForwardProblem, forward/_problem.py:
+ * 18-59): slot (device, 3 n_points) holds each component's index among the
+ * free ones or -1 for a fixed one; p_free and the vector outputs have one
+ * entry per free component, u is full. */
+int agb_model_eval_free(agb_model* model, unsigned flags, const int32_t* slot, const void* u, const void* p_free,
+                        double* energy, void* grad, void* hess_diag, void* hess_prod, double* hess_quad,
+                        void* stream);
 
 /* Free/fixed DOF maps over the flattened n_points x 3 vector
  * (DofMap.to_free / to_free_grad / to_free_hess_diag / to_full /
