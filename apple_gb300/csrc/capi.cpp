@@ -1068,7 +1068,8 @@ int agb_solver_reset(agb_solver* sv, const void* u, void* stream) {
 // Capture into `graph` after `deps` (which may be empty): the three passes
 // of one iteration (refresh = false) or the two refresh passes as plain
 // launches (refresh = true); for resident iterations their launch and the
-// refresh passes.
+// refresh passes; for ARAP the main passes or the fallback passes (refresh =
+// true).
 // Iterations per body of agb_solver_iterate's WHILE loop: the second of two
 // is guarded (its passes return at once when the first ended the run), its
 // direction pass a programmatic dependent of the first's vertex pass, and
@@ -1085,6 +1086,12 @@ static cudaError_t capture_into(agb_solver* sv, cudaGraph_t graph, const cudaGra
   if (sv->resident.shape) {
     cudaError_t le = run_resident(sv, a, cs);
     if (le == cudaSuccess) le = launch_solver_refresh(a, cs, false);
+    cudaGraph_t captured = nullptr;
+    e = cudaStreamEndCapture(cs, &captured);
+    return e == cudaSuccess ? le : e;
+  }
+  if (a.fv.material == AGB_ARAP) {
+    cudaError_t le = launch_solver_arap_part(a, refresh, cs);
     cudaGraph_t captured = nullptr;
     e = cudaStreamEndCapture(cs, &captured);
     return e == cudaSuccess ? le : e;
@@ -1122,6 +1129,10 @@ static cudaError_t add_conditional(cudaGraph_t g, const cudaGraphNode_t* deps, s
 // the refresh only if it was asked for) continues the outer loop and re-arms
 // the inner one unless the solve ended or reached the limit.
 // Resident iterations: WHILE(outer) { resident run; refresh passes }.
+// ARAP: WHILE(outer) { WHILE(c) { direction, speculative gradient, vertex };
+// trial passes, gradient, vertex }: the inner loop runs while alpha_0 is
+// accepted, so the five fallback passes are launched only after a rejection
+// (idle, they took 25 of 268 us per iteration on 1,966,080 tets).
 static int build_loop_graph(agb_solver* sv) {
   cudaGraph_t g = nullptr;
   AGB_CHECK_CUDA(cudaGraphCreate(&g, 0));
@@ -1136,7 +1147,7 @@ static int build_loop_graph(agb_solver* sv) {
     SolveArgs ar = a;
     ar.cond_outer = (unsigned long long)h_out;
     if (e == cudaSuccess) e = capture_into(sv, body_out, nullptr, 0, ar, true);
-  } else if (a.delta) {
+  } else if (a.delta || a.fv.material == AGB_ARAP) {
     e = cudaGraphConditionalHandleCreate(&h_out, g, 1u, cudaGraphCondAssignDefault);
     if (e == cudaSuccess) e = add_conditional(g, nullptr, 0, h_out, cudaGraphCondTypeWhile, &w_out, &body_out);
     if (e == cudaSuccess) e = cudaGraphConditionalHandleCreate(&h_in, body_out, 1u, cudaGraphCondAssignDefault);
@@ -1144,7 +1155,7 @@ static int build_loop_graph(agb_solver* sv) {
     if (e == cudaSuccess) {
       SolveArgs ai = a;
       ai.cond = (unsigned long long)h_in;
-      ai.refresh_exits = 1;
+      ai.refresh_exits = a.delta;
       e = capture_into(sv, body_in, nullptr, 0, ai, false);
     }
     if (e == cudaSuccess) {

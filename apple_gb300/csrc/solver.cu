@@ -234,6 +234,13 @@ __global__ void __launch_bounds__(kGradThreads, 4) solver_grad_spec_kernel(Solve
 // ---------------------------------------------------------------------------
 // vertex pass
 // ---------------------------------------------------------------------------
+// the loop condition, and in the pass that ends an outer loop's body (ARAP's
+// fallback) both loops'
+__device__ __forceinline__ void set_loop(const SolveArgs& a, bool go) {
+  cudaGraphSetConditional((cudaGraphConditionalHandle)a.cond, go ? 1u : 0u);
+  if (a.cond_outer) cudaGraphSetConditional((cudaGraphConditionalHandle)a.cond_outer, go ? 1u : 0u);
+}
+
 // phase (ARAP): 1 after the speculative gradient pass, running only if its
 // step was accepted; 2 after the fallback passes, running only if it was not;
 // 0 otherwise (always runs)
@@ -252,14 +259,18 @@ __global__ void __launch_bounds__(kVThreads, kVertexCtasPerSM) solver_vertex_ker
   pdl_wait();
   SolverState* st = a.st;
   if (st->done) {
-    if (use_cond && blockIdx.x == 0 && threadIdx.x == 0)
-      cudaGraphSetConditional((cudaGraphConditionalHandle)a.cond, 0u);
+    if (use_cond && blockIdx.x == 0 && threadIdx.x == 0) set_loop(a, false);
     return;
   }
   if (guard_skip(a, st)) return;  // the loop condition stays as the direction pass left it: 0
   // ARAP: the pass after the speculative gradient pass, or the one after the
-  // fallback passes, whichever applies (the other leaves the condition alone)
-  if ((phase == 1 && !st->spec_ok) || (phase == 2 && st->spec_ok)) return;
+  // fallback passes, whichever applies (a rejected step leaves the inner
+  // loop's condition as the direction pass left it: 0)
+  if (phase == 1 && !st->spec_ok) return;
+  if (phase == 2 && st->spec_ok) {  // the inner loop ended with the run
+    if (use_cond && a.cond_outer && blockIdx.x == 0 && threadIdx.x == 0) set_loop(a, false);
+    return;
+  }
   const R t = to_real<R>(st->t);
   const V4<R>* P = p_cur<R>(a, st->pbuf);
   // 0 gPg 1 gPy 2 yPy 3 sum|d| 4 count 5 zgg 6 zgy 7 zyy 8 y.p 9 p.g 10 g.g 11 ext energy
@@ -288,9 +299,7 @@ __global__ void __launch_bounds__(kVThreads, kVertexCtasPerSM) solver_vertex_ker
   if (threadIdx.x == 0) {
     if (a.svd) sst.sbuf ^= 1;  // the gradient pass's SVDs are those at the new x
     const bool go = !sst.done && sst.iter < sst.iter_limit;
-    if (use_cond)
-      cudaGraphSetConditional((cudaGraphConditionalHandle)a.cond,
-                              (go && !(a.refresh_exits && sst.refresh)) ? 1u : 0u);
+    if (use_cond) set_loop(a, go && !(a.refresh_exits && sst.refresh));
   }
   __syncthreads();
   if ((int)threadIdx.x < kStateWords) ((uint32_t*)st)[threadIdx.x] = ((const uint32_t*)&sst)[threadIdx.x];
@@ -354,11 +363,15 @@ __global__ void __launch_bounds__(kVThreads, kVertexCtasPerSM) solver_vertex_bul
   pdl_wait();
   SolverState* st = a.st;
   if (st->done) {
-    if (use_cond && blockIdx.x == 0 && tid == 0) cudaGraphSetConditional((cudaGraphConditionalHandle)a.cond, 0u);
+    if (use_cond && blockIdx.x == 0 && tid == 0) set_loop(a, false);
     return;
   }
   if (guard_skip(a, st)) return;
-  if ((phase == 1 && !st->spec_ok) || (phase == 2 && st->spec_ok)) return;
+  if (phase == 1 && !st->spec_ok) return;
+  if (phase == 2 && st->spec_ok) {  // the inner loop ended with the run
+    if (use_cond && a.cond_outer && blockIdx.x == 0 && tid == 0) set_loop(a, false);
+    return;
+  }
   const R t = to_real<R>(st->t);
   const V4<R>* P = p_cur<R>(a, st->pbuf);
   const V4<R>* XA = (const V4<R>*)a.xa;
@@ -462,9 +475,7 @@ __global__ void __launch_bounds__(kVThreads, kVertexCtasPerSM) solver_vertex_bul
     else if (a.svd)
       sst.sbuf ^= 1;
     const bool go = !sst.done && sst.iter < sst.iter_limit;
-    if (use_cond)
-      cudaGraphSetConditional((cudaGraphConditionalHandle)a.cond,
-                              (go && !(a.refresh_exits && sst.refresh)) ? 1u : 0u);
+    if (use_cond) set_loop(a, go && !(a.refresh_exits && sst.refresh));
   }
   __syncthreads();
   if (tid < kStateWords) ((uint32_t*)st)[tid] = ((const uint32_t*)&sst)[tid];
@@ -674,25 +685,33 @@ static cudaError_t launch_vertex(const SolveArgs& a, int use_cond, int phase, cu
     return launch_pdl(solver_vertex_kernel<R, DELTA>, dim3(a.vblocks), dim3(kVThreads), 0, s, a, use_cond, phase);
 }
 
+// part (ARAP): the whole iteration, or in agb_solver_iterate's graph the
+// passes every iteration runs and those that follow a rejected step
+constexpr int kWhole = 0, kArapMain = 1, kArapFallback = 2;
+
 template <class R, int MAT, bool DELTA>
-static cudaError_t launch_iteration_d(const SolveArgs& a, bool use_cond, bool first, int max_bt,
+static cudaError_t launch_iteration_d(const SolveArgs& a, bool use_cond, bool first, int max_bt, int part,
                                       cudaStream_t s) {
   const dim3 eg(a.fv.n_tiles), eb(kElemThreads);
   if (!first) {
     // a guarded iteration follows another one: its direction pass is a
     // programmatic dependent of that iteration's vertex pass
-    cudaError_t e = launch_dir<R, MAT>(a, use_cond ? 1 : 0, a.guard != 0, s);
+    cudaError_t e = cudaSuccess;
+    if (part != kArapFallback) e = launch_dir<R, MAT>(a, use_cond ? 1 : 0, a.guard != 0, s);
     if (e != cudaSuccess) return e;
     if constexpr (MAT == AGB_ARAP) {
       // speculative gradient pass at alpha_0 and its vertex pass; when the
       // step is rejected, trial passes from alpha_0 / 2, then the gradient
       // and vertex passes at the step they decide (each of these returns at
       // once when the speculative step was accepted)
-      const dim3 gb(kGradThreads), vg(a.vblocks), vb(kVThreads);
+      const dim3 gb(kGradThreads);
       const int uc = use_cond ? 1 : 0;
-      cudaError_t e = launch_pdl(solver_grad_spec_kernel<R>, eg, gb, grad_spec_smem_bytes<R>(), s, a);
-      if (e == cudaSuccess) e = launch_vertex<R, DELTA>(a, uc, 1, s);
-      if (e != cudaSuccess) return e;
+      cudaError_t e = cudaSuccess;
+      if (part != kArapFallback) {
+        e = launch_pdl(solver_grad_spec_kernel<R>, eg, gb, grad_spec_smem_bytes<R>(), s, a);
+        if (e == cudaSuccess) e = launch_vertex<R, DELTA>(a, uc, 1, s);
+      }
+      if (e != cudaSuccess || part == kArapMain) return e;
       for (int j0 = 1; j0 <= max_bt; j0 += 3)
         solver_trial_kernel<R><<<eg, eb, 0, s>>>(a, j0, max_bt - j0 + 1 < 3 ? max_bt - j0 + 1 : 3);
       e = launch_pdl(solver_grad_kernel<R, MAT, DELTA>, eg, gb, grad_smem_bytes<R>(), s, a, 1);
@@ -706,34 +725,34 @@ static cudaError_t launch_iteration_d(const SolveArgs& a, bool use_cond, bool fi
 }
 
 template <class R, int MAT>
-static cudaError_t launch_iteration_t(const SolveArgs& a, bool use_cond, bool first, int max_bt,
+static cudaError_t launch_iteration_t(const SolveArgs& a, bool use_cond, bool first, int max_bt, int part,
                                       cudaStream_t s) {
   if (a.delta) {  // the reference-state kernels read x_ref and g(x_ref)
     if (!kRefDelta<R, MAT> || !a.xref || !a.gref) return cudaErrorInvalidValue;
-    return launch_iteration_d<R, MAT, kRefDelta<R, MAT>>(a, use_cond, first, max_bt, s);
+    return launch_iteration_d<R, MAT, kRefDelta<R, MAT>>(a, use_cond, first, max_bt, part, s);
   }
-  return launch_iteration_d<R, MAT, false>(a, use_cond, first, max_bt, s);
+  return launch_iteration_d<R, MAT, false>(a, use_cond, first, max_bt, part, s);
 }
 
 
-static cudaError_t launch_iteration(const SolveArgs& a, bool use_cond, bool first, cudaStream_t s) {
+static cudaError_t launch_iteration(const SolveArgs& a, bool use_cond, bool first, int part, cudaStream_t s) {
   if (a.fv.n_tiles == 0) return cudaErrorInvalidValue;
   const int max_bt = a.max_bt;
   cudaError_t e;
   if (a.precision == AGB_F64) {
     if (a.fv.material == AGB_ARAP)
-      e = launch_iteration_t<double, AGB_ARAP>(a, use_cond, first, max_bt, s);
+      e = launch_iteration_t<double, AGB_ARAP>(a, use_cond, first, max_bt, part, s);
     else if (a.fv.material == AGB_STABLE_NEO_HOOKEAN_MUSCLE)
-      e = launch_iteration_t<double, AGB_STABLE_NEO_HOOKEAN_MUSCLE>(a, use_cond, first, max_bt, s);
+      e = launch_iteration_t<double, AGB_STABLE_NEO_HOOKEAN_MUSCLE>(a, use_cond, first, max_bt, part, s);
     else
-      e = launch_iteration_t<double, AGB_STABLE_NEO_HOOKEAN>(a, use_cond, first, max_bt, s);
+      e = launch_iteration_t<double, AGB_STABLE_NEO_HOOKEAN>(a, use_cond, first, max_bt, part, s);
   } else {
     if (a.fv.material == AGB_ARAP)
-      e = launch_iteration_t<float, AGB_ARAP>(a, use_cond, first, max_bt, s);
+      e = launch_iteration_t<float, AGB_ARAP>(a, use_cond, first, max_bt, part, s);
     else if (a.fv.material == AGB_STABLE_NEO_HOOKEAN_MUSCLE)
-      e = launch_iteration_t<float, AGB_STABLE_NEO_HOOKEAN_MUSCLE>(a, use_cond, first, max_bt, s);
+      e = launch_iteration_t<float, AGB_STABLE_NEO_HOOKEAN_MUSCLE>(a, use_cond, first, max_bt, part, s);
     else
-      e = launch_iteration_t<float, AGB_STABLE_NEO_HOOKEAN>(a, use_cond, first, max_bt, s);
+      e = launch_iteration_t<float, AGB_STABLE_NEO_HOOKEAN>(a, use_cond, first, max_bt, part, s);
   }
   if (e != cudaSuccess) return e;
   return cudaGetLastError();
@@ -780,11 +799,15 @@ cudaError_t launch_solver_pass(const SolveArgs& a, int which, cudaStream_t s) {
 }
 
 cudaError_t launch_solver_iteration(const SolveArgs& a, bool use_cond, cudaStream_t s) {
-  return launch_iteration(a, use_cond, false, s);
+  return launch_iteration(a, use_cond, false, kWhole, s);
+}
+
+cudaError_t launch_solver_arap_part(const SolveArgs& a, bool fallback, cudaStream_t s) {
+  return launch_iteration(a, true, false, fallback ? kArapFallback : kArapMain, s);
 }
 
 cudaError_t launch_solver_first(const SolveArgs& a, cudaStream_t s) {
-  return launch_iteration(a, false, true, s);
+  return launch_iteration(a, false, true, kWhole, s);
 }
 
 cudaError_t launch_solver_unpack_x(const SolveArgs& a, const void*, const int32_t* uoi, void* u,

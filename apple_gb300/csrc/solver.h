@@ -114,6 +114,10 @@ cudaError_t launch_solver_init(const SolveArgs& a, const void* u_user, const voi
 cudaError_t launch_solver_set_limit(const SolveArgs& a, int n_steps, cudaStream_t s);
 // one PNCG iteration: direction pass, [ARAP trial passes], gradient pass, vertex pass
 cudaError_t launch_solver_iteration(const SolveArgs& a, bool use_cond, cudaStream_t s);
+// ARAP, in agb_solver_iterate's graph: the passes every iteration runs, which
+// repeat in the loop a.cond while alpha_0 is accepted, or the fallback passes
+// after that loop, which decide whether the loop a.cond_outer around both goes on
+cudaError_t launch_solver_arap_part(const SolveArgs& a, bool fallback, cudaStream_t s);
 // gradient + vertex pass at t = 0 (initial g_0, diag_0)
 cudaError_t launch_solver_first(const SolveArgs& a, cudaStream_t s);
 cudaError_t launch_solver_unpack_x(const SolveArgs& a, const void* fixed_unused,
