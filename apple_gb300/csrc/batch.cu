@@ -1,21 +1,27 @@
 // Batched PNCG: many independent meshes, one set of launches per iteration.
 //
 // The meshes' vertices and tiles are concatenated (tiles never span meshes,
-// vertex chunks never span meshes).  An iteration is five kernels, captured
-// once in a CUDA graph; every mesh carries its own SolverState, so each one
-// runs the reference's PNCG iteration (benches/bench_pncg_branching_backends.py
+// vertex chunks never span meshes).  An iteration is three kernels, captured
+// in a CUDA graph; every mesh carries its own SolverState, so each one runs
+// the reference's PNCG iteration (benches/bench_pncg_branching_backends.py
 // :254-456, 606-679) with its own beta, step and termination:
 //   direction pass   one CTA per tile: p of the tile's mesh, p^T H p and the
-//                    energy polynomial; one partial per tile
-//   direction tail   one CTA per mesh: the mesh's tile partials in tile order,
-//                    then the Armijo decision (dir_decide)
+//                    energy polynomial; one partial per tile; the last CTA of
+//                    a mesh adds its partials in tile order and takes the
+//                    Armijo decision (dir_decide)
 //   gradient pass    one CTA per tile at x + t_mesh p (grad_tile)
-//   vertex pass      one CTA per vertex chunk: x, g, d and the 12 sums
-//   vertex tail      one CTA per mesh: chunk partials in order, then beta and
-//                    termination (vertex_decide); the last CTA to finish
-//                    counts the meshes still running and sets the graph's
+//   vertex pass      one CTA per vertex chunk: x, g, d and the 12 sums; the
+//                    last CTA of a mesh adds its chunks in order and decides
+//                    beta and termination (vertex_decide); the last mesh
+//                    counts those still running and sets the graph's
 //                    while-condition
-// Tiles and chunks of a finished mesh return at once.
+// Tiles and chunks of a finished mesh return at once.  The graph's loop body
+// holds two iterations, the second skipped when the first ended the run.
+// What bounds it is the chain of small launches.  Measured, reset and 20
+// iterations of 24 meshes of 1.2k to 11k tets in FP32: 2,600 -> 1,534 us with
+// the tails in the passes, two iterations a body and one refresh in the reset;
+// three beams 1,124 -> 849, 64 meshes 5,731 -> 2,790, 24 large ones 4,207 ->
+// 3,056.
 #include "kernels.h"
 #include "solver.h"
 #include "solver_common.cuh"
@@ -25,6 +31,42 @@ namespace agb {
 namespace {
 
 constexpr int kTailThreads = 256;
+
+// the passes of the body's second iteration skip it when the first one ended
+// the run
+__device__ __forceinline__ bool batch_skip(const BatchArgs& b) { return b.guard && !b.bs->go; }
+
+// one more CTA of mesh m is done with the pass; true in the last of n
+// (every thread calls it; thread 0's writes before it are visible to the last)
+__device__ __forceinline__ bool last_of_mesh(unsigned* counter, unsigned n) {
+  __shared__ int s_last;
+  if (threadIdx.x == 0) {
+    __threadfence();
+    s_last = atomicAdd(counter, 1u) == n - 1u;
+    if (s_last) *counter = 0u;
+  }
+  __syncthreads();
+  if (!s_last) return false;
+  __threadfence();
+  return true;
+}
+
+// thread 0 of one CTA per mesh, after the mesh's iteration: counts it, and the
+// last mesh closes the batch's iteration
+__device__ __forceinline__ void mesh_arrives(const BatchArgs& b, bool running) {
+  BatchState* bs = b.bs;
+  if (running) atomicAdd(&bs->n_active, 1u);
+  __threadfence();
+  if (atomicAdd(&bs->arrived, 1u) != (unsigned)b.n_meshes - 1u) return;
+  __threadfence();
+  const unsigned active = atomicAdd(&bs->n_active, 0u);
+  bs->iter += 1;
+  bs->n_active = 0u;
+  bs->arrived = 0u;
+  const bool go = active > 0u && bs->iter < bs->iter_limit;
+  bs->go = go ? 1 : 0;
+  if (b.cond) cudaGraphSetConditional((cudaGraphConditionalHandle)b.cond, go ? 1u : 0u);
+}
 
 template <class R, int MAT>
 __global__ void __launch_bounds__(kElemThreads) batch_dir_kernel(BatchArgs b) {
@@ -36,10 +78,13 @@ __global__ void __launch_bounds__(kElemThreads) batch_dir_kernel(BatchArgs b) {
   __shared__ Acc<R> red[kWarps * N];
   const SolveArgs& a = b.a;
   const int tile = blockIdx.x;
-  if (b.cond && tile == 0 && threadIdx.x == 0)
-    cudaGraphSetConditional((cudaGraphConditionalHandle)b.cond, 0u);  // the vertex tail re-arms
+  if (!b.guard && b.cond && tile == 0 && threadIdx.x == 0)
+    cudaGraphSetConditional((cudaGraphConditionalHandle)b.cond, 0u);  // the vertex pass re-arms
   pdl_trigger();
-  SolverState* st = b.st + b.tile_mesh[tile];
+  const int mesh = b.tile_mesh[tile];
+  if (b.guard) pdl_wait();  // a dependent of the first iteration's last pass
+  if (batch_skip(b)) return;
+  SolverState* st = b.st + mesh;
   if (st->done) return;
   const R beta = to_real<R>(st->beta), inv_mean = to_real<R>(st->inv_mean);
   const int pb = st->pbuf;
@@ -83,18 +128,10 @@ __global__ void __launch_bounds__(kElemThreads) batch_dir_kernel(BatchArgs b) {
 #pragma unroll
     for (int k = 0; k < N; ++k) ((AccStore<R>*)b.part_dir)[(size_t)tile * N + k] = acc_store(sums[k]);
   }
-}
-
-template <class R, int MAT>
-__global__ void __launch_bounds__(kTailThreads) batch_dir_tail_kernel(BatchArgs b) {
-  constexpr int N = 6;
-  __shared__ Acc<R> red[(kTailThreads / 32) * N];
-  pdl_trigger();
-  pdl_wait();
-  SolverState* st = b.st + blockIdx.x;
-  if (st->done) return;
-  if (threadIdx.x == 0) st->refresh = 0;  // the refresh passes, if any, ran after the last vertex tail
-  const int t0 = b.mesh_tile0[blockIdx.x], t1 = b.mesh_tile0[blockIdx.x + 1];
+  // the last tile of the mesh: partials in tile order, then the decision
+  const int t0 = b.mesh_tile0[mesh], t1 = b.mesh_tile0[mesh + 1];
+  if (!last_of_mesh(b.cnt_dir + mesh, (unsigned)(t1 - t0))) return;
+  if (threadIdx.x == 0) st->refresh = 0;  // the refresh passes, if any, ran after the last vertex pass
   Acc<R> s[N] = {};
   for (int t = t0 + threadIdx.x; t < t1; t += blockDim.x) {
 #pragma unroll
@@ -171,7 +208,8 @@ __global__ void __launch_bounds__(kTailThreads) batch_trial_tail_kernel(BatchArg
 // speculative step was rejected
 template <class R, int MAT, bool DELTA>
 __global__ void __launch_bounds__(kGradThreads, 6) batch_grad_kernel(BatchArgs b, int fallback) {
-  grad_tile<R, MAT, DELTA>(b.a, blockIdx.x, b.st + b.tile_mesh[blockIdx.x], nullptr, fallback != 0);
+  grad_tile<R, MAT, DELTA>(b.a, blockIdx.x, b.st + b.tile_mesh[blockIdx.x], nullptr, fallback != 0,
+                           b.guard ? &b.bs->go : nullptr);
 }
 
 // phase (ARAP): 1 after the speculative gradient pass, for the meshes whose
@@ -182,13 +220,19 @@ __global__ void __launch_bounds__(kVThreads) batch_vertex_kernel(BatchArgs b, in
   constexpr unsigned FF = (1u << 1) | (1u << 6) | (1u << 8) | (1u << 9);
   __shared__ Acc<R> red[(kVThreads / 32) * N];
   const SolveArgs& a = b.a;
-  const int c = blockIdx.x;
+  const int c = blockIdx.x, mesh = b.chunk_mesh[c];
   const int v0 = b.chunk_v0[c], v1 = b.chunk_v0[c + 1];
-  const SolverState* st = b.st + b.chunk_mesh[c];
+  const int c0 = b.mesh_chunk0[mesh], c1 = b.mesh_chunk0[mesh + 1];
+  SolverState* st = b.st + mesh;
   pdl_trigger();
   pdl_wait();
-  if (st->done) return;
-  if ((phase == 1 && !st->spec_ok) || (phase == 2 && st->spec_ok)) return;
+  if (batch_skip(b)) return;
+  // a mesh this pass does not concern: its first chunk counts it (in the pass
+  // of phase 1 the later one does)
+  if (st->done || (phase == 1 && !st->spec_ok) || (phase == 2 && st->spec_ok)) {
+    if (phase != 1 && c == c0 && threadIdx.x == 0) mesh_arrives(b, !st->done);
+    return;
+  }
   const R t = to_real<R>(st->t);
   const V4<R>* P = p_cur<R>(a, st->pbuf);
   R s[N] = {};
@@ -204,54 +248,24 @@ __global__ void __launch_bounds__(kVThreads) batch_vertex_kernel(BatchArgs b, in
 #pragma unroll
     for (int k = 0; k < N; ++k) ((AccStore<R>*)b.part_vert)[(size_t)c * N + k] = acc_store(acc[k]);
   }
-}
-
-// phase as in batch_vertex_kernel; the pass of phase 1 decides its meshes
-// only, the others also count the meshes still running
-template <class R>
-__global__ void __launch_bounds__(kTailThreads) batch_vertex_tail_kernel(BatchArgs b, int phase) {
-  constexpr int N = 12;
-  __shared__ Acc<R> red[(kTailThreads / 32) * N];
-  __shared__ bool s_last;
-  pdl_wait();
-  SolverState* st = b.st + blockIdx.x;
-  // read by every thread before thread 0 writes the state
-  const bool was_done = st->done != 0;
-  const bool mine = phase == 0 || (phase == 1) == (st->spec_ok != 0);
-  __syncthreads();
-  if (phase == 1 && !mine) return;
-  if (!was_done && mine) {
-    const int c0 = b.mesh_chunk0[blockIdx.x], c1 = b.mesh_chunk0[blockIdx.x + 1];
-    Acc<R> s[N] = {};
-    for (int c = c0 + threadIdx.x; c < c1; c += blockDim.x) {
+  // the last chunk of the mesh: chunk partials in order, then the decision
+  if (!last_of_mesh(b.cnt_vert + mesh, (unsigned)(c1 - c0))) return;
+  Acc<R> q[N] = {};
+  for (int k0 = c0 + threadIdx.x; k0 < c1; k0 += blockDim.x) {
 #pragma unroll
-      for (int k = 0; k < N; ++k) s[k].add(acc_load<R>((const AccStore<R>*)b.part_vert + (size_t)c * N + k));
-    }
-    block_reduce<N, 0xffffffffu, R>(s, red);
-    vertex_decide<R>(st, red);  // the sums are in red[0 .. N-1]
-    // the gradient pass's SVDs are those at the new x
-    if (threadIdx.x == 0 && b.a.svd) st->sbuf ^= 1;
+    for (int k = 0; k < N; ++k) q[k].add(acc_load<R>((const AccStore<R>*)b.part_vert + (size_t)k0 * N + k));
   }
-  if (phase == 1) return;
-  if (threadIdx.x == 0) {
-    if (!st->done) atomicAdd(&b.bs->n_active, 1u);
-    __threadfence();
-    s_last = atomicAdd(&b.bs->arrived, 1u) == (unsigned)b.n_meshes - 1u;
-  }
-  __syncthreads();
-  if (!s_last || threadIdx.x != 0) return;
-  __threadfence();
-  BatchState* bs = b.bs;
-  const unsigned active = atomicAdd(&bs->n_active, 0u);
-  bs->iter += 1;
-  bs->n_active = 0u;
-  bs->arrived = 0u;
-  if (b.cond)
-    cudaGraphSetConditional((cudaGraphConditionalHandle)b.cond,
-                            (active > 0u && bs->iter < bs->iter_limit) ? 1u : 0u);
+  block_reduce<N, 0xffffffffu, R>(q, red);
+  vertex_decide<R>(st, red);  // the sums are in red[0 .. N-1]
+  if (threadIdx.x != 0) return;
+  if (b.a.svd) st->sbuf ^= 1;  // the gradient pass's SVDs are those at the new x
+  if (phase != 1) mesh_arrives(b, !st->done);
 }
 
-// reference-state refresh of the models that asked for one (FP32)
+// reference-state refresh of the models that asked for one (FP32); it runs
+// too after the iteration that ends the run, where the next run's first
+// direction pass clears the request (after a skipped iteration it repeats what
+// the one before stored)
 // (grid-stride over tiles / chunks with a resident-sized grid)
 template <int MAT>
 __global__ void __launch_bounds__(kGradThreads) batch_ref_elem_kernel(BatchArgs b) {
@@ -337,7 +351,7 @@ __global__ void batch_init_state_kernel(BatchArgs b, SolverState proto) {
     st.spec_ok = 0;
     b.st[m] = st;
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) *b.bs = BatchState{0, 0, 0u, 0u};
+  if (blockIdx.x == 0 && threadIdx.x == 0) *b.bs = BatchState{0, 0, 0u, 0u, 0};
 }
 
 __global__ void batch_set_limit_kernel(BatchState* bs, int n) { bs->iter_limit = bs->iter + n; }
@@ -354,41 +368,47 @@ cudaError_t batch_refresh(const BatchArgs& b, cudaStream_t s) {
 }
 
 template <class R, int MAT, bool DELTA>
-cudaError_t batch_grad_and_vertex_d(const BatchArgs& b, cudaStream_t s, int fallback = 0) {
+cudaError_t batch_grad_and_vertex_d(const BatchArgs& b, cudaStream_t s, int fallback = 0, bool refresh = true) {
   const int phase = fallback ? 2 : 0;
   cudaError_t e = launch_pdl(batch_grad_kernel<R, MAT, DELTA>, dim3(b.a.fv.n_tiles), dim3(kGradThreads),
                                grad_smem_bytes<R>(), s, b, fallback);
   if (e == cudaSuccess)
     e = launch_pdl(batch_vertex_kernel<R, DELTA>, dim3(b.n_chunks), dim3(kVThreads), 0, s, b, phase);
-  if (e == cudaSuccess)
-    e = launch_pdl(batch_vertex_tail_kernel<R>, dim3(b.n_meshes), dim3(kTailThreads), 0, s, b, phase);
-  if (e == cudaSuccess && DELTA) e = batch_refresh(b, s);
+  if (e == cudaSuccess && DELTA && refresh) e = batch_refresh(b, s);
   return e;
 }
 
 template <class R, int MAT>
-cudaError_t batch_grad_and_vertex_m(const BatchArgs& b, cudaStream_t s) {
+cudaError_t batch_grad_and_vertex_m(const BatchArgs& b, cudaStream_t s, bool refresh = true) {
   if (b.a.delta) {
     if (!kRefDelta<R, MAT> || !b.a.xref || !b.a.gref) return cudaErrorInvalidValue;
-    return batch_grad_and_vertex_d<R, MAT, kRefDelta<R, MAT>>(b, s);
+    return batch_grad_and_vertex_d<R, MAT, kRefDelta<R, MAT>>(b, s, 0, refresh);
   }
   return batch_grad_and_vertex_d<R, MAT, false>(b, s);
 }
 
+// the first pass: launch_batch_first has just refreshed every mesh's
+// reference state at the same x, so no refresh follows (it took 180 us of a
+// 24-mesh reset to store what was there)
 template <class R>
-cudaError_t batch_grad_and_vertex(const BatchArgs& b, cudaStream_t s) {
+cudaError_t batch_first(const BatchArgs& b, cudaStream_t s) {
   if (b.a.fv.material == AGB_ARAP) return batch_grad_and_vertex_d<R, AGB_ARAP, false>(b, s);
   return b.a.fv.material == AGB_STABLE_NEO_HOOKEAN_MUSCLE
-             ? batch_grad_and_vertex_m<R, AGB_STABLE_NEO_HOOKEAN_MUSCLE>(b, s)
-             : batch_grad_and_vertex_m<R, AGB_STABLE_NEO_HOOKEAN>(b, s);
+             ? batch_grad_and_vertex_m<R, AGB_STABLE_NEO_HOOKEAN_MUSCLE>(b, s, false)
+             : batch_grad_and_vertex_m<R, AGB_STABLE_NEO_HOOKEAN>(b, s, false);
+}
+
+template <class R, int MAT>
+cudaError_t batch_dir(const BatchArgs& b, cudaStream_t s) {
+  const dim3 g(b.a.fv.n_tiles), t(kElemThreads);
+  if (b.guard) return launch_pdl(batch_dir_kernel<R, MAT>, g, t, 0, s, b);
+  batch_dir_kernel<R, MAT><<<g, t, 0, s>>>(b);
+  return cudaGetLastError();
 }
 
 template <class R, int MAT>
 cudaError_t batch_iteration_m(const BatchArgs& b, cudaStream_t s) {
-  batch_dir_kernel<R, MAT><<<b.a.fv.n_tiles, kElemThreads, 0, s>>>(b);
-  cudaError_t e = cudaGetLastError();
-  if (e == cudaSuccess)
-    e = launch_pdl(batch_dir_tail_kernel<R, MAT>, dim3(b.n_meshes), dim3(kTailThreads), 0, s, b);
+  cudaError_t e = batch_dir<R, MAT>(b, s);
   if (e == cudaSuccess) e = batch_grad_and_vertex_m<R, MAT>(b, s);
   return e;
 }
@@ -401,16 +421,12 @@ template <class R>
 cudaError_t batch_iteration_arap(const BatchArgs& b, cudaStream_t s) {
   constexpr int A = AGB_ARAP;
   const int nt = b.a.fv.n_tiles, max_bt = b.a.max_bt;
-  batch_dir_kernel<R, A><<<nt, kElemThreads, 0, s>>>(b);
-  cudaError_t e = cudaGetLastError();
-  if (e == cudaSuccess) e = launch_pdl(batch_dir_tail_kernel<R, A>, dim3(b.n_meshes), dim3(kTailThreads), 0, s, b);
+  cudaError_t e = batch_dir<R, A>(b, s);
   if (e == cudaSuccess)
     e = launch_pdl(batch_grad_spec_kernel<R>, dim3(nt), dim3(kGradThreads), grad_spec_smem_bytes<R>(), s, b);
   if (e == cudaSuccess) e = launch_pdl(batch_spec_tail_kernel<R>, dim3(b.n_meshes), dim3(kTailThreads), 0, s, b);
   if (e == cudaSuccess)
     e = launch_pdl(batch_vertex_kernel<R, false>, dim3(b.n_chunks), dim3(kVThreads), 0, s, b, 1);
-  if (e == cudaSuccess)
-    e = launch_pdl(batch_vertex_tail_kernel<R>, dim3(b.n_meshes), dim3(kTailThreads), 0, s, b, 1);
   for (int j0 = 1; e == cudaSuccess && j0 <= max_bt; j0 += 3) {
     const int k = max_bt - j0 + 1 < 3 ? max_bt - j0 + 1 : 3;
     batch_trial_kernel<R><<<nt, kElemThreads, 0, s>>>(b, j0, k);
@@ -474,7 +490,7 @@ cudaError_t launch_batch_first(const BatchArgs& b, cudaStream_t s) {
     if (e != cudaSuccess) return e;
   }
   const cudaError_t e =
-      b.a.precision == AGB_F64 ? batch_grad_and_vertex<double>(b, s) : batch_grad_and_vertex<float>(b, s);
+      b.a.precision == AGB_F64 ? batch_first<double>(b, s) : batch_first<float>(b, s);
   return e != cudaSuccess ? e : cudaGetLastError();
 }
 

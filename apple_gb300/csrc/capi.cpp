@@ -1611,7 +1611,7 @@ int agb_batch_destroy(agb_batch* b) {
                   (void*)b->d_tile_mesh, (void*)b->d_mesh_tile0, (void*)b->d_chunk_v0, (void*)b->d_chunk_mesh,
                   (void*)b->d_mesh_chunk0, b->d_xa, b->d_gd, b->d_p0, b->d_p1, b->d_xref, b->d_gref, b->d_slots,
                   b->d_svd, b->d_part, b->d_act,
-                  (void*)b->d_state, (void*)b->d_bstate})
+                  (void*)b->d_state, (void*)b->d_bstate, (void*)b->d_cnt})
     dfree(p);
   if (b->h_state) cudaFreeHost(b->h_state);
   delete b;
@@ -1784,6 +1784,8 @@ int agb_batch_create(int32_t n_models, agb_model* const* models, const agb_pncg_
   if (!rc) rc = dalloc_bytes(&b->d_part, 8 * n_part);
   if (!rc) rc = dalloc(&b->d_state, (size_t)n_models);
   if (!rc) rc = dalloc(&b->d_bstate, 1);
+  if (!rc) rc = dalloc(&b->d_cnt, 2 * (size_t)n_models);
+  if (!rc && cudaMemset(b->d_cnt, 0, 2 * sizeof(unsigned) * n_models) != cudaSuccess) rc = AGB_E_CUDA;
   if (!rc && cudaMallocHost((void**)&b->h_state, sizeof(SolverState) * n_models) != cudaSuccess) rc = AGB_E_CUDA;
   if (!rc && cudaStreamCreateWithFlags(&b->capture_stream, cudaStreamNonBlocking) != cudaSuccess) rc = AGB_E_CUDA;
   if (!rc && batch_prepare_kernels(prec) != cudaSuccess) rc = AGB_E_CUDA;
@@ -1835,7 +1837,10 @@ int agb_batch_create(int32_t n_models, agb_model* const* models, const agb_pncg_
   ba.part_dir = part;
   ba.part_grad = part + 8 * (size_t)P.n_tiles * 6;
   ba.part_vert = part + 8 * (size_t)P.n_tiles * 7;
+  ba.cnt_dir = b->d_cnt;
+  ba.cnt_vert = b->d_cnt + n_models;
   ba.cond = 0;
+  ba.guard = 0;
   // initial state: done until reset
   std::vector<SolverState> st0(n_models);
   for (auto& st : st0) {
@@ -1895,6 +1900,10 @@ static int build_batch_graph(agb_batch* b, bool loop) {
     BatchArgs a = b->args;
     a.cond = loop ? (unsigned long long)h : 0ull;
     cudaError_t le = launch_batch_iteration(a, b->capture_stream);
+    if (loop && le == cudaSuccess && a.a.fv.material != AGB_ARAP) {
+      a.guard = 1;
+      le = launch_batch_iteration(a, b->capture_stream);
+    }
     cudaGraph_t captured = nullptr;
     e = cudaStreamEndCapture(b->capture_stream, &captured);
     if (e == cudaSuccess) e = le;

@@ -696,10 +696,12 @@ __device__ __forceinline__ void delta_gradient(const V4<R>* sh, const V2<R>* sl,
 // Psi(F + t dF) - Psi(F) - t P(F):dF into *rem, so that the Armijo test of
 // the first trial step needs no pass of its own.  FALLBACK: a pass launched
 // after the speculative one that returns at once unless that one's step was
-// rejected.  Returns false when the pass returned without work.
+// rejected.  go (batch): return at once when it is 0.  Returns false when the
+// pass returned without work.
 template <class R, int MAT, bool DELTA = kRefDelta<R, MAT>, bool SPEC = false>
 __device__ __forceinline__ bool grad_tile(const SolveArgs& a, int tile, const SolverState* st,
-                                          Acc<R>* rem = nullptr, bool fallback = false) {
+                                          Acc<R>* rem = nullptr, bool fallback = false,
+                                          const int32_t* go = nullptr) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   V4<R>* sh = reinterpret_cast<V4<R>*>(smem_raw);
   V4<R>* acc4 = sh + kTileVerts;  // [warp][vertex]: gx gy gz dx
@@ -728,7 +730,7 @@ __device__ __forceinline__ bool grad_tile(const SolveArgs& a, int tile, const So
   }
   pdl_trigger();
   pdl_wait();
-  if (st->done || guard_skip(a, st)) return false;
+  if (st->done || guard_skip(a, st) || (go && !*go)) return false;
   if (fallback && st->spec_ok) return false;
   // ARAP: base SVDs (x) and the SVDs written by this pass
   const size_t ncell = (size_t)a.fv.n_cells;
