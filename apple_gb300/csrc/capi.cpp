@@ -1058,7 +1058,8 @@ int agb_solver_reset(agb_solver* sv, const void* u, void* stream) {
                   "solver_init"));
   if (sv->whole.delta) {  // x_ref = x_0 and g(x_0) in FP64 before the first gradient pass
     RC(check_launch(launch_solver_force_refresh(sv->whole, s), "solver_refresh"));
-    RC(check_launch(launch_solver_refresh(sv->whole, s), "solver_refresh"));
+    // on the iterations' tiles: split ones spread a small mesh's FP64 work
+    RC(check_launch(launch_solver_refresh(sv->args, s, false), "solver_refresh"));
   }
   RC(check_launch(launch_solver_first(sv->whole, s), "solver_first"));
   sv->has_state = true;
