@@ -51,6 +51,7 @@ struct TilePlan {
   std::vector<int32_t> tile_gstart;  // n_tiles + 1, warp-group ranges
   std::vector<int32_t> group_estart; // n_groups + 1, element ranges of conflict-free warp groups
   std::vector<int32_t> tv_vid;       // n_tv, internal vertex id
+  std::vector<uint8_t> tv_rank;      // n_tv, the vertex's place in its tile in ascending order of ids
   std::vector<int32_t> elem_user;    // internal element -> caller's cell index
   std::vector<uint32_t> ids;         // packed 4 x 8-bit local corner ids
   std::vector<double> D;             // 9 x n_cells, rows 1..3 of dhdX (component-major)
@@ -78,6 +79,23 @@ int region_compute(int n_cells, const int32_t* cells, const double* points,
 int build_tiles(int n_cells, const int32_t* cells_int, const double* centroid_xyz,
                 const double* D9, const double* mudv, const double* lamdv, int tile_elems,
                 TilePlan* plan);
+
+// Renumber each tile's local vertices, inside blocks of 32 consecutive ones
+// (a warp still stages the same 32 vertices, so its global loads stay as
+// coalesced as they were), so that the lanes of a warp group meet less often on
+// a shared-memory bank when they gather and add their corners' vertices: every
+// vertex in turn takes the free position where its corners meet the fewest
+// lanes.  The tile passes are bound by those accesses.  Nothing that is
+// computed changes: tiles, groups, elements and corner orders stay, and a tile
+// vertex's sums do not depend on its position.  Cycles per access against a
+// conflict-free one, 138k-tet grid: 2.52 -> 2.15 (16 bytes), 2.89 -> 2.39 (8).
+// Measured: evaluation of 1.5M tets 96.3 -> 89.8 us, 40 PNCG iterations on them
+// 5,677 -> 5,515, on 138k 1,163 -> 1,144, 40 adjoint CG steps there 723 -> 694.
+void spread_banks(TilePlan* plan);
+
+// The plan's vertex lists and corner ids with each tile's vertices in ascending
+// order, as build_tiles leaves them.
+void sorted_labels(const TilePlan& plan, std::vector<int32_t>* tv_vid, std::vector<uint32_t>* ids);
 
 // Cut the tiles of a plan with at most sms * per_sm of them into as many
 // pieces (of at least 8 warp groups, each with its tile's vertex list), for

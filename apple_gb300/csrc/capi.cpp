@@ -216,8 +216,13 @@ uint64_t solver_fingerprint(const agb_model* m, const agb_pncg_params& prm, int 
     f.val(fe->material);
     f.vec(fe->plan.tile_estart);
     f.vec(fe->plan.tile_vstart);
-    f.vec(fe->plan.tv_vid);
-    f.vec(fe->plan.ids);
+    // the labels in ascending order: their spread over the banks is no part of
+    // what a checkpoint depends on
+    std::vector<int32_t> tv_vid;
+    std::vector<uint32_t> ids;
+    sorted_labels(fe->plan, &tv_vid, &ids);
+    f.vec(tv_vid);
+    f.vec(ids);
     f.vec(fe->plan.D);
     f.vec(fe->plan.mudv);
     f.vec(fe->plan.lamdv);
@@ -408,6 +413,7 @@ int agb_fem_create(agb_space* space, int material, int precision, int32_t n_cell
   f->precision = precision;
   int rc = build_tiles(n_cells, cells_int.data(), centroid.data(), D9.data(), mudv.data(),
                        lamdv.data(), tile_elems, &f->plan);
+  if (!rc) spread_banks(&f->plan);
   std::vector<SlotMap> sm;
   if (!rc) {
     build_slots(np, {&f->plan}, &sm, &f->own_off);
@@ -477,6 +483,7 @@ int agb_plan_tiles(int32_t n_points, int32_t n_cells, const int32_t* cells, cons
     }
   TilePlan P;
   RC(build_tiles(n_cells, cells_int.data(), centroid.data(), D9.data(), zero.data(), zero.data(), tile_elems, &P));
+  spread_banks(&P);
   *n_tiles = P.n_tiles;
   *n_groups = (int32_t)P.group_estart.size() - 1;
   for (int t = 0; t < P.n_tiles; ++t) {

@@ -121,7 +121,7 @@ int build_tiles(int n_cells, const int32_t* cells, const double* centroid, const
 
   int n_points = 0;
   for (int e = 0; e < 4 * n_cells; ++e) n_points = std::max(n_points, cells[e] + 1);
-  std::vector<int32_t> stamp(n_points, -1);
+  std::vector<int32_t> stamp(n_points, -1), local_of(n_points, 0);
 
   plan->n_cells = n_cells;
   plan->tile_estart.assign(1, 0);
@@ -129,6 +129,7 @@ int build_tiles(int n_cells, const int32_t* cells, const double* centroid, const
   plan->tile_gstart.assign(1, 0);
   plan->group_estart.clear();
   plan->tv_vid.clear();
+  plan->tv_rank.clear();
   plan->elem_user.clear();
   plan->elem_user.reserve(n_cells);
   plan->ids.assign(n_cells, 0);
@@ -145,9 +146,8 @@ int build_tiles(int n_cells, const int32_t* cells, const double* centroid, const
     std::sort(tile_verts.begin(), tile_verts.end());
     const int nv = (int)tile_verts.size();
     // local ids by sorted vertex order
-    auto local = [&](int32_t v) {
-      return (int)(std::lower_bound(tile_verts.begin(), tile_verts.end(), v) - tile_verts.begin());
-    };
+    for (int i = 0; i < nv; ++i) local_of[tile_verts[i]] = i;
+    auto local = [&](int32_t v) { return (int)local_of[v]; };
     // element order inside the tile: warp groups of <= 32 elements in which
     // no vertex occurs more than 4 times (first fit along a strided walk of
     // the Morton order), then, per group, a corner order for every element
@@ -262,7 +262,10 @@ int build_tiles(int n_cells, const int32_t* cells, const double* centroid, const
       }
     }
     plan->tile_gstart.push_back((int32_t)plan->group_estart.size());
-    for (int i = 0; i < nv; ++i) plan->tv_vid.push_back(tile_verts[i]);
+    for (int i = 0; i < nv; ++i) {
+      plan->tv_vid.push_back(tile_verts[i]);
+      plan->tv_rank.push_back((uint8_t)i);
+    }
     plan->tile_estart.push_back((int32_t)plan->elem_user.size());
     plan->tile_vstart.push_back((int32_t)plan->tv_vid.size());
     tile_elems_list.clear();
@@ -295,6 +298,115 @@ int build_tiles(int n_cells, const int32_t* cells, const double* centroid, const
   plan->n_tiles = (int)plan->tile_estart.size() - 1;
   plan->n_tv = (int)plan->tv_vid.size();
   return AGB_OK;
+}
+
+void spread_banks(TilePlan* plan) {
+  constexpr int kBlock = 32;
+  // Per warp group and corner, the lanes that one shared-memory cycle serves:
+  // a unit is a quarter warp (16-byte accesses, bank = position mod 8), a pair
+  // of units a half warp (8-byte accesses, position mod 16).  A word holds
+  // eight 8-bit counts of the lanes on a bank (at most 8 or 16 each).
+  std::vector<uint64_t> by8, by16;
+  std::vector<int32_t> inc, start(kTileVerts + 1), cursor;
+  std::vector<int32_t> pos, vid;
+  // (called once, on the ascending order that build_tiles leaves)
+  for (int t = 0; t < plan->n_tiles; ++t) {
+    const int vs = plan->tile_vstart[t], nv = plan->tile_vstart[t + 1] - vs;
+    const int g0 = plan->tile_gstart[t], g1 = plan->tile_gstart[t + 1];
+    const int ea = plan->tile_estart[t], eb = plan->tile_estart[t + 1];
+    // the units that touch each local vertex
+    std::fill(start.begin(), start.end(), 0);
+    for (int e = ea; e < eb; ++e)
+      for (int k = 0; k < 4; ++k) ++start[((plan->ids[e] >> (8 * k)) & 0xffu) + 1];
+    for (int i = 0; i < kTileVerts; ++i) start[i + 1] += start[i];
+    inc.resize(4 * (size_t)(eb - ea));
+    cursor.assign(start.begin(), start.end() - 1);
+    for (int g = g0; g < g1; ++g)
+      for (int e = plan->group_estart[g]; e < plan->group_estart[g + 1]; ++e)
+        for (int k = 0; k < 4; ++k)
+          inc[cursor[(plan->ids[e] >> (8 * k)) & 0xffu]++] = ((g - g0) * 4 + k) * 4 + (e - plan->group_estart[g]) / 8;
+    const size_t units = 16 * (size_t)(g1 - g0);
+    by8.assign(units, 0);
+    by16.assign(units, 0);
+    auto count = [&](int v, int p, bool add) {
+      const uint64_t one = 1ull << (8 * (p % 8));
+      for (int q = start[v]; q < start[v + 1]; ++q) {
+        uint64_t& a = by8[inc[q]];
+        uint64_t& b = by16[(inc[q] & ~1) + (p % 16) / 8];
+        a = add ? a + one : a - one;
+        b = add ? b + one : b - one;
+      }
+    };
+    pos.resize(nv);
+    for (int i = 0; i < nv; ++i) {
+      pos[i] = i;
+      count(i, i, true);
+    }
+    for (int b0 = 0; b0 < nv; b0 += kBlock) {
+      const int b1 = std::min(nv, b0 + kBlock);
+      int next[16], left[16] = {};  // per position mod 16: the next free one, how many
+      for (int i = b1 - 1; i >= b0; --i) {
+        count(i, i, false);
+        next[i % 16] = i;
+        ++left[i % 16];
+      }
+      for (int i = b0; i < b1; ++i) {
+        // the lanes that vertex i would meet on each bank; [odd] holds the odd
+        // banks' sums, 16 bits each
+        constexpr uint64_t kEven = 0x00ff00ff00ff00ffull;
+        uint64_t m8[2] = {}, m16[2][2] = {};
+        for (int q = start[i]; q < start[i + 1]; ++q) {
+          const uint64_t a = by8[inc[q]], lo = by16[inc[q] & ~1], hi = by16[inc[q] | 1];
+          m8[0] += a & kEven;
+          m8[1] += (a >> 8) & kEven;
+          m16[0][0] += lo & kEven;
+          m16[0][1] += (lo >> 8) & kEven;
+          m16[1][0] += hi & kEven;
+          m16[1][1] += (hi >> 8) & kEven;
+        }
+        int best = -1, least = 0;
+        for (int r = 0; r < 16; ++r) {
+          if (!left[r]) continue;
+          const int sh = 16 * ((r % 8) / 2);
+          // two 16-byte cycles for each 8-byte one
+          const int meets = 2 * (int)((m8[r & 1] >> sh) & 0xffff) + (int)((m16[r / 8][r & 1] >> sh) & 0xffff);
+          if (best < 0 || meets < least) {
+            best = r;
+            least = meets;
+          }
+        }
+        pos[i] = next[best];
+        next[best] += 16;
+        --left[best];
+        count(i, pos[i], true);
+      }
+    }
+    for (int e = ea; e < eb; ++e) {
+      uint32_t packed = 0;
+      for (int k = 0; k < 4; ++k) packed |= (uint32_t)pos[(plan->ids[e] >> (8 * k)) & 0xffu] << (8 * k);
+      plan->ids[e] = packed;
+    }
+    vid.assign(plan->tv_vid.begin() + vs, plan->tv_vid.begin() + vs + nv);
+    for (int i = 0; i < nv; ++i) {
+      plan->tv_vid[vs + pos[i]] = vid[i];
+      plan->tv_rank[vs + pos[i]] = (uint8_t)i;
+    }
+  }
+}
+
+void sorted_labels(const TilePlan& plan, std::vector<int32_t>* tv_vid, std::vector<uint32_t>* ids) {
+  tv_vid->resize(plan.tv_vid.size());
+  ids->resize(plan.ids.size());
+  for (int t = 0; t < plan.n_tiles; ++t) {
+    const int vs = plan.tile_vstart[t], nv = plan.tile_vstart[t + 1] - vs;
+    const uint8_t* rank = plan.tv_rank.data() + vs;
+    for (int i = 0; i < nv; ++i) (*tv_vid)[vs + rank[i]] = plan.tv_vid[vs + i];
+    for (int e = plan.tile_estart[t]; e < plan.tile_estart[t + 1]; ++e) {
+      const uint32_t p = plan.ids[e];
+      (*ids)[e] = (uint32_t)rank[p & 0xffu] | (uint32_t)rank[(p >> 8) & 0xffu] << 8 |
+                  (uint32_t)rank[(p >> 16) & 0xffu] << 16 | (uint32_t)rank[p >> 24] << 24;
+    }
+  }
 }
 
 void split_tiles(const TilePlan& plan, int sms, int per_sm, TilePlan* out) {
