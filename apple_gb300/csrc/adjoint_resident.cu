@@ -119,7 +119,7 @@ __global__ void __launch_bounds__(32 * NW, 2) cg_resident_kernel(CgArgs c, int m
     }
     word(MASK, j) = ((const V4<R>*)a.xa)[2 * v].w;
   }
-  if constexpr (REC) keep_records<MAT>(a.fv, tile, max_elems, srec, sgrp);
+  if constexpr (REC) keep_records<MAT>(a.fv, tile, max_elems, srec, sgrp, threadIdx.x, blockDim.x);
   const GroupLoader<R, MAT, REC> load{a.fv, gs, max_elems, srec, sgrp};
   const int w0 = decision_warp<NW>();
   __syncthreads();
@@ -370,7 +370,7 @@ using CgKernel = void (*)(CgArgs, int, void*, void*, unsigned*);
 
 struct Shape {
   CgKernel kernel;
-  int threads;
+  int blocks, threads;
   size_t smem;
 };
 
@@ -382,7 +382,7 @@ Shape shape(const ResidentPlan& p, int n_tiles) {
   // up to one tile per SM: more shared memory than half an SM's, so that no
   // two CTAs share an SM while others idle
   if (n_tiles <= kSMs) smem = std::max(smem, (size_t)120 * 1024);
-  return Shape{cg_resident_kernel<R, MAT, NW, REC>, 32 * NW, smem};
+  return Shape{cg_resident_kernel<R, MAT, NW, REC>, n_tiles, 32 * NW, smem};
 }
 
 template <int MAT>
@@ -412,7 +412,7 @@ cudaError_t launch_cg_resident(const CgArgs& c, const ResidentPlan& p, void* par
                                cudaStream_t s) {
   if (!p.shape) return cudaErrorInvalidValue;
   const Shape sh = shape_of(c.a, p);
-  return launch_cooperative(sh.kernel, c.a.fv.n_tiles, sh.threads, sh.smem, s, c, p.max_elems, part_p, part_v, counters);
+  return launch_cooperative(sh.kernel, sh.blocks, sh.threads, sh.smem, s, c, p.max_elems, part_p, part_v, counters);
 }
 
 }  // namespace agb

@@ -105,6 +105,11 @@ void sorted_labels(const TilePlan& plan, std::vector<int32_t>* tv_vid, std::vect
 // and corner ids are the plan's.
 void split_tiles(const TilePlan& plan, int sms, int per_sm, TilePlan* out);
 
+// Two tiles for each of `sms` SMs, -1 for none: of the `sms` tiles with the
+// most warp groups the smallest go with the largest of the others, the largest
+// stay alone.
+std::vector<int32_t> pair_tiles(const TilePlan& plan, int sms);
+
 // One slot map over several plans (a model); plans[k]->n_tv entries each.
 void build_slots(int n_points, const std::vector<const TilePlan*>& plans,
                  std::vector<SlotMap>* per_plan, std::vector<int32_t>* off);

@@ -794,7 +794,8 @@ int agb_solver_destroy(agb_solver* sv) {
                   sv->d_p1, sv->d_xref, sv->d_gref, sv->d_svd, sv->d_slots, sv->d_part, (void*)sv->d_cnt,
                   (void*)sv->d_state, sv->d_u_tmp, sv->d_act, sv->d_res_part, (void*)sv->d_res_counters,
                   (void*)sv->d_piece_estart, (void*)sv->d_piece_vstart, (void*)sv->d_piece_gstart,
-                  (void*)sv->d_piece_vid, (void*)sv->d_piece_slot, (void*)sv->d_piece_off})
+                  (void*)sv->d_piece_vid, (void*)sv->d_piece_slot, (void*)sv->d_piece_off,
+                  (void*)sv->d_piece_order})
     dfree(p);
   if (sv->h_state) cudaFreeHost(sv->h_state);
   delete sv;
@@ -1036,9 +1037,13 @@ int agb_solver_create(agb_model* m, const agb_pncg_params* params, agb_solver** 
     largest_tile(pieces, &sv->resident);
     const int n_whole = m->fems.size() == 1 ? m->fems[0]->plan.n_tiles : sv->plan.n_tiles;
     sv->resident.whole = n_whole > kResidentMaxTiles / 2 ? kResidentMaxTiles / 2 : 0;
-    rc = check_launch(resident_prepare(a, &sv->resident), "resident_prepare");
+    if (sv->precision == AGB_F64 && pieces.n_tiles > kResidentMaxTiles / 2) {
+      rc = dupload(&sv->d_piece_order, pair_tiles(pieces, kResidentMaxTiles / 2));
+      sv->resident.order = sv->d_piece_order;
+    }
+    if (!rc) rc = check_launch(resident_prepare(a, &sv->resident), "resident_prepare");
     const bool fits = sv->resident.shape != 0;
-    if (!rc && fits) rc = dalloc_bytes(&sv->d_res_part, 8 * 18 * nt);
+    if (!rc && fits) rc = dalloc_bytes(&sv->d_res_part, 8 * 18 * (size_t)kResidentMaxTiles);
     if (!rc && fits) rc = dalloc(&sv->d_res_counters, kResidentCounters);
     if (!rc && fits && cudaMemset(sv->d_res_counters, 0, kResidentCounters * sizeof(unsigned)) != cudaSuccess) rc = AGB_E_CUDA;
     if (rc) {
@@ -1053,7 +1058,7 @@ int agb_solver_create(agb_model* m, const agb_pncg_params* params, agb_solver** 
 
 // the solver's iterations up to its limit, or a due refresh, in one launch
 static cudaError_t run_resident(agb_solver* sv, const SolveArgs& a, cudaStream_t s) {
-  return launch_resident(a, sv->resident, sv->d_res_part, (char*)sv->d_res_part + 8 * 6 * (size_t)a.fv.n_tiles,
+  return launch_resident(a, sv->resident, sv->d_res_part, (char*)sv->d_res_part + 8 * 6 * (size_t)kResidentMaxTiles,
                          sv->d_res_counters, s);
 }
 

@@ -440,6 +440,19 @@ void split_tiles(const TilePlan& plan, int sms, int per_sm, TilePlan* out) {
   out->n_tv = (int)out->tv_vid.size();
 }
 
+std::vector<int32_t> pair_tiles(const TilePlan& plan, int sms) {
+  std::vector<int32_t> order(plan.n_tiles);
+  for (int t = 0; t < plan.n_tiles; ++t) order[t] = t;
+  auto groups = [&](int32_t t) { return plan.tile_gstart[t + 1] - plan.tile_gstart[t]; };
+  std::stable_sort(order.begin(), order.end(), [&](int32_t a, int32_t b) { return groups(a) > groups(b); });
+  std::vector<int32_t> paired;
+  for (int k = 0; k < sms; ++k) {
+    paired.push_back(sms - 1 - k < plan.n_tiles ? order[sms - 1 - k] : -1);
+    paired.push_back(sms + k < plan.n_tiles ? order[sms + k] : -1);
+  }
+  return paired;
+}
+
 void build_slots(int n_points, const std::vector<const TilePlan*>& plans,
                  std::vector<SlotMap>* per_plan, std::vector<int32_t>* off) {
   std::vector<int32_t> count(n_points + 1, 0);

@@ -1,5 +1,6 @@
 // Shared by the resident kernels (solver_resident.cu, adjoint_resident.cu):
-// one tile per CTA for a whole run, two CTAs per SM, cooperative launch.
+// every tile stays on one CTA for a whole run, two tiles per SM, cooperative
+// launch.
 #pragma once
 
 #include "gridsync.cuh"
@@ -11,7 +12,7 @@ namespace agb {
 
 static_assert(kResidentCounters == 2 + kPlaceWords, "barrier and placement");
 
-// Warps per tile (two CTAs per SM): 8 in FP32; FP64 is bound by its
+// Warps per tile (two tiles per SM): 8 in FP32; FP64 is bound by its
 // arithmetic pipe, which 8 warps per SM fill: 4.  Meshes with fewer tiles
 // than CTAs are cut finer first (split_tiles in prep.cpp): a whole tile's
 // groups are issue-bound on one SM while others idle.
@@ -60,19 +61,20 @@ size_t records_bytes(const ResidentPlan& p) {
 }
 
 template <int MAT>
-__device__ __forceinline__ void keep_records(const FemView& fv, int tile, int max_elems, float4* srec, int* sgrp) {
+__device__ __forceinline__ void keep_records(const FemView& fv, int tile, int max_elems, float4* srec, int* sgrp,
+                                             int tid, int threads) {
   const int e0 = fv.tile_estart[tile], ne = fv.tile_estart[tile + 1] - e0;
   const int gs = fv.tile_gstart[tile], ge = fv.tile_gstart[tile + 1];
   const float4* rec = static_cast<const float4*>(fv.rec);
   const float4* act = static_cast<const float4*>(fv.act);
   const size_t nc = (size_t)fv.n_cells;
-  for (int i = threadIdx.x; i < ne; i += blockDim.x) {
+  for (int i = tid; i < ne; i += threads) {
 #pragma unroll
     for (int k = 0; k < 3; ++k) srec[(size_t)k * max_elems + i] = __ldg(rec + k * nc + e0 + i);
 #pragma unroll
     for (int k = 3; k < kRecStreams<MAT>; ++k) srec[(size_t)k * max_elems + i] = __ldg(act + (k - 3) * nc + e0 + i);
   }
-  for (int i = threadIdx.x; i <= ge - gs; i += blockDim.x) sgrp[i] = fv.group_estart[gs + i] - e0;
+  for (int i = tid; i <= ge - gs; i += threads) sgrp[i] = fv.group_estart[gs + i] - e0;
 }
 
 // The record of this lane in warp group q, and the group's size: from shared
@@ -111,7 +113,7 @@ struct GroupLoader {
 };
 
 // The first shape (1: FP32 records in shared memory; 2, or 1 in FP64: not)
-// whose CTAs, one per tile, fit the device at once, into p->shape; 0 if none
+// whose CTAs fit the device at once, into p->shape; 0 if none
 // does (too many tiles, or tiles with too many elements).
 template <class ShapeOf>
 cudaError_t choose_shape(const SolveArgs& a, ResidentPlan* p, ShapeOf shape_of) {
@@ -133,7 +135,7 @@ cudaError_t choose_shape(const SolveArgs& a, ResidentPlan* p, ShapeOf shape_of) 
     e = allow_max_smem(sh.kernel);
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, sh.kernel, sh.threads, sh.smem);
     if (e != cudaSuccess) return e;
-    if ((int64_t)a.fv.n_tiles <= (int64_t)occ * sms) {
+    if ((int64_t)sh.blocks <= (int64_t)occ * sms) {
       p->shape = k;
       return cudaSuccess;
     }

@@ -143,13 +143,14 @@ cudaError_t launch_solver_force_refresh(const SolveArgs& a, cudaStream_t s);
 // the iteration limit, termination or a due refresh.  resident_prepare fills
 // `shape` when every tile's CTA fits the device at once (0: it does not) from
 // the largest tile's elements and warp groups; part_d and part_v hold 6 and
-// 12 partials per tile, counters kResidentCounters zeroed words.
+// 12 partials for kResidentMaxTiles CTAs, counters kResidentCounters zeroed words.
 constexpr int kResidentMaxTiles = 2 * 152;  // two CTAs on each of the 152 SMs
 struct ResidentPlan {
   int shape = 0;
   int max_elems = 0;
   int max_groups = 0;
-  int whole = 0;  // the first tiles are this many whole ones, the others cut (0: all alike)
+  int whole = 0;  // FP32: the first tiles are this many whole ones, the others cut (0: all alike)
+  const int32_t* order = nullptr;  // FP64 with more tiles than SMs: pair_tiles()
 };
 // words of `counters` below
 constexpr int kResidentCounters = 4 + 256;
@@ -313,6 +314,7 @@ struct agb_solver {
   int32_t* d_piece_vid = nullptr;
   int32_t* d_piece_slot = nullptr;
   int32_t* d_piece_off = nullptr;
+  int32_t* d_piece_order = nullptr;
   bool has_state = false;  // vertex state written (reset or checkpoint load)
   uint64_t fingerprint = 0;  // of the model and parameters, checked by agb_solver_load
 };

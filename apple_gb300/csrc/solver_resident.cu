@@ -13,7 +13,7 @@
 //   -- barrier: sums, alpha_0, Armijo step t --
 //   gradient    x <- x + t p; forces and clamped diagonal -> slots
 //   -- barrier --
-//   vertex      the first tile that holds a vertex sums its slots, writes
+//   vertex      one of the tiles that hold a vertex sums its slots, writes
 //               (g, d) and adds the 12 dot products
 //   -- barrier: sums, beta, preconditioner mean, termination --
 //
@@ -26,11 +26,13 @@
 // for bit.
 //
 // Measured (40 iterations with the reset and the refreshes): 5,000-tet cube in
-// FP32 833 us against 1,369 with the three-kernel loop, 138,240 tets 1,176
-// against 1,976; 20 iterations of 138,240 tets in FP64 4,458 against 7,306.
+// FP32 807 us against 1,371 with the three-kernel loop, 138,240 tets 1,139
+// against 1,968; 20 iterations of 138,240 tets in FP64 3,955 against 7,303.
 // An iteration of the cube takes 15.7 us, of which the three barriers are 4,
 // the element groups 3, the sums 1.3 and the two decisions 2.5.
 #include <math.h>
+
+#include <algorithm>
 
 #include "gridsync.cuh"
 #include "resident.cuh"
@@ -57,14 +59,27 @@ constexpr size_t resident_smem(int nw) {
 
 // REC: the tile's element records stay in shared memory after the first read;
 // otherwise each group's records are loaded one group ahead.
-template <class R, int MAT, bool DELTA, int NW, bool REC>
-__global__ void __launch_bounds__(32 * NW, 2) solver_resident_kernel(SolveArgs a, int max_elems, int whole,
-                                                                                     void* part_d, void* part_v,
-                                                                                     unsigned* counters) {
-  constexpr int T = 32 * NW, ND = 6, NVT = 12, kSlotBatch = 4;
+//
+// SHARE: how tiles share an SM.  kTwoCtas, FP32: two CTAs of a tile each, which
+// run apart between the barriers (as halves of one CTA 108k tets took 1,117
+// against 1,086 us, 138k 1,158 against 1,144).  kTwoTiles, FP64 with more tiles
+// than SMs: the halves of one CTA hold a tile each, paired by their size.  The
+// SM has one FP64 pipe (19 cycles per warp instruction from four warps on), and
+// the CTA takes the grid's sums and the decisions once: with the vertex sums packed (below) 138k tets
+// 4,153 -> 3,955 us for 20 iterations, 80k 5,910 -> 5,297 for 40.  kAlone, FP64 with at
+// most a tile per SM.
+enum Share { kAlone, kTwoCtas, kTwoTiles };
+
+template <class R, int MAT, bool DELTA, int NW, bool REC, Share SHARE>
+__global__ void __launch_bounds__(32 * NW * (SHARE == kTwoTiles ? 2 : 1), SHARE == kTwoCtas ? 2 : 1)
+    solver_resident_kernel(SolveArgs a, int max_elems, int tile_smem, int whole, const int32_t* __restrict__ order,
+                           void* part_d, void* part_v, unsigned* counters) {
+  constexpr int T = 32 * NW, ND = 6, NVT = 12, kSlotBatch = 4;  // T threads per tile
+  constexpr int TILES = SHARE == kTwoTiles ? 2 : 1, TC = T * TILES;
   constexpr unsigned FFD = 0x2u, FFV = (1u << 1) | (1u << 6) | (1u << 8) | (1u << 9);
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  V4<R>* s4 = reinterpret_cast<V4<R>*>(smem_raw);           // staging
+  const int half = TILES == 2 ? (int)threadIdx.x / T : 0;
+  V4<R>* s4 = reinterpret_cast<V4<R>*>(smem_raw + (size_t)half * tile_smem);  // staging
   V4<R>* acc4 = s4 + kTileVerts;                            // [warp][vertex]: gx gy gz dx
   V2<R>* s2 = reinterpret_cast<V2<R>*>(acc4 + NW * kTileVerts);
   V2<R>* acc2 = s2 + kTileVerts;                            // [warp][vertex]: dy dz
@@ -72,10 +87,14 @@ __global__ void __launch_bounds__(32 * NW, 2) solver_resident_kernel(SolveArgs a
   int* vi = reinterpret_cast<int*>(vw + kVertexWords<DELTA> * kTileVerts);  // vertex, slot, first and end slot
   float4* srec = reinterpret_cast<float4*>(vi + 4 * kTileVerts);  // REC: [stream][element]
   int* sgrp = reinterpret_cast<int*>(srec + (size_t)kRecStreams<MAT> * max_elems);  // REC: group starts
-  R* const rows = reinterpret_cast<R*>(acc4);  // the block sums' terms, while no accumulation runs
-  static_assert(NW * kTileVerts * sizeof(V4<R>) >= (NVT + 1) * T * sizeof(R), "rows fit the accumulators");
+  // the block sums' terms, in the first tile's accumulators while no accumulation runs
+  R* const rows = reinterpret_cast<R*>(reinterpret_cast<V4<R>*>(smem_raw) + kTileVerts);
+  static_assert(NW * kTileVerts * sizeof(V4<R>) >= (NVT + 1) * TC * sizeof(R), "rows fit the accumulators");
   __shared__ Acc<R> tot[NVT];
   __shared__ SolverState sst;
+  __shared__ uint8_t s_own[TILES][kTileVerts];  // the tile vertices that this tile sums
+  __shared__ int s_owned[TILES][NW];
+  uint8_t* const own = s_own[half];
   R* const xh = vw;
   R* const xl = vw + 3 * kTileVerts;
   R* const vp = vw + 6 * kTileVerts;
@@ -84,15 +103,23 @@ __global__ void __launch_bounds__(32 * NW, 2) solver_resident_kernel(SolveArgs a
   R* const xr = vw + 13 * kTileVerts;  // DELTA only
 
   if (a.st->done) return;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  __shared__ int s_tile;
-  if (tid == 0) s_tile = whole > 0 ? place_cta(counters, whole, gridDim.x) : (int)blockIdx.x;
-  __syncthreads();
-  const int tile = s_tile;
-  const int gs = a.fv.tile_gstart[tile], ge = a.fv.tile_gstart[tile + 1];
-  const int vs = a.fv.tile_vstart[tile], nv = a.fv.tile_vstart[tile + 1] - vs;
+  const int tid = (int)threadIdx.x - half * T, warp = tid >> 5, lane = tid & 31;  // within the tile's threads
+  int tile = blockIdx.x;
+  if constexpr (SHARE == kTwoCtas) {
+    __shared__ int s_tile;
+    if (whole > 0) {
+      if (threadIdx.x == 0) s_tile = place_cta(counters, whole, gridDim.x);
+      __syncthreads();
+      tile = s_tile;
+    }
+  } else if constexpr (SHARE == kTwoTiles) {
+    tile = order[2 * blockIdx.x + half];  // -1: the half takes part in the CTA's sums and barriers only
+  }
+  const int gs = tile < 0 ? 0 : a.fv.tile_gstart[tile], ge = tile < 0 ? 0 : a.fv.tile_gstart[tile + 1];
+  const int vs = tile < 0 ? 0 : a.fv.tile_vstart[tile], nv = tile < 0 ? 0 : a.fv.tile_vstart[tile + 1] - vs;
+  const int me = SHARE == kTwoCtas ? tile : (int)blockIdx.x;  // the place of the CTA's partials
   GridBar bar{counters, kResidentCounters, gridDim.x, 0};
-  if (tid < kStateWords) ((uint32_t*)&sst)[tid] = ((const uint32_t*)a.st)[tid];
+  if (threadIdx.x < kStateWords) ((uint32_t*)&sst)[threadIdx.x] = ((const uint32_t*)a.st)[threadIdx.x];
   __syncthreads();
   const V4<R>* XA = (const V4<R>*)a.xa;
   V4<R>* GD = (V4<R>*)a.gd;
@@ -126,12 +153,30 @@ __global__ void __launch_bounds__(32 * NW, 2) solver_resident_kernel(SolveArgs a
       }
     }
   }
-  if constexpr (REC) keep_records<MAT>(a.fv, tile, max_elems, srec, sgrp);
+  // FP64 sums its vertices without the gaps that other tiles' ones leave in the
+  // warps (FP32 takes a tile's vertices in one turn anyhow)
+  constexpr bool PACK = sizeof(R) == 8;
+  int n_own = PACK ? 0 : nv;
+  for (int i0 = 0; PACK && i0 < kTileVerts; i0 += T) {  // both halves take every turn
+    const int i = i0 + tid;
+    const bool mine = i < nv && vi[2 * kTileVerts + i] != vi[3 * kTileVerts + i];  // this thread's own stores
+    const unsigned m = __ballot_sync(0xffffffffu, mine);
+    if (lane == 0) s_owned[half][warp] = __popc(m);
+    __syncthreads();
+    int k = n_own + __popc(m & ((1u << lane) - 1u));
+    for (int w = 0; w < NW; ++w) {
+      if (w < warp) k += s_owned[half][w];
+      n_own += s_owned[half][w];
+    }
+    if (mine) own[k] = (uint8_t)i;
+    __syncthreads();
+  }
+  if (REC && tile >= 0) keep_records<MAT>(a.fv, tile, max_elems, srec, sgrp, tid, T);
   const GroupLoader<R, MAT, REC> load_group{a.fv, gs, max_elems, srec, sgrp};
   // The accumulators are cleared while a barrier is waited for: those that
   // the block sums' rows overlay after the direction pass, the others after
   // the vertex pass.
-  constexpr int kRowCopies = (int)(((NVT + 1) * T * sizeof(R) + kTileVerts * sizeof(V4<R>) - 1) /
+  constexpr int kRowCopies = (int)(((NVT + 1) * TC * sizeof(R) + kTileVerts * sizeof(V4<R>) - 1) /
                                    (kTileVerts * sizeof(V4<R>)));
   auto zero4 = [&](int w) {
     for (int i = tid; i < nv; i += T) acc4[w * kTileVerts + i] = V4<R>{R(0), R(0), R(0), R(0)};
@@ -143,9 +188,10 @@ __global__ void __launch_bounds__(32 * NW, 2) solver_resident_kernel(SolveArgs a
   };
   zero_rest();
   __syncthreads();  // every thread has read sst.pbuf; records and groups are in place
-  if (tid == 0) sst.refresh = 0;  // the refresh passes, if any, ran after the last vertex pass
+  if (threadIdx.x == 0) sst.refresh = 0;  // the refresh passes, if any, ran after the last vertex pass
 
-  const int w0 = decision_warp<NW>();
+  // two CTAs of an SM decide on different schedulers
+  const int w0 = SHARE == kTwoCtas ? decision_warp<NW>() : 0;
 
   bool ok = true;
   for (;;) {
@@ -216,7 +262,7 @@ __global__ void __launch_bounds__(32 * NW, 2) solver_resident_kernel(SolveArgs a
       } else {
         plain[1] = c2acc.v;
       }
-      cta_partials<ND, FFD, sizeof(R) == 4 ? 1 : -1, T, R>(plain, lo, rows, (AccStore<R>*)part_d, gridDim.x, tile);
+      cta_partials<ND, FFD, sizeof(R) == 4 ? 1 : -1, TC, R>(plain, lo, rows, (AccStore<R>*)part_d, gridDim.x, me);
     }
     bar.arrive();
     for (int w = 0; w < kRowCopies; ++w) zero4(w);
@@ -225,8 +271,8 @@ __global__ void __launch_bounds__(32 * NW, 2) solver_resident_kernel(SolveArgs a
     g = gs + warp;
     n = 0;
     if (!REC && g < ge) load_group(g, n, geo, ids);
-    grid_totals<ND, T, R>((const AccStore<R>*)part_d, gridDim.x, tot);
-    if (warp == w0) dir_decide<MAT, R>(&sst, tot);
+    grid_totals<ND, TC, R>((const AccStore<R>*)part_d, gridDim.x, tot);
+    if (threadIdx.x / 32 == w0) dir_decide<MAT, R>(&sst, tot);
     __syncthreads();
     const R t = to_real<R>(sst.t);
 
@@ -339,25 +385,25 @@ __global__ void __launch_bounds__(32 * NW, 2) solver_resident_kernel(SolveArgs a
     // ---- vertex ----
     {
       R s[NVT] = {};
-      for (int i = tid; i < nv; i += T) {
-        const int s0 = vi[2 * kTileVerts + i], s1 = vi[3 * kTileVerts + i];
+      for (int k = tid; k < n_own; k += T) {
+        const int i = PACK ? own[k] : k, s0 = vi[2 * kTileVerts + i], s1 = vi[3 * kTileVerts + i];
         if (s0 == s1) continue;  // another tile's vertex
         const int v = vi[i];
         V4<R> r{}, f{};
         if constexpr (DELTA) r = ldg4((const V4<R>*)a.gref + v);
         if (a.force) f = ldg4((const V4<R>*)a.force + v);
         R ss[3] = {R(0), R(0), R(0)}, ds[3] = {R(0), R(0), R(0)};
-        for (int k = s0; k < s1; k += kSlotBatch) {  // a batch of slots in flight together
+        for (int b = s0; b < s1; b += kSlotBatch) {  // a batch of slots in flight together
           V4<R> sg[kSlotBatch], sd[kSlotBatch];
 #pragma unroll
           for (int q = 0; q < kSlotBatch; ++q)
-            if (k + q < s1) {
-              sg[q] = ldcg4(slots + 2 * (size_t)(k + q));
-              sd[q] = ldcg4(slots + 2 * (size_t)(k + q) + 1);
+            if (b + q < s1) {
+              sg[q] = ldcg4(slots + 2 * (size_t)(b + q));
+              sd[q] = ldcg4(slots + 2 * (size_t)(b + q) + 1);
             }
 #pragma unroll
           for (int q = 0; q < kSlotBatch; ++q)
-            if (k + q < s1) {
+            if (b + q < s1) {
               ss[0] += sg[q].x;
               ss[1] += sg[q].y;
               ss[2] += sg[q].z;
@@ -377,12 +423,12 @@ __global__ void __launch_bounds__(32 * NW, 2) solver_resident_kernel(SolveArgs a
         GD[2 * v] = V4<R>{gn[0], gn[1], gn[2], R(0)};
         GD[2 * v + 1] = V4<R>{dn[0], dn[1], dn[2], R(0)};
       }
-      cta_partials<NVT, FFV, -1, T, R>(s, R(0), rows, (AccStore<R>*)part_v, gridDim.x, tile);
+      cta_partials<NVT, FFV, -1, TC, R>(s, R(0), rows, (AccStore<R>*)part_v, gridDim.x, me);
     }
     bar.arrive();
     zero_rest();
     if (!(ok = bar.wait())) break;
-    grid_totals<NVT, T, R>((const AccStore<R>*)part_v, gridDim.x, tot);
+    grid_totals<NVT, TC, R>((const AccStore<R>*)part_v, gridDim.x, tot);
     vertex_decide<R>(&sst, tot, w0);
     __syncthreads();
     if (sst.done || sst.iter >= sst.iter_limit || sst.refresh) break;
@@ -399,42 +445,53 @@ __global__ void __launch_bounds__(32 * NW, 2) solver_resident_kernel(SolveArgs a
       X[2 * v + 1] = V4<R>{xl[i], xl[kTileVerts + i], xl[2 * kTileVerts + i], R(0)};
       P[v] = V4<R>{vp[i], vp[kTileVerts + i], vp[2 * kTileVerts + i], R(0)};
     }
-  } else if (tid == 0) {  // a barrier gave up: the solve stops with a device error
+  } else if (threadIdx.x == 0) {  // a barrier gave up: the solve stops with a device error
     atomicMax(&a.st->error, 3);
     a.st->done = 1;
   }
   bar.leave();
 }
 
-using ResidentKernel = void (*)(SolveArgs, int, int, void*, void*, unsigned*);
+using ResidentKernel = void (*)(SolveArgs, int, int, int, const int32_t*, void*, void*, unsigned*);
 
 struct Shape {
   ResidentKernel kernel;
-  int threads;
+  int blocks, threads;
   size_t smem;
+  int tile_smem;
 };
 
 template <class R, int MAT, bool DELTA, int NW, bool REC>
-Shape shape(const ResidentPlan& p) {
+Shape shape(const ResidentPlan& p, int n_tiles) {
   size_t smem = resident_smem<R, DELTA>(NW);
   if (REC) smem += records_bytes<MAT>(p);
-  return Shape{solver_resident_kernel<R, MAT, DELTA, NW, REC>, 32 * NW, smem};
+  smem = (smem + 15) & ~(size_t)15;
+  if constexpr (sizeof(R) == 4) {
+    return Shape{solver_resident_kernel<R, MAT, DELTA, NW, REC, kTwoCtas>, n_tiles, 32 * NW, smem, 0};
+  } else if (n_tiles > kSMs) {
+    return Shape{solver_resident_kernel<R, MAT, DELTA, NW, REC, kTwoTiles>, kSMs, 64 * NW, 2 * smem, (int)smem};
+  } else {
+    // more shared memory than half an SM's: no two CTAs share an SM while others idle
+    return Shape{solver_resident_kernel<R, MAT, DELTA, NW, REC, kAlone>, n_tiles, 32 * NW,
+                 std::max(smem, (size_t)120 * 1024), 0};
+  }
 }
 
 template <int MAT, bool DELTA>
-Shape shape_f32(const ResidentPlan& p) {
+Shape shape_f32(const ResidentPlan& p, int nt) {
   constexpr int W = kResidentWarps<float>;
-  return p.shape == 1 ? shape<float, MAT, DELTA, W, true>(p) : shape<float, MAT, DELTA, W, false>(p);
+  return p.shape == 1 ? shape<float, MAT, DELTA, W, true>(p, nt) : shape<float, MAT, DELTA, W, false>(p, nt);
 }
 
 Shape shape_of(const SolveArgs& a, const ResidentPlan& p) {
   constexpr int SNH = AGB_STABLE_NEO_HOOKEAN, MU = AGB_STABLE_NEO_HOOKEAN_MUSCLE;
   const bool mu = a.fv.material == MU;
+  const int nt = a.fv.n_tiles;
   if (a.precision == AGB_F64)
-    return mu ? shape<double, MU, false, kResidentWarps<double>, false>(p)
-              : shape<double, SNH, false, kResidentWarps<double>, false>(p);
-  if (a.delta) return mu ? shape_f32<MU, true>(p) : shape_f32<SNH, true>(p);
-  return mu ? shape_f32<MU, false>(p) : shape_f32<SNH, false>(p);
+    return mu ? shape<double, MU, false, kResidentWarps<double>, false>(p, nt)
+              : shape<double, SNH, false, kResidentWarps<double>, false>(p, nt);
+  if (a.delta) return mu ? shape_f32<MU, true>(p, nt) : shape_f32<SNH, true>(p, nt);
+  return mu ? shape_f32<MU, false>(p, nt) : shape_f32<SNH, false>(p, nt);
 }
 
 }  // namespace
@@ -453,7 +510,7 @@ cudaError_t launch_resident(const SolveArgs& a, const ResidentPlan& p, void* par
                             cudaStream_t s) {
   if (!p.shape) return cudaErrorInvalidValue;
   const Shape sh = shape_of(a, p);
-  return launch_cooperative(sh.kernel, a.fv.n_tiles, sh.threads, sh.smem, s, a, p.max_elems, p.whole, part_d, part_v,
+  return launch_cooperative(sh.kernel, sh.blocks, sh.threads, sh.smem, s, a, p.max_elems, sh.tile_smem, p.whole, p.order, part_d, part_v,
                             counters);
 }
 
