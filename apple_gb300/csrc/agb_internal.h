@@ -156,16 +156,21 @@ struct agb_fem {
   int material = 0;
   int precision = 0;
   agb::TilePlan plan;
-  agb::SlotMap own_slots;         // slots when used on its own
-  std::vector<int32_t> own_off;
+  // what the evaluation passes run over: in FP64, when all its pieces fit on
+  // the SMs two at a time, the plan cut by split_tiles; else empty, the plan
+  agb::TilePlan pieces;
+  const agb::TilePlan& eval_plan() const { return pieces.n_tiles > 0 ? pieces : plan; }
   // device
   int32_t* d_tile_estart = nullptr;
   int32_t* d_tile_vstart = nullptr;
   int32_t* d_tile_gstart = nullptr;
   int32_t* d_group_estart = nullptr;
   int32_t* d_tv_vid = nullptr;
+  int32_t* d_piece_vstart = nullptr;
+  int32_t* d_piece_gstart = nullptr;
+  int32_t* d_piece_user = nullptr;
   int32_t* d_tv_user = nullptr;   // tile-vertex -> caller's point id
-  int32_t* d_own_slot = nullptr;  // tile-vertex -> slot (standalone)
+  int32_t* d_own_slot = nullptr;  // eval_plan's tile-vertex -> slot (standalone)
   int32_t* d_own_off = nullptr;   // n_points + 1
   void* d_rec = nullptr;
   uint32_t* d_ids = nullptr;
@@ -180,6 +185,7 @@ struct agb_fem {
   double* d_partials = nullptr;
   unsigned* d_counter = nullptr;
   agb::FemView view() const;
+  agb::FemView eval_view() const;
 };
 
 struct agb_model {
@@ -195,7 +201,10 @@ struct agb_model {
   std::vector<double> force_internal;  // n_points x 3 (summed per vertex)
   // device
   int32_t* d_off = nullptr;
+  // evaluation passes (the potentials' eval_plan)
   std::vector<int32_t*> d_slot_of_tv;  // per potential
+  int32_t* d_eval_off = nullptr;
+  int32_t n_eval_slots = 0;
   void* d_fixed = nullptr;             // V4<R> n_points: fixed values, w = mask bits
   void* d_force = nullptr;             // V4<R> n_points or null
   void* d_slots = nullptr;             // up to 9 R per slot

@@ -257,6 +257,19 @@ FemView agb_fem::view() const {
   return v;
 }
 
+FemView agb_fem::eval_view() const {
+  FemView v = view();
+  if (pieces.n_tiles > 0) {
+    v.n_tiles = pieces.n_tiles;
+    v.tile_vstart = d_piece_vstart;
+    v.tile_gstart = d_piece_gstart;
+    v.tv_user = d_piece_user;
+    v.tile_estart = nullptr;  // not read by the evaluation passes
+    v.tv_vid = nullptr;
+  }
+  return v;
+}
+
 extern "C" {
 
 const char* agb_last_error(void) { return agb::last_error(); }
@@ -334,6 +347,7 @@ int agb_fem_destroy(agb_fem* f) {
   if (!f) return AGB_OK;
   for (void* p : {(void*)f->d_tile_estart, (void*)f->d_tile_vstart, (void*)f->d_tile_gstart,
                   (void*)f->d_group_estart, (void*)f->d_tv_vid, (void*)f->d_tv_user,
+                  (void*)f->d_piece_vstart, (void*)f->d_piece_gstart, (void*)f->d_piece_user,
                   (void*)f->d_own_slot, (void*)f->d_own_off, f->d_rec, (void*)f->d_ids, f->d_slots, (void*)f->d_partials, (void*)f->d_counter,
                   (void*)f->d_elem_user, f->d_vol, f->d_act, (void*)f->d_D, (void*)f->d_act_user})
     dfree(p);
@@ -415,30 +429,43 @@ int agb_fem_create(agb_space* space, int material, int precision, int32_t n_cell
                        lamdv.data(), tile_elems, &f->plan);
   if (!rc) spread_banks(&f->plan);
   std::vector<SlotMap> sm;
+  std::vector<int32_t> own_off;
   if (!rc) {
-    build_slots(np, {&f->plan}, &sm, &f->own_off);
-    f->own_slots = sm[0];
+    // An SM's FP64 work goes through one pipe: 214 whole tiles leave some SMs
+    // with two and some with one.
+    if (precision == AGB_F64 && f->plan.n_tiles > 0 && f->plan.n_tiles <= kResidentMaxTiles)
+      split_tiles(f->plan, kResidentMaxTiles / 2, 2, &f->pieces);
+    build_slots(np, {&f->eval_plan()}, &sm, &own_off);
     f->vol_internal.resize(n_cells);
     for (int e = 0; e < n_cells; ++e) f->vol_internal[e] = vol[f->plan.elem_user[e]];
   }
   const TilePlan& P = f->plan;
-  const size_t n_part = (size_t)std::max(P.n_tiles, unpack_blocks(np)) * 2;
+  const TilePlan& E = f->eval_plan();
+  const size_t n_part = (size_t)std::max(E.n_tiles, unpack_blocks(np)) * 2;
   if (!rc) rc = dupload(&f->d_tile_estart, P.tile_estart);
   if (!rc) rc = dupload(&f->d_tile_vstart, P.tile_vstart);
   if (!rc) rc = dupload(&f->d_tile_gstart, P.tile_gstart);
   if (!rc) rc = dupload(&f->d_group_estart, P.group_estart);
   if (!rc) rc = dupload(&f->d_tv_vid, P.tv_vid);
   if (!rc) {
-    std::vector<int32_t> tv_user(P.tv_vid.size());
-    for (size_t i = 0; i < tv_user.size(); ++i) tv_user[i] = space->user_of_internal[P.tv_vid[i]];
-    rc = dupload(&f->d_tv_user, tv_user);
+    auto users = [&](const std::vector<int32_t>& vid, int32_t** out) {
+      std::vector<int32_t> tv_user(vid.size());
+      for (size_t i = 0; i < tv_user.size(); ++i) tv_user[i] = space->user_of_internal[vid[i]];
+      return dupload(out, tv_user);
+    };
+    rc = users(P.tv_vid, &f->d_tv_user);
+    if (!rc && &E != &P) rc = users(E.tv_vid, &f->d_piece_user);
   }
-  if (!rc) rc = dupload(&f->d_own_slot, f->own_slots.slot_of_tv);
-  if (!rc) rc = dupload(&f->d_own_off, f->own_off);
+  if (!rc && &E != &P) {
+    rc = dupload(&f->d_piece_vstart, E.tile_vstart);
+    if (!rc) rc = dupload(&f->d_piece_gstart, E.tile_gstart);
+  }
+  if (!rc) rc = dupload(&f->d_own_slot, sm[0].slot_of_tv);
+  if (!rc) rc = dupload(&f->d_own_off, own_off);
   if (!rc) rc = upload_records(P, precision, &f->d_rec, &f->d_ids);
   if (!rc && material == AGB_STABLE_NEO_HOOKEAN_MUSCLE)
     rc = upload_act(std::vector<double>(6 * (size_t)n_cells, 0.0), (size_t)n_cells, precision, &f->d_act);
-  if (!rc) rc = dalloc_bytes(&f->d_slots, 9 * real_bytes(precision) * (size_t)P.n_tv);
+  if (!rc) rc = dalloc_bytes(&f->d_slots, 9 * real_bytes(precision) * (size_t)E.n_tv);
   if (!rc) rc = dalloc(&f->d_partials, n_part);
   if (!rc) rc = dalloc(&f->d_counter, 1);
   if (!rc && cudaMemset(f->d_counter, 0, sizeof(unsigned)) != cudaSuccess) rc = AGB_E_CUDA;
@@ -550,13 +577,13 @@ static int fem_eval(agb_fem* f, unsigned flags, const void* u, const void* p, do
     if (flags & AGB_FUN) AGB_CHECK_CUDA(cudaMemsetAsync(energy, 0, sizeof(double), s));
     if (flags & AGB_HESS_QUAD) AGB_CHECK_CUDA(cudaMemsetAsync(quad, 0, sizeof(double), s));
   }
-  RC(check_launch(launch_fem_eval(f->precision, f->view(), flags, u, p, nullptr, f->d_own_slot, f->d_slots,
-                                  f->plan.n_tv, f->d_partials, f->d_counter, energy, quad, assign, s),
+  RC(check_launch(launch_fem_eval(f->precision, f->eval_view(), flags, u, p, nullptr, f->d_own_slot, f->d_slots,
+                                  f->eval_plan().n_tv, f->d_partials, f->d_counter, energy, quad, assign, s),
                   "fem_eval"));
   const unsigned vec = flags & (AGB_GRAD | AGB_HESS_DIAG | AGB_HESS_PROD);
   if (vec)
     RC(check_launch(launch_unpack(f->precision, np, f->space->d_user_of_internal, f->d_own_off, f->d_slots,
-                                  f->plan.n_tv, vec, grad, diag, prod, nullptr, assign, nullptr, u, f->d_partials, f->d_counter,
+                                  f->eval_plan().n_tv, vec, grad, diag, prod, nullptr, assign, nullptr, u, f->d_partials, f->d_counter,
                                   nullptr, s),
                     "unpack"));
   return AGB_OK;
@@ -594,7 +621,7 @@ int agb_fem_hess_quad(agb_fem* f, const void* u, const void* p, double* out, voi
 int agb_model_destroy(agb_model* m) {
   if (!m) return AGB_OK;
   for (int32_t* p : m->d_slot_of_tv) dfree(p);
-  for (void* p : {(void*)m->d_off, m->d_fixed, m->d_force, m->d_slots,
+  for (void* p : {(void*)m->d_off, (void*)m->d_eval_off, m->d_fixed, m->d_force, m->d_slots,
                   (void*)m->d_partials, (void*)m->d_counter})
     dfree(p);
   delete m;
@@ -654,8 +681,17 @@ int agb_model_create(agb_space* space, int precision, int32_t n_pot, agb_fem* co
   m->n_force = n_force;
   const size_t v4 = v4_bytes(prec);
   int rc = dupload(&m->d_off, m->off);
-  m->d_slot_of_tv.assign(n_pot, nullptr);
-  for (int k = 0; k < n_pot && !rc; ++k) rc = dupload(&m->d_slot_of_tv[k], m->slots[k].slot_of_tv);
+  {
+    std::vector<const TilePlan*> eval_plans;
+    for (agb_fem* f : m->fems) eval_plans.push_back(&f->eval_plan());
+    std::vector<SlotMap> maps;
+    std::vector<int32_t> off;
+    build_slots(np, eval_plans, &maps, &off);
+    m->n_eval_slots = off[np];
+    m->d_slot_of_tv.assign(n_pot, nullptr);
+    if (!rc) rc = dupload(&m->d_eval_off, off);
+    for (int k = 0; k < n_pot && !rc; ++k) rc = dupload(&m->d_slot_of_tv[k], maps[k].slot_of_tv);
+  }
   if (!rc) rc = dalloc_bytes(&m->d_fixed, v4 * np);
   if (!rc) {
     if (prec == AGB_F64) {
@@ -679,9 +715,9 @@ int agb_model_create(agb_space* space, int precision, int32_t n_pot, agb_fem* co
     }
   }
   int max_tiles = 0;
-  for (agb_fem* f : m->fems) max_tiles = std::max(max_tiles, f->plan.n_tiles);
+  for (agb_fem* f : m->fems) max_tiles = std::max(max_tiles, f->eval_plan().n_tiles);
   const size_t n_part = (size_t)std::max(max_tiles, unpack_blocks(np)) * 2;
-  if (!rc) rc = dalloc_bytes(&m->d_slots, 9 * real_bytes(prec) * (size_t)m->n_slots);
+  if (!rc) rc = dalloc_bytes(&m->d_slots, 9 * real_bytes(prec) * (size_t)m->n_eval_slots);
   if (!rc) rc = dalloc(&m->d_partials, n_part);
   if (!rc) rc = dalloc(&m->d_counter, 1);
   if (!rc && cudaMemset(m->d_counter, 0, sizeof(unsigned)) != cudaSuccess) rc = AGB_E_CUDA;
@@ -738,15 +774,15 @@ static int model_eval(agb_model* m, unsigned flags, const int32_t* slot, const v
   if (!flags) return AGB_OK;
   int assign = 1;
   for (size_t k = 0; k < m->fems.size(); ++k) {
-    RC(check_launch(launch_fem_eval(m->precision, m->fems[k]->view(), flags, u, p, slot, m->d_slot_of_tv[k], m->d_slots,
-                                    m->n_slots, m->d_partials, m->d_counter, energy, quad, assign, s),
+    RC(check_launch(launch_fem_eval(m->precision, m->fems[k]->eval_view(), flags, u, p, slot, m->d_slot_of_tv[k], m->d_slots,
+                                    m->n_eval_slots, m->d_partials, m->d_counter, energy, quad, assign, s),
                     "fem_eval"));
     if (m->fems[k]->plan.n_tiles > 0) assign = 0;
   }
   const unsigned vec = flags & (AGB_GRAD | AGB_HESS_DIAG | AGB_HESS_PROD | AGB_FUN);
   const bool ext = m->d_force != nullptr;
   if ((vec & ~AGB_FUN) || (ext && (flags & AGB_FUN)))
-    RC(check_launch(launch_unpack(m->precision, np, m->space->d_user_of_internal, m->d_off, m->d_slots, m->n_slots,
+    RC(check_launch(launch_unpack(m->precision, np, m->space->d_user_of_internal, m->d_eval_off, m->d_slots, m->n_eval_slots,
                                   vec, grad, diag, prod, slot, 1, m->d_force, u, m->d_partials, m->d_counter, energy, s),
                     "unpack"));
   return AGB_OK;

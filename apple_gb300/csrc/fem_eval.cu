@@ -96,9 +96,9 @@ constexpr size_t eval_smem_bytes(int warps) {
 // with the vector branches compiled in, the invariants are formed the same
 // way, and the energy and p^T H p have the same element values whatever else
 // is asked for.
-// Measured, all five quantities on the 1.5M-tet grid in FP32: element pass 81 us
-// (119 us with shared-memory float atomics on one accumulator), the call
-// 130 us (170 us with that, a packing pass and separate zeroing).
+// Measured, all five quantities on the 1.5M-tet grid in FP32: the call 90 us
+// (170 us with shared-memory float atomics on one accumulator, a packing pass
+// and separate zeroing).
 template <class R, int MAT, int NVEC, int MAXT>
 __global__ void __launch_bounds__(MAXT, MAXT == 128 ? (sizeof(R) == 4 ? 5 : 2) : 1) fem_eval_kernel(
     FemView fv, unsigned flags, const R* __restrict__ u, const R* __restrict__ p,
@@ -376,11 +376,15 @@ unsigned vec_mask(unsigned flags) {
 
 // Warps per tile.  With at least two tiles per SM, four (five CTAs per SM
 // keep the SM busy, and fewer accumulator copies are summed); below that the
-// SMs have room, and more warps shorten each tile's chain of groups: 8 up to
-// two tiles per SM, 16 (FP32; 8 in FP64, by shared memory) up to one.
+// SMs have room, and in FP32 more warps shorten each tile's chain of groups: 8
+// up to two tiles per SM, 16 up to one.  FP64 tiles arrive cut (eval_view):
+// four warps, which fill the pipe, so that two CTAs share an SM, and 8 up to
+// one tile per SM.  All five quantities of 138k tets in FP64: 245 us with 214
+// whole tiles of 8 warps, 184 us with 275 pieces of 4.
 int eval_warps(int precision, int n_tiles) {
   if (n_tiles > 2 * kSMs) return 4;
-  return n_tiles > kSMs || precision == AGB_F64 ? 8 : 16;
+  if (precision == AGB_F64) return n_tiles > kSMs ? 4 : 8;
+  return n_tiles > kSMs ? 8 : 16;
 }
 
 template <class R, int MAT, int NVEC, int MAXT>

@@ -65,9 +65,9 @@ constexpr size_t resident_smem(int nw) {
 // against 1,086 us, 138k 1,158 against 1,144).  kTwoTiles, FP64 with more tiles
 // than SMs: the halves of one CTA hold a tile each, paired by their size.  The
 // SM has one FP64 pipe (19 cycles per warp instruction from four warps on), and
-// the CTA takes the grid's sums and the decisions once: with the vertex sums packed (below) 138k tets
-// 4,153 -> 3,955 us for 20 iterations, 80k 5,910 -> 5,297 for 40.  kAlone, FP64 with at
-// most a tile per SM.
+// the CTA takes the grid's sums and the decisions once: with the vertex sums
+// packed (below) 138k tets 4,153 -> 3,955 us for 20 iterations, 80k 5,910 ->
+// 5,297 for 40.  kAlone, FP64 with at most a tile per SM.
 enum Share { kAlone, kTwoCtas, kTwoTiles };
 
 template <class R, int MAT, bool DELTA, int NW, bool REC, Share SHARE>
