@@ -1114,6 +1114,16 @@ int agb_solver_reset(agb_solver* sv, const void* u, void* stream) {
   return AGB_OK;
 }
 
+// ARAP: whether alpha_0 is expected to be accepted, so that the fallback
+// passes belong outside the loop.  On a quadratic, overstep s times the
+// minimiser decreases the energy by s (1 - s / 2) |g.p| alpha, enough for
+// Armijo while s <= 2 (1 - c).  20 iterations, passes apart against in one
+// body: accepted steps 882 / 979 us on 5k tets and 2,095 / 2,252 on 737k;
+// every step rejected (s = 4) 2,039 / 1,869 and 4,516 / 4,270.
+static bool arap_apart(const agb_solver* sv) {
+  return sv->args.fv.material == AGB_ARAP && sv->params.overstep <= 2.0 * (1.0 - sv->params.armijo_c);
+}
+
 // Capture into `graph` after `deps` (which may be empty): the three passes
 // of one iteration (refresh = false) or the two refresh passes as plain
 // launches (refresh = true); for resident iterations their launch and the
@@ -1139,7 +1149,7 @@ static cudaError_t capture_into(agb_solver* sv, cudaGraph_t graph, const cudaGra
     e = cudaStreamEndCapture(cs, &captured);
     return e == cudaSuccess ? le : e;
   }
-  if (a.fv.material == AGB_ARAP) {
+  if (arap_apart(sv)) {
     cudaError_t le = launch_solver_arap_part(a, refresh, cs);
     cudaGraph_t captured = nullptr;
     e = cudaStreamEndCapture(cs, &captured);
@@ -1181,7 +1191,8 @@ static cudaError_t add_conditional(cudaGraph_t g, const cudaGraphNode_t* deps, s
 // ARAP: WHILE(outer) { WHILE(c) { direction, speculative gradient, vertex };
 // trial passes, gradient, vertex }: the inner loop runs while alpha_0 is
 // accepted, so the five fallback passes are launched only after a rejection
-// (idle, they took 25 of 268 us per iteration on 1,966,080 tets).
+// (idle, they took 25 of 268 us per iteration on 1,966,080 tets); in one body
+// where alpha_0 is expected to be rejected (arap_apart).
 static int build_loop_graph(agb_solver* sv) {
   cudaGraph_t g = nullptr;
   AGB_CHECK_CUDA(cudaGraphCreate(&g, 0));
@@ -1196,7 +1207,7 @@ static int build_loop_graph(agb_solver* sv) {
     SolveArgs ar = a;
     ar.cond_outer = (unsigned long long)h_out;
     if (e == cudaSuccess) e = capture_into(sv, body_out, nullptr, 0, ar, true);
-  } else if (a.delta || a.fv.material == AGB_ARAP) {
+  } else if (a.delta || arap_apart(sv)) {
     e = cudaGraphConditionalHandleCreate(&h_out, g, 1u, cudaGraphCondAssignDefault);
     if (e == cudaSuccess) e = add_conditional(g, nullptr, 0, h_out, cudaGraphCondTypeWhile, &w_out, &body_out);
     if (e == cudaSuccess) e = cudaGraphConditionalHandleCreate(&h_in, body_out, 1u, cudaGraphCondAssignDefault);
