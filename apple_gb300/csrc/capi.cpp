@@ -814,14 +814,24 @@ void agb_pncg_default_params(agb_pncg_params* p) {
   p->refresh_ratio = -1.0;
 }
 
-int agb_solver_destroy(agb_solver* sv) {
-  if (!sv) return AGB_OK;
-  if (sv->loop_exec) cudaGraphExecDestroy(sv->loop_exec);
-  if (sv->cg_exec) cudaGraphExecDestroy(sv->cg_exec);
+// the adjoint CG's buffers, as before its first call
+static void cg_release(agb_solver* sv) {
   for (void* p : {sv->d_cg, sv->d_cg_part, (void*)sv->d_cg_cnt, (void*)sv->d_cg_state, sv->d_cg_res_part,
                   (void*)sv->d_cg_res_counters})
     dfree(p);
   if (sv->h_cg_state) cudaFreeHost(sv->h_cg_state);
+  sv->d_cg = sv->d_cg_part = sv->d_cg_res_part = nullptr;
+  sv->d_cg_cnt = sv->d_cg_res_counters = nullptr;
+  sv->d_cg_state = sv->h_cg_state = nullptr;
+  sv->cg_resident = ResidentPlan{};
+  sv->cg_ready = false;
+}
+
+int agb_solver_destroy(agb_solver* sv) {
+  if (!sv) return AGB_OK;
+  if (sv->loop_exec) cudaGraphExecDestroy(sv->loop_exec);
+  if (sv->cg_exec) cudaGraphExecDestroy(sv->cg_exec);
+  cg_release(sv);
   if (sv->step_exec) cudaGraphExecDestroy(sv->step_exec);
   if (sv->capture_stream) cudaStreamDestroy(sv->capture_stream);
   for (void* p : {(void*)sv->d_tile_estart, (void*)sv->d_tile_vstart, (void*)sv->d_tile_gstart,
@@ -1520,7 +1530,7 @@ void agb_cg_default_params(agb_cg_params* p) {
 }
 
 static int cg_setup(agb_solver* sv) {
-  if (sv->d_cg) return AGB_OK;
+  if (sv->cg_ready) return AGB_OK;
   clear_error();
   const int np = sv->args.n_points;
   const size_t v4 = v4_bytes(sv->precision);
@@ -1545,6 +1555,7 @@ static int cg_setup(agb_solver* sv) {
   }
   if (rc) {
     if (rc == AGB_E_CUDA && agb::last_error()[0] == 0) set_error("agb_solver_adjoint: CUDA allocation failed");
+    cg_release(sv);  // the next call starts afresh
     return rc;
   }
   CgArgs& c = sv->cg;
@@ -1562,6 +1573,7 @@ static int cg_setup(agb_solver* sv) {
   c.cs = sv->d_cg_state;
   c.vblocks = vblocks;
   c.cond = 0;
+  sv->cg_ready = true;
   return AGB_OK;
 }
 

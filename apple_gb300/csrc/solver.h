@@ -288,6 +288,7 @@ struct agb_solver {
   agb::SolveArgs args{};   // the iterations' tiles (split ones for resident iterations)
   agb::SolveArgs whole{};  // the whole tiles: reset, energy, adjoint CG
   // adjoint CG (allocated on first use)
+  bool cg_ready = false;           // the buffers and arguments below are complete
   void* d_cg = nullptr;            // lam, res, q, minv, p0, p1: 6 x V4<R> x n_points
   void* d_cg_part = nullptr;
   unsigned* d_cg_cnt = nullptr;
