@@ -38,15 +38,20 @@ int upload(void* d, const void* h, size_t bytes) {
   return AGB_OK;
 }
 
+void dfree(void* p) {
+  if (p) cudaFree(p);
+}
+
+// a new device array with h's contents
 template <class T>
 int dupload(T** d, const std::vector<T>& h) {
   int rc = dalloc(d, h.size());
-  if (rc) return rc;
-  return upload(*d, h.data(), h.size() * sizeof(T));
-}
-
-void dfree(void* p) {
-  if (p) cudaFree(p);
+  if (!rc) rc = upload(*d, h.data(), h.size() * sizeof(T));
+  if (rc) {  // *d is null or complete
+    dfree(*d);
+    *d = nullptr;
+  }
+  return rc;
 }
 
 #define RC(call)           \
@@ -153,15 +158,11 @@ std::vector<R> pack_v4(const std::vector<double>& xyz, const std::vector<uint8_t
 
 // internal -> caller cell index and dV * fraction on the device (first use)
 int ensure_vjp_tables(agb_fem* f) {
-  if (f->d_elem_user) return AGB_OK;
-  RC(dupload(&f->d_elem_user, f->plan.elem_user));
-  if (f->precision == AGB_F64) {
-    RC(dalloc_bytes(&f->d_vol, 8 * f->vol_internal.size()));
-    return upload(f->d_vol, f->vol_internal.data(), 8 * f->vol_internal.size());
-  }
-  std::vector<float> v(f->vol_internal.begin(), f->vol_internal.end());
-  RC(dalloc_bytes(&f->d_vol, 4 * v.size()));
-  return upload(f->d_vol, v.data(), 4 * v.size());
+  if (!f->d_elem_user) RC(dupload(&f->d_elem_user, f->plan.elem_user));
+  if (f->d_vol) return AGB_OK;
+  const std::vector<double>& v = f->vol_internal;
+  if (f->precision == AGB_F64) return dupload((double**)&f->d_vol, v);
+  return dupload((float**)&f->d_vol, std::vector<float>(v.begin(), v.end()));
 }
 
 // the activation per internal element (6 each) of a muscle potential, read

@@ -67,6 +67,53 @@ int main() {
 }
 """
 
+MATERIAL_GRADIENT = r"""
+#include "host_fakes.h"
+using namespace agb;
+static int launches = 0, bad = 0;
+static bool has(const void* p) { return p && fake::live.count((void*)p); }
+namespace agb {
+cudaError_t launch_param_vjp(const FemView& fv, int precision, const void*, const void*, const void* vol,
+                             const int32_t* elem_user, void*, void*, cudaStream_t) {
+  ++launches;
+  if (!has(vol) || !has(elem_user)) ++bad;
+  else if (elem_user[0] < 0 || elem_user[0] >= fv.n_cells) ++bad;
+  else if ((precision == AGB_F64 ? *(const double*)vol : *(const float*)vol) <= 0) ++bad;
+  return cudaSuccess;
+}
+}
+
+int main() {
+  FakeMesh m(2);
+  for (int precision : {AGB_F32, AGB_F64})
+    for (int k = 1;; ++k) {
+      agb_space* s = nullptr; agb_fem* f = nullptr;
+      if (agb_space_create(m.n_points(), m.points.data(), &s)) return 1;
+      if (agb_fem_create(s, AGB_STABLE_NEO_HOOKEAN, precision, m.n_cells(), m.cells.data(), m.points.data(), nullptr,
+                         nullptr, nullptr, m.mu.data(), m.lam.data(), 0, &f)) return 2;
+      double x[1] = {0};
+      launches = 0;
+      fake::fail_at = k;
+      const int rc = agb_fem_grad_param_vjp(f, x, x, x, x, nullptr);
+      const bool failed = fake::fail_at == 0;
+      fake::fail_at = 0;
+      if (failed && (rc == AGB_OK || launches)) { printf("allocation %d: rc %d\n", k, rc); return 5; }
+      if (agb_fem_grad_param_vjp(f, x, x, x, x, nullptr) || bad || !launches) {
+        printf("allocation %d: the next call ran on half-made tables\n", k);
+        return 7;
+      }
+      agb_fem_destroy(f);
+      agb_space_destroy(s);
+      if (!fake::live.empty()) return 6;
+      if (!failed) {
+        if (k < 3) return 8;
+        break;
+      }
+    }
+  return 0;
+}
+"""
+
 
 def _run(tmp_path, program):
     cpp = tmp_path / "check.cpp"
@@ -81,6 +128,6 @@ def _run(tmp_path, program):
     assert r.returncode == 0, (r.returncode, r.stdout)
 
 
-@pytest.mark.parametrize("program", [ADJOINT], ids=["adjoint"])
+@pytest.mark.parametrize("program", [ADJOINT, MATERIAL_GRADIENT], ids=["adjoint", "material_gradient"])
 def test_a_failed_allocation_leaves_nothing_half_made(tmp_path, program):
     _run(tmp_path, program)
