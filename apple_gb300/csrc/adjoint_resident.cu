@@ -58,7 +58,7 @@ __device__ __forceinline__ void bar_arrive(int id, int threads) {
 
 template <class R, int MAT, int NW, bool REC>
 __global__ void __launch_bounds__(32 * NW, 2) cg_resident_kernel(CgArgs c, int max_elems, void* part_p, void* part_v,
-                                                                unsigned* counters) {
+                                                                unsigned* counters, uint64_t wait_ns) {
   constexpr int T = 32 * NW, TURNS = NW / kCopies, kSlotBatch = 4;
   static_assert(TURNS == 1 || TURNS == 2, "one or two warps per accumulator copy");
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(32 * NW, 2) cg_resident_kernel(CgArgs c, int m
   const int n = a.n_points, chunks = (n + 31) / 32;
   const int mine = (chunks - tile + (int)gridDim.x - 1) / (int)gridDim.x;  // chunks tile, tile + grid, ...
   if (tid == 0) cs = *c.cs;
-  GridBar bar{counters, kResidentCounters, gridDim.x, 0};
+  GridBar bar{counters, kResidentCounters, wait_ns, gridDim.x, 0};
   V4<R>* slots = (V4<R>*)a.slots;
   V4<R>* Z = (V4<R>*)c.q;  // z = M^-1 r of the current residual
   for (int i = tid; i < nv; i += T) {
@@ -359,14 +359,14 @@ __global__ void __launch_bounds__(32 * NW, 2) cg_resident_kernel(CgArgs c, int m
       if (v < n) ((V4<R>*)c.lam)[v] = V4<R>{word(LAM, j), word(LAM + 1, j), word(LAM + 2, j), R(0)};
     }
     if (tile == 0 && tid == 0) *c.cs = cs;
-  } else if (tid == 0) {  // a barrier gave up
+  }
+  if (bar.leave()) {  // a barrier gave up
     c.cs->done = 1;
     c.cs->result = AGB_E_DEVICE;
   }
-  bar.leave();
 }
 
-using CgKernel = void (*)(CgArgs, int, void*, void*, unsigned*);
+using CgKernel = void (*)(CgArgs, int, void*, void*, unsigned*, uint64_t);
 
 struct Shape {
   CgKernel kernel;
@@ -412,7 +412,8 @@ cudaError_t launch_cg_resident(const CgArgs& c, const ResidentPlan& p, void* par
                                cudaStream_t s) {
   if (!p.shape) return cudaErrorInvalidValue;
   const Shape sh = shape_of(c.a, p);
-  return launch_cooperative(sh.kernel, sh.blocks, sh.threads, sh.smem, s, c, p.max_elems, part_p, part_v, counters);
+  return launch_cooperative(sh.kernel, sh.blocks, sh.threads, sh.smem, s, c, p.max_elems, part_p, part_v, counters,
+                            p.wait_ns);
 }
 
 }  // namespace agb

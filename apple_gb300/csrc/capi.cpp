@@ -825,6 +825,7 @@ static void cg_release(agb_solver* sv) {
   sv->d_cg_cnt = sv->d_cg_res_counters = nullptr;
   sv->d_cg_state = sv->h_cg_state = nullptr;
   sv->cg_resident = ResidentPlan{};
+  sv->cg_resident.wait_ns = sv->resident.wait_ns;
   sv->cg_ready = false;
 }
 
@@ -1133,6 +1134,16 @@ int agb_solver_reset(agb_solver* sv, const void* u, void* stream) {
 // every step rejected (s = 4) 2,039 / 1,869 and 4,516 / 4,270.
 static bool arap_apart(const agb_solver* sv) {
   return sv->args.fv.material == AGB_ARAP && sv->params.overstep <= 2.0 * (1.0 - sv->params.armijo_c);
+}
+
+int agb_solver_set_wait_limit(agb_solver* sv, int64_t ns) {
+  AGB_REQUIRE(sv && ns >= 0, AGB_E_INVALID, "agb_solver_set_wait_limit: bad argument");
+  sv->resident.wait_ns = sv->cg_resident.wait_ns = (uint64_t)ns;
+  for (cudaGraphExec_t* g : {&sv->loop_exec, &sv->step_exec}) {  // they hold the launch's arguments
+    if (*g) AGB_CHECK_CUDA(cudaGraphExecDestroy(*g));
+    *g = nullptr;
+  }
+  return AGB_OK;
 }
 
 // Capture into `graph` after `deps` (which may be empty): the three passes

@@ -1,9 +1,11 @@
 // Barrier and deterministic sums across the CTAs of a cooperative launch.
 //
 // The barrier is a counter of arrivals: CTA thread 0 adds one and polls until
-// every CTA has arrived `round` times.  The wait is bounded: after about two
-// seconds it gives up, the caller reports a device error and returns.  The
-// last CTA to leave the kernel resets the counters for the next launch.
+// every CTA has arrived `round` times.  The wait is bounded: at its limit it
+// polls once more, gives up and notes that in a counter of its own; its CTA
+// returns, and the others' next waits give up too.  The last CTA to leave the
+// kernel learns whether any wait gave up, after everything the others wrote,
+// and resets the counters for the next launch.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -14,10 +16,13 @@
 
 namespace agb {
 
+// words of `counters`, zero before the first launch
+constexpr int kArrived = 0, kLeft = 1, kGaveUp = 2, kPlaceWord = 3;
+
 struct GridBar {
-  static constexpr uint64_t kLimit = 2000000000ull;  // ns
-  unsigned* counters;  // [0] arrivals, [1] exits; `words` of them, zero before the first launch
+  unsigned* counters;
   int words;           // reset by the last CTA to leave
+  uint64_t limit;      // of a wait, ns
   unsigned n;          // CTAs
   unsigned round;      // barriers passed
 
@@ -29,7 +34,7 @@ struct GridBar {
     __syncthreads();
     if (threadIdx.x == 0) {
       __threadfence();
-      atomicAdd(&counters[0], 1u);
+      atomicAdd(&counters[kArrived], 1u);
     }
   }
 
@@ -41,10 +46,12 @@ struct GridBar {
       const uint64_t t0 = global_ns();
       bool ok = true;
       for (;;) {
+        const bool late = global_ns() - t0 >= limit;  // read before the load, which may come long after it
         unsigned v;
-        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(counters) : "memory");
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(counters + kArrived) : "memory");
         if ((int)(v - want) >= 0) break;  // the counter may wrap
-        if (global_ns() - t0 > kLimit) {
+        if (late) {
+          atomicExch(&counters[kGaveUp], 1u);
           ok = false;
           break;
         }
@@ -55,13 +62,17 @@ struct GridBar {
     return s_ok != 0;
   }
 
-  // every CTA once, after its last sync()
-  __device__ __forceinline__ void leave() {
+  // every CTA once, after its last wait(), whether that gave up or not; true
+  // in thread 0 of the last CTA when a wait gave up anywhere
+  __device__ __forceinline__ bool leave() {
     __syncthreads();
-    if (threadIdx.x != 0) return;
+    if (threadIdx.x != 0) return false;
     __threadfence();
-    if (atomicAdd(&counters[1], 1u) == n - 1u)
-      for (int k = 0; k < words; ++k) counters[k] = 0u;
+    if (atomicAdd(&counters[kLeft], 1u) != n - 1u) return false;
+    __threadfence();
+    const bool gave_up = atomicAdd(&counters[kGaveUp], 0u) != 0u;
+    for (int k = 0; k < words; ++k) counters[k] = 0u;
+    return gave_up;
   }
 };
 
@@ -139,8 +150,8 @@ __device__ __forceinline__ void grid_totals(const AccStore<R>* part, int n, Acc<
 // The work item of this CTA when the first `whole` of n items are large: the
 // first CTA to arrive on an SM takes the next large one, a second CTA there
 // the next of the others, so that no SM holds two large items while another
-// holds none.  counters[2], [3]: items taken; counters[4 + k]: CTAs on SM k
-// (kPlaceWords words after the barrier's two, zero before the launch).
+// holds none.  counters[kPlaceWord] and the next: items taken; those after:
+// CTAs on each SM (kPlaceWords words in all, zero before the launch).
 // Called by one thread.
 constexpr int kPlaceSms = 256;
 constexpr int kPlaceWords = 2 + kPlaceSms;
@@ -148,15 +159,16 @@ constexpr int kPlaceWords = 2 + kPlaceSms;
 __device__ __forceinline__ int place_cta(unsigned* counters, int whole, int n) {
   unsigned sm;
   asm volatile("mov.u32 %0, %%smid;" : "=r"(sm));
-  const bool first = atomicAdd(&counters[4 + (sm & (kPlaceSms - 1))], 1u) == 0u;
+  counters += kPlaceWord;
+  const bool first = atomicAdd(&counters[2 + (sm & (kPlaceSms - 1))], 1u) == 0u;
   if (first) {
-    const int k = (int)atomicAdd(&counters[2], 1u);
+    const int k = (int)atomicAdd(&counters[0], 1u);
     if (k < whole) return k;
-    return min(whole + (int)atomicAdd(&counters[3], 1u), n - 1);
+    return min(whole + (int)atomicAdd(&counters[1], 1u), n - 1);
   }
-  const int k = (int)atomicAdd(&counters[3], 1u);
+  const int k = (int)atomicAdd(&counters[1], 1u);
   if (whole + k < n) return whole + k;
-  return min((int)atomicAdd(&counters[2], 1u), n - 1);
+  return min((int)atomicAdd(&counters[0], 1u), n - 1);
 }
 
 }  // namespace agb

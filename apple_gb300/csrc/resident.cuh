@@ -10,7 +10,7 @@
 
 namespace agb {
 
-static_assert(kResidentCounters == 2 + kPlaceWords, "barrier and placement");
+static_assert(kResidentCounters == kPlaceWord + kPlaceWords, "barrier and placement");
 
 // Warps per tile (two tiles per SM): 8 in FP32; FP64 is bound by its
 // arithmetic pipe, which 8 warps per SM fill: 4.  Meshes with fewer tiles

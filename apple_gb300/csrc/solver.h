@@ -151,9 +151,10 @@ struct ResidentPlan {
   int max_groups = 0;
   int whole = 0;  // FP32: the first tiles are this many whole ones, the others cut (0: all alike)
   const int32_t* order = nullptr;  // FP64 with more tiles than SMs: pair_tiles()
+  uint64_t wait_ns = 2000000000;   // limit of a grid barrier's wait
 };
 // words of `counters` below
-constexpr int kResidentCounters = 4 + 256;
+constexpr int kResidentCounters = 5 + 256;
 cudaError_t resident_prepare(const SolveArgs& a, ResidentPlan* p);
 cudaError_t launch_resident(const SolveArgs& a, const ResidentPlan& p, void* part_d, void* part_v, unsigned* counters,
                             cudaStream_t s);

@@ -73,7 +73,7 @@ enum Share { kAlone, kTwoCtas, kTwoTiles };
 template <class R, int MAT, bool DELTA, int NW, bool REC, Share SHARE>
 __global__ void __launch_bounds__(32 * NW * (SHARE == kTwoTiles ? 2 : 1), SHARE == kTwoCtas ? 2 : 1)
     solver_resident_kernel(SolveArgs a, int max_elems, int tile_smem, int whole, const int32_t* __restrict__ order,
-                           void* part_d, void* part_v, unsigned* counters) {
+                           void* part_d, void* part_v, unsigned* counters, uint64_t wait_ns) {
   constexpr int T = 32 * NW, ND = 6, NVT = 12, kSlotBatch = 4;  // T threads per tile
   constexpr int TILES = SHARE == kTwoTiles ? 2 : 1, TC = T * TILES;
   constexpr unsigned FFD = 0x2u, FFV = (1u << 1) | (1u << 6) | (1u << 8) | (1u << 9);
@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(32 * NW * (SHARE == kTwoTiles ? 2 : 1), SHARE 
   const int gs = tile < 0 ? 0 : a.fv.tile_gstart[tile], ge = tile < 0 ? 0 : a.fv.tile_gstart[tile + 1];
   const int vs = tile < 0 ? 0 : a.fv.tile_vstart[tile], nv = tile < 0 ? 0 : a.fv.tile_vstart[tile + 1] - vs;
   const int me = SHARE == kTwoCtas ? tile : (int)blockIdx.x;  // the place of the CTA's partials
-  GridBar bar{counters, kResidentCounters, gridDim.x, 0};
+  GridBar bar{counters, kResidentCounters, wait_ns, gridDim.x, 0};
   if (threadIdx.x < kStateWords) ((uint32_t*)&sst)[threadIdx.x] = ((const uint32_t*)a.st)[threadIdx.x];
   __syncthreads();
   const V4<R>* XA = (const V4<R>*)a.xa;
@@ -445,14 +445,14 @@ __global__ void __launch_bounds__(32 * NW * (SHARE == kTwoTiles ? 2 : 1), SHARE 
       X[2 * v + 1] = V4<R>{xl[i], xl[kTileVerts + i], xl[2 * kTileVerts + i], R(0)};
       P[v] = V4<R>{vp[i], vp[kTileVerts + i], vp[2 * kTileVerts + i], R(0)};
     }
-  } else if (threadIdx.x == 0) {  // a barrier gave up: the solve stops with a device error
-    atomicMax(&a.st->error, 3);
+  }
+  if (bar.leave()) {  // a barrier gave up: the solve stops with a device error
+    a.st->error = 3;
     a.st->done = 1;
   }
-  bar.leave();
 }
 
-using ResidentKernel = void (*)(SolveArgs, int, int, int, const int32_t*, void*, void*, unsigned*);
+using ResidentKernel = void (*)(SolveArgs, int, int, int, const int32_t*, void*, void*, unsigned*, uint64_t);
 
 struct Shape {
   ResidentKernel kernel;
@@ -510,8 +510,8 @@ cudaError_t launch_resident(const SolveArgs& a, const ResidentPlan& p, void* par
                             cudaStream_t s) {
   if (!p.shape) return cudaErrorInvalidValue;
   const Shape sh = shape_of(a, p);
-  return launch_cooperative(sh.kernel, sh.blocks, sh.threads, sh.smem, s, a, p.max_elems, sh.tile_smem, p.whole, p.order, part_d, part_v,
-                            counters);
+  return launch_cooperative(sh.kernel, sh.blocks, sh.threads, sh.smem, s, a, p.max_elems, sh.tile_smem, p.whole,
+                            p.order, part_d, part_v, counters, p.wait_ns);
 }
 
 }  // namespace agb

@@ -317,6 +317,12 @@ int agb_solver_read_reductions(agb_solver* solver, double* out5, void* stream);
 int agb_solver_checkpoint_size(agb_solver* solver, size_t* bytes);
 int agb_solver_save(agb_solver* solver, void* host, void* stream);
 int agb_solver_load(agb_solver* solver, const void* host, size_t bytes, void* stream);
+/* Small and medium meshes run their iterations and their adjoint CG in one
+ * cooperative launch, whose grid barriers wait at most `ns` nanoseconds (2 s
+ * by default).  A wait that runs out ends the launch, and agb_solver_read or
+ * agb_solver_adjoint reports AGB_E_DEVICE; agb_solver_reset starts afresh.
+ * Call it while no launch of this solver is in flight. */
+int agb_solver_set_wait_limit(agb_solver* solver, int64_t ns);
 /* Diagnostics: time each pass of an iteration on its own with CUDA events on
  * `stream`, `reps` launches each (direction, gradient, vertex pass), writing
  * `flush_bytes` of the device buffer `flush` (may be NULL) before every launch
