@@ -1,27 +1,28 @@
 // Batched PNCG: many independent meshes, one set of launches per iteration.
 //
 // The meshes' vertices and tiles are concatenated (tiles never span meshes,
-// vertex chunks never span meshes).  An iteration is three kernels, captured
-// in a CUDA graph; every mesh carries its own SolverState, so each one runs
-// the reference's PNCG iteration (benches/bench_pncg_branching_backends.py
+// vertex chunks never span meshes).  An iteration is five kernels (three in
+// small batches, batch_fused below), captured in a CUDA graph; every mesh
+// carries its own SolverState, so each one runs the reference's PNCG iteration (benches/bench_pncg_branching_backends.py
 // :254-456, 606-679) with its own beta, step and termination:
 //   direction pass   one CTA per tile: p of the tile's mesh, p^T H p and the
-//                    energy polynomial; one partial per tile; the last CTA of
-//                    a mesh adds its partials in tile order and takes the
-//                    Armijo decision (dir_decide)
+//                    energy polynomial; one partial per tile
+//   direction tail   one CTA per mesh: the mesh's tile partials in tile order,
+//                    then the Armijo decision (dir_decide)
 //   gradient pass    one CTA per tile at x + t_mesh p (grad_tile)
-//   vertex pass      one CTA per vertex chunk: x, g, d and the 12 sums; the
-//                    last CTA of a mesh adds its chunks in order and decides
-//                    beta and termination (vertex_decide); the last mesh
-//                    counts those still running and sets the graph's
+//   vertex pass      one CTA per vertex chunk: x, g, d and the 12 sums
+//   vertex tail      one CTA per mesh: chunk partials in order, then beta and
+//                    termination (vertex_decide); the last CTA to finish
+//                    counts the meshes still running and sets the graph's
 //                    while-condition
 // Tiles and chunks of a finished mesh return at once.  The graph's loop body
 // holds two iterations, the second skipped when the first ended the run.
-// What bounds it is the chain of small launches.  Measured, reset and 20
-// iterations of 24 meshes of 1.2k to 11k tets in FP32: 2,600 -> 1,534 us with
-// the tails in the passes, two iterations a body and one refresh in the reset;
-// three beams 1,124 -> 849, 64 meshes 5,731 -> 2,790, 24 large ones 4,207 ->
-// 3,056.
+// What bounds it: the passes' throughput, and for a few small meshes the chain
+// of launches.  An iteration in FP32 with the reference-state correction, us:
+// 24 meshes (318k tets) 65, 64 meshes (1.0M) 121, 64 (4.2M) 306, 160 (8.4M)
+// 584, 320 (18.7M) 1,227.  With the tails taken by the last CTA of a mesh in
+// the passes themselves (an arrival counter in every CTA): 65, 122, 319, 610,
+// 1,288.
 #include "kernels.h"
 #include "solver.h"
 #include "solver_common.cuh"
@@ -32,11 +33,19 @@ namespace {
 
 constexpr int kTailThreads = 256;
 
+// FUSED: the last CTA of a mesh takes the mesh's tail in the pass itself.
+// Up to a tile per SM the chain of launches is the longer part; above, the
+// arrival counter in every CTA costs as much as the two launches saved, and
+// more with several waves of CTAs (the times above).  An iteration in FP32,
+// fused against separate: 5 tiles 30.5 / 32.4 us, 113 tiles 44.9 / 48.5, 181
+// tiles 60.1 / 60.7, 478 tiles 61.5 / 60.9; in FP64 113 tiles 281 / 305.
+bool batch_fused(const BatchArgs& b) { return b.a.fv.n_tiles <= kSMs; }
+
 // the passes of the body's second iteration skip it when the first one ended
 // the run
 __device__ __forceinline__ bool batch_skip(const BatchArgs& b) { return b.guard && !b.bs->go; }
 
-// one more CTA of mesh m is done with the pass; true in the last of n
+// one more CTA of a mesh is done with the pass; true in the last of n
 // (every thread calls it; thread 0's writes before it are visible to the last)
 __device__ __forceinline__ bool last_of_mesh(unsigned* counter, unsigned n) {
   __shared__ int s_last;
@@ -51,7 +60,7 @@ __device__ __forceinline__ bool last_of_mesh(unsigned* counter, unsigned n) {
   return true;
 }
 
-// thread 0 of one CTA per mesh, after the mesh's iteration: counts it, and the
+// thread 0 of a mesh's tail, after the mesh's iteration: counts it, and the
 // last mesh closes the batch's iteration
 __device__ __forceinline__ void mesh_arrives(const BatchArgs& b, bool running) {
   BatchState* bs = b.bs;
@@ -68,7 +77,41 @@ __device__ __forceinline__ void mesh_arrives(const BatchArgs& b, bool running) {
   if (b.cond) cudaGraphSetConditional((cudaGraphConditionalHandle)b.cond, go ? 1u : 0u);
 }
 
-template <class R, int MAT>
+// the direction tail of a mesh, by a whole CTA: its tiles' partials in tile
+// order, then the Armijo decision
+template <class R, int MAT, int THREADS>
+__device__ __forceinline__ void dir_tail(const BatchArgs& b, int mesh, SolverState* st) {
+  constexpr int N = 6;
+  __shared__ Acc<R> red[(THREADS / 32) * N];
+  if (threadIdx.x == 0) st->refresh = 0;  // the refresh passes, if any, ran after the last vertex tail
+  const int t0 = b.mesh_tile0[mesh], t1 = b.mesh_tile0[mesh + 1];
+  Acc<R> s[N] = {};
+  for (int t = t0 + threadIdx.x; t < t1; t += THREADS) {
+#pragma unroll
+    for (int k = 0; k < N; ++k) s[k].add(acc_load<R>((const AccStore<R>*)b.part_dir + (size_t)t * N + k));
+  }
+  block_reduce<N, 0xffffffffu, R>(s, red);
+  if (threadIdx.x < 32) dir_decide<MAT, R>(st, red);  // the sums are in red[0 .. N-1]
+}
+
+// the vertex tail of a mesh, by a whole CTA: its chunks' partials in order,
+// then beta and termination
+template <class R, int THREADS>
+__device__ __forceinline__ void vertex_tail(const BatchArgs& b, int mesh, SolverState* st) {
+  constexpr int N = 12;
+  __shared__ Acc<R> red[(THREADS / 32) * N];
+  const int c0 = b.mesh_chunk0[mesh], c1 = b.mesh_chunk0[mesh + 1];
+  Acc<R> s[N] = {};
+  for (int c = c0 + threadIdx.x; c < c1; c += THREADS) {
+#pragma unroll
+    for (int k = 0; k < N; ++k) s[k].add(acc_load<R>((const AccStore<R>*)b.part_vert + (size_t)c * N + k));
+  }
+  block_reduce<N, 0xffffffffu, R>(s, red);
+  vertex_decide<R>(st, red);  // the sums are in red[0 .. N-1]
+  if (threadIdx.x == 0 && b.a.svd) st->sbuf ^= 1;  // the gradient pass's SVDs are those at the new x
+}
+
+template <class R, int MAT, bool FUSED>
 __global__ void __launch_bounds__(kElemThreads) batch_dir_kernel(BatchArgs b) {
   constexpr int N = 6;
   // float-float warp tree for c2 (terms of both signs); ARAP sums p^T H p only
@@ -79,11 +122,10 @@ __global__ void __launch_bounds__(kElemThreads) batch_dir_kernel(BatchArgs b) {
   const SolveArgs& a = b.a;
   const int tile = blockIdx.x;
   if (!b.guard && b.cond && tile == 0 && threadIdx.x == 0)
-    cudaGraphSetConditional((cudaGraphConditionalHandle)b.cond, 0u);  // the vertex pass re-arms
+    cudaGraphSetConditional((cudaGraphConditionalHandle)b.cond, 0u);  // the vertex tail re-arms
   pdl_trigger();
-  const int mesh = b.tile_mesh[tile];
-  if (b.guard) pdl_wait();  // a dependent of the first iteration's last pass
   if (batch_skip(b)) return;
+  const int mesh = b.tile_mesh[tile];
   SolverState* st = b.st + mesh;
   if (st->done) return;
   const R beta = to_real<R>(st->beta), inv_mean = to_real<R>(st->inv_mean);
@@ -128,17 +170,20 @@ __global__ void __launch_bounds__(kElemThreads) batch_dir_kernel(BatchArgs b) {
 #pragma unroll
     for (int k = 0; k < N; ++k) ((AccStore<R>*)b.part_dir)[(size_t)tile * N + k] = acc_store(sums[k]);
   }
-  // the last tile of the mesh: partials in tile order, then the decision
-  const int t0 = b.mesh_tile0[mesh], t1 = b.mesh_tile0[mesh + 1];
-  if (!last_of_mesh(b.cnt_dir + mesh, (unsigned)(t1 - t0))) return;
-  if (threadIdx.x == 0) st->refresh = 0;  // the refresh passes, if any, ran after the last vertex pass
-  Acc<R> s[N] = {};
-  for (int t = t0 + threadIdx.x; t < t1; t += blockDim.x) {
-#pragma unroll
-    for (int k = 0; k < N; ++k) s[k].add(acc_load<R>((const AccStore<R>*)b.part_dir + (size_t)t * N + k));
+  if constexpr (FUSED) {
+    if (last_of_mesh(b.cnt_dir + mesh, (unsigned)(b.mesh_tile0[mesh + 1] - b.mesh_tile0[mesh])))
+      dir_tail<R, MAT, kElemThreads>(b, mesh, st);
   }
-  block_reduce<N, 0xffffffffu, R>(s, red);
-  if (threadIdx.x < 32) dir_decide<MAT, R>(st, red);  // the sums are in red[0 .. N-1]
+}
+
+template <class R, int MAT>
+__global__ void __launch_bounds__(kTailThreads) batch_dir_tail_kernel(BatchArgs b) {
+  pdl_trigger();
+  pdl_wait();
+  if (batch_skip(b)) return;
+  SolverState* st = b.st + blockIdx.x;
+  if (st->done) return;
+  dir_tail<R, MAT, kTailThreads>(b, blockIdx.x, st);
 }
 
 // ARAP: the gradient pass at the first trial step x + alpha_0 p of each
@@ -214,7 +259,7 @@ __global__ void __launch_bounds__(kGradThreads, 6) batch_grad_kernel(BatchArgs b
 
 // phase (ARAP): 1 after the speculative gradient pass, for the meshes whose
 // alpha_0 was accepted; 2 after the fallback passes, for the others; 0: all
-template <class R, bool DELTA>
+template <class R, bool DELTA, bool FUSED>
 __global__ void __launch_bounds__(kVThreads) batch_vertex_kernel(BatchArgs b, int phase) {
   constexpr int N = 12;
   constexpr unsigned FF = (1u << 1) | (1u << 6) | (1u << 8) | (1u << 9);
@@ -227,10 +272,10 @@ __global__ void __launch_bounds__(kVThreads) batch_vertex_kernel(BatchArgs b, in
   pdl_trigger();
   pdl_wait();
   if (batch_skip(b)) return;
-  // a mesh this pass does not concern: its first chunk counts it (in the pass
-  // of phase 1 the later one does)
+  // a mesh this pass does not concern: fused, its first chunk counts it (in
+  // the pass of phase 1 the later one does)
   if (st->done || (phase == 1 && !st->spec_ok) || (phase == 2 && st->spec_ok)) {
-    if (phase != 1 && c == c0 && threadIdx.x == 0) mesh_arrives(b, !st->done);
+    if (FUSED && phase != 1 && c == c0 && threadIdx.x == 0) mesh_arrives(b, !st->done);
     return;
   }
   const R t = to_real<R>(st->t);
@@ -248,18 +293,28 @@ __global__ void __launch_bounds__(kVThreads) batch_vertex_kernel(BatchArgs b, in
 #pragma unroll
     for (int k = 0; k < N; ++k) ((AccStore<R>*)b.part_vert)[(size_t)c * N + k] = acc_store(acc[k]);
   }
-  // the last chunk of the mesh: chunk partials in order, then the decision
-  if (!last_of_mesh(b.cnt_vert + mesh, (unsigned)(c1 - c0))) return;
-  Acc<R> q[N] = {};
-  for (int k0 = c0 + threadIdx.x; k0 < c1; k0 += blockDim.x) {
-#pragma unroll
-    for (int k = 0; k < N; ++k) q[k].add(acc_load<R>((const AccStore<R>*)b.part_vert + (size_t)k0 * N + k));
+  if constexpr (FUSED) {
+    if (!last_of_mesh(b.cnt_vert + mesh, (unsigned)(c1 - c0))) return;
+    vertex_tail<R, kVThreads>(b, mesh, st);
+    if (phase != 1 && threadIdx.x == 0) mesh_arrives(b, !st->done);
   }
-  block_reduce<N, 0xffffffffu, R>(q, red);
-  vertex_decide<R>(st, red);  // the sums are in red[0 .. N-1]
-  if (threadIdx.x != 0) return;
-  if (b.a.svd) st->sbuf ^= 1;  // the gradient pass's SVDs are those at the new x
-  if (phase != 1) mesh_arrives(b, !st->done);
+}
+
+// phase as in batch_vertex_kernel; the pass of phase 1 decides its meshes
+// only, the others also count the meshes still running
+template <class R>
+__global__ void __launch_bounds__(kTailThreads) batch_vertex_tail_kernel(BatchArgs b, int phase) {
+  pdl_trigger();
+  pdl_wait();
+  if (batch_skip(b)) return;
+  SolverState* st = b.st + blockIdx.x;
+  // read by every thread before thread 0 writes the state
+  const bool was_done = st->done != 0;
+  const bool mine = phase == 0 || (phase == 1) == (st->spec_ok != 0);
+  __syncthreads();
+  if (phase == 1 && !mine) return;
+  if (!was_done && mine) vertex_tail<R, kTailThreads>(b, blockIdx.x, st);
+  if (phase != 1 && threadIdx.x == 0) mesh_arrives(b, !st->done);
 }
 
 // reference-state refresh of the models that asked for one (FP32); it runs
@@ -356,14 +411,31 @@ __global__ void batch_init_state_kernel(BatchArgs b, SolverState proto) {
 
 __global__ void batch_set_limit_kernel(BatchState* bs, int n) { bs->iter_limit = bs->iter + n; }
 
+// The element pass is a plain launch: as a programmatic dependent its CTAs
+// fill the SMs in the order in which the pass before drains them, four
+// consecutive ones to an SM, so that the tiles of the one mesh that refreshes
+// share a few FP64 pipes (64 meshes, 1.0M tets: a step with a refresh 150 us
+// against 150 to 290, one without it the same).
 cudaError_t batch_refresh(const BatchArgs& b, cudaStream_t s) {
-  cudaError_t e = b.a.fv.material == AGB_STABLE_NEO_HOOKEAN_MUSCLE
-                      ? launch_pdl(batch_ref_elem_kernel<AGB_STABLE_NEO_HOOKEAN_MUSCLE>,
-                                     dim3(ref_blocks(b.a.fv.n_tiles)), dim3(kGradThreads), ref_smem_bytes(), s, b)
-                      : launch_pdl(batch_ref_elem_kernel<AGB_STABLE_NEO_HOOKEAN>, dim3(ref_blocks(b.a.fv.n_tiles)),
-                                     dim3(kGradThreads), ref_smem_bytes(), s, b);
+  const int eb = ref_blocks(b.a.fv.n_tiles);
+  if (b.a.fv.material == AGB_STABLE_NEO_HOOKEAN_MUSCLE)
+    batch_ref_elem_kernel<AGB_STABLE_NEO_HOOKEAN_MUSCLE><<<eb, kGradThreads, ref_smem_bytes(), s>>>(b);
+  else
+    batch_ref_elem_kernel<AGB_STABLE_NEO_HOOKEAN><<<eb, kGradThreads, ref_smem_bytes(), s>>>(b);
+  cudaError_t e = cudaGetLastError();
   const int vb = b.n_chunks < kSMs * 8 ? b.n_chunks : kSMs * 8;
   if (e == cudaSuccess) e = launch_pdl(batch_ref_vertex_kernel, dim3(vb > 0 ? vb : 1), dim3(kVThreads), 0, s, b);
+  return e;
+}
+
+// the vertex pass and its tail
+template <class R, bool DELTA>
+cudaError_t batch_vertex(const BatchArgs& b, int phase, cudaStream_t s) {
+  if (batch_fused(b))
+    return launch_pdl(batch_vertex_kernel<R, DELTA, true>, dim3(b.n_chunks), dim3(kVThreads), 0, s, b, phase);
+  cudaError_t e = launch_pdl(batch_vertex_kernel<R, DELTA, false>, dim3(b.n_chunks), dim3(kVThreads), 0, s, b, phase);
+  if (e == cudaSuccess)
+    e = launch_pdl(batch_vertex_tail_kernel<R>, dim3(b.n_meshes), dim3(kTailThreads), 0, s, b, phase);
   return e;
 }
 
@@ -371,9 +443,8 @@ template <class R, int MAT, bool DELTA>
 cudaError_t batch_grad_and_vertex_d(const BatchArgs& b, cudaStream_t s, int fallback = 0, bool refresh = true) {
   const int phase = fallback ? 2 : 0;
   cudaError_t e = launch_pdl(batch_grad_kernel<R, MAT, DELTA>, dim3(b.a.fv.n_tiles), dim3(kGradThreads),
-                               grad_smem_bytes<R>(), s, b, fallback);
-  if (e == cudaSuccess)
-    e = launch_pdl(batch_vertex_kernel<R, DELTA>, dim3(b.n_chunks), dim3(kVThreads), 0, s, b, phase);
+                             grad_smem_bytes<R>(), s, b, fallback);
+  if (e == cudaSuccess) e = batch_vertex<R, DELTA>(b, phase, s);
   if (e == cudaSuccess && DELTA && refresh) e = batch_refresh(b, s);
   return e;
 }
@@ -398,12 +469,20 @@ cudaError_t batch_first(const BatchArgs& b, cudaStream_t s) {
              : batch_grad_and_vertex_m<R, AGB_STABLE_NEO_HOOKEAN>(b, s, false);
 }
 
+// the direction pass, in both iterations of the loop's body a plain launch (as a
+// programmatic dependent of the first iteration the second took 64 meshes of
+// 4.2M tets from 319 to 337 us an iteration), and its tail
 template <class R, int MAT>
 cudaError_t batch_dir(const BatchArgs& b, cudaStream_t s) {
-  const dim3 g(b.a.fv.n_tiles), t(kElemThreads);
-  if (b.guard) return launch_pdl(batch_dir_kernel<R, MAT>, g, t, 0, s, b);
-  batch_dir_kernel<R, MAT><<<g, t, 0, s>>>(b);
-  return cudaGetLastError();
+  if (batch_fused(b)) {
+    batch_dir_kernel<R, MAT, true><<<b.a.fv.n_tiles, kElemThreads, 0, s>>>(b);
+    return cudaGetLastError();
+  }
+  batch_dir_kernel<R, MAT, false><<<b.a.fv.n_tiles, kElemThreads, 0, s>>>(b);
+  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess)
+    e = launch_pdl(batch_dir_tail_kernel<R, MAT>, dim3(b.n_meshes), dim3(kTailThreads), 0, s, b);
+  return e;
 }
 
 template <class R, int MAT>
@@ -425,8 +504,7 @@ cudaError_t batch_iteration_arap(const BatchArgs& b, cudaStream_t s) {
   if (e == cudaSuccess)
     e = launch_pdl(batch_grad_spec_kernel<R>, dim3(nt), dim3(kGradThreads), grad_spec_smem_bytes<R>(), s, b);
   if (e == cudaSuccess) e = launch_pdl(batch_spec_tail_kernel<R>, dim3(b.n_meshes), dim3(kTailThreads), 0, s, b);
-  if (e == cudaSuccess)
-    e = launch_pdl(batch_vertex_kernel<R, false>, dim3(b.n_chunks), dim3(kVThreads), 0, s, b, 1);
+  if (e == cudaSuccess) e = batch_vertex<R, false>(b, 1, s);
   for (int j0 = 1; e == cudaSuccess && j0 <= max_bt; j0 += 3) {
     const int k = max_bt - j0 + 1 < 3 ? max_bt - j0 + 1 : 3;
     batch_trial_kernel<R><<<nt, kElemThreads, 0, s>>>(b, j0, k);

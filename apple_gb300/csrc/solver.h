@@ -202,7 +202,7 @@ cudaError_t launch_cg_resident(const CgArgs& c, const ResidentPlan& p, void* par
 struct BatchState {
   int32_t iter;        // iterations of the batch loop
   int32_t iter_limit;
-  uint32_t n_active;   // meshes still running after this iteration (vertex pass)
+  uint32_t n_active;   // meshes still running after this iteration (vertex tail)
   uint32_t arrived;    // meshes done with it (the last one sets the condition)
   int32_t go;          // the loop goes on
 };
@@ -221,8 +221,8 @@ struct BatchArgs {
   void* part_dir;              // n_tiles x 6
   void* part_grad;             // n_tiles energy partials (on demand)
   void* part_vert;             // n_chunks x 12
-  unsigned* cnt_dir;           // n_meshes: tiles done with the direction pass
-  unsigned* cnt_vert;          // n_meshes: chunks done with the vertex pass
+  unsigned* cnt_dir;           // n_meshes: tiles done with the direction pass (small batches)
+  unsigned* cnt_vert;          // n_meshes: chunks done with the vertex pass (small batches)
   unsigned long long cond;
   int guard;                   // second iteration of the loop's body
 };
@@ -230,7 +230,8 @@ struct BatchArgs {
 cudaError_t batch_prepare_kernels(int precision);
 cudaError_t launch_batch_init(const BatchArgs& b, const void* u_user, const void* fixed,
                               const int32_t* user_of_internal, const SolverState& proto, cudaStream_t s);
-// one iteration of every running mesh: direction, gradient and vertex pass
+// one iteration of every running mesh: direction pass + tail, gradient pass,
+// vertex pass + tail
 cudaError_t launch_batch_iteration(const BatchArgs& b, cudaStream_t s);
 // gradient + vertex pass at t = 0 (g_0, diag_0 of every mesh)
 cudaError_t launch_batch_first(const BatchArgs& b, cudaStream_t s);
