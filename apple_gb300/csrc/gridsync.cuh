@@ -80,9 +80,10 @@ struct GridBar {
 // thread's terms; lo: the low word of quantity LO (float-float), or unused
 // with LO < 0.  The terms go through shared memory (`rows`: N + 1 rows of
 // THREADS reals) so that one warp adds one quantity, instead of every warp
-// reducing all N by shuffles: quantities in FF in float-float, the others
-// (sums of same-sign terms) in R.
-template <int N, unsigned FF, int LO, int THREADS, class R>
+// reducing all N by shuffles, in float-float from the threads' terms on.
+// (Same-sign sums in plain FP32 above the threads had several times the
+// rounding error and were no faster: 14.0 us an iteration of the 5k-tet cube.)
+template <int N, int LO, int THREADS, class R>
 __device__ __forceinline__ void cta_partials(const R (&x)[N], R lo, R* rows, AccStore<R>* part, int n, int block) {
   constexpr int NW = THREADS / 32;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -93,24 +94,16 @@ __device__ __forceinline__ void cta_partials(const R (&x)[N], R lo, R* rows, Acc
   for (int k = warp; k < N; k += NW) {
     const R* row = rows + k * THREADS;
     Acc<R> s{};
-    if ((FF >> k) & 1u) {
 #pragma unroll 4
-      for (int j = 0; j < NW; ++j) s.add(row[lane + 32 * j]);
-      if (k == LO) {
-        R l = R(0);
+    for (int j = 0; j < NW; ++j) s.add(row[lane + 32 * j]);
+    if (k == LO) {
+      R l = R(0);
 #pragma unroll 4
-        for (int j = 0; j < NW; ++j) l += rows[N * THREADS + lane + 32 * j];
-        s.add(l);
-      }
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1) s.add(s.shfl_down(off));
-    } else {
-      R p = R(0);
-#pragma unroll 4
-      for (int j = 0; j < NW; ++j) p += row[lane + 32 * j];
-      s.add(p);
-      s.warp_plain_sum();
+      for (int j = 0; j < NW; ++j) l += rows[N * THREADS + lane + 32 * j];
+      s.add(l);
     }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) s.add(s.shfl_down(off));
     if (lane == 0) part[(size_t)k * n + block] = acc_store(s);
   }
 }

@@ -76,7 +76,6 @@ __global__ void __launch_bounds__(32 * NW * (SHARE == kTwoTiles ? 2 : 1), SHARE 
                            void* part_d, void* part_v, unsigned* counters, uint64_t wait_ns) {
   constexpr int T = 32 * NW, ND = 6, NVT = 12, kSlotBatch = 4;  // T threads per tile
   constexpr int TILES = SHARE == kTwoTiles ? 2 : 1, TC = T * TILES;
-  constexpr unsigned FFD = 0x2u, FFV = (1u << 1) | (1u << 6) | (1u << 8) | (1u << 9);
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int half = TILES == 2 ? (int)threadIdx.x / T : 0;
   V4<R>* s4 = reinterpret_cast<V4<R>*>(smem_raw + (size_t)half * tile_smem);  // staging
@@ -262,7 +261,7 @@ __global__ void __launch_bounds__(32 * NW * (SHARE == kTwoTiles ? 2 : 1), SHARE 
       } else {
         plain[1] = c2acc.v;
       }
-      cta_partials<ND, FFD, sizeof(R) == 4 ? 1 : -1, TC, R>(plain, lo, rows, (AccStore<R>*)part_d, gridDim.x, me);
+      cta_partials<ND, sizeof(R) == 4 ? 1 : -1, TC, R>(plain, lo, rows, (AccStore<R>*)part_d, gridDim.x, me);
     }
     bar.arrive();
     for (int w = 0; w < kRowCopies; ++w) zero4(w);
@@ -423,7 +422,7 @@ __global__ void __launch_bounds__(32 * NW * (SHARE == kTwoTiles ? 2 : 1), SHARE 
         GD[2 * v] = V4<R>{gn[0], gn[1], gn[2], R(0)};
         GD[2 * v + 1] = V4<R>{dn[0], dn[1], dn[2], R(0)};
       }
-      cta_partials<NVT, FFV, -1, TC, R>(s, R(0), rows, (AccStore<R>*)part_v, gridDim.x, me);
+      cta_partials<NVT, -1, TC, R>(s, R(0), rows, (AccStore<R>*)part_v, gridDim.x, me);
     }
     bar.arrive();
     zero_rest();
