@@ -381,7 +381,7 @@ Shape shape(const ResidentPlan& p, int n_tiles) {
   if (REC) smem += records_bytes<MAT>(p);
   // up to one tile per SM: more shared memory than half an SM's, so that no
   // two CTAs share an SM while others idle
-  if (n_tiles <= kSMs) smem = std::max(smem, (size_t)120 * 1024);
+  if (n_tiles <= p.sms) smem = std::max(smem, (size_t)120 * 1024);
   return Shape{cg_resident_kernel<R, MAT, NW, REC>, n_tiles, 32 * NW, smem};
 }
 

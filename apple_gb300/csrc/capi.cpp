@@ -135,6 +135,16 @@ int upload_records(const TilePlan& plan, int precision, void** d_rec, uint32_t**
   return dupload(d_ids, plan.ids);
 }
 
+// the SMs that tiles are cut and paired for: the device's, at most
+// kResidentMaxTiles / 2
+int resident_sms(int* out) {
+  int dev = 0;
+  AGB_CHECK_CUDA(cudaGetDevice(&dev));
+  AGB_CHECK_CUDA(cudaDeviceGetAttribute(out, cudaDevAttrMultiProcessorCount, dev));
+  *out = std::min(*out, kResidentMaxTiles / 2);
+  return AGB_OK;
+}
+
 cudaStream_t as_stream(void* s) { return static_cast<cudaStream_t>(s); }
 
 int check_launch(cudaError_t e, const char* what) {
@@ -431,11 +441,13 @@ int agb_fem_create(agb_space* space, int material, int precision, int32_t n_cell
   if (!rc) spread_banks(&f->plan);
   std::vector<SlotMap> sm;
   std::vector<int32_t> own_off;
+  int sms = 0;
+  if (!rc) rc = resident_sms(&sms);
   if (!rc) {
     // An SM's FP64 work goes through one pipe: 214 whole tiles leave some SMs
     // with two and some with one.
-    if (precision == AGB_F64 && f->plan.n_tiles > 0 && f->plan.n_tiles <= kResidentMaxTiles)
-      split_tiles(f->plan, kResidentMaxTiles / 2, 2, &f->pieces);
+    if (precision == AGB_F64 && f->plan.n_tiles > 0 && f->plan.n_tiles <= 2 * sms)
+      split_tiles(f->plan, sms, 2, &f->pieces);
     build_slots(np, {&f->eval_plan()}, &sm, &own_off);
     f->vol_internal.resize(n_cells);
     for (int e = 0; e < n_cells; ++e) f->vol_internal[e] = vol[f->plan.elem_user[e]];
@@ -970,12 +982,14 @@ int agb_solver_create(agb_model* m, const agb_pncg_params* params, agb_solver** 
   // there, so such a mesh keeps the three-kernel iteration)
   bool covered = true;
   for (int v = 0; v < np && covered; ++v) covered = m->off[v + 1] > m->off[v];
-  const bool small = covered && mat != AGB_ARAP && sv->fv.n_tiles > 0 && sv->fv.n_tiles <= kResidentMaxTiles;
+  int sms = 0;
+  if (!rc) rc = resident_sms(&sms);
+  const bool small = covered && mat != AGB_ARAP && sv->fv.n_tiles > 0 && sv->fv.n_tiles <= 2 * sms;
   TilePlan pieces;
   FemView fv = sv->fv;
   int32_t n_slots = m->n_slots;
   if (!rc && small) {
-    split_tiles(m->fems.size() == 1 ? m->fems[0]->plan : sv->plan, kResidentMaxTiles / 2, 2, &pieces);
+    split_tiles(m->fems.size() == 1 ? m->fems[0]->plan : sv->plan, sms, 2, &pieces);
     std::vector<SlotMap> sm;
     std::vector<int32_t> off;
     build_slots(np, {&pieces}, &sm, &off);
@@ -1084,13 +1098,15 @@ int agb_solver_create(agb_model* m, const agb_pncg_params* params, agb_solver** 
   if (small) {
     largest_tile(pieces, &sv->resident);
     const int n_whole = m->fems.size() == 1 ? m->fems[0]->plan.n_tiles : sv->plan.n_tiles;
-    sv->resident.whole = n_whole > kResidentMaxTiles / 2 ? kResidentMaxTiles / 2 : 0;
-    if (sv->precision == AGB_F64 && pieces.n_tiles > kResidentMaxTiles / 2) {
-      rc = dupload(&sv->d_piece_order, pair_tiles(pieces, kResidentMaxTiles / 2));
+    sv->resident.sms = sms;
+    sv->resident.whole = n_whole > sms ? sms : 0;
+    if (sv->precision == AGB_F64 && pieces.n_tiles > sms) {
+      rc = dupload(&sv->d_piece_order, pair_tiles(pieces, sms));
       sv->resident.order = sv->d_piece_order;
     }
     if (!rc) rc = check_launch(resident_prepare(a, &sv->resident), "resident_prepare");
     const bool fits = sv->resident.shape != 0;
+    if (!fits) a = sv->whole;  // the three-kernel iteration: cut tiles would only add slots
     if (!rc && fits) rc = dalloc_bytes(&sv->d_res_part, 8 * 18 * (size_t)kResidentMaxTiles);
     if (!rc && fits) rc = dalloc(&sv->d_res_counters, kResidentCounters);
     if (!rc && fits && cudaMemset(sv->d_res_counters, 0, kResidentCounters * sizeof(unsigned)) != cudaSuccess) rc = AGB_E_CUDA;
@@ -1557,7 +1573,8 @@ static int cg_setup(agb_solver* sv) {
   if (!rc && cg_prepare_kernels(sv->precision) != cudaSuccess) rc = AGB_E_CUDA;
   if (!rc) {
     largest_tile(sv->model->fems.size() == 1 ? sv->model->fems[0]->plan : sv->plan, &sv->cg_resident);
-    rc = check_launch(cg_resident_prepare(sv->whole, &sv->cg_resident), "cg_resident_prepare");
+    rc = resident_sms(&sv->cg_resident.sms);
+    if (!rc) rc = check_launch(cg_resident_prepare(sv->whole, &sv->cg_resident), "cg_resident_prepare");
   }
   if (!rc && sv->cg_resident.shape) {
     rc = dalloc_bytes(&sv->d_cg_res_part, 8 * 3 * (size_t)sv->fv.n_tiles);

@@ -149,6 +149,7 @@ struct ResidentPlan {
   int shape = 0;
   int max_elems = 0;
   int max_groups = 0;
+  int sms = 0;    // the SMs that the tiles are cut and paired for
   int whole = 0;  // FP32: the first tiles are this many whole ones, the others cut (0: all alike)
   const int32_t* order = nullptr;  // FP64 with more tiles than SMs: pair_tiles()
   uint64_t wait_ns = 2000000000;   // limit of a grid barrier's wait

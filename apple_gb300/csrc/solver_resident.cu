@@ -467,8 +467,8 @@ Shape shape(const ResidentPlan& p, int n_tiles) {
   smem = (smem + 15) & ~(size_t)15;
   if constexpr (sizeof(R) == 4) {
     return Shape{solver_resident_kernel<R, MAT, DELTA, NW, REC, kTwoCtas>, n_tiles, 32 * NW, smem, 0};
-  } else if (n_tiles > kSMs) {
-    return Shape{solver_resident_kernel<R, MAT, DELTA, NW, REC, kTwoTiles>, kSMs, 64 * NW, 2 * smem, (int)smem};
+  } else if (n_tiles > p.sms) {
+    return Shape{solver_resident_kernel<R, MAT, DELTA, NW, REC, kTwoTiles>, p.sms, 64 * NW, 2 * smem, (int)smem};
   } else {
     // more shared memory than half an SM's: no two CTAs share an SM while others idle
     return Shape{solver_resident_kernel<R, MAT, DELTA, NW, REC, kAlone>, n_tiles, 32 * NW,
