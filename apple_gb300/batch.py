@@ -20,7 +20,17 @@ import torch
 
 from . import _lib
 from .fem import ptr, stream_ptr
+from .model import DofMap, Model
 from .pncg import PNCG, Solution
+
+
+def _initial_u(model) -> torch.Tensor:
+    """``model.init().u``; for this package's own model and map without the
+    launch: the fixed values, zero elsewhere."""
+    dof_map = model.dof_map
+    if type(model) is Model and type(dof_map) is DofMap and "init" not in vars(model):
+        return dof_map._fill_for(model.dtype).reshape(-1, 3)
+    return model.init().u
 
 
 class BatchedForward:
@@ -60,9 +70,7 @@ class BatchedForward:
         return npt.value, nc.value
 
     def initial_u(self, device="cuda") -> torch.Tensor:
-        # Model.init() of each: the fixed values, zero elsewhere
-        parts = [m.dof_map._fill_for(m.dtype).reshape(-1, 3).to(device) for m in self.models]
-        return torch.cat(parts, 0).contiguous()
+        return torch.cat([_initial_u(m).to(device) for m in self.models], 0).contiguous()
 
     def reset(self, u: torch.Tensor | None = None) -> None:
         u = self.initial_u() if u is None else u
