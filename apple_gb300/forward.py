@@ -7,7 +7,7 @@ import functools
 
 import torch
 
-from .model import DofMap, DofMapBuilder, Model, ModelBuilder
+from .model import DofMap, DofMapBuilder, Model, ModelBuilder, WarpModel
 from .pncg import PNCG, ConvergenceCriteria, LineSearch, Solution
 
 # the names of liblaf.apple.forward (forward/__init__.pyi)
@@ -60,7 +60,9 @@ class ForwardProblem:
 
 
 def _eval_free(model, u: torch.Tensor, what: str, p: torch.Tensor | None = None):
-    if type(model) is not Model or type(model.dof_map) is not DofMap:
+    wm = getattr(model, "warp_model", None)
+    if type(model) is not Model or type(model.dof_map) is not DofMap or type(wm) is not WarpModel \
+            or what in vars(model) or what in vars(wm):
         return None
     return model.eval_free(u, what, p)
 

@@ -277,8 +277,9 @@ class Model:
         if not isinstance(u, torch.Tensor) or not u.is_cuda or u.device != dm.slot.device or dm.dim != 3 \
                 or dm.n_points != wm.n_points or dm.n_free == 0:
             return None
-        if p is not None and not (isinstance(p, torch.Tensor) and p.dtype == wm.dtype and p.device == u.device
-                                  and p.numel() == dm.n_free and p.is_contiguous()):
+        if what in ("hess_prod", "hess_quad") and not (
+                isinstance(p, torch.Tensor) and p.dtype == wm.dtype and p.device == u.device
+                and p.numel() == dm.n_free and p.is_contiguous()):
             return None
         check_vec(u, wm.n_points, wm.dtype, "u")
         quad = what == "hess_quad"
