@@ -785,7 +785,15 @@ static int model_eval(agb_model* m, unsigned flags, const int32_t* slot, const v
   if ((flags & AGB_FUN) && !any_tiles) AGB_CHECK_CUDA(cudaMemsetAsync(energy, 0, sizeof(double), s));
   if ((flags & AGB_HESS_QUAD) && !any_tiles) AGB_CHECK_CUDA(cudaMemsetAsync(quad, 0, sizeof(double), s));
   if (!flags) return AGB_OK;
-  int assign = 1;
+  // outputs that are one buffer receive their sum: zeroed, then accumulated into
+  const bool g = flags & AGB_GRAD, d = flags & AGB_HESS_DIAG, h = flags & AGB_HESS_PROD;
+  const bool one_vector = !slot && ((g && d && grad == diag) || (g && h && grad == prod) || (d && h && diag == prod));
+  const bool one_scalar = (flags & AGB_FUN) && (flags & AGB_HESS_QUAD) && energy == quad;
+  if (one_scalar && any_tiles) AGB_CHECK_CUDA(cudaMemsetAsync(energy, 0, sizeof(double), s));
+  if (one_vector)
+    for (void* out : {g ? grad : nullptr, d ? diag : nullptr, h ? prod : nullptr})
+      if (out) AGB_CHECK_CUDA(cudaMemsetAsync(out, 0, 3 * (size_t)np * real_bytes(m->precision), s));
+  int assign = one_scalar ? 0 : 1;
   for (size_t k = 0; k < m->fems.size(); ++k) {
     RC(check_launch(launch_fem_eval(m->precision, m->fems[k]->eval_view(), flags, u, p, slot, m->d_slot_of_tv[k], m->d_slots,
                                     m->n_eval_slots, m->d_partials, m->d_counter, energy, quad, assign, s),
@@ -796,7 +804,7 @@ static int model_eval(agb_model* m, unsigned flags, const int32_t* slot, const v
   const bool ext = m->d_force != nullptr;
   if ((vec & ~AGB_FUN) || (ext && (flags & AGB_FUN)))
     RC(check_launch(launch_unpack(m->precision, np, m->space->d_user_of_internal, m->d_eval_off, m->d_slots, m->n_eval_slots,
-                                  vec, grad, diag, prod, slot, 1, m->d_force, u, m->d_partials, m->d_counter, energy, s),
+                                  vec, grad, diag, prod, slot, one_vector ? 0 : 1, m->d_force, u, m->d_partials, m->d_counter, energy, s),
                     "unpack"));
   return AGB_OK;
 }
