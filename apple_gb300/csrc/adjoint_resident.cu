@@ -121,7 +121,6 @@ __global__ void __launch_bounds__(32 * NW, 2) cg_resident_kernel(CgArgs c, int m
   }
   if constexpr (REC) keep_records<MAT>(a.fv, tile, max_elems, srec, sgrp, threadIdx.x, blockDim.x);
   const GroupLoader<R, MAT, REC> load{a.fv, gs, max_elems, srec, sgrp};
-  const int w0 = decision_warp<NW>();
   __syncthreads();
 
   bool ok = true;
@@ -250,7 +249,7 @@ __global__ void __launch_bounds__(32 * NW, 2) cg_resident_kernel(CgArgs c, int m
     bar.arrive();
     if (!(ok = bar.wait())) break;
     grid_totals<1, T, R>((const AccStore<R>*)part_p, gridDim.x, tot);
-    if (warp == w0) {
+    if (warp == 0) {
       const double pq = tot[0].value();
       const bool pos = positive_finite(pq);  // else H is not positive definite along p, or NaN
       const double al = pos ? cs.rz / pq : 0.0;
@@ -305,7 +304,7 @@ __global__ void __launch_bounds__(32 * NW, 2) cg_resident_kernel(CgArgs c, int m
     bar.arrive();
     if (!(ok = bar.wait())) break;
     grid_totals<2, T, R>((const AccStore<R>*)part_v, gridDim.x, tot);
-    if (warp == w0) {
+    if (warp == 0) {
       const double rz = tot[0].value();
       const double b = cs.rz > 0.0 ? rz / cs.rz : 0.0;
       __syncwarp();
@@ -314,7 +313,7 @@ __global__ void __launch_bounds__(32 * NW, 2) cg_resident_kernel(CgArgs c, int m
         cs.rz = rz;
         s_beta = to_real<R>(b);
       }
-    } else if (warp == w0 + 1) {
+    } else if (warp == 1) {
       const double rr = tot[1].value();
       const double rn = sqrt(rr);
       const bool small = rn <= fmax(cs.atol, cs.rtol * sqrt(cs.rr0));

@@ -16,7 +16,7 @@
 namespace agb {
 
 // FP64 arithmetic is the bound of every FP64 pass (GB300: one FP64 warp
-// instruction per 16 cycles and SM), so the double forms below share
+// instruction per 19 cycles and SM, measured), so the double forms below share
 // subexpressions that the FP32 ones leave to the compiler, and clamp in the
 // integer pipe.  Measured: 20 FP64 iterations of 138,240 tets 4,458 -> 4,168 us,
 // 40,000 tets 2,400 -> 2,160; the FP64 refresh of the reference state on the

@@ -34,21 +34,6 @@ __device__ __forceinline__ V4<double> ldcg4<double>(const V4<double>* p) {
   return V4<double>{a.x, a.y, b.x, b.y};
 }
 
-// The first warp of the scalar decisions: the second CTA of an SM uses other
-// schedulers' FP64 pipes than the first.  Every thread calls it; a
-// __syncthreads before it and one after.
-template <int NW>
-__device__ __forceinline__ int decision_warp() {
-  __shared__ int s_w0;
-  if (threadIdx.x == 0) {
-    unsigned slot;
-    asm volatile("mov.u32 %0, %%warpid;" : "=r"(slot));
-    s_w0 = (int)((slot / NW) & 1u);
-  }
-  __syncthreads();
-  return s_w0;
-}
-
 // Element records kept in shared memory (FP32): the float4 streams of the
 // tile, [stream][element], and its groups' first elements.  A barrier's
 // acquire leaves nothing in L1, so every pass would fetch them from L2.

@@ -26,11 +26,11 @@ __device__ __forceinline__ bool guard_skip(const SolveArgs& a, const SolverState
 
 // Scalar decisions.  A GB300 warp issues one FP64 instruction per 65 cycles,
 // whatever its lanes and its parallelism (measured: 65.4 cycles per DFMA in
-// one chain or in four; a division 690, a square root 706), and its four
-// schedulers work independently.  The decisions therefore convert all sums in
-// one instruction (a sum per lane), test signs, finiteness and magnitudes in
-// the integer pipe, and give independent quotients and roots to different
-// warps.
+// one chain or in four; a division 690, a square root 706); the SM's one FP64
+// pipe takes one per 19 cycles, so three warps do not slow each other.  The
+// decisions therefore convert all sums in one instruction (a sum per lane),
+// test signs, finiteness and magnitudes in the integer pipe, and give
+// independent quotients and roots to three warps.
 __device__ __forceinline__ bool finite_bits(double x) {
   return (__double2hiint(x) & 0x7ff00000) != 0x7ff00000;
 }
@@ -416,17 +416,17 @@ __device__ __forceinline__ void trial_decide(SolverState* st, double a0, int j0,
 // After the vertex pass, by every thread of the CTA (at least 96): Dai-Kou
 // beta, preconditioner mean, descent check and termination from the 12 sums
 // 0 gPg 1 gPy 2 yPy 3 sum|d| 4 count 5 zgg 6 zgy 7 zyy 8 y.p 9 p.g 10 g.g 11 ext energy
-// Of three warps from `w0` on, the first forms the mean fill and its three
+// Of the first three warps, the first forms the mean fill and its three
 // products, the second 1 / y.p, the third the gradient norm and its tests; the
 // first finishes.
 template <class R>
-__device__ __forceinline__ void vertex_decide(SolverState* st, const Acc<R>* tot, int w0 = 0) {
+__device__ __forceinline__ void vertex_decide(SolverState* st, const Acc<R>* tot) {
   constexpr unsigned ALL = 0xffffffffu;
   __shared__ double s_d[3];
   __shared__ int s_flags;
-  const int lane = threadIdx.x & 31, warp = (int)(threadIdx.x >> 5) - w0;
+  const int lane = threadIdx.x & 31, warp = (int)(threadIdx.x >> 5);
   double v = 0.0, inv_m = 1.0, filled = 0.0;
-  if (warp >= 0 && warp < 3) v = tot[lane < 12 ? lane : 0].value();
+  if (warp < 3) v = tot[lane < 12 ? lane : 0].value();
   if (warp == 0) {
     const double sad = __shfl_sync(ALL, v, 3), cnt = __shfl_sync(ALL, v, 4);
     const double mean = cnt / sad;

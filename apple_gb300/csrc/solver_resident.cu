@@ -189,9 +189,6 @@ __global__ void __launch_bounds__(32 * NW * (SHARE == kTwoTiles ? 2 : 1), SHARE 
   __syncthreads();  // every thread has read sst.pbuf; records and groups are in place
   if (threadIdx.x == 0) sst.refresh = 0;  // the refresh passes, if any, ran after the last vertex pass
 
-  // two CTAs of an SM decide on different schedulers
-  const int w0 = SHARE == kTwoCtas ? decision_warp<NW>() : 0;
-
   bool ok = true;
   for (;;) {
     // ---- direction ----
@@ -271,7 +268,7 @@ __global__ void __launch_bounds__(32 * NW * (SHARE == kTwoTiles ? 2 : 1), SHARE 
     n = 0;
     if (!REC && g < ge) load_group(g, n, geo, ids);
     grid_totals<ND, TC, R>((const AccStore<R>*)part_d, gridDim.x, tot);
-    if (threadIdx.x / 32 == w0) dir_decide<MAT, R>(&sst, tot);
+    if (threadIdx.x < 32) dir_decide<MAT, R>(&sst, tot);
     __syncthreads();
     const R t = to_real<R>(sst.t);
 
@@ -428,7 +425,7 @@ __global__ void __launch_bounds__(32 * NW * (SHARE == kTwoTiles ? 2 : 1), SHARE 
     zero_rest();
     if (!(ok = bar.wait())) break;
     grid_totals<NVT, TC, R>((const AccStore<R>*)part_v, gridDim.x, tot);
-    vertex_decide<R>(&sst, tot, w0);
+    vertex_decide<R>(&sst, tot);
     __syncthreads();
     if (sst.done || sst.iter >= sst.iter_limit || sst.refresh) break;
   }
