@@ -1317,6 +1317,13 @@ static int build_step_graph(agb_solver* sv) {
   return check_launch(e, "solver step graph");
 }
 
+int agb_solver_info(const agb_solver* sv, int32_t* resident_iterations, int32_t* resident_adjoint) {
+  AGB_REQUIRE(sv, AGB_E_INVALID, "agb_solver_info: null handle");
+  if (resident_iterations) *resident_iterations = sv->resident.shape != 0;
+  if (resident_adjoint) *resident_adjoint = sv->cg_ready ? sv->cg_resident.shape != 0 : -1;
+  return AGB_OK;
+}
+
 int agb_solver_step_kernels(agb_solver* sv, int32_t* n_kernels) {
   AGB_REQUIRE(sv && n_kernels, AGB_E_INVALID, "agb_solver_step_kernels: null argument");
   if (!sv->step_exec) RC(build_step_graph(sv));

@@ -202,10 +202,17 @@ class DeviceSolver:
         return {"hess_quad": out[0], "gd": out[1], "grad_norm": out[2], "precond_fill_inv": out[3], "beta": out[4]}
 
     def step_kernels(self) -> int:
-        """Kernels one iteration launches (the nodes of the step graph)."""
+        """Kernels one :meth:`step` launches (the nodes of the step graph)."""
         n = ctypes.c_int32()
         _lib.call("agb_solver_step_kernels", self.handle, ctypes.byref(n))
         return n.value
+
+    def info(self) -> dict:
+        """Whether the iterations and the adjoint CG (None before its first
+        call) run in one cooperative launch."""
+        it, cg = ctypes.c_int32(), ctypes.c_int32()
+        _lib.call("agb_solver_info", self.handle, ctypes.byref(it), ctypes.byref(cg))
+        return {"resident_iterations": bool(it.value), "resident_adjoint": None if cg.value < 0 else bool(cg.value)}
 
     def read(self, u_out: torch.Tensor | None = None) -> Solution:
         st = _lib.PncgStats()

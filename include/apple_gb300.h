@@ -268,15 +268,22 @@ int agb_solver_reset(agb_solver* solver, const void* u, void* stream);
 /* run up to n_steps iterations (fewer if the solve terminates); the loop
  * runs on the device as one CUDA graph launch (conditional while node; with
  * the FP32 correction on, the two refresh passes sit in an outer while loop
- * and run only when a refresh is due). */
+ * and run only when a refresh is due), or where iterations are resident and
+ * the correction is off as one cooperative launch. */
 int agb_solver_iterate(agb_solver* solver, int32_t n_steps, void* stream);
 /* exactly one iteration as one graph launch (benchmark building block); with
  * the FP32 correction on, the two refresh passes follow and return at once
  * unless a refresh is due */
 int agb_solver_step(agb_solver* solver, void* stream);
-/* number of kernels one iteration of agb_solver_step launches (the three
- * passes, plus the two refresh passes when the FP32 correction is on) */
+/* number of kernels one iteration of agb_solver_step launches: the three
+ * passes, or where iterations are resident (agb_solver_info) the limit and the
+ * cooperative launch; plus the two refresh passes when the FP32 correction is
+ * on */
 int agb_solver_step_kernels(agb_solver* solver, int32_t* n_kernels);
+/* The form that this solver's work takes, 1: one cooperative launch, 0: a
+ * kernel per pass: of its iterations, and of its adjoint CG (-1 before the
+ * first agb_solver_adjoint).  Host only; either pointer may be NULL. */
+int agb_solver_info(const agb_solver* solver, int32_t* resident_iterations, int32_t* resident_adjoint);
 /* copy u out (device, caller order) and the stats (host); synchronises stream */
 int agb_solver_read(agb_solver* solver, void* u_out, agb_pncg_stats* stats, void* stream);
 /* the search direction p of the last iteration (the step taken was
@@ -388,7 +395,8 @@ void agb_cg_default_params(agb_cg_params* params);
  * positive ones as in the PNCG preconditioner).  H is the sum of the model's
  * hess_prod (warp/fem/_base.py:326-351); fixed components of lam are 0.
  * rhs and lam: device, caller order, n_points x 3 of the solver precision.
- * The CG loop runs on the device as one CUDA graph launch; stats on the host.
+ * The CG loop runs on the device as one CUDA graph launch or one cooperative
+ * launch (agb_solver_info); stats on the host.
  * The solver's PNCG state is not modified.  Only for models whose potentials
  * share one material (the solver's element passes). */
 int agb_solver_adjoint(agb_solver* solver, const void* rhs, void* lam, const agb_cg_params* params,
