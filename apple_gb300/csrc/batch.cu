@@ -3,8 +3,9 @@
 // The meshes' vertices and tiles are concatenated (tiles never span meshes,
 // vertex chunks never span meshes).  An iteration is five kernels (three in
 // small batches, batch_fused below), captured in a CUDA graph; every mesh
-// carries its own SolverState, so each one runs the reference's PNCG iteration (benches/bench_pncg_branching_backends.py
-// :254-456, 606-679) with its own beta, step and termination:
+// carries its own SolverState, so each one runs the reference's PNCG iteration
+// (benches/bench_pncg_branching_backends.py:254-456, 606-679) with its own
+// beta, step and termination:
 //   direction pass   one CTA per tile: p of the tile's mesh, p^T H p and the
 //                    energy polynomial; one partial per tile
 //   direction tail   one CTA per mesh: the mesh's tile partials in tile order,

@@ -104,10 +104,9 @@ int upload_act(const std::vector<double>& act, size_t n, int precision, void** d
   return upload(*d_act, v.data(), v.size() * sizeof(double));
 }
 
-int upload_records(const TilePlan& plan, int precision, void** d_rec, uint32_t** d_ids,
-                   const std::vector<double>* D_override = nullptr) {
+int upload_records(const TilePlan& plan, int precision, void** d_rec, uint32_t** d_ids) {
   const size_t n = (size_t)plan.n_cells;
-  const std::vector<double>& D = D_override ? *D_override : plan.D;
+  const std::vector<double>& D = plan.D;
   if (precision == AGB_F32) {
     std::vector<float> rec(12 * n);
     for (size_t e = 0; e < n; ++e) {
@@ -359,8 +358,9 @@ int agb_fem_destroy(agb_fem* f) {
   for (void* p : {(void*)f->d_tile_estart, (void*)f->d_tile_vstart, (void*)f->d_tile_gstart,
                   (void*)f->d_group_estart, (void*)f->d_tv_vid, (void*)f->d_tv_user,
                   (void*)f->d_piece_vstart, (void*)f->d_piece_gstart, (void*)f->d_piece_user,
-                  (void*)f->d_own_slot, (void*)f->d_own_off, f->d_rec, (void*)f->d_ids, f->d_slots, (void*)f->d_partials, (void*)f->d_counter,
-                  (void*)f->d_elem_user, f->d_vol, f->d_act, (void*)f->d_D, (void*)f->d_act_user})
+                  (void*)f->d_own_slot, (void*)f->d_own_off, f->d_rec, (void*)f->d_ids, f->d_slots,
+                  (void*)f->d_partials, (void*)f->d_counter, (void*)f->d_elem_user, f->d_vol, f->d_act,
+                  (void*)f->d_D, (void*)f->d_act_user})
     dfree(p);
   delete f;
   return AGB_OK;
@@ -596,8 +596,8 @@ static int fem_eval(agb_fem* f, unsigned flags, const void* u, const void* p, do
   const unsigned vec = flags & (AGB_GRAD | AGB_HESS_DIAG | AGB_HESS_PROD);
   if (vec)
     RC(check_launch(launch_unpack(f->precision, np, f->space->d_user_of_internal, f->d_own_off, f->d_slots,
-                                  f->eval_plan().n_tv, vec, grad, diag, prod, nullptr, assign, nullptr, u, f->d_partials, f->d_counter,
-                                  nullptr, s),
+                                  f->eval_plan().n_tv, vec, grad, diag, prod, nullptr, assign, nullptr, u,
+                                  f->d_partials, f->d_counter, nullptr, s),
                     "unpack"));
   return AGB_OK;
 }
@@ -795,16 +795,17 @@ static int model_eval(agb_model* m, unsigned flags, const int32_t* slot, const v
       if (out) AGB_CHECK_CUDA(cudaMemsetAsync(out, 0, 3 * (size_t)np * real_bytes(m->precision), s));
   int assign = one_scalar ? 0 : 1;
   for (size_t k = 0; k < m->fems.size(); ++k) {
-    RC(check_launch(launch_fem_eval(m->precision, m->fems[k]->eval_view(), flags, u, p, slot, m->d_slot_of_tv[k], m->d_slots,
-                                    m->n_eval_slots, m->d_partials, m->d_counter, energy, quad, assign, s),
+    RC(check_launch(launch_fem_eval(m->precision, m->fems[k]->eval_view(), flags, u, p, slot, m->d_slot_of_tv[k],
+                                    m->d_slots, m->n_eval_slots, m->d_partials, m->d_counter, energy, quad, assign, s),
                     "fem_eval"));
     if (m->fems[k]->plan.n_tiles > 0) assign = 0;
   }
   const unsigned vec = flags & (AGB_GRAD | AGB_HESS_DIAG | AGB_HESS_PROD | AGB_FUN);
   const bool ext = m->d_force != nullptr;
   if ((vec & ~AGB_FUN) || (ext && (flags & AGB_FUN)))
-    RC(check_launch(launch_unpack(m->precision, np, m->space->d_user_of_internal, m->d_eval_off, m->d_slots, m->n_eval_slots,
-                                  vec, grad, diag, prod, slot, one_vector ? 0 : 1, m->d_force, u, m->d_partials, m->d_counter, energy, s),
+    RC(check_launch(launch_unpack(m->precision, np, m->space->d_user_of_internal, m->d_eval_off, m->d_slots,
+                                  m->n_eval_slots, vec, grad, diag, prod, slot, one_vector ? 0 : 1, m->d_force, u,
+                                  m->d_partials, m->d_counter, energy, s),
                     "unpack"));
   return AGB_OK;
 }
@@ -1117,7 +1118,8 @@ int agb_solver_create(agb_model* m, const agb_pncg_params* params, agb_solver** 
     if (!fits) a = sv->whole;  // the three-kernel iteration: cut tiles would only add slots
     if (!rc && fits) rc = dalloc_bytes(&sv->d_res_part, 8 * 18 * (size_t)kResidentMaxTiles);
     if (!rc && fits) rc = dalloc(&sv->d_res_counters, kResidentCounters);
-    if (!rc && fits && cudaMemset(sv->d_res_counters, 0, kResidentCounters * sizeof(unsigned)) != cudaSuccess) rc = AGB_E_CUDA;
+    if (!rc && fits && cudaMemset(sv->d_res_counters, 0, kResidentCounters * sizeof(unsigned)) != cudaSuccess)
+      rc = AGB_E_CUDA;
     if (rc) {
       if (rc == AGB_E_CUDA && agb::last_error()[0] == 0) set_error("agb_solver_create: CUDA allocation failed");
       agb_solver_destroy(sv);

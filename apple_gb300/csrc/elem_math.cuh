@@ -511,73 +511,73 @@ __device__ void svd_rv(const R (&G)[3][3], R jm1, Svd<R>& out) {
       for (int j = i; j < 3; ++j) A[i][j] = A[j][i] = V[0][i] * EV[0][j] + V[1][i] * EV[1][j] + V[2][i] * EV[2][j];
   } else {
 #pragma unroll
-      for (int i = 0; i < 3; ++i)
+    for (int i = 0; i < 3; ++i)
 #pragma unroll
-        for (int j = 0; j < 3; ++j) V[i][j] = (i == j) ? R(1) : R(0);
-    }
-    const R eps = sizeof(R) == 4 ? R(1e-7) : R(1e-15);
-    for (int sweep = 0; sweep < 8; ++sweep) {
-      const R off = A[0][1] * A[0][1] + A[0][2] * A[0][2] + A[1][2] * A[1][2];
-      const R dia = A[0][0] * A[0][0] + A[1][1] * A[1][1] + A[2][2] * A[2][2];
-      if (off <= eps * eps * (dia + R(1e-30))) break;
-      jacobi_rotate(A, V, 0, 1);
-      jacobi_rotate(A, V, 0, 2);
-      jacobi_rotate(A, V, 1, 2);
-    }
-    R e[3] = {A[0][0], A[1][1], A[2][2]};
-    if (e[0] < e[1]) swap_cols(V, e, 0, 1);
-    if (e[0] < e[2]) swap_cols(V, e, 0, 2);
-    if (e[1] < e[2]) swap_cols(V, e, 1, 2);
-    // F v_i = v_i + G v_i
-    R b0[3], b1[3];
+      for (int j = 0; j < 3; ++j) V[i][j] = (i == j) ? R(1) : R(0);
+  }
+  const R eps = sizeof(R) == 4 ? R(1e-7) : R(1e-15);
+  for (int sweep = 0; sweep < 8; ++sweep) {
+    const R off = A[0][1] * A[0][1] + A[0][2] * A[0][2] + A[1][2] * A[1][2];
+    const R dia = A[0][0] * A[0][0] + A[1][1] * A[1][1] + A[2][2] * A[2][2];
+    if (off <= eps * eps * (dia + R(1e-30))) break;
+    jacobi_rotate(A, V, 0, 1);
+    jacobi_rotate(A, V, 0, 2);
+    jacobi_rotate(A, V, 1, 2);
+  }
+  R e[3] = {A[0][0], A[1][1], A[2][2]};
+  if (e[0] < e[1]) swap_cols(V, e, 0, 1);
+  if (e[0] < e[2]) swap_cols(V, e, 0, 2);
+  if (e[1] < e[2]) swap_cols(V, e, 1, 2);
+  // F v_i = v_i + G v_i
+  R b0[3], b1[3];
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      b0[k] = V[k][0] + G[k][0] * V[0][0] + G[k][1] * V[1][0] + G[k][2] * V[2][0];
-      b1[k] = V[k][1] + G[k][0] * V[0][1] + G[k][1] * V[1][1] + G[k][2] * V[2][1];
-    }
-    normalize3(b0, R(1));
-    const R proj = b0[0] * b1[0] + b0[1] * b1[1] + b0[2] * b1[2];
+  for (int k = 0; k < 3; ++k) {
+    b0[k] = V[k][0] + G[k][0] * V[0][0] + G[k][1] * V[1][0] + G[k][2] * V[2][0];
+    b1[k] = V[k][1] + G[k][0] * V[0][1] + G[k][1] * V[1][1] + G[k][2] * V[2][1];
+  }
+  normalize3(b0, R(1));
+  const R proj = b0[0] * b1[0] + b0[1] * b1[1] + b0[2] * b1[2];
 #pragma unroll
-    for (int k = 0; k < 3; ++k) b1[k] -= proj * b0[k];
-    {
-      const R n2 = b1[0] * b1[0] + b1[1] * b1[1] + b1[2] * b1[2];
-      if (n2 > R(1e-30)) {
-        const R r = rsqrt_(n2);
-        b1[0] *= r;
-        b1[1] *= r;
-        b1[2] *= r;
-      } else {  // rank <= 1: any unit vector orthogonal to b0
-        R a[3] = {R(0), R(0), R(0)};
-        const int k = (fabs(b0[0]) <= fabs(b0[1]) && fabs(b0[0]) <= fabs(b0[2]))
-                          ? 0
-                          : (fabs(b0[1]) <= fabs(b0[2]) ? 1 : 2);
-        a[k] = R(1);
-        b1[0] = b0[1] * a[2] - b0[2] * a[1];
-        b1[1] = b0[2] * a[0] - b0[0] * a[2];
-        b1[2] = b0[0] * a[1] - b0[1] * a[0];
-        normalize3(b1, R(0));
-      }
+  for (int k = 0; k < 3; ++k) b1[k] -= proj * b0[k];
+  {
+    const R n2 = b1[0] * b1[0] + b1[1] * b1[1] + b1[2] * b1[2];
+    if (n2 > R(1e-30)) {
+      const R r = rsqrt_(n2);
+      b1[0] *= r;
+      b1[1] *= r;
+      b1[2] *= r;
+    } else {  // rank <= 1: any unit vector orthogonal to b0
+      R a[3] = {R(0), R(0), R(0)};
+      const int k = (fabs(b0[0]) <= fabs(b0[1]) && fabs(b0[0]) <= fabs(b0[2]))
+                        ? 0
+                        : (fabs(b0[1]) <= fabs(b0[2]) ? 1 : 2);
+      a[k] = R(1);
+      b1[0] = b0[1] * a[2] - b0[2] * a[1];
+      b1[1] = b0[2] * a[0] - b0[0] * a[2];
+      b1[2] = b0[0] * a[1] - b0[1] * a[0];
+      normalize3(b1, R(0));
     }
+  }
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      out.U[k][0] = b0[k];
-      out.U[k][1] = b1[k];
+  for (int k = 0; k < 3; ++k) {
+    out.U[k][0] = b0[k];
+    out.U[k][1] = b1[k];
+  }
+  out.U[0][2] = b0[1] * b1[2] - b0[2] * b1[1];
+  out.U[1][2] = b0[2] * b1[0] - b0[0] * b1[2];
+  out.U[2][2] = b0[0] * b1[1] - b0[1] * b1[0];
+  const bool inverted = (R(1) + jm1) < R(0);
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const R ei = fmax(e[i], R(-1));
+    const R si = sqrt_ge0(R(1) + ei);
+    if (i == 2 && inverted) {
+      out.s[i] = -si;
+      out.sm1[i] = -si - R(1);
+    } else {
+      out.s[i] = si;
+      out.sm1[i] = quick_div(ei, si + R(1));
     }
-    out.U[0][2] = b0[1] * b1[2] - b0[2] * b1[1];
-    out.U[1][2] = b0[2] * b1[0] - b0[0] * b1[2];
-    out.U[2][2] = b0[0] * b1[1] - b0[1] * b1[0];
-    const bool inverted = (R(1) + jm1) < R(0);
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-      const R ei = fmax(e[i], R(-1));
-      const R si = sqrt_ge0(R(1) + ei);
-      if (i == 2 && inverted) {
-        out.s[i] = -si;
-        out.sm1[i] = -si - R(1);
-      } else {
-        out.s[i] = si;
-        out.sm1[i] = quick_div(ei, si + R(1));
-      }
   }
 }
 

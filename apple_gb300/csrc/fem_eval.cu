@@ -102,8 +102,8 @@ constexpr size_t eval_smem_bytes(int warps) {
 template <class R, int MAT, int NVEC, int MAXT>
 __global__ void __launch_bounds__(MAXT, MAXT == 128 ? (sizeof(R) == 4 ? 5 : 2) : 1) fem_eval_kernel(
     FemView fv, unsigned flags, const R* __restrict__ u, const R* __restrict__ p,
-    const int32_t* __restrict__ p_slot, const int32_t* __restrict__ slot_of_tv, void* __restrict__ slots, int n_slots, AccStore<R>* __restrict__ partials,
-    unsigned* counter, double* energy, double* quad, int assign) {
+    const int32_t* __restrict__ p_slot, const int32_t* __restrict__ slot_of_tv, void* __restrict__ slots,
+    int n_slots, AccStore<R>* __restrict__ partials, unsigned* counter, double* energy, double* quad, int assign) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   V4<R>* sx = reinterpret_cast<V4<R>*>(smem_raw);
   V2<R>* sq = reinterpret_cast<V2<R>*>(sx + kTileVerts);
@@ -307,8 +307,8 @@ constexpr int kUnpackThreads = 256;
 template <class R, int NVEC>
 __global__ void __launch_bounds__(kUnpackThreads) unpack_kernel(
     int n, const int32_t* __restrict__ uoi, const int32_t* __restrict__ off, const void* __restrict__ slots,
-    int n_slots, R* o0, R* o1, R* o2, const int32_t* __restrict__ out_slot, int assign, int force_grad, int force_fun, const V4<R>* __restrict__ force,
-    const R* __restrict__ u, AccStore<R>* partials, unsigned* counter, double* energy) {
+    int n_slots, R* o0, R* o1, R* o2, const int32_t* __restrict__ out_slot, int assign, int force_grad,
+    int force_fun, const V4<R>* __restrict__ force, const R* __restrict__ u, AccStore<R>* partials, unsigned* counter, double* energy) {
   __shared__ Acc<R> red[kUnpackThreads / 32];
   const VecArrays<R, NVEC> in{(unsigned char*)slots, (size_t)n_slots};
   Acc<R> ext[1] = {};
@@ -389,8 +389,8 @@ int eval_warps(int precision, int n_tiles) {
 
 template <class R, int MAT, int NVEC, int MAXT>
 cudaError_t eval_launch(const FemView& fv, int warps, unsigned flags, const void* u, const void* p,
-                        const int32_t* p_slot, const int32_t* slot_of_tv, void* slots, int32_t n_slots, void* partials, unsigned* counter,
-                        double* energy, double* quad, int assign, cudaStream_t s) {
+                        const int32_t* p_slot, const int32_t* slot_of_tv, void* slots, int32_t n_slots,
+                        void* partials, unsigned* counter, double* energy, double* quad, int assign, cudaStream_t s) {
   const bool vectors = flags & (AGB_GRAD | AGB_HESS_DIAG | AGB_HESS_PROD);
   const size_t smem = vectors ? eval_smem_bytes<R, NVEC>(warps) : eval_stage_bytes<R>();
   if (smem > 48 * 1024) {  // above the default limit the kernel has to opt in
@@ -461,28 +461,29 @@ int unpack_blocks(int n_points) {
 }
 
 cudaError_t launch_fem_eval(int precision, const FemView& fv, unsigned flags, const void* u, const void* p,
-                            const int32_t* p_slot, const int32_t* slot_of_tv, void* slots, int32_t n_slots, void* partials,
-                            unsigned* counter, double* energy, double* quad, int assign, cudaStream_t stream) {
+                            const int32_t* p_slot, const int32_t* slot_of_tv, void* slots, int32_t n_slots,
+                            void* partials, unsigned* counter, double* energy, double* quad, int assign,
+                            cudaStream_t stream) {
   if (fv.n_tiles == 0) return cudaSuccess;
   const int nvec = popcount3(vec_mask(flags)), warps = eval_warps(precision, fv.n_tiles);
   if (precision == AGB_F64)
-    return eval_material<double>(nvec, fv, warps, flags, u, p, p_slot, slot_of_tv, slots, n_slots, partials, counter, energy,
-                                 quad, assign, stream);
-  return eval_material<float>(nvec, fv, warps, flags, u, p, p_slot, slot_of_tv, slots, n_slots, partials, counter, energy,
-                              quad, assign, stream);
+    return eval_material<double>(nvec, fv, warps, flags, u, p, p_slot, slot_of_tv, slots, n_slots, partials, counter,
+                                 energy, quad, assign, stream);
+  return eval_material<float>(nvec, fv, warps, flags, u, p, p_slot, slot_of_tv, slots, n_slots, partials, counter,
+                              energy, quad, assign, stream);
 }
 
 cudaError_t launch_unpack(int precision, int n, const int32_t* uoi, const int32_t* off, const void* slots,
                           int32_t n_slots, unsigned flags, void* grad, void* diag, void* prod,
-                          const int32_t* out_slot, int assign, const void* force, const void* u, void* partials, unsigned* counter, double* energy,
-                          cudaStream_t stream) {
+                          const int32_t* out_slot, int assign, const void* force, const void* u, void* partials,
+                          unsigned* counter, double* energy, cudaStream_t stream) {
   if (n <= 0) return cudaSuccess;
   const int nvec = popcount3(vec_mask(flags));
   if (precision == AGB_F64)
-    return unpack_vectors<double>(nvec, n, uoi, off, slots, n_slots, flags, grad, diag, prod, out_slot, assign, force, u,
-                                  partials, counter, energy, stream);
-  return unpack_vectors<float>(nvec, n, uoi, off, slots, n_slots, flags, grad, diag, prod, out_slot, assign, force, u, partials,
-                               counter, energy, stream);
+    return unpack_vectors<double>(nvec, n, uoi, off, slots, n_slots, flags, grad, diag, prod, out_slot, assign, force,
+                                  u, partials, counter, energy, stream);
+  return unpack_vectors<float>(nvec, n, uoi, off, slots, n_slots, flags, grad, diag, prod, out_slot, assign, force, u,
+                               partials, counter, energy, stream);
 }
 
 // ---------------------------------------------------------------------------
@@ -492,8 +493,9 @@ cudaError_t launch_unpack(int precision, int n, const int32_t* uoi, const int32_
 // host: D is read and the records are written once each, coalesced; only the
 // 48-byte activation rows are gathered (cells in the caller's order).
 // Measured on 138,240 cells in FP32: set_activation, energy, gradient and
-// diagonal, and the three VJPs together take 743 us; with host loops and
-// whole-record uploads in place of this kernel they took 4,697 us.
+// diagonal, and the three VJPs together take 286 us; with host loops and
+// whole-record uploads in place of this kernel they took 4,697 us (743 with
+// the evaluation of that time).
 // ---------------------------------------------------------------------------
 template <class R>
 __global__ void __launch_bounds__(256) muscle_records_kernel(int n, const int32_t* __restrict__ elem_user,

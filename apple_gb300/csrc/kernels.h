@@ -20,8 +20,9 @@ inline size_t v4_bytes(int precision) { return 4 * real_bytes(precision); }
 // product (at most 9 reals of each of n_slots); scalar results are added to
 // *energy / *quad by the last block, or with `assign` stored there.
 cudaError_t launch_fem_eval(int precision, const FemView& fv, unsigned flags, const void* u, const void* p,
-                            const int32_t* p_slot, const int32_t* slot_of_tv, void* slots, int32_t n_slots, void* partials,
-                            unsigned* counter, double* energy, double* quad, int assign, cudaStream_t stream);
+                            const int32_t* p_slot, const int32_t* slot_of_tv, void* slots, int32_t n_slots,
+                            void* partials, unsigned* counter, double* energy, double* quad, int assign,
+                            cudaStream_t stream);
 
 // After launch_fem_eval with the same vector flags, in the same stream: sum
 // slots per vertex (CSR `off`) and add them to the caller's (n_points, 3)

@@ -74,7 +74,8 @@ int main() {
             if (iter_args.fv.n_tiles != tiles || iter_args.fv.tv_vid != whole_args.fv.tv_vid ||
                 iter_args.slot_of_tv != whole_args.slot_of_tv || iter_args.off != whole_args.off ||
                 iter_args.n_slots != whole_args.n_slots) {
-              printf("n %d sms %d: no resident form, but %d tiles in place of %d\n", n, sms, iter_args.fv.n_tiles, tiles);
+              printf("n %d sms %d: no resident form, but %d tiles in place of %d\n", n, sms, iter_args.fv.n_tiles,
+                     tiles);
               return 9;
             }
           } else if (precision == AGB_F32 && n == 16 && iter_args.fv.n_tiles <= tiles) {
