@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(32 * NW, 2) cg_resident_kernel(CgArgs c, int m
   const int n = a.n_points, chunks = (n + 31) / 32;
   const int mine = (chunks - tile + (int)gridDim.x - 1) / (int)gridDim.x;  // chunks tile, tile + grid, ...
   if (tid == 0) cs = *c.cs;
-  GridBar bar{counters, kResidentCounters, wait_ns, gridDim.x, 0};
+  GridBar bar{counters, kResidentCounters, wait_ns, gridDim.x, 0, false};
   V4<R>* slots = (V4<R>*)a.slots;
   V4<R>* Z = (V4<R>*)c.q;  // z = M^-1 r of the current residual
   for (int i = tid; i < nv; i += T) {

@@ -2,10 +2,10 @@
 //
 // The barrier is a counter of arrivals: CTA thread 0 adds one and polls until
 // every CTA has arrived `round` times.  The wait is bounded: at its limit it
-// polls once more, gives up and notes that in a counter of its own; its CTA
-// returns, and the others' next waits give up too.  The last CTA to leave the
-// kernel learns whether any wait gave up, after everything the others wrote,
-// and resets the counters for the next launch.
+// polls once more and gives up; its CTA leaves, and the others' next waits give
+// up too.  The counter of CTAs that left also counts those that gave up, so the
+// last one to leave learns of it, after everything the others wrote; it resets
+// the counters for the next launch.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -17,7 +17,8 @@
 namespace agb {
 
 // words of `counters`, zero before the first launch
-constexpr int kArrived = 0, kLeft = 1, kGaveUp = 2, kPlaceWord = 3;
+constexpr int kArrived = 0, kLeft = 1, kPlaceWord = 2;
+constexpr unsigned kGaveUp = 1u << 16;  // in kLeft, above the CTAs that left
 
 struct GridBar {
   unsigned* counters;
@@ -25,6 +26,7 @@ struct GridBar {
   uint64_t limit;      // of a wait, ns
   unsigned n;          // CTAs
   unsigned round;      // barriers passed
+  bool gave_up;        // thread 0: its wait ran out
 
   // every thread of the CTA calls it; what the CTA wrote before is visible to
   // the others after their wait().  Work that needs nothing from them can go
@@ -51,8 +53,8 @@ struct GridBar {
         asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(counters + kArrived) : "memory");
         if ((int)(v - want) >= 0) break;  // the counter may wrap
         if (late) {
-          atomicExch(&counters[kGaveUp], 1u);
           ok = false;
+          gave_up = true;
           break;
         }
       }
@@ -68,11 +70,12 @@ struct GridBar {
     __syncthreads();
     if (threadIdx.x != 0) return false;
     __threadfence();
-    if (atomicAdd(&counters[kLeft], 1u) != n - 1u) return false;
-    __threadfence();
-    const bool gave_up = atomicAdd(&counters[kGaveUp], 0u) != 0u;
+    const unsigned before = atomicAdd(&counters[kLeft], gave_up ? 1u + kGaveUp : 1u);
+    if (before % kGaveUp != n - 1u) return false;
     for (int k = 0; k < words; ++k) counters[k] = 0u;
-    return gave_up;
+    if (before < kGaveUp && !gave_up) return false;
+    __threadfence();  // what the others wrote comes before what the caller reports
+    return true;
   }
 };
 

@@ -155,7 +155,7 @@ struct ResidentPlan {
   uint64_t wait_ns = 2000000000;   // limit of a grid barrier's wait
 };
 // words of `counters` below
-constexpr int kResidentCounters = 5 + 256;
+constexpr int kResidentCounters = 4 + 256;
 cudaError_t resident_prepare(const SolveArgs& a, ResidentPlan* p);
 cudaError_t launch_resident(const SolveArgs& a, const ResidentPlan& p, void* part_d, void* part_v, unsigned* counters,
                             cudaStream_t s);
