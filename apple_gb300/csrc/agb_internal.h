@@ -140,6 +140,8 @@ struct FemView {
   const int32_t* group_estart;
   const int32_t* tv_vid;
   const int32_t* tv_user;  // the caller's point id of each tile vertex (evaluation API)
+  int packed;              // evaluation API, FP64: batches of 32 elements instead of warp groups
+  int max_batches;         // evaluation API: the most batches of a tile
   // FP32: rec = float4[3][n_cells]; FP64: rec = double[11][n_cells] + ids
   const void* rec;
   const uint32_t* ids;
@@ -159,6 +161,8 @@ struct agb_fem {
   // what the evaluation passes run over: in FP64, when all its pieces fit on
   // the SMs two at a time, the plan cut by split_tiles; else empty, the plan
   agb::TilePlan pieces;
+  bool packed = false;     // FemView::packed, max_batches
+  int max_batches = 0;
   const agb::TilePlan& eval_plan() const { return pieces.n_tiles > 0 ? pieces : plan; }
   // device
   int32_t* d_tile_estart = nullptr;

@@ -87,11 +87,12 @@ constexpr size_t eval_smem_bytes(int warps) {
 
 // Bound: the shared-memory pipe and latency in FP32 (staging, gathers and
 // read-modify-writes of 3 NVEC reals per corner), the FP64 pipe in FP64.  The
-// records of a warp's next group are loaded while the current one computes.
-// MAXT 128: four warps per tile and five CTAs per SM in FP32, for meshes with
-// enough tiles to fill the SMs; MAXT 512 (FP64: 256): 8 or 16 warps per tile (blockDim),
-// for meshes with fewer tiles than SMs, where one tile's serial chain of
-// groups is the whole pass (eval_warps below).
+// records of a warp's next batch of elements (a warp group) are loaded while
+// the current one computes.
+// MAXT 128 (FP32): four warps per tile and five CTAs per SM, for meshes with
+// enough tiles to fill the SMs; MAXT 512 (FP64: 256): up to 16 (8) warps per
+// tile (blockDim), for meshes with fewer tiles than SMs, where one tile's
+// serial chain of batches is the whole pass (eval_warps below).
 // A call for scalars alone runs the NVEC 1 kernel without its accumulators:
 // with the vector branches compiled in, the invariants are formed the same
 // way, and the energy and p^T H p have the same element values whatever else
@@ -99,8 +100,15 @@ constexpr size_t eval_smem_bytes(int warps) {
 // Measured, all five quantities on the 1.5M-tet grid in FP32: the call 90 us
 // (170 us with shared-memory float atomics on one accumulator, a packing pass
 // and separate zeroing).
-template <class R, int MAT, int NVEC, int MAXT>
-__global__ void __launch_bounds__(MAXT, MAXT == 128 ? (sizeof(R) == 4 ? 5 : 2) : 1) fem_eval_kernel(
+// PACK (FP64): a batch is 32 consecutive elements, scattered group by group.
+// FP64 pays for idle lanes, and the warp groups of small tiles are half empty
+// (10 elements a group with 64 elements a tile, 27 with 256).  All five
+// quantities of 138k tets in FP64: 254 us against 482 by groups with 64
+// elements a tile, 207 against 238 with 256, 184.5 against 183.5 with the
+// default tiles; ARAP 568 against 1,481, 541 against 671, 595 against 595.
+// FemView::packed chooses.
+template <class R, int MAT, int NVEC, int MAXT, bool PACK>
+__global__ void __launch_bounds__(MAXT, MAXT == 128 ? 5 : 1) fem_eval_kernel(
     FemView fv, unsigned flags, const R* __restrict__ u, const R* __restrict__ p,
     const int32_t* __restrict__ p_slot, const int32_t* __restrict__ slot_of_tv, void* __restrict__ slots,
     int n_slots, AccStore<R>* __restrict__ partials, unsigned* counter, double* energy, double* quad, int assign) {
@@ -117,13 +125,19 @@ __global__ void __launch_bounds__(MAXT, MAXT == 128 ? (sizeof(R) == 4 ? 5 : 2) :
 
   const int tile = blockIdx.x;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
-  const int ge = fv.tile_gstart[tile + 1];
-  int g = fv.tile_gstart[tile] + warp, n = 0;
+  const int gs = fv.tile_gstart[tile], gend = fv.tile_gstart[tile + 1];
+  // the warp's batches of elements, b = g, g + warps, ... below ge
+  const int ea = PACK ? fv.group_estart[gs] : 0, eb = PACK ? fv.group_estart[gend] : 0;
+  const int ge = PACK ? (eb - ea + 31) / 32 : gend;
+  auto batch = [&](int b, int& e0, int& count) {
+    e0 = PACK ? ea + 32 * b : fv.group_estart[b];
+    count = PACK ? min(32, eb - e0) : fv.group_estart[b + 1] - e0;
+  };
+  int g = (PACK ? 0 : gs) + warp, e0 = 0, n = 0, h = gs;  // h (PACK): the group of the batch's first element
   ElemGeo<R> geo;
   uint32_t ids = 0;
   if (g < ge) {
-    const int e0 = fv.group_estart[g];
-    n = fv.group_estart[g + 1] - e0;
+    batch(g, e0, n);
     if (lane < n) load_elem_m<R, MAT>(fv, e0 + lane, geo, ids);
   }
   const int vs = fv.tile_vstart[tile], nv = fv.tile_vstart[tile + 1] - vs;
@@ -154,13 +168,19 @@ __global__ void __launch_bounds__(MAXT, MAXT == 128 ? (sizeof(R) == 4 ? 5 : 2) :
   Acc<R> sums[2] = {};
   while (g < ge) {
     const int gn = g + warps;
-    int nn = 0;
+    int e0n = 0, nn = 0;
     ElemGeo<R> geon;
     uint32_t idsn = 0;
     if (gn < ge) {
-      const int e0n = fv.group_estart[gn];
-      nn = fv.group_estart[gn + 1] - e0n;
+      batch(gn, e0n, nn);
       if (lane < nn) load_elem_m<R, MAT>(fv, e0n + lane, geon, idsn);
+    }
+    // PACK: the end of the group that the batch begins in, and of the next one
+    int end0 = 0, end1 = 0;
+    if (PACK && vectors) {
+      while (fv.group_estart[h + 1] <= e0) ++h;
+      end0 = fv.group_estart[h + 1];
+      end1 = fv.group_estart[min(h + 2, gend)];
     }
     const int l[4] = {corner(ids, 0), corner(ids, 1), corner(ids, 2), corner(ids, 3)};
     // f[q]: corner values of the q-th requested vector
@@ -252,23 +272,37 @@ __global__ void __launch_bounds__(MAXT, MAXT == 128 ? (sizeof(R) == 4 ? 5 : 2) :
       }
     }
     if (vectors) {
-      // corner k of the group's lanes is a distinct vertex for every lane
+      // corner k of a group's lanes is a distinct vertex for every lane
+      auto scatter = [&](bool mine) {
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        __syncwarp();
-        if (lane < n) {
-          R x[9];
-          my.load(l[k], x);
+        for (int k = 0; k < 4; ++k) {
+          __syncwarp();
+          if (mine) {
+            R x[9];
+            my.load(l[k], x);
 #pragma unroll
-          for (int q = 0; q < NVEC; ++q)
+            for (int q = 0; q < NVEC; ++q)
 #pragma unroll
-            for (int c = 0; c < 3; ++c) x[3 * q + c] += f[q][k][c];
-          my.store(l[k], x);
+              for (int c = 0; c < 3; ++c) x[3 * q + c] += f[q][k][c];
+            my.store(l[k], x);
+          }
         }
+        __syncwarp();
+      };
+      if constexpr (PACK) {
+        const int e = e0 + lane;
+        scatter(lane < n && e < end0);
+        for (int q = h + 1, from = end0, to = end1; from < e0 + n; ++q) {
+          scatter(lane < n && e >= from && e < to);
+          from = to;
+          to = fv.group_estart[min(q + 2, gend)];
+        }
+      } else {
+        scatter(lane < n);
       }
-      __syncwarp();
     }
     g = gn;
+    e0 = e0n;
     n = nn;
     geo = geon;
     ids = idsn;
@@ -308,7 +342,8 @@ template <class R, int NVEC>
 __global__ void __launch_bounds__(kUnpackThreads) unpack_kernel(
     int n, const int32_t* __restrict__ uoi, const int32_t* __restrict__ off, const void* __restrict__ slots,
     int n_slots, R* o0, R* o1, R* o2, const int32_t* __restrict__ out_slot, int assign, int force_grad,
-    int force_fun, const V4<R>* __restrict__ force, const R* __restrict__ u, AccStore<R>* partials, unsigned* counter, double* energy) {
+    int force_fun, const V4<R>* __restrict__ force, const R* __restrict__ u, AccStore<R>* partials,
+    unsigned* counter, double* energy) {
   __shared__ Acc<R> red[kUnpackThreads / 32];
   const VecArrays<R, NVEC> in{(unsigned char*)slots, (size_t)n_slots};
   Acc<R> ext[1] = {};
@@ -379,25 +414,38 @@ unsigned vec_mask(unsigned flags) {
 // SMs have room, and in FP32 more warps shorten each tile's chain of groups: 8
 // up to two tiles per SM, 16 up to one.  FP64 tiles arrive cut (eval_view):
 // four warps, which fill the pipe, so that two CTAs share an SM, and 8 up to
-// one tile per SM.  All five quantities of 138k tets in FP64: 245 us with 214
-// whole tiles of 8 warps, 184 us with 275 pieces of 4.
-int eval_warps(int precision, int n_tiles) {
-  if (n_tiles > 2 * kSMs) return 4;
-  if (precision == AGB_F64) return n_tiles > kSMs ? 4 : 8;
-  return n_tiles > kSMs ? 8 : 16;
+// one tile per SM or for ARAP's scalars and single vectors, where the SVDs wait
+// rather than compute (the energy of 138k tets with 384 elements a tile 343 us,
+// 433 with four; the gradient with 192 elements 341 and 381).  All five
+// quantities of 138k tets in FP64: 245 us with 214 whole tiles of 8 warps, 184
+// us with 275 pieces of 4.
+int eval_warps(int precision, const FemView& fv, int nvec) {
+  if (precision == AGB_F64) return fv.n_tiles > kSMs && (nvec > 1 || fv.material != AGB_ARAP) ? 4 : 8;
+  return fv.n_tiles > 2 * kSMs ? 4 : (fv.n_tiles > kSMs ? 8 : 16);
 }
 
-template <class R, int MAT, int NVEC, int MAXT>
+// No more warps than the largest tile has batches: the others' accumulators
+// would be cleared and summed and take the shared memory and, in FP64, the
+// registers of further CTAs.  Packed batches are dealt out evenly.
+int used_warps(int warps, const FemView& fv) {
+  if (fv.max_batches < 1) return 1;
+  if (!fv.packed) return std::min(warps, fv.max_batches);
+  const int rounds = (fv.max_batches + warps - 1) / warps;
+  return (fv.max_batches + rounds - 1) / rounds;
+}
+
+template <class R, int MAT, int NVEC, int MAXT, bool PACK>
 cudaError_t eval_launch(const FemView& fv, int warps, unsigned flags, const void* u, const void* p,
                         const int32_t* p_slot, const int32_t* slot_of_tv, void* slots, int32_t n_slots,
                         void* partials, unsigned* counter, double* energy, double* quad, int assign, cudaStream_t s) {
   const bool vectors = flags & (AGB_GRAD | AGB_HESS_DIAG | AGB_HESS_PROD);
+  if (vectors || sizeof(R) == 8) warps = used_warps(warps, fv);
   const size_t smem = vectors ? eval_smem_bytes<R, NVEC>(warps) : eval_stage_bytes<R>();
-  if (smem > 48 * 1024) {  // above the default limit the kernel has to opt in
-    const cudaError_t e = allow_max_smem(fem_eval_kernel<R, MAT, NVEC, MAXT>);
+  if (smem + 1024 > 48 * 1024) {  // with its static arrays above the default limit the kernel has to opt in
+    const cudaError_t e = allow_max_smem(fem_eval_kernel<R, MAT, NVEC, MAXT, PACK>);
     if (e != cudaSuccess) return e;
   }
-  fem_eval_kernel<R, MAT, NVEC, MAXT><<<fv.n_tiles, 32 * warps, smem, s>>>(
+  fem_eval_kernel<R, MAT, NVEC, MAXT, PACK><<<fv.n_tiles, 32 * warps, smem, s>>>(
       fv, flags, (const R*)u, (const R*)p, p_slot, slot_of_tv, slots, n_slots, (AccStore<R>*)partials, counter, energy,
       quad, assign);
   return cudaGetLastError();
@@ -405,8 +453,15 @@ cudaError_t eval_launch(const FemView& fv, int warps, unsigned flags, const void
 
 template <class R, int MAT, int NVEC, class... A>
 cudaError_t eval_warps_of(const FemView& fv, int warps, A... args) {
-  return warps == 4 ? eval_launch<R, MAT, NVEC, 128>(fv, warps, args...)
-                    : eval_launch<R, MAT, NVEC, sizeof(R) == 4 ? 512 : 256>(fv, warps, args...);
+  if constexpr (sizeof(R) == 8) {
+    if constexpr (MAT != AGB_ARAP) {  // ARAP is always packed
+      if (!fv.packed) return eval_launch<R, MAT, NVEC, 256, false>(fv, warps, args...);
+    }
+    return eval_launch<R, MAT, NVEC, 256, true>(fv, warps, args...);
+  } else {
+    return warps == 4 ? eval_launch<R, MAT, NVEC, 128, false>(fv, warps, args...)
+                      : eval_launch<R, MAT, NVEC, 512, false>(fv, warps, args...);
+  }
 }
 
 template <class R, int MAT, class... A>
@@ -465,7 +520,7 @@ cudaError_t launch_fem_eval(int precision, const FemView& fv, unsigned flags, co
                             void* partials, unsigned* counter, double* energy, double* quad, int assign,
                             cudaStream_t stream) {
   if (fv.n_tiles == 0) return cudaSuccess;
-  const int nvec = popcount3(vec_mask(flags)), warps = eval_warps(precision, fv.n_tiles);
+  const int nvec = popcount3(vec_mask(flags)), warps = eval_warps(precision, fv, nvec);
   if (precision == AGB_F64)
     return eval_material<double>(nvec, fv, warps, flags, u, p, p_slot, slot_of_tv, slots, n_slots, partials, counter,
                                  energy, quad, assign, stream);
