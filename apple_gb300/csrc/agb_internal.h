@@ -182,6 +182,7 @@ struct agb_fem {
   void* d_act = nullptr;             // muscle: S stream (FemView::act)
   double* d_D = nullptr;             // muscle: D of the plan (9 x n_cells), allocated by set_activation
   double* d_act_user = nullptr;      // muscle: activation as set (n_cells x 6, the caller's cell order)
+  std::vector<double> act_user;      // the same, of small potentials
   int32_t* d_elem_user = nullptr;    // internal -> caller's cell index (on first use)
   void* d_vol = nullptr;             // R per internal element (on first use)
   // scratch for the standalone evaluation API
