@@ -270,7 +270,9 @@ class WarpPotentialFem(WarpPotential):
         check_vec(u, self.n_points, self.dtype, "u")
         w = check_vec(w.to(self.dtype), self.n_points, self.dtype, "w")
         n = self.cells.shape[0]
-        dmu, dlam = torch.zeros((2, n), dtype=self.dtype, device=u.device)
+        # two tensors: rows of one could not be changed in place under autograd
+        dmu = torch.zeros(n, dtype=self.dtype, device=u.device)
+        dlam = torch.zeros(n, dtype=self.dtype, device=u.device)
         _lib.call("agb_fem_grad_param_vjp", self._standalone(), ptr(u), ptr(w), ptr(dmu), ptr(dlam),
                   stream_ptr(u.device))
         out = {"mu": dmu}
