@@ -1304,7 +1304,11 @@ static int build_loop_graph(agb_solver* sv) {
 // correction the two refresh passes follow as programmatic dependents and
 // return at once unless a refresh is due (an IF node around them costs more
 // than their idle launches: 130.8 against 124 us per iteration measured on
-// the 1.5M-tet grid).
+// the 1.5M-tet grid).  Where iterations are resident the step is a run with a
+// limit of one, although each run stages the records and the vertex state
+// again: among others, 5k tets 23.0 us against 27.1 with three kernels, 138k
+// 36.4 against 43.5 (with the correction), 138k in FP64 193 against 351, 40
+// tets 20.9 against 21.1.
 static int build_step_graph(agb_solver* sv) {
   cudaGraph_t g = nullptr;
   AGB_CHECK_CUDA(cudaGraphCreate(&g, 0));

@@ -466,7 +466,7 @@ def batched_record(n=64, dims=(4, 40), max_steps=2000, rtol=1e-6, n_check=3, see
         err_b.append(float(np.abs(us[k].double().cpu().numpy() - u_ref).max()) / diag[k])
         err_p.append(float(np.abs(plain_u[k].double().cpu().numpy() - u_ref).max()) / diag[k])
     iters = [s.n_steps for s in sols]
-    # the device loop's fixed cost per iteration (five kernels in a graph
+    # the device loop's fixed cost per iteration (three kernels in a graph
     # WHILE node): the same loop over two 4x4x4-cell grids, where the kernels
     # have almost no work; a persistent kernel with grid barriers between the
     # phases could save at most this much per iteration
