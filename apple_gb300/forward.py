@@ -60,11 +60,11 @@ class ForwardProblem:
 
 
 def _eval_free(model, u: torch.Tensor, what: str, p: torch.Tensor | None = None):
-    wm = getattr(model, "warp_model", None)
-    if type(model) is not Model or type(model.dof_map) is not DofMap or type(wm) is not WarpModel \
-            or what in vars(model) or what in vars(wm):
-        return None
-    return model.eval_free(u, what, p)
+    if type(model) is Model and what not in model.__dict__ and type(model.dof_map) is DofMap:
+        wm = model.warp_model
+        if type(wm) is WarpModel and what not in wm.__dict__:
+            return model.eval_free(u, what, p)
+    return None
 
 
 class Forward:
